@@ -148,6 +148,19 @@ def test_gemm_simt_row_does_not_depend_on_the_batch(ops):
     assert torch.equal(full[17:18], one)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 17, 60), (9, 16, 2048), (16, 1100, 4100), (17, 63, 256), (65, 65, 2052), (70, 130, 8196)])
+def test_gemm_simt_rows_and_tiles(ops, M, N, K):
+    """32-bit operands in whole 16-byte pieces: rows that are not full, tails of a k-tile, stage and segment; a row is
+    the same alone (the rows kernel) as among the others (the tiles kernel from 17 rows on)."""
+    a, w = rnd(M, K, s=0.5), rnd(N, K, s=0.5, seed=1)
+    want = a.double() @ w.double().T
+    got = ops.gemm_simt(a, w, torch.float32)
+    close(got, want, torch.float32, scale=math.sqrt(K))
+    close(ops.gemm_simt(a, w, torch.bfloat16, softcap=3.0, out_scale=0.5), 1.5 * torch.tanh(want / 3.0), torch.bfloat16, scale=4.0)
+    i = M - 1
+    assert torch.equal(got[i:i + 1], ops.gemm_simt(a[i:i + 1].contiguous(), w, torch.float32))
+
+
 @pytest.mark.parametrize("odt", DT)
 @pytest.mark.parametrize("M,N,K", [(1, 128, 64), (3, 40, 72), (16, 384, 96), (17, 130, 64), (64, 2304, 2048),
                                    (100, 512, 520), (128, 256, 64), (129, 256, 64), (300, 520, 200),
