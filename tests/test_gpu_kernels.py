@@ -148,6 +148,31 @@ def test_gemm_simt_row_does_not_depend_on_the_batch(ops):
     assert torch.equal(full[17:18], one)
 
 
+@pytest.mark.parametrize("heads,P,N,groups,lens,span", [(2, 64, 128, 1, [128], 1.0), (3, 8, 8, 1, [65, 1, 7], 0.1), (4, 72, 40, 2, [129, 300], 1.0),
+                                                        (2, 64, 64, 2, [3, 127, 513], 30.0), (1, 16, 120, 1, [64], 1e4)])
+def test_mamba2_prompts_as_products(ops, heads, P, N, groups, lens, span):
+    """The product form against the recurrence (which a step that does not say its longest prompt takes): the same
+    convolution, so the states differ by the order of 32-bit sums (up to N + 128 terms and as many products, in rms
+    about 1e-6) and the outputs by that and one bfloat16 rounding.  ``span``: how far the decays reach."""
+    T, B, inner, ch = sum(lens), len(lens), heads * P, heads * P + 2 * groups * N
+    proj, dt = rnd(T, inner + ch, dt=torch.bfloat16), rnd(T, heads, seed=1)
+    small = [rnd(ch, 4, s=0.3, seed=2), rnd(ch, s=0.1, seed=3), rnd(heads, seed=4) - 2, rnd(heads, s=0.5, seed=5) + math.log(span), rnd(heads, seed=6)]
+    norm = rnd(inner, s=0.1, seed=7) + 1
+    first = rnd(B + 1, ops.mamba2_state_size(heads, P, N, groups, 4), seed=8)
+    starts = torch.tensor([sum(lens[:i]) for i in range(B + 1)], dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).to("cuda", torch.int32)
+    slots = torch.arange(B, 0, -1, dtype=torch.int32, device="cuda")
+    got = []
+    for longest in (0, max(lens)):
+        state = first.clone()
+        out = ops.mamba2(proj, dt, heads, P, N, groups, 4, 1, *small, norm, 1e-6, state, starts, seq, slots, B, False, longest)
+        got.append((out.double(), state.double()))
+    assert torch.equal(got[0][1][0], got[1][1][0])                       # a slot that is not in the step
+    assert (got[1][1] - got[0][1]).norm() <= 3e-6 * got[0][1].norm()
+    assert (got[1][0] - got[0][0]).norm() <= 3e-3 * got[0][0].norm()
+    assert torch.isfinite(got[1][0]).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 17, 60), (9, 16, 2048), (16, 1100, 4100), (17, 63, 256), (65, 65, 2052), (70, 130, 8196)])
 def test_gemm_simt_rows_and_tiles(ops, M, N, K):
     """32-bit operands in whole 16-byte pieces: rows that are not full, tails of a k-tile, stage and segment; a row is

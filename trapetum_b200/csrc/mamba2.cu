@@ -16,6 +16,8 @@
 //                        its decays, a second launch starts every chunk from what the chunks before it left
 //                        (S_c = D_(c-1) S_(c-1) + E_(c-1), folded by the chunk itself) and writes y.  Twice the
 //                        arithmetic, chunks times the parallelism; the same sums in another order.
+//   tb_mamba2_chunks     the same for prompts in bfloat16, as matrix products over chunks of 128 tokens (mma.sync; see
+//                        "Prompts as products" below)
 //   tb_mamba2_gate_norm  out = groupnorm(y * silu(z)) * w, the norm over `norm_groups` equal parts of a row.
 //
 // The state of a sequence is one 32-bit row: [heads][P][N] of S, then [taps-1][channels] of conv inputs
@@ -48,6 +50,9 @@ struct Mamba2Args {
     float* chunk_state; float* chunk_decay; int chunk_len; int n_chunks;
 };
 
+// The argument block's size, for the Python mirror's check.
+extern "C" int tb_mamba2_args_bytes() { return (int)sizeof(Mamba2Args); }
+
 // ---------------------------------------------------------------------------------------------------------
 template <typename T, typename TW>
 __global__ void mamba2_conv_kernel(Mamba2Args a) {
@@ -70,6 +75,76 @@ __global__ void mamba2_conv_kernel(Mamba2Args a) {
         acc += to_f<TW>(w[j]) * v;
     }
     ((T*)a.xbc)[(size_t)t * ch + c] = from_f<T>(silu_f(acc));
+}
+
+// Four taps in bfloat16: a thread takes four neighbouring channels of eight tokens in a row, whose inputs are on their way
+// together, 8 bytes a load: 18 us for 2,048 tokens x 4,352 channels, cold (a thread per number: 76; eight channels a thread,
+// whose registers leave half the warps: 26; its 36 MB are 5.4).
+constexpr int CONV_TOK = 8;
+__device__ __forceinline__ void unpack4(const uint2& v, float* f) {
+    f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+    f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *(uint32_t*)&h;
+}
+__global__ void __launch_bounds__(128, 6) mamba2_conv4_kernel(Mamba2Args a) {
+    pdl_launch_dependents();
+    const int inner = a.heads * a.P, ch = inner + 2 * a.groups * a.N;
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    const int t0 = blockIdx.x * CONV_TOK, nt = min(CONV_TOK, a.n_tokens - t0);
+    if (c >= ch) return;
+    float w[4][4], bias[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const float4 x = *(const float4*)((const float*)a.conv_w + (size_t)(c + e) * 4);
+        w[e][0] = x.x; w[e][1] = x.y; w[e][2] = x.z; w[e][3] = x.w;
+        bias[e] = ((const float*)a.conv_b)[c + e];
+    }
+    int b = a.token_seq[t0], i = t0 - a.seq_start[b];     // (a step's integers are there before its first kernel)
+    pdl_wait();
+    const bf16* in = (const bf16*)a.proj + inner + c;
+    uint2 rows[CONV_TOK + 3];                        // tokens t0 - 3 .. t0 + 7 (earlier ones only of the same sequence)
+#pragma unroll
+    for (int r = 0; r < CONV_TOK + 3; r++) {
+        rows[r] = make_uint2(0, 0);
+        if (r < 3 ? i >= 3 - r : r - 3 < nt) rows[r] = *(const uint2*)(in + (size_t)(t0 + r - 3) * a.proj_stride);
+    }
+    float h[3][4];                                   // the three inputs before the token
+    auto from_state = [&](int k, int row) {          // h[k] from row `row` of the sequence's state
+        const float* st = a.state + (size_t)a.slot_ids[b] * a.state_stride + (size_t)a.heads * a.P * a.N + (size_t)row * ch + c;
+#pragma unroll
+        for (int e = 0; e < 4; e++) h[k][e] = st[e];
+    };
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        if (i >= 3 - k) unpack4(rows[k], h[k]);
+        else from_state(k, k + i);                   // index i - 3 + k < 0: row 3 + (i - 3 + k) of the state
+    }
+#pragma unroll
+    for (int r = 0; r < CONV_TOK; r++) {
+        if (r >= nt) break;
+        if (r > 0) {
+            const int nb = a.token_seq[t0 + r];
+            if (nb != b) {                           // the next sequence's first token
+                b = nb;
+#pragma unroll
+                for (int k = 0; k < 3; k++) from_state(k, k);
+            }
+        }
+        float cur[4], acc[4];
+        unpack4(rows[r + 3], cur);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            acc[e] = bias[e] + w[e][0] * h[0][e];
+            acc[e] += w[e][1] * h[1][e];
+            acc[e] += w[e][2] * h[2][e];
+            acc[e] = silu_f(acc[e] + w[e][3] * cur[e]);
+            h[0][e] = h[1][e]; h[1][e] = h[2][e]; h[2][e] = cur[e];
+        }
+        *(uint2*)((bf16*)a.xbc + (size_t)(t0 + r) * ch + c) = make_uint2(pack2(acc[0], acc[1]), pack2(acc[2], acc[3]));
+    }
 }
 
 // After a step of several tokens: the state keeps the last taps-1 inputs of each sequence.  One thread owns a
@@ -342,6 +417,313 @@ __global__ void __launch_bounds__(SCAN_NS * PT / SCAN_PP) mamba2_scan_kernel(Mam
 }
 
 // ---------------------------------------------------------------------------------------------------------
+// Prompts as products (bfloat16, N up to 128).  With the step sizes dt, the log2 decays l = max(A dt log2 e, -300) and
+// their running sums c within a chunk of 128 tokens, S the state before it:
+//     y_i = sum_{j <= i} (C_i . B_j) 2^(c_i - c_j) dt_j x_j  +  2^(c_i) S C_i  +  D x_i
+//     S'  = 2^(c_last) S + sum_j 2^(c_last - c_j) dt_j x_j B_j^T
+// in three launches: each chunk's own sum E, the states before the chunks (a scan over chunks, element by element), the
+// outputs.  x, B and C are bfloat16 numbers; what meets them (the weighted scores, the weighted x, the state) is 32-bit and
+// enters as the sum of three bfloat16 numbers, 24 bits, so every product is that of the recurrence and only the order of the
+// 32-bit sums differs.  The running sums are kept as two 32-bit numbers (c_i - c_j of near tokens keeps its digits); a
+// decay below 2^-300 is 0 in any product.  A non-finite x reaches the up to 15 tokens before it too (0 times it).
+// 2,048 tokens, 64 heads of 64 x 128: 31 + 20 + 56 us cold (the recurrence in chunks: 167 + 235); the tensor pipe and the
+// three-way splits share the time of the third launch.  All of ops.mamba2: 486 -> 129 us.
+// ---------------------------------------------------------------------------------------------------------
+constexpr int MC = 128, MCT = 256;                    // tokens of a chunk, threads
+constexpr int MP = 64, MXPITCH = MP * 2 + 16;         // values of P a CTA takes; bytes of a shared row of them (no bank conflicts)
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
+    const int n = valid ? 16 : 0;                     // 0 source bytes: the 16 destination bytes become zero
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int K> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(K) : "memory"); }
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Two 32-bit numbers as sums of three bfloat16 numbers each: the remainders are exact, the last one holds what is left.
+__device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    hi = pack2(x, y);
+    x -= __uint_as_float(hi << 16); y -= __uint_as_float(hi & 0xffff0000u);
+    mid = pack2(x, y);
+    lo = pack2(x - __uint_as_float(mid << 16), y - __uint_as_float(mid & 0xffff0000u));
+}
+__device__ __forceinline__ float exp2_fast(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+
+struct ChunkPlace { int t0, n, c, b, slot; };         // first token, tokens, index in its sequence, sequence, scratch slot
+// A sequence's chunks lie from slot floor(seq_start / 128) + b on, which leaves every sequence enough of them.
+__device__ __forceinline__ ChunkPlace chunk_place(const Mamba2Args& a, int z) {
+    ChunkPlace p;
+    p.b = z / a.n_chunks; p.c = z % a.n_chunks;
+    const int s0 = a.seq_start[p.b], s1 = a.seq_start[p.b + 1];
+    p.t0 = s0 + p.c * MC; p.n = min(MC, s1 - p.t0); p.slot = s0 / MC + p.b + p.c;
+    return p;
+}
+
+// dt and the running sums of the log2 decays of a chunk's tokens (past its end: no step, no decay) into shared memory.
+__device__ __forceinline__ void chunk_decays(const Mamba2Args& a, const ChunkPlace& p, int h, float* sdt, float2* scum, double* red) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    double l = 0.0;
+    if (tid < MC) {
+        float dt = 0.f;
+        if (tid < p.n) {
+            const float* q = a.dt + (size_t)(p.t0 + tid) * a.dt_stride + h;
+            dt = q[0];
+            for (int sp = 1; sp < a.dt_splits; sp++) dt += q[(size_t)sp * a.dt_split_stride];
+            dt = softplus_f(dt + ((const float*)a.dt_bias)[h]);
+            l = fmax((double)-expf(((const float*)a.A_log)[h]) * (double)dt * 1.4426950408889634, -300.0);
+        }
+        sdt[tid] = dt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, l, o);
+            if (lane >= o) l += up;
+        }
+        if (lane == 31) red[tid >> 5] = l;
+    }
+    __syncthreads();
+    if (tid < MC) {
+        for (int w = 0; w < tid >> 5; w++) l += red[w];
+        const float hi = (float)l;
+        scum[tid] = make_float2(hi, (float)(l - (double)hi));
+    }
+    __syncthreads();
+}
+
+// 128 rows of COLS bfloat16 columns, of which `cols` exist, into padded shared rows; rows from n on become zero.
+template <int COLS>
+__device__ __forceinline__ void load_chunk(uint8_t* dst, const bf16* src, long long stride, int n, int cols) {
+    constexpr int CPR = COLS / 8, PITCH = COLS * 2 + 16;
+#pragma unroll 4
+    for (int c = threadIdx.x; c < MC * CPR; c += MCT) {
+        const int r = c / CPR, k = (c % CPR) * 8;
+        const bool ok = r < n && k < cols;
+        cp_async16(dst + r * PITCH + k * 2, src + (ok ? (size_t)r * stride + k : 0), ok);
+    }
+}
+
+// E = sum_j 2^(c_last - c_j) dt_j x_j B_j^T: 64 values of P of one head, all N.  Warp w: 16 rows of P, half of N.
+template <int NP>
+__global__ void __launch_bounds__(MCT) mamba2_chunk_sum_kernel(Mamba2Args a) {
+    pdl_launch_dependents();
+    constexpr int BPITCH = NP * 2 + 16, NT = NP / 16;  // 8-column pieces a warp
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t* sB = smem;                               // [128][BPITCH]
+    uint8_t* sx = sB + MC * BPITCH;                   // [128][MXPITCH]
+    float2* scum = (float2*)(sx + MC * MXPITCH);      // [128]
+    float* sdt = (float*)(scum + MC);                 // [128], then the weights
+    __shared__ double red[4];
+    const int h = blockIdx.y, p0 = blockIdx.x * MP, N = a.N, P = a.P;
+    const int inner = a.heads * P, ch = inner + 2 * a.groups * N, g_of = h / (a.heads / a.groups);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    pdl_wait();
+    const ChunkPlace pl = chunk_place(a, blockIdx.z);
+    if (pl.n <= 0) return;
+    const bf16* row = (const bf16*)a.xbc + (size_t)pl.t0 * ch;
+    load_chunk<NP>(sB, row + inner + g_of * N, ch, pl.n, N);
+    load_chunk<MP>(sx, row + h * P + p0, ch, pl.n, P - p0);
+    cp_async_commit();
+    chunk_decays(a, pl, h, sdt, scum, red);
+    const float2 last = scum[MC - 1];
+    if (threadIdx.x < MC) sdt[threadIdx.x] *= exp2_fast((last.x - scum[threadIdx.x].x) + (last.y - scum[threadIdx.x].y));
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.chunk_decay[(size_t)pl.slot * a.heads + h] = exp2_fast(last.x + last.y);
+    cp_async_wait<0>();
+    __syncthreads();
+    const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * (NP / 2);
+    float acc[NT][4];
+#pragma unroll
+    for (int j = 0; j < NT; j++) { acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f; }
+    const int steps = (pl.n + 15) / 16;
+    for (int kk = 0; kk < steps; kk++) {
+        const float2 wa = *(const float2*)(sdt + kk * 16 + 2 * t), wb = *(const float2*)(sdt + kk * 16 + 2 * t + 8);
+        uint32_t x[4], hi[4], mid[4], lo[4];
+        ldsm_x4_t(smem_addr(sx + (kk * 16 + (lane >> 4) * 8 + (lane & 7)) * MXPITCH + (m0 + ((lane >> 3) & 1) * 8) * 2), x);
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            split3(__uint_as_float(x[e] << 16) * (e < 2 ? wa.x : wb.x), __uint_as_float(x[e] & 0xffff0000u) * (e < 2 ? wa.y : wb.y), hi[e], mid[e], lo[e]);
+#pragma unroll
+        for (int j = 0; j < NT; j += 2) {
+            uint32_t f[4];
+            ldsm_x4_t(smem_addr(sB + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * BPITCH + (n0 + j * 8 + (lane >> 4) * 8) * 2), f);
+            mma_bf16(acc[j], lo, f[0], f[1]); mma_bf16(acc[j + 1], lo, f[2], f[3]);
+            mma_bf16(acc[j], mid, f[0], f[1]); mma_bf16(acc[j + 1], mid, f[2], f[3]);
+            mma_bf16(acc[j], hi, f[0], f[1]); mma_bf16(acc[j + 1], hi, f[2], f[3]);
+        }
+    }
+    float* E = a.chunk_state + (size_t)pl.slot * a.heads * P * N + (size_t)h * P * N;
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        const int n = n0 + j * 8 + 2 * t, p = p0 + m0 + g;
+        if (n >= N) continue;                         // (N is even)
+        if (p < P) *(float2*)(E + (size_t)p * N + n) = make_float2(acc[j][0], acc[j][1]);
+        if (p + 8 < P) *(float2*)(E + (size_t)(p + 8) * N + n) = make_float2(acc[j][2], acc[j][3]);
+    }
+}
+
+// Every chunk's own sum becomes the state before the chunk; the sequence's state becomes the one after its last token.
+__global__ void __launch_bounds__(256) mamba2_chunk_fold_kernel(Mamba2Args a) {
+    pdl_launch_dependents();
+    const int b = blockIdx.y, per = a.P * a.N;
+    const size_t hpn = (size_t)a.heads * per;
+    const size_t e = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (e >= hpn) return;
+    const int h = (int)(e / per);
+    pdl_wait();
+    const int s0 = a.seq_start[b], len = a.seq_start[b + 1] - s0, n = (len + MC - 1) / MC, slot = s0 / MC + b;
+    if (n <= 0) return;
+    float* st = a.state + (size_t)a.slot_ids[b] * a.state_stride + e;
+    float4 s = *(const float4*)st;
+    float* E = a.chunk_state + (size_t)slot * hpn + e;
+    const float* D = a.chunk_decay + (size_t)slot * a.heads + h;
+    for (int c0 = 0; c0 < n; c0 += 8) {               // eight chunks' sums on their way together
+        float4 x[8]; float d[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) if (c0 + u < n) { x[u] = *(const float4*)(E + (c0 + u) * hpn); d[u] = D[(size_t)(c0 + u) * a.heads]; }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (c0 + u < n) {
+                *(float4*)(E + (c0 + u) * hpn) = s;
+                s.x = fmaf(d[u], s.x, x[u].x); s.y = fmaf(d[u], s.y, x[u].y); s.z = fmaf(d[u], s.z, x[u].z); s.w = fmaf(d[u], s.w, x[u].w);
+            }
+    }
+    *(float4*)st = s;
+}
+
+// y of 128 tokens of one head, 64 values of P.  Warp w: 16 tokens.
+template <int NP>
+__global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) {
+    pdl_launch_dependents();
+    constexpr int BPITCH = NP * 2 + 16, KS = NP / 16;
+    constexpr int FIRST = MC * BPITCH > 3 * MP * BPITCH ? MC * BPITCH : 3 * MP * BPITCH;
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t* sS = smem;                               // [128][BPITCH] C, then [3][64][BPITCH] the state's three parts
+    uint8_t* sB = sS + FIRST;                         // [128][BPITCH]
+    uint8_t* sx = sB + MC * BPITCH;                   // [128][MXPITCH]
+    float2* scum = (float2*)(sx + MC * MXPITCH);      // [128]
+    float* sdt = (float*)(scum + MC);                 // [128]
+    __shared__ double red[4];
+    const int h = blockIdx.y, p0 = blockIdx.x * MP, N = a.N, P = a.P;
+    const int inner = a.heads * P, ch = inner + 2 * a.groups * N, g_of = h / (a.heads / a.groups);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    pdl_wait();
+    const ChunkPlace pl = chunk_place(a, blockIdx.z);
+    if (pl.n <= 0) return;
+    const bf16* row = (const bf16*)a.xbc + (size_t)pl.t0 * ch;
+    load_chunk<NP>(sS, row + inner + (a.groups + g_of) * N, ch, pl.n, N);
+    cp_async_commit();
+    load_chunk<NP>(sB, row + inner + g_of * N, ch, pl.n, N);
+    load_chunk<MP>(sx, row + h * P + p0, ch, pl.n, P - p0);
+    cp_async_commit();
+    // the state, on its way through registers meanwhile: thread (p, part of n)
+    const float* S = a.chunk_state + (size_t)pl.slot * a.heads * P * N + ((size_t)h * P + p0) * N;
+    constexpr int Q = MP * NP / 4 / MCT;              // groups of four a thread
+    float4 sv[Q];
+#pragma unroll
+    for (int u = 0; u < Q; u++) {
+        const int i = tid + u * MCT, p = i / (NP / 4), n = (i % (NP / 4)) * 4;
+        sv[u] = (p0 + p < P && n < N) ? *(const float4*)(S + (size_t)p * N + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    chunk_decays(a, pl, h, sdt, scum, red);
+    cp_async_wait<1>();
+    __syncthreads();
+    uint32_t q[KS][4];
+#pragma unroll
+    for (int ks = 0; ks < KS; ks++) ldsm_x4(smem_addr(sS + (warp * 16 + (lane & 15)) * BPITCH + (ks * 16 + (lane >> 4) * 8) * 2), q[ks]);
+    __syncthreads();                                  // C is in registers: its place takes the state
+#pragma unroll
+    for (int u = 0; u < Q; u++) {
+        const int i = tid + u * MCT, p = i / (NP / 4), n = (i % (NP / 4)) * 4;
+        uint2 part[3];
+        split3(sv[u].x, sv[u].y, part[0].x, part[1].x, part[2].x);
+        split3(sv[u].z, sv[u].w, part[0].y, part[1].y, part[2].y);
+#pragma unroll
+        for (int k = 0; k < 3; k++) *(uint2*)(sS + (k * MP + p) * BPITCH + n * 2) = part[k];
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    // ---- what the state before the chunk gives
+    float o[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; j++) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
+    if (warp * 16 < pl.n) {                           // (rows past the end: nothing to write)
+#pragma unroll
+        for (int k = 2; k >= 0; k--)
+#pragma unroll
+            for (int ks = 0; ks < KS; ks++)
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    uint32_t f[4];
+                    ldsm_x4(smem_addr(sS + (k * MP + j * 8 + (lane >> 4) * 8 + (lane & 7)) * BPITCH + (ks * 16 + ((lane >> 3) & 1) * 8) * 2), f);
+                    mma_bf16(o[j], q[ks], f[0], f[1]);
+                    mma_bf16(o[j + 1], q[ks], f[2], f[3]);
+                }
+        const int ra = warp * 16 + g, rb = ra + 8;
+        const float2 ca = scum[ra], cb = scum[rb];
+        {
+            const float fa = exp2_fast(ca.x + ca.y), fb = exp2_fast(cb.x + cb.y);
+#pragma unroll
+            for (int j = 0; j < 8; j++) { o[j][0] *= fa; o[j][1] *= fa; o[j][2] *= fb; o[j][3] *= fb; }
+        }
+        // ---- the chunk's own tokens, 16 keys at a time up to this warp's last row
+        for (int kk = 0; kk <= warp; kk++) {
+            float s[2][4];
+#pragma unroll
+            for (int n = 0; n < 2; n++) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
+#pragma unroll
+            for (int ks = 0; ks < KS; ks++) {
+                uint32_t f[4];
+                ldsm_x4(smem_addr(sB + (kk * 16 + (lane >> 4) * 8 + (lane & 7)) * BPITCH + (ks * 16 + ((lane >> 3) & 1) * 8) * 2), f);
+                mma_bf16(s[0], q[ks], f[0], f[1]);
+                mma_bf16(s[1], q[ks], f[2], f[3]);
+            }
+            uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+            for (int n = 0; n < 2; n++) {
+                const int j = kk * 16 + n * 8 + 2 * t;
+                const float4 cj = *(const float4*)(scum + j);          // tokens j and j + 1
+                const float2 dj = *(const float2*)(sdt + j);
+                const float x0 = j <= ra ? s[n][0] * (exp2_fast((ca.x - cj.x) + (ca.y - cj.y)) * dj.x) : 0.f;
+                const float x1 = j + 1 <= ra ? s[n][1] * (exp2_fast((ca.x - cj.z) + (ca.y - cj.w)) * dj.y) : 0.f;
+                const float x2 = j <= rb ? s[n][2] * (exp2_fast((cb.x - cj.x) + (cb.y - cj.y)) * dj.x) : 0.f;
+                const float x3 = j + 1 <= rb ? s[n][3] * (exp2_fast((cb.x - cj.z) + (cb.y - cj.w)) * dj.y) : 0.f;
+                split3(x0, x1, hi[n * 2], mid[n * 2], lo[n * 2]);
+                split3(x2, x3, hi[n * 2 + 1], mid[n * 2 + 1], lo[n * 2 + 1]);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                uint32_t f[4];
+                ldsm_x4_t(smem_addr(sx + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * MXPITCH + (j * 8 + (lane >> 4) * 8) * 2), f);
+                mma_bf16(o[j], lo, f[0], f[1]); mma_bf16(o[j + 1], lo, f[2], f[3]);
+                mma_bf16(o[j], mid, f[0], f[1]); mma_bf16(o[j + 1], mid, f[2], f[3]);
+                mma_bf16(o[j], hi, f[0], f[1]); mma_bf16(o[j + 1], hi, f[2], f[3]);
+            }
+        }
+        const float Dh = ((const float*)a.D)[h];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int r = e ? rb : ra;
+            if (r >= pl.n) continue;
+            float* y = a.y + (size_t)(pl.t0 + r) * inner + h * P + p0;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int p = j * 8 + 2 * t;
+                if (p0 + p >= P) continue;            // (P is even)
+                const uint32_t xv = *(const uint32_t*)(sx + r * MXPITCH + p * 2);
+                *(float2*)(y + p) = make_float2(o[j][2 * e] + Dh * __uint_as_float(xv << 16), o[j][2 * e + 1] + Dh * __uint_as_float(xv & 0xffff0000u));
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------
 // out = groupnorm(y * silu(z)) * w: one CTA per (token, norm group).
 template <typename T, typename TW>
 __global__ void mamba2_gate_norm_kernel(Mamba2Args a) {
@@ -367,36 +749,38 @@ __global__ void mamba2_gate_norm_kernel(Mamba2Args a) {
     }
 }
 
-// The same for few tokens, where the launch's time is its chain of memory round trips: a thread keeps its NV groups
-// of four columns in registers, so y and z are read once (group sizes up to 1,024 x 4 x NV that are multiples of 4).
-template <typename T, typename TW, int NV>
-__global__ void __launch_bounds__(1024) mamba2_gate_norm_few_kernel(Mamba2Args a) {
+// The same where a thread can keep its NV groups of four columns in registers, so that y and z are read once, 16 bytes of y
+// and four values of z a load (group sizes that are multiples of 4).  Few tokens (the launch's time is a chain of memory
+// round trips): a group a thread.  Many: 256 threads a row, 2,048 rows of 4,096 in 15 us (read twice: 37; 67 MB are 10).
+__device__ __forceinline__ float4 four(const float* p) { return *(const float4*)p; }
+__device__ __forceinline__ float4 four(const bf16* p) {
+    const uint2 u = *(const uint2*)p;
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void store4(float* p, float4 v) { *(float4*)p = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v) { *(uint2*)p = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w)); }
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(NV == 1 ? 1024 : NV == 2 ? 512 : 256) mamba2_gate_norm_rows_kernel(Mamba2Args a) {
     pdl_launch_dependents();
     __shared__ float red[33];
     const int inner = a.heads * a.P, gs = inner / a.norm_groups;
     const int t = blockIdx.x, c0 = blockIdx.y * gs;
-    float w[NV][4], v[NV][4];
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-        const int i = (threadIdx.x + k * blockDim.x) * 4;
-#pragma unroll
-        for (int e = 0; e < 4; e++) w[k][e] = i < gs ? to_f<TW>(((const TW*)a.norm_w)[c0 + i + e]) : 0.f;
-    }
     pdl_wait();
     const float* y = a.y + (size_t)t * inner + c0;
     const T* z = (const T*)a.proj + (size_t)t * a.proj_stride + c0;
-    float ss = 0.f;
+    float4 v[NV], u[NV];
 #pragma unroll
     for (int k = 0; k < NV; k++) {
         const int i = (threadIdx.x + k * blockDim.x) * 4;
+        v[k] = u[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < gs) { v[k] = four(y + i); u[k] = four(z + i); }
+    }
+    float ss = 0.f;
 #pragma unroll
-        for (int e = 0; e < 4; e++) v[k][e] = 0.f;
-        if (i < gs) {
-            const float4 yy = *(const float4*)(y + i);
-            const float ye[4] = {yy.x, yy.y, yy.z, yy.w};
-#pragma unroll
-            for (int e = 0; e < 4; e++) { v[k][e] = ye[e] * silu_f(to_f<T>(z[i + e])); ss += v[k][e] * v[k][e]; }
-        }
+    for (int k = 0; k < NV; k++) {
+        v[k].x *= silu_f(u[k].x); v[k].y *= silu_f(u[k].y); v[k].z *= silu_f(u[k].z); v[k].w *= silu_f(u[k].w);
+        ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
     }
     ss = block_sum(ss, red);
     const float r = 1.0f / sqrtf(ss / (float)gs + a.eps);
@@ -405,8 +789,8 @@ __global__ void __launch_bounds__(1024) mamba2_gate_norm_few_kernel(Mamba2Args a
     for (int k = 0; k < NV; k++) {
         const int i = (threadIdx.x + k * blockDim.x) * 4;
         if (i < gs) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) out[i + e] = from_f<T>(v[k][e] * r * w[k][e]);
+            const float4 w = four((const float*)a.norm_w + c0 + i);
+            store4(out + i, make_float4(v[k].x * r * w.x, v[k].y * r * w.y, v[k].z * r * w.z, v[k].w * r * w.w));
         }
     }
 }
@@ -442,7 +826,10 @@ extern "C" int tb_mamba2_conv(const Mamba2Args* args, int dtype, int w_dtype, in
         DISPATCH2(dtype, w_dtype, tb_launch(mamba2_conv_step_kernel<T, TW>, dim3(a.batch, gy), dim3(128), 0, stream, a));
         return tb_launch_status();
     }
-    DISPATCH2(dtype, w_dtype, tb_launch(mamba2_conv_kernel<T, TW>, dim3(a.n_tokens, gy), dim3(128), 0, stream, a));
+    const bool wide = dtype == TB_BF16 && w_dtype == TB_F32 && a.taps == 4 && ch % 4 == 0 && (a.heads * a.P) % 4 == 0 && a.proj_stride % 4 == 0 &&
+                      ((uintptr_t)a.proj & 7) == 0 && ((uintptr_t)a.xbc & 7) == 0 && ((uintptr_t)a.conv_w & 15) == 0;
+    if (wide) tb_launch(mamba2_conv4_kernel, dim3((a.n_tokens + CONV_TOK - 1) / CONV_TOK, (ch / 4 + 127) / 128), dim3(128), 0, stream, a);
+    else DISPATCH2(dtype, w_dtype, tb_launch(mamba2_conv_kernel<T, TW>, dim3(a.n_tokens, gy), dim3(128), 0, stream, a));
     int st = tb_launch_status();
     if (st) return st;
     if (a.taps > 1) {
@@ -522,6 +909,48 @@ extern "C" int tb_mamba2_scan(const Mamba2Args* args, int dtype, int w_dtype, cu
     return tb_launch_status();
 }
 
+// Whether the product form takes these sizes: bfloat16, whole 16-byte pieces of x, B and C.
+extern "C" int tb_mamba2_chunks_takes(int dtype, int heads, int P, int N, int groups) {
+    return dtype == TB_BF16 && heads > 0 && groups > 0 && heads <= 65535 && P > 0 && P % 8 == 0 && N >= 8 && N <= 128 && N % 8 == 0;
+}
+
+// Scratch slots of a step: every sequence's chunks lie from slot floor(seq_start / 128) + its index on.
+extern "C" int tb_mamba2_chunk_slots(int batch, int n_tokens) { return n_tokens / MC + batch; }
+
+template <int NP>
+static int run_chunks(const Mamba2Args& a, cudaStream_t stream) {
+    constexpr int BPITCH = NP * 2 + 16, TAIL = MC * MXPITCH + MC * 12;
+    constexpr int SUM = MC * BPITCH + TAIL, OUT = (MC * BPITCH > 3 * MP * BPITCH ? MC * BPITCH : 3 * MP * BPITCH) + MC * BPITCH + TAIL;
+    cudaError_t e = cudaFuncSetAttribute(mamba2_chunk_sum_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SUM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(mamba2_chunk_out_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT);
+    if (e != cudaSuccess) return (int)e;
+    const dim3 grid((a.P + MP - 1) / MP, a.heads, a.batch * a.n_chunks);
+    tb_launch(mamba2_chunk_sum_kernel<NP>, grid, dim3(MCT), SUM, stream, a);
+    int st = tb_launch_status();
+    if (st) return st;
+    const long long quads = (long long)a.heads * a.P * a.N / 4;
+    tb_launch(mamba2_chunk_fold_kernel, dim3((unsigned)((quads + 255) / 256), a.batch), dim3(256), 0, stream, a);
+    st = tb_launch_status();
+    if (st) return st;
+    tb_launch(mamba2_chunk_out_kernel<NP>, grid, dim3(MCT), OUT, stream, a);
+    return tb_launch_status();
+}
+
+// n_chunks: of the longest sequence; chunk_state [slots][heads * P * N], chunk_decay [slots][heads].
+extern "C" int tb_mamba2_chunks(const Mamba2Args* args, int dtype, int w_dtype, cudaStream_t stream) {
+    const Mamba2Args& a = *args;
+    if (a.n_tokens <= 0 || a.batch <= 0) return 0;
+    if (check(a)) return -1;
+    const int ch = a.heads * a.P + 2 * a.groups * a.N;
+    if (!tb_mamba2_chunks_takes(dtype, a.heads, a.P, a.N, a.groups) || w_dtype != TB_F32)
+        return tb_refuse("mamba2: the product form takes bfloat16 with P and N in multiples of 8, N up to 128 (got P=%d N=%d)", a.P, a.N);
+    if (a.chunk_state == nullptr || a.chunk_decay == nullptr || a.n_chunks < 1 || (long long)a.batch * a.n_chunks > 65535)
+        return tb_refuse("mamba2: the product form needs its scratch, and at most 65535 chunks (%d sequences of %d)", a.batch, a.n_chunks);
+    if (((uintptr_t)a.xbc & 15) || ch % 8 || ((uintptr_t)a.state & 15) || a.state_stride % 4 || ((uintptr_t)a.chunk_state & 15) || ((uintptr_t)a.y & 7))
+        return tb_refuse("mamba2: the product form needs 16-byte aligned rows and states");
+    return a.N <= 64 ? run_chunks<64>(a, stream) : run_chunks<128>(a, stream);
+}
+
 extern "C" int tb_mamba2_gate_norm(const Mamba2Args* args, int dtype, int w_dtype, cudaStream_t stream) {
     Mamba2Args a = *args;
     if (a.n_tokens <= 0) return 0;
@@ -530,14 +959,18 @@ extern "C" int tb_mamba2_gate_norm(const Mamba2Args* args, int dtype, int w_dtyp
     int threads = (gs + 31) / 32 * 32;
     threads = threads < 64 ? 64 : (threads > 512 ? 512 : threads);
     if (a.norm_groups > 65535) return tb_refuse("mamba2: too many norm groups");
-    if (a.n_tokens <= 64 && gs % 4 == 0 && gs <= 1024 * 4 * 4 && (a.heads * a.P) % 4 == 0 && ((uintptr_t)a.y & 15) == 0) {
-        const int groups4 = gs / 4;
-        const int nvv = groups4 <= 1024 ? 1 : groups4 <= 2048 ? 2 : 4;
-        int th = ((groups4 + nvv - 1) / nvv + 31) / 32 * 32;
+    const int es = dtype == TB_BF16 ? 2 : 4;
+    if (w_dtype == TB_F32 && gs % 4 == 0 && gs <= 16384 && a.proj_stride % 4 == 0 && ((uintptr_t)a.y & 15) == 0 && ((uintptr_t)a.norm_w & 15) == 0 &&
+        ((uintptr_t)a.proj & (4 * es - 1)) == 0 && ((uintptr_t)a.out & (4 * es - 1)) == 0) {
+        const int quads = gs / 4, want = a.n_tokens <= 64 ? 1024 : 256;
+        int nv = 1;
+        while (nv < 16 && quads > nv * (nv == 1 ? 1024 : nv == 2 ? 512 : 256)) nv *= 2;
+        while (nv < 16 && quads > nv * want) nv *= 2;
+        int th = ((quads + nv - 1) / nv + 31) / 32 * 32;
         if (th < 64) th = 64;
-#define FEW(NV_) DISPATCH2(dtype, w_dtype, tb_launch(mamba2_gate_norm_few_kernel<T, TW, NV_>, dim3(a.n_tokens, a.norm_groups), dim3(th), 0, stream, a))
-        if (nvv == 1) FEW(1); else if (nvv == 2) FEW(2); else FEW(4);
-#undef FEW
+#define ROWS(NV_) TB_DISPATCH_1(dtype, T, tb_launch(mamba2_gate_norm_rows_kernel<T, NV_>, dim3(a.n_tokens, a.norm_groups), dim3(th), 0, stream, a))
+        if (nv == 1) ROWS(1); else if (nv == 2) ROWS(2); else if (nv == 4) ROWS(4); else if (nv == 8) ROWS(8); else ROWS(16);
+#undef ROWS
         return tb_launch_status();
     }
     DISPATCH2(dtype, w_dtype, tb_launch(mamba2_gate_norm_kernel<T, TW>, dim3(a.n_tokens, a.norm_groups), dim3(threads), 0, stream, a));

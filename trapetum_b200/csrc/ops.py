@@ -81,7 +81,7 @@ def _check(lib, status: int, what: str, kernels: int = 1) -> None:
 def args_mirrors():
     """(library, function that returns the C side's size, Python structure) of the argument blocks that have such a
     function: a mirror that has drifted from its C struct makes a kernel read garbage pointers."""
-    return (("gla", "tb_gla_args_bytes", _GlaArgs), ("retention", "tb_retention_args_bytes", _RetentionArgs),
+    return (("gla", "tb_gla_args_bytes", _GlaArgs), ("mamba2", "tb_mamba2_args_bytes", _Mamba2Args), ("retention", "tb_retention_args_bytes", _RetentionArgs),
             ("projnorm_kv", "tb_projnorm_kv_args_bytes", _ProjNormKvArgs), ("norm", "tb_add_terms_args_bytes", _AddTermsArgs),
             ("dyt", "tb_dyt_args_bytes", _DytArgs), ("moe", "tb_moe_route_args_bytes", _MoeRouteArgs),
             ("moe", "tb_moe_expert_args_bytes", _MoeExpertArgs), ("moe", "tb_moe_grouped_args_bytes", _MoeGroupedArgs))
@@ -723,6 +723,12 @@ class _Mamba2Args(ctypes.Structure):
                 ("chunk_state", c_void_p), ("chunk_decay", c_void_p), ("chunk_len", c_int), ("n_chunks", c_int)]
 
 
+# Tokens of the longest prompt from which prompts run as products over chunks: 48 / 64 / 96 / 256 tokens take 30.2 / 31.2 /
+# 38.5 / 50.1 us, as a recurrence 30.7 / 36.5 / 52.3 / 111.9 (64 heads of 64 x 128)
+MAMBA2_PRODUCTS_FROM = 64
+MAMBA2_PRODUCTS_BYTES = 1 << 30     # ... as long as the states between the chunks (16 KB a token of the medium sizes) stay within this
+
+
 def mamba2_state_size(heads: int, P: int, N: int, groups: int, taps: int) -> int:
     """32-bit numbers of one sequence's state: S [heads, P, N], then the last taps-1 conv inputs [taps-1, channels]."""
     return heads * P * N + (taps - 1) * (heads * P + 2 * groups * N)
@@ -770,8 +776,17 @@ def mamba2(proj: torch.Tensor, dt_raw: torch.Tensor, heads: int, P: int, N: int,
     a.seq_start = seq_start.data_ptr(); a.token_seq = token_seq.data_ptr(); a.slot_ids = slot_ids.data_ptr()
     a.xbc = xbc.data_ptr(); a.y = y.data_ptr(); a.out = out.data_ptr(); a.batch = batch; a.n_tokens = T
     lib = build.load("mamba2")
-    scan_launches = 1
-    if not one_token_each and max_seq_len > 0:
+    scan_launches, products = 1, False
+    if not one_token_each and max_seq_len >= MAMBA2_PRODUCTS_FROM and lib.tb_mamba2_chunks_takes(c_int(code(dt)), c_int(heads), c_int(P), c_int(N), c_int(groups)) \
+            and state.data_ptr() % 16 == 0 and state.stride(0) % 4 == 0:
+        # whole prompts as products over chunks; not where the chunks' states would take more than MAMBA2_PRODUCTS_BYTES
+        slots, n_chunks = int(lib.tb_mamba2_chunk_slots(c_int(batch), c_int(T))), (max_seq_len + 127) // 128
+        products = slots * heads * P * N * 4 <= MAMBA2_PRODUCTS_BYTES and batch * n_chunks <= 65535
+        if products:
+            chunk_state = torch.empty((slots, heads * P * N), dtype=torch.float32, device=proj.device)
+            chunk_decay = torch.empty((slots, heads), dtype=torch.float32, device=proj.device)
+            a.chunk_state = chunk_state.data_ptr(); a.chunk_decay = chunk_decay.data_ptr(); a.n_chunks = n_chunks
+    if not products and not one_token_each and max_seq_len > 0:
         chunk_len = c_int(0)
         n_chunks = int(lib.tb_mamba2_plan(c_int(heads), c_int(P), c_int(batch), c_int(int(max_seq_len)), ctypes.byref(chunk_len)))
         if n_chunks > 1:
@@ -783,7 +798,10 @@ def mamba2(proj: torch.Tensor, dt_raw: torch.Tensor, heads: int, P: int, N: int,
     cd, cw = c_int(code(dt)), c_int(code(wd))
     _check(lib, lib.tb_mamba2_conv(ctypes.byref(a), cd, cw, c_int(int(bool(one_token_each))), _stream()), "mamba2_conv",
            1 if one_token_each or taps == 1 else 2)
-    _check(lib, lib.tb_mamba2_scan(ctypes.byref(a), cd, cw, _stream()), "mamba2_scan", scan_launches)
+    if products:
+        _check(lib, lib.tb_mamba2_chunks(ctypes.byref(a), cd, cw, _stream()), "mamba2_chunks", 3)
+    else:
+        _check(lib, lib.tb_mamba2_scan(ctypes.byref(a), cd, cw, _stream()), "mamba2_scan", scan_launches)
     _check(lib, lib.tb_mamba2_gate_norm(ctypes.byref(a), cd, cw, _stream()), "mamba2_gate_norm")
     return out
 
