@@ -173,6 +173,30 @@ def test_mamba2_prompts_as_products(ops, heads, P, N, groups, lens, span):
     assert torch.isfinite(got[1][0]).all()
 
 
+@pytest.mark.parametrize("heads,D,V,lens,span", [(8, 128, 256, [700, 15], 1.0), (2, 72, 128, [16, 33, 1], 0.01), (3, 64, 128, [32], 30.0),
+                                                 (1, 8, 144, [300, 257], 1.0), (2, 128, 256, [65], 1e3)])
+def test_gla_prompts_in_blocks(ops, monkeypatch, heads, D, V, lens, span):
+    """The block form against the recurrence (which a step that does not say its longest prompt takes): states by the
+    order of 32-bit sums, outputs by that and one bfloat16 rounding.  ``span``: how far the decays reach."""
+    monkeypatch.setattr(ops, "GLA_BLOCKS_FROM", 1)                       # also where the recurrence is the faster one
+    T, B, rank = sum(lens), len(lens), 16
+    proj, low = rnd(T, 2 * heads * (D + V), dt=torch.bfloat16), rnd(1, T, rank, seed=1)
+    a2, bias, norm = rnd(heads * D, rank, s=0.3, seed=2), rnd(heads * D, seed=3) + 2, rnd(V, s=0.1, seed=4) + 1
+    first = rnd(B + 1, heads * D * V, seed=5)
+    starts = torch.tensor([sum(lens[:i]) for i in range(B + 1)], dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).to("cuda", torch.int32)
+    slots = torch.arange(B, 0, -1, dtype=torch.int32, device="cuda")
+    got = []
+    for longest in (0, max(lens)):
+        state = first.clone()
+        out = ops.gla(proj, low, a2, bias, 8.0 / span, D ** -0.5, norm, 1e-6, heads, D, V, state, starts, seq, slots, B, longest)
+        got.append((out.double(), state.double()))
+    assert torch.equal(got[0][1][0], got[1][1][0])                       # a slot that is not in the step
+    assert (got[1][1] - got[0][1]).norm() <= 3e-6 * got[0][1].norm()
+    assert (got[1][0] - got[0][0]).norm() <= 3e-3 * got[0][0].norm()
+    assert torch.isfinite(got[1][0]).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 17, 60), (9, 16, 2048), (16, 1100, 4100), (17, 63, 256), (65, 65, 2052), (70, 130, 8196)])
 def test_gemm_simt_rows_and_tiles(ops, M, N, K):
     """32-bit operands in whole 16-byte pieces: rows that are not full, tails of a k-tile, stage and segment; a row is
