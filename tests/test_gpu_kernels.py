@@ -197,6 +197,30 @@ def test_gla_prompts_in_blocks(ops, monkeypatch, heads, D, V, lens, span):
     assert torch.isfinite(got[1][0]).all()
 
 
+@pytest.mark.parametrize("B,heads,C,R,longest,window", [(1, 5, 64, 16, 33, 0), (1, 16, 448, 64, 700, 0), (3, 20, 96, 0, 500, 0), (8, 16, 512, 64, 900, 0),
+                                                        (40, 16, 128, 64, 300, 0), (40, 3, 448, 64, 640, 200), (2, 33, 512, 512, 130, 0)])
+def test_latent_decode_pieces(ops, B, heads, C, R, longest, window):
+    """Every way of cutting the keys (alone, clusters, the folding launch), heads and rows that fill no tile, one to two
+    tiles a ring.  The pool holds NaN wherever no key of the step lies.  Weights and result are rounded to bfloat16 once each."""
+    KD, lens = C + R, [max(1, longest - 37 * b % longest) for b in range(B)]
+    pages = (longest + PAGE - 1) // PAGE
+    pool = torch.full((B * pages, 1, PAGE, KD), float("nan"), dtype=torch.bfloat16, device="cuda")
+    table = torch.arange(B * pages, dtype=torch.int32, device="cuda").flip(0).view(B, pages).contiguous()
+    q, sink, rows = rnd(B, heads * KD, dt=torch.bfloat16), rnd(heads, seed=1), rnd(B, longest, KD, dt=torch.bfloat16, seed=2)
+    want = torch.empty(B, heads * C, dtype=torch.float64, device="cuda")
+    for b, n in enumerate(lens):
+        first = max(0, n - window) if window else 0
+        view = pool[table[b].long()].reshape(-1, KD)
+        view[first:n] = rows[b, first:n]
+        pool[table[b].long()] = view.view(pages, 1, PAGE, KD)
+        k = rows[b, first:n].double()
+        s = torch.cat([q[b].double().view(heads, KD) @ k.T * 0.1, sink.double()[:, None]], -1)
+        want[b] = (torch.softmax(s, -1)[:, :-1] @ k[:, :C]).reshape(-1)
+    got = ops.latent_decode(q, pool, table, torch.tensor(lens, dtype=torch.int32, device="cuda"), sink, heads, C, R, 0.1, longest, window)
+    assert (got.double() - want).norm() <= 4e-3 * want.norm()
+    assert ops.kernel_errors() == {}
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 17, 60), (9, 16, 2048), (16, 1100, 4100), (17, 63, 256), (65, 65, 2052), (70, 130, 8196)])
 def test_gemm_simt_rows_and_tiles(ops, M, N, K):
     """32-bit operands in whole 16-byte pieces: rows that are not full, tails of a k-tile, stage and segment; a row is

@@ -15,7 +15,12 @@
 //   tb_latent_decode   one query per sequence and head against the cached rows, the key range cut into
 //                      splits; softmax with a sink: the denominator also holds exp(sink_h), which has no
 //                      key and no value; partial (max, sum, o) per split are folded in split order
+#include <cooperative_groups.h>
+#include <cuda.h>
 #include "common.cuh"
+#include "async.cuh"
+
+namespace cg = cooperative_groups;
 
 TB_EXPORT_ERROR()
 
@@ -346,25 +351,29 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(LatentDecodeArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// The same decode on tensor cores (bfloat16): one CTA takes up to 16 heads of a sequence and a range of its
-// keys, so that a cached row is fetched once for all of them.  Rows arrive 32 at a time (half a page, one
-// contiguous piece of memory) by cp.async into a two-stage ring; S = Q' K^T with the heads as the 16
-// rows of mma.sync m16n8k16 (each warp 8 of the 32 keys), the softmax of a head's 32 scores by one warp (four heads
-// each), then O += P C with every warp taking a share of the latent's columns.  Partial (max, sum, o) go to the
-// scratch that latent_combine_kernel folds (it also adds the sink).
+// The same decode on tensor cores (bfloat16): one CTA an SM takes up to 16 heads of a sequence and a range of its keys, so
+// that a cached row is fetched once for all of them.  A warp of its own brings rows by tiled TMA copies (boxes of 32 rows x 64
+// numbers with the 128-byte swizzle; a bulk copy a row came to 24 GB/s an SM), half a page at a time, into a ring that fills
+// the shared memory (6 stages of 32 KB for rows of 512 numbers); KG groups of four warps take the tiles in turn, each with a
+// softmax and sums of its own, so that one group's chain of instructions (scores, softmax, outputs; two barriers of the group)
+// runs beside the others' and the copies never stop.  S = Q' K^T with 16 heads as the rows of mma.sync m16n8k16: a warp
+// takes a quarter of the row's numbers for all 32 keys, so that its queries stay in registers and a row is read once (a
+// quarter of the keys each read the queries from shared memory for every tile, most of its traffic); the four parts are
+// added on the way into the softmax (eight threads a head).  O += P C with every warp taking a share of the latent's columns.
+// The groups' sums meet in shared memory; the pieces of a sequence, as the CTAs of a cluster, in distributed shared memory
+// (with the sink), or else as partial (max, sum, o) that latent_combine_kernel folds.
+// 64 sequences of 1,536 to 2,048 rows of 448 + 64 numbers, 16 heads: 70 -> 42 us, at twice the rows 128 -> 68 (3.5 TB/s; the
+// kernel before: a two-stage cp.async ring, all warps meeting at four barriers a tile); 32 heads take the rows twice (the
+// second time from L2): 93 -> 68.  The copies alone would take 29 us, the groups' chains alone 35.
 // ---------------------------------------------------------------------------
-constexpr int LD_BN = 32;
+constexpr int LD_BN = 32, LD_SP = LD_BN + 4, LD_PP = LD_BN * 2 + 16;       // keys a tile; pitches of scores (floats) and weights (bytes)
+constexpr int LD_H = 16, LD_GT = 128, LD_GW = 4;                           // heads of a CTA; threads and warps of a group
+
+__device__ int g_latent_error = 0;
 
 __device__ __forceinline__ uint32_t ld_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ld_cp16(void* dst, const void* src, bool valid) {
-    const int n = valid ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ld_smem(dst)), "l"(src), "r"(n) : "memory");
-}
 __device__ __forceinline__ void ld_ldsm4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
-}
-__device__ __forceinline__ void ld_ldsm2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
 }
 __device__ __forceinline__ void ld_ldsm4_t(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
@@ -373,189 +382,379 @@ __device__ __forceinline__ void ld_mma(float* d, const uint32_t* a, uint32_t b0,
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void ld_box(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
+}
+// Byte offset of (row, 16-byte piece) in a tile: boxes of 64 numbers, [32 rows][128 bytes] each, pieces swizzled by the row.
+constexpr int LD_BOX = LD_BN * 128;
+__device__ __forceinline__ int ld_off(int row, int piece) { return (piece >> 3) * LD_BOX + row * 128 + (((piece & 7) ^ (row & 7)) << 4); }
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(LD_GT) : "memory"); }
 
-// MT: tiles of 16 heads per CTA (1 or 2), with 4 * MT warps.  NP: pairs of 8-column tiles of the latent per warp
-// (C <= NP * 16 * warps).  A warp scores 8 keys for 16 heads (four sums side by side, so that no product waits for the
-// one before it), takes the softmax of four heads, and adds its share of the latent's columns for all heads.
-template <int NP, int MT>
-__global__ void __launch_bounds__(MT * 128) latent_decode_mma_kernel(LatentDecodeArgs a) {
+// Bytes of a CTA's shared memory before the ring (1024: the ring's alignment), and of a tile of the ring.
+template <int KG>
+__host__ __device__ constexpr int ld_head_bytes() { return KG * LD_H * (4 * LD_SP * 4 + LD_PP + 4 + 8) + 256 + 1024; }
+__host__ __device__ constexpr int ld_tile_bytes(int KD) { return (KD + 63) / 64 * LD_BOX; }
+
+// NP: pairs of 8-column tiles of the latent per warp (C <= NP * 64).  KS: steps of 16 numbers of a row that a warp scores
+// (C + R <= KS * 64).  CL: up to how many pieces meet in a cluster.  stages: tiles the ring holds (2 .. 16).
+template <int NP, int KS, int KG, int CL>
+__global__ void __launch_bounds__((LD_GW * KG + 1) * 32, 1)
+latent_decode_mma_kernel(LatentDecodeArgs a, const __grid_constant__ CUtensorMap rows, int stages, int in_cluster) {
     pdl_launch_dependents();
-    constexpr int WARPS = 4 * MT, HEADS = 16 * MT, THREADS = WARPS * 32;
-    extern __shared__ __align__(16) unsigned char sm[];
-    const int KD = a.C + a.R, C = a.C;
-    const int pitch = KD * 2 + 16;
-    constexpr int PP = LD_BN * 2 + 16;
-    unsigned char* q_s = sm;                                        // [HEADS][pitch]
-    unsigned char* k_s = q_s + HEADS * pitch;                       // [2][LD_BN][pitch]
-    float* s_s = (float*)(k_s + 2 * LD_BN * pitch);                 // [HEADS][LD_BN]
-    unsigned char* p_s = (unsigned char*)(s_s + HEADS * LD_BN);     // [HEADS][PP]
-    float* corr_s = (float*)(p_s + HEADS * PP);                     // [HEADS]
-    const int b = blockIdx.x, hg = blockIdx.y, split = blockIdx.z;
+    constexpr int HEADS = LD_H, MMA_WARPS = LD_GW * KG;
+    extern __shared__ __align__(128) unsigned char sm[];
+    const int KD = a.C + a.R, C = a.C, boxes = (KD + 63) / 64, tile = boxes * LD_BOX;
+    uint64_t* full = (uint64_t*)sm;                                 // [16] the tile is there
+    uint64_t* empty = full + 16;                                    // [16] its group has read it
+    float* s_all = (float*)(sm + 256);                              // [KG][4][HEADS][LD_SP] parts of the scores
+    float* corr_all = s_all + KG * 4 * HEADS * LD_SP;               // [KG][HEADS]
+    float* ml_s = corr_all + KG * HEADS;                            // [KG][HEADS][2] maximum and sum
+    unsigned char* p_all = (unsigned char*)(ml_s + KG * HEADS * 2); // [KG][HEADS][LD_PP] weights
+    unsigned char* ring = (unsigned char*)(((uintptr_t)(p_all + KG * HEADS * LD_PP) + 1023) & ~(uintptr_t)1023);   // [stages] tiles, in the end [KG - 1][HEADS][C] sums
+    const int b = blockIdx.x, h0 = blockIdx.y * HEADS, nh = min(HEADS, a.heads - h0), split = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h0 = hg * HEADS, nh = min(HEADS, a.heads - h0);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < stages; i++) { mbar_init(full + i, 1); mbar_init(empty + i, LD_GW); }
+        mbar_init_fence();
+    }
     pdl_wait();
     const int len = a.len_after[b];
     const int lo = latent_first_key(a.window, len), lo32 = lo / LD_BN * LD_BN;
     int per = (len - lo32 + a.n_splits - 1) / a.n_splits;
     per = (per + LD_BN - 1) / LD_BN * LD_BN;
     const int beg = lo32 + split * per, end = min(len, beg + per);
-    const int* pt = a.page_table + (size_t)b * a.pt_stride;
-    const bf16* pool = (const bf16*)a.pool;
-    const int chunks = KD / 8;                                      // 16-byte pieces of a row
-    auto load = [&](int stage, int j0) {
-        const int r0 = a.ring_rows > 0 ? j0 % a.ring_rows : j0;       // 32 rows that start at a multiple of 32 lie in one page
-        const bf16* src = pool + ((size_t)pt[r0 / a.page_rows] * a.page_rows + (r0 % a.page_rows)) * KD;
-        unsigned char* dst = k_s + (size_t)stage * LD_BN * pitch;
-        for (int c = threadIdx.x; c < LD_BN * chunks; c += THREADS) {
-            const int r = c / chunks, ch = c % chunks;
-            ld_cp16(dst + r * pitch + ch * 16, src + (size_t)r * KD + ch * 8, j0 + r < end && j0 + r >= lo);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    if (beg < end) load(0, beg);
-    {   // the queries of this CTA's heads (rows past the last head: zeros)
-        const bf16* q = (const bf16*)a.q + (size_t)b * a.q_stride + (size_t)h0 * KD;
-        for (int c = threadIdx.x; c < HEADS * chunks; c += THREADS) {
-            const int r = c / chunks, ch = c % chunks;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (r < nh) v = *(const uint4*)(q + (size_t)r * KD + ch * 8);
-            *(uint4*)(q_s + r * pitch + ch * 16) = v;
-        }
-    }
-    float o[MT][NP * 2][4];
-#pragma unroll
-    for (int m = 0; m < MT; m++)
-#pragma unroll
-        for (int n = 0; n < NP * 2; n++) { o[m][n][0] = o[m][n][1] = o[m][n][2] = o[m][n][3] = 0.f; }
-    float m_run[4], l_run[4];                                       // of heads 4 * warp + i (every lane holds a copy)
-#pragma unroll
-    for (int i = 0; i < 4; i++) { m_run[i] = -INFINITY; l_run[i] = 0.f; }
-    const int sm_tile = warp / 4, sn_tile = warp % 4;               // scores: this warp's 16 heads and 8 keys
     const int n_tiles = beg < end ? (end - beg + LD_BN - 1) / LD_BN : 0;
-    for (int it = 0; it < n_tiles; it++) {
-        const int j0 = beg + it * LD_BN;
-        if (it + 1 < n_tiles) { load((it + 1) & 1, j0 + LD_BN); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-        else asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        const unsigned char* kt = k_s + (size_t)(it & 1) * LD_BN * pitch;
-        // ---- scores
-        float sc[4][4];
+    __syncthreads();
+    bool bad = false;                                               // a wait ran out: no more waiting, the result is void
+    auto wait = [&](uint64_t* bar, int use) {                       // the use-th completion of the barrier, counted from 0
+        if (!bad && !mbar_wait(bar, use & 1)) { bad = true; g_latent_error = 1; }
+    };
+    float o[NP * 2][4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) { sc[u][0] = sc[u][1] = sc[u][2] = sc[u][3] = 0.f; }
-        const uint32_t qa = ld_smem(q_s + (sm_tile * 16 + (lane & 15)) * pitch + (lane >> 4) * 16);
-        const uint32_t ka = ld_smem(kt + (sn_tile * 8 + (lane & 7)) * pitch + ((lane >> 3) & 1) * 16);
-        const int ksteps = KD / 16;
-        for (int ks = 0; ks < ksteps; ks += 4) {
+    for (int n = 0; n < NP * 2; n++) { o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f; }
+    const int kg = warp / LD_GW, w = warp % LD_GW, gt = threadIdx.x - kg * LD_GT;
+    if (warp == MMA_WARPS) {
+        // ---- the copies: a lane a box; the page numbers of 32 tiles at a time, asked for together
+        const int* pt = a.page_table + (size_t)b * a.pt_stride;
+        int row_of = 0;
+        for (int it = 0; it < n_tiles; it++) {
+            if (it % 32 == 0 && it + lane < n_tiles) {
+                const int j = beg + (it + lane) * LD_BN, r = a.ring_rows > 0 ? j % a.ring_rows : j;    // 32 rows from a multiple of 32 on lie in one page
+                row_of = pt[r / a.page_rows] * a.page_rows + r % a.page_rows;
+            }
+            const int st = it % stages, row = __shfl_sync(0xffffffffu, row_of, it % 32);
+            if (it >= stages) wait(empty + st, it / stages - 1);
+            if (lane == 0) mbar_expect_tx(full + st, (uint32_t)tile);
+            __syncwarp();
+            if (lane < boxes) ld_box(ring + (size_t)st * tile + lane * LD_BOX, &rows, full + st, lane * 64, row);
+        }
+        // every copy has landed before the ring becomes something else
+        for (int it = max(0, n_tiles - stages); it < n_tiles; it++)
+            if (!mbar_wait(full + it % stages, (it / stages) & 1)) g_latent_error = 1;
+    } else {
+        float* s_s = s_all + kg * 4 * HEADS * LD_SP;
+        float* corr_s = corr_all + kg * HEADS;
+        unsigned char* p_s = p_all + kg * HEADS * LD_PP;
+        const int hr = gt >> 3, k4 = (gt & 7) * 4;                  // softmax: this thread's head and four keys
+        float m_run = -INFINITY, l_run = 0.f;                       // (every one of a head's eight threads)
+        const int first = w * KS, steps = min(KS, KD / 16 - first); // this warp's 16-number steps of a row
+        uint32_t q[KS][4];                                          // its part of the queries (heads past the last one: zeros)
+        {
+            const int ra = lane >> 2, c = (lane & 3) * 2;
+            const bf16* qa = (const bf16*)a.q + (size_t)b * a.q_stride + (size_t)(h0 + ra) * KD + first * 16 + c;
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (ks + u < ksteps) {
-                    uint32_t fa[4], b0, b1;
-                    ld_ldsm4(qa + (ks + u) * 32, fa[0], fa[1], fa[2], fa[3]);
-                    ld_ldsm2(ka + (ks + u) * 32, b0, b1);
-                    ld_mma(sc[u], fa, b0, b1);
-                }
+            for (int ks = 0; ks < KS; ks++) {
+                const bool in = ks < steps, ia = in && ra < nh, ib = in && ra + 8 < nh;
+                q[ks][0] = ia ? *(const uint32_t*)(qa + ks * 16) : 0u;
+                q[ks][1] = ib ? *(const uint32_t*)(qa + (size_t)8 * KD + ks * 16) : 0u;
+                q[ks][2] = ia ? *(const uint32_t*)(qa + ks * 16 + 8) : 0u;
+                q[ks][3] = ib ? *(const uint32_t*)(qa + (size_t)8 * KD + ks * 16 + 8) : 0u;
             }
         }
-        {
-            const int r = sm_tile * 16 + (lane >> 2), cc = sn_tile * 8 + (lane & 3) * 2;
-            s_s[r * LD_BN + cc] = (sc[0][0] + sc[1][0] + sc[2][0] + sc[3][0]) * a.scale;
-            s_s[r * LD_BN + cc + 1] = (sc[0][1] + sc[1][1] + sc[2][1] + sc[3][1]) * a.scale;
-            s_s[(r + 8) * LD_BN + cc] = (sc[0][2] + sc[1][2] + sc[2][2] + sc[3][2]) * a.scale;
-            s_s[(r + 8) * LD_BN + cc + 1] = (sc[0][3] + sc[1][3] + sc[2][3] + sc[3][3]) * a.scale;
-        }
-        __syncthreads();
-        // ---- softmax of four heads per warp over the tile's 32 keys (one key per lane)
+        for (int it = kg; it < n_tiles; it += KG) {
+            const int st = it % stages, j0 = beg + it * LD_BN;
+            unsigned char* kt = ring + (size_t)st * tile;
+            wait(full + st, it / stages);
+            if (j0 < lo || j0 + LD_BN > end) {                      // rows that are not the sequence's keys: whatever the page holds there stays out
+                for (int r = 0; r < LD_BN; r++)
+                    if (j0 + r < lo || j0 + r >= end)
+                        for (int c = gt; c < boxes * 8; c += LD_GT) *(uint4*)(kt + ld_off(r, c)) = make_uint4(0, 0, 0, 0);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // (before a later copy into this place)
+                group_sync(kg);
+            }
+            // ---- this warp's part of the scores: 16 heads x 32 keys
+            const uint32_t kb = ld_smem(kt);
+            float sc[4][4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int r = warp * 4 + i;
-            const float v = (j0 + lane < end && j0 + lane >= lo) ? s_s[r * LD_BN + lane] : -INFINITY;
-            const float mn = fmaxf(m_run[i], warp_max(v));
-            const float corr = (m_run[i] == -INFINITY) ? 0.f : expf(m_run[i] - mn);
-            const float p = (v == -INFINITY) ? 0.f : expf(v - mn);
-            l_run[i] = l_run[i] * corr + warp_sum(p);
-            m_run[i] = mn;
-            *(bf16*)(p_s + r * PP + lane * 2) = __float2bfloat16_rn(p);
-            if (lane == 0) corr_s[r] = corr;
-        }
-        __syncthreads();
-        // ---- O = O * corr + P C, this warp's share of the latent's columns, for every tile of heads
+            for (int n = 0; n < 4; n++) { sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f; }
 #pragma unroll
-        for (int m = 0; m < MT; m++) {
-            const float ca = corr_s[m * 16 + (lane >> 2)], cb = corr_s[m * 16 + (lane >> 2) + 8];
+            for (int ks = 0; ks < KS; ks++) {
+                if (ks >= steps) break;                             // (the same in every lane)
+#pragma unroll
+                for (int n = 0; n < 4; n += 2) {
+                    uint32_t f[4];
+                    ld_ldsm4(kb + ld_off(n * 8 + (lane >> 4) * 8 + (lane & 7), (first + ks) * 2 + ((lane >> 3) & 1)), f[0], f[1], f[2], f[3]);
+                    ld_mma(sc[n], q[ks], f[0], f[1]);
+                    ld_mma(sc[n + 1], q[ks], f[2], f[3]);
+                }
+            }
+            {
+                float* d = s_s + (w * HEADS + (lane >> 2)) * LD_SP + (lane & 3) * 2;
+#pragma unroll
+                for (int n = 0; n < 4; n++) {
+                    *(float2*)(d + n * 8) = make_float2(sc[n][0], sc[n][1]);
+                    *(float2*)(d + n * 8 + 8 * LD_SP) = make_float2(sc[n][2], sc[n][3]);
+                }
+            }
+            group_sync(kg);
+            // ---- softmax: eight threads a head, four keys each
+            {
+                float4 sv[4];
+#pragma unroll
+                for (int x = 0; x < 4; x++) sv[x] = *(const float4*)(s_s + (x * HEADS + hr) * LD_SP + k4);
+                float v[4] = {((sv[0].x + sv[1].x) + (sv[2].x + sv[3].x)) * a.scale, ((sv[0].y + sv[1].y) + (sv[2].y + sv[3].y)) * a.scale,
+                              ((sv[0].z + sv[1].z) + (sv[2].z + sv[3].z)) * a.scale, ((sv[0].w + sv[1].w) + (sv[2].w + sv[3].w)) * a.scale};
+                float mx = -INFINITY;
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int j = j0 + k4 + e;
+                    if (j >= end || j < lo) v[e] = -INFINITY;
+                    mx = fmaxf(mx, v[e]);
+                }
+#pragma unroll
+                for (int x = 1; x < 8; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+                const float mn = fmaxf(m_run, mx);
+                const float corr = (m_run == -INFINITY) ? 0.f : expf(m_run - mn);
+                float sum = 0.f;
+#pragma unroll
+                for (int e = 0; e < 4; e++) { v[e] = (v[e] == -INFINITY) ? 0.f : expf(v[e] - mn); sum += v[e]; }
+#pragma unroll
+                for (int x = 1; x < 8; x <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+                l_run = l_run * corr + sum;
+                m_run = mn;
+                __nv_bfloat162 pa = __floats2bfloat162_rn(v[0], v[1]), pb = __floats2bfloat162_rn(v[2], v[3]);
+                *(uint2*)(p_s + hr * LD_PP + k4 * 2) = make_uint2(*(uint32_t*)&pa, *(uint32_t*)&pb);
+                if ((gt & 7) == 0) corr_s[hr] = corr;
+            }
+            group_sync(kg);
+            // ---- O = O * corr + P C, this warp's share of the latent's columns
+            const float ca = corr_s[lane >> 2], cb = corr_s[(lane >> 2) + 8];
             uint32_t pa[LD_BN / 16][4];
 #pragma unroll
             for (int kk = 0; kk < LD_BN / 16; kk++)
-                ld_ldsm4(ld_smem(p_s + (m * 16 + (lane & 15)) * PP + (kk * 16 + (lane >> 4) * 8) * 2), pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3]);
+                ld_ldsm4(ld_smem(p_s + (lane & 15) * LD_PP + (kk * 16 + (lane >> 4) * 8) * 2), pa[kk][0], pa[kk][1], pa[kk][2], pa[kk][3]);
 #pragma unroll
             for (int j = 0; j < NP; j++) {
-                const int col0 = (j * WARPS + warp) * 16;
+                const int col0 = (j * LD_GW + w) * 16;
                 if (col0 >= C) continue;
-                float* oa = o[m][2 * j]; float* ob = o[m][2 * j + 1];
+                float* oa = o[2 * j]; float* ob = o[2 * j + 1];
                 oa[0] *= ca; oa[1] *= ca; oa[2] *= cb; oa[3] *= cb; ob[0] *= ca; ob[1] *= ca; ob[2] *= cb; ob[3] *= cb;
 #pragma unroll
                 for (int kk = 0; kk < LD_BN / 16; kk++) {
                     uint32_t b0, b1, b2, b3;
-                    ld_ldsm4_t(ld_smem(kt + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * pitch + (col0 + (lane >> 4) * 8) * 2), b0, b1, b2, b3);
+                    ld_ldsm4_t(kb + ld_off(kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), col0 / 8 + (lane >> 4)), b0, b1, b2, b3);
                     ld_mma(oa, pa[kk], b0, b1);
                     ld_mma(ob, pa[kk], b2, b3);
                 }
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty + st);
         }
-        __syncthreads();                                            // the load after next overwrites this stage; s_s and p_s are free
+        if ((gt & 7) == 0) { ml_s[(kg * HEADS + hr) * 2] = m_run; ml_s[(kg * HEADS + hr) * 2 + 1] = l_run; }
     }
-    // ---- partial results: [b][h][split][C + 2]
-#pragma unroll
-    for (int m = 0; m < MT; m++) {
-        const int ra = m * 16 + (lane >> 2), rb = ra + 8;
+    // ---- the groups' sums meet: the ring becomes [KG - 1][HEADS][C] floats, the first group adds them to its own
+    __syncthreads();
+    float* o_s = (float*)ring;
+    auto each = [&](auto&& f) {                                     // f(second of its two heads, head of the CTA, column, two neighbouring sums)
 #pragma unroll
         for (int j = 0; j < NP; j++) {
-            const int col0 = (j * WARPS + warp) * 16;
+            const int col0 = (j * LD_GW + w) * 16;
             if (col0 >= C) continue;
 #pragma unroll
-            for (int half = 0; half < 2; half++) {
-                const int col = col0 + half * 8 + (lane & 3) * 2;
-                const float* acc = o[m][2 * j + half];
-                if (ra < nh) { float* p = a.partial + (((size_t)b * a.heads + h0 + ra) * a.n_splits + split) * (C + 2); p[col] = acc[0]; p[col + 1] = acc[1]; }
-                if (rb < nh) { float* p = a.partial + (((size_t)b * a.heads + h0 + rb) * a.n_splits + split) * (C + 2); p[col] = acc[2]; p[col + 1] = acc[3]; }
-            }
-        }
-    }
-    if (lane == 0) {
+            for (int half = 0; half < 2; half++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int r = warp * 4 + i;
-            if (r < nh) { float* p = a.partial + (((size_t)b * a.heads + h0 + r) * a.n_splits + split) * (C + 2); p[C] = m_run[i]; p[C + 1] = l_run[i]; }
+                for (int e = 0; e < 2; e++)
+                    f(e, (lane >> 2) + e * 8, col0 + half * 8 + (lane & 3) * 2, o[2 * j + half][2 * e], o[2 * j + half][2 * e + 1]);
         }
+    };
+    if (warp < MMA_WARPS && kg > 0)
+        each([&](int, int r, int c, float& x, float& y) { *(float2*)(o_s + ((size_t)(kg - 1) * HEADS + r) * C + c) = make_float2(x, y); });
+    __syncthreads();
+    if (warp < LD_GW) {
+        float f[2][KG];                                             // the groups' factors for this thread's heads
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int r = (lane >> 2) + e * 8;
+            float M = -INFINITY;
+#pragma unroll
+            for (int k = 0; k < KG; k++) M = fmaxf(M, ml_s[(k * HEADS + r) * 2]);
+#pragma unroll
+            for (int k = 0; k < KG; k++) { const float mk = ml_s[(k * HEADS + r) * 2]; f[e][k] = mk == -INFINITY ? 0.f : expf(mk - M); }
+        }
+        each([&](int e, int r, int c, float& x, float& y) {
+            x *= f[e][0]; y *= f[e][0];
+#pragma unroll
+            for (int k = 1; k < KG; k++) {
+                const float2 z = *(const float2*)(o_s + ((size_t)(k - 1) * HEADS + r) * C + c);
+                x = fmaf(z.x, f[e][k], x); y = fmaf(z.y, f[e][k], y);
+            }
+        });
     }
+    __syncthreads();                                                // (maxima and sums have been read)
+    if (threadIdx.x < HEADS) {
+        float M = -INFINITY, L = 0.f;
+#pragma unroll
+        for (int k = 0; k < KG; k++) M = fmaxf(M, ml_s[(k * HEADS + threadIdx.x) * 2]);
+#pragma unroll
+        for (int k = 0; k < KG; k++) { const float mk = ml_s[(k * HEADS + threadIdx.x) * 2]; if (mk != -INFINITY) L += ml_s[(k * HEADS + threadIdx.x) * 2 + 1] * expf(mk - M); }
+        ml_s[threadIdx.x * 2] = M; ml_s[threadIdx.x * 2 + 1] = L;   // (group 0's place: each head's thread reads it before)
+    }
+    if (!in_cluster) {
+        // ---- partial results: [b][h][split][C + 2]
+        __syncthreads();
+        float* p = a.partial + (((size_t)b * a.heads + h0) * a.n_splits + split) * (C + 2);
+        const size_t step = (size_t)a.n_splits * (C + 2);
+        if (warp < LD_GW) each([&](int, int r, int c, float& x, float& y) { if (r < nh) { p[r * step + c] = x; p[r * step + c + 1] = y; } });
+        if (threadIdx.x < nh) { p[threadIdx.x * step + C] = ml_s[threadIdx.x * 2]; p[threadIdx.x * step + C + 1] = ml_s[threadIdx.x * 2 + 1]; }
+        return;
+    }
+    // ---- the pieces of the sequence meet: every CTA of the cluster adds and writes a slice of the outputs
+    if (warp < LD_GW) each([&](int, int r, int c, float& x, float& y) { *(float2*)(o_s + (size_t)r * C + c) = make_float2(x, y); });
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const int S = a.n_splits, rank = (int)cluster.block_rank();
+    float* f_s = s_all;                                             // [HEADS][CL]: every piece's share of the result (the scores are done with)
+    if (threadIdx.x < nh) {
+        const int r = threadIdx.x;
+        const float sink = (a.sink != nullptr) ? a.sink[h0 + r] : -INFINITY;
+        float m[CL], l[CL], M = sink;
+#pragma unroll
+        for (int k = 0; k < CL; k++) {
+            m[k] = -INFINITY; l[k] = 0.f;
+            if (k < S) { const float2 ml = *(const float2*)(cluster.map_shared_rank(ml_s, k) + r * 2); m[k] = ml.x; l[k] = ml.y; }
+        }
+#pragma unroll
+        for (int k = 0; k < CL; k++) M = fmaxf(M, m[k]);
+        float L = (sink != -INFINITY) ? expf(sink - M) : 0.f;
+#pragma unroll
+        for (int k = 0; k < CL; k++) { m[k] = m[k] == -INFINITY ? 0.f : expf(m[k] - M); L += l[k] * m[k]; }
+#pragma unroll
+        for (int k = 0; k < CL; k++) f_s[r * CL + k] = m[k] / L;
+    }
+    __syncthreads();
+    const int quads = C / 4, per_cta = (nh * quads + S - 1) / S;    // four neighbouring columns a thread and turn
+    for (int i = rank * per_cta + threadIdx.x; i < min(nh * quads, (rank + 1) * per_cta); i += blockDim.x) {
+        const int r = i / quads, c = (i - r * quads) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < CL; k++)
+            if (k < S) {
+                const float4 x = *(const float4*)(cluster.map_shared_rank(o_s, k) + (size_t)r * C + c);
+                const float f = f_s[r * CL + k];
+                v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
+            }
+        bf16* out = (bf16*)a.out + (size_t)b * a.out_stride + (size_t)(h0 + r) * a.out_dim + c;
+        out[0] = __float2bfloat16_rn(v.x); out[1] = __float2bfloat16_rn(v.y); out[2] = __float2bfloat16_rn(v.z); out[3] = __float2bfloat16_rn(v.w);
+    }
+    cluster.sync();                                                 // nobody leaves while its sums are being read
 }
 
 extern "C" int tb_latent_decode_mma_takes(int C, int R) {
     return C > 0 && C % 16 == 0 && (C + R) % 16 == 0 && C <= 512 && (C + R) <= 1024;
 }
 
+// Reads and clears the error word (1: a bounded wait on a copy of rows ran out; that launch's results are void).  Synchronises.
+extern "C" int tb_latent_decode_error() {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_latent_error, sizeof v) != cudaSuccess) return -1;
+    if (v) cudaMemcpyToSymbol(g_latent_error, &zero, sizeof zero);
+    return v;
+}
+
+// Which pieces meet in a cluster: one, two or four (three leave SMs of a GPC empty), eight where that is up to 64 CTAs
+// (128 sequences' pieces in clusters of eight take two rounds).
+static int latent_units(int batch, int heads) { return batch * ((heads + LD_H - 1) / LD_H); }
+static bool latent_in_cluster(int pieces, int units) { return pieces == 1 || pieces == 2 || pieces == 4 || (pieces == 8 && units <= 8); }
+extern "C" int tb_latent_decode_folds(int pieces, int batch, int heads) { return !latent_in_cluster(pieces, latent_units(batch, heads)); }
+// In how many pieces a launch of `batch` sequences of up to `rows` keys cuts each: the count that wastes least of the last
+// round of CTAs (one an SM), a piece's start and end being worth five turns of its three groups (2.5 us each), with a launch that
+// folds ten; clusters of four and eight do not fill more than one round well (96 units of 3,000 rows in four: 95 us, in three: 79).
+extern "C" int tb_latent_decode_pieces(int batch, int heads, int rows, int sms) {
+    const int units = latent_units(batch, heads), tiles = (rows + LD_BN - 1) / LD_BN;
+    int best = 1;
+    double best_eff = 0.0;
+    for (int s = 1; s <= 64 && s * 3 <= tiles + 2; s++) {
+        const long long ctas = (long long)units * s;
+        const double turns = (double)((tiles + s - 1) / s + 2) / 3;
+        const bool cluster = latent_in_cluster(s, units);
+        double eff = (double)ctas / ((double)((ctas + sms - 1) / sms) * sms) * turns / (turns + (cluster ? 5.0 : 10.0));
+        if (cluster && s >= 4 && ctas > sms) eff *= 0.85;
+        if (eff > best_eff + 1e-9) { best = s; best_eff = eff; }
+    }
+    return best;
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// The pool as a matrix of rows of KD numbers (how many is not known here: the page table decides which are read); numbers
+// past a row's end come as zeros.
+static int rows_map(CUtensorMap* m, const void* pool, int KD) {
+    static EncodeTiledFn fn = nullptr;
+    if (!fn) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = (EncodeTiledFn)p;
+        if (!fn) return tb_refuse("latent_decode: the driver does not provide cuTensorMapEncodeTiled");
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)KD, (cuuint64_t)0x7fffff00}, strides[1] = {(cuuint64_t)KD * 2};
+    const cuuint32_t box[2] = {64, LD_BN}, one[2] = {1, 1};
+    const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)pool, dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : tb_refuse("latent_decode: cuTensorMapEncodeTiled failed with %d", (int)r);
+}
+
+template <int NP, int KS, int KG, int CL>
+static int run_latent_mma(const LatentDecodeArgs& a, int batch, cudaStream_t stream) {
+    const int KD = a.C + a.R, head = ld_head_bytes<KG>(), tile = ld_tile_bytes(KD);
+    int stages = (227 * 1024 - head) / tile;
+    stages = stages > 16 ? 16 : stages;
+    if (stages < 2) return tb_refuse("latent_decode_mma: rows of %d numbers leave no room for two tiles", KD);
+    const int smem = head + stages * tile;
+    const bool in_cluster = latent_in_cluster(a.n_splits, latent_units(batch, a.heads));
+    const cudaError_t e = cudaFuncSetAttribute(latent_decode_mma_kernel<NP, KS, KG, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(batch, (a.heads + LD_H - 1) / LD_H, a.n_splits); cfg.blockDim = dim3((LD_GW * KG + 1) * 32);
+    cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = in_cluster ? a.n_splits : 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    CUtensorMap rows;
+    if (rows_map(&rows, a.pool, KD)) return -1;
+    cudaLaunchKernelEx(&cfg, latent_decode_mma_kernel<NP, KS, KG, CL>, a, rows, stages, (int)in_cluster);
+    int st = tb_launch_status();
+    if (st || in_cluster) return st;
+    tb_launch(latent_combine_kernel<bf16>, dim3(batch, a.heads), dim3(128), 0, stream, a);
+    return tb_launch_status();
+}
+
 extern "C" int tb_latent_decode_mma(const LatentDecodeArgs* args, int batch, cudaStream_t stream) {
     if (batch <= 0) return 0;
     const LatentDecodeArgs& a = *args;
     if (!tb_latent_decode_mma_takes(a.C, a.R)) return tb_refuse("latent_decode_mma: C=%d R=%d (multiples of 16, C <= 512)", a.C, a.R);
-    if (a.partial == nullptr || a.n_splits < 1 || a.n_splits > 65535 || a.out_dim < a.C || a.page_rows % LD_BN)
+    if (a.n_splits < 1 || a.n_splits > 65535 || (a.partial == nullptr && !latent_in_cluster(a.n_splits, latent_units(batch, a.heads))) || a.out_dim < a.C || a.page_rows % LD_BN)
         return tb_refuse("latent_decode_mma: n_splits=%d needs scratch; pages of %d rows", a.n_splits, a.page_rows);
     if (((uintptr_t)a.q & 15) || (a.q_stride % 8) || ((uintptr_t)a.pool & 15)) return tb_refuse("latent_decode_mma: rows must be 16-byte aligned");
-    const int KD = a.C + a.R, pitch = KD * 2 + 16;
-    const int mt = a.heads > 16 ? 2 : 1, heads_cta = 16 * mt, warps = 4 * mt;
-    const size_t smem = (size_t)heads_cta * pitch + 2 * (size_t)LD_BN * pitch + heads_cta * LD_BN * 4 + heads_cta * (LD_BN * 2 + 16) + heads_cta * 4;
-    const int np = (a.C + 16 * warps - 1) / (16 * warps);
-    dim3 grid(batch, (a.heads + heads_cta - 1) / heads_cta, a.n_splits);
-#define LD_MMA(N, M) do { \
-        static bool set = false; \
-        if (!set) { cudaError_t e = cudaFuncSetAttribute(latent_decode_mma_kernel<N, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
-                    if (e != cudaSuccess) return (int)e; set = true; } \
-        tb_launch(latent_decode_mma_kernel<N, M>, dim3(grid), dim3(warps * 32), smem, stream, a); } while (0)
-    if (mt == 1) { if (np <= 2) LD_MMA(2, 1); else if (np <= 4) LD_MMA(4, 1); else LD_MMA(8, 1); }
-    else { if (np <= 1) LD_MMA(1, 2); else if (np <= 2) LD_MMA(2, 2); else LD_MMA(4, 2); }
-    int st = tb_launch_status();
-    if (st) return st;
-    tb_launch(latent_combine_kernel<bf16>, dim3(batch, a.heads), dim3(128), 0, stream, a);
-    return tb_launch_status();
+    const int KD = a.C + a.R;
+#define LD_RUN(N, K, G) (a.n_splits == 8 ? run_latent_mma<N, K, G, 8>(a, batch, stream) : run_latent_mma<N, K, G, 4>(a, batch, stream))
+    return KD <= 256 ? LD_RUN(4, 4, 3) : KD <= 512 ? LD_RUN(8, 8, 3) : LD_RUN(8, 16, 2);
+#undef LD_RUN
 }
 
 extern "C" int tb_latent_decode(const LatentDecodeArgs* args, int dtype, int batch, cudaStream_t stream) {

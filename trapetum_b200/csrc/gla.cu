@@ -768,7 +768,7 @@ static int run_blocks(const GlaArgs& a, cudaStream_t stream) {
     const int smem = BlockSmem<DP>::bytes(a.V);
     const dim3 grid(a.heads, a.batch * a.n_chunks), block(a.V * 2);
     auto launch = [&](void (*kern)(GlaArgs)) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BlockSmem<DP>::bytes(256));
         if (e != cudaSuccess) return (int)e;
         tb_launch(kern, grid, block, smem, stream, a);
         return tb_launch_status();

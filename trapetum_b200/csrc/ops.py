@@ -1078,6 +1078,8 @@ def kernel_errors() -> dict:
         out["gemm_tc"] = "a bounded wait ran out"
     if "attention_decode" in loaded and attn_decode_error():
         out["attention_decode"] = "a bounded wait ran out"
+    if "attention_latent" in loaded and int(build.load("attention_latent").tb_latent_decode_error()):
+        out["attention_latent"] = "a bounded wait ran out"
     for name in loaded:
         if name.startswith("attention_prefill_tc@"):
             v = int(build.load(name).tb_attn_prefill_tc_error())
@@ -1783,12 +1785,14 @@ def latent_decode(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Tensor,
     lib = build.load("attention_latent")
     mma = q.dtype == torch.bfloat16 and bool(lib.tb_latent_decode_mma_takes(c_int(C), c_int(R))) and q.stride(0) % 8 == 0 \
         and q.data_ptr() % 16 == 0
-    # pieces: enough CTAs for about two per SM, none shorter than 128 keys (256 on the generic kernel)
-    units = B * ((heads + 31) // 32 if heads > 16 else 1) if mma else B * heads          # the tensor-core kernel: up to 32 heads a CTA
-    shortest = 128 if mma else 256
-    pieces = max(1, min((len_bucket + shortest - 1) // shortest, max(1, (2 * sm_count(q.device)) // max(1, units))))
+    if mma:         # one CTA an SM, up to 16 heads of a sequence each
+        pieces = int(lib.tb_latent_decode_pieces(c_int(B), c_int(heads), c_int(int(len_bucket)), c_int(sm_count(q.device))))
+    else:           # enough CTAs for about two per SM, none shorter than 256 keys
+        pieces = max(1, min((len_bucket + 255) // 256, max(1, (2 * sm_count(q.device)) // max(1, B * heads))))
     out = torch.empty((B, heads * C), dtype=q.dtype, device=q.device)
-    scratch = torch.empty(B * heads * pieces * (C + 2), dtype=torch.float32, device=q.device) if (pieces > 1 or mma) else None
+    # (few pieces of the tensor-core kernel meet in a cluster)
+    folded = bool(lib.tb_latent_decode_folds(c_int(pieces), c_int(B), c_int(heads))) if mma else pieces > 1
+    scratch = torch.empty(B * heads * pieces * (C + 2), dtype=torch.float32, device=q.device) if folded else None
     a = _LatentDecodeArgs()
     a.q = q.data_ptr(); a.q_stride = q.stride(0); a.pool = pool.data_ptr()
     a.page_table = page_table.data_ptr(); a.pt_stride = page_table.stride(0); a.page_rows = PAGE_ROWS
@@ -1797,7 +1801,7 @@ def latent_decode(q: torch.Tensor, pool: torch.Tensor, page_table: torch.Tensor,
     a.heads = heads; a.C = C; a.R = R; a.out_dim = C; a.n_splits = pieces; a.scale = scale
     a.window = window or 0; a.ring_rows = ring_rows
     if mma:
-        _check(lib, lib.tb_latent_decode_mma(ctypes.byref(a), c_int(B), _stream()), "latent_decode_mma", 2)
+        _check(lib, lib.tb_latent_decode_mma(ctypes.byref(a), c_int(B), _stream()), "latent_decode_mma", 2 if folded else 1)
     else:
         _check(lib, lib.tb_latent_decode(ctypes.byref(a), c_int(code(q.dtype)), c_int(B), _stream()), "latent_decode",
                2 if pieces > 1 else 1)
