@@ -735,6 +735,40 @@ def test_sample_draws_follow_the_inverse_cdf(ops, V, temperature, top_p):
         assert lo - 1e-4 <= float(u[i]) <= float(cdf[tok]) + 1e-4
 
 
+@pytest.mark.parametrize("V", [16384, 40001, 256000])
+@pytest.mark.parametrize("kind", ["equal", "three values", "masked", "flat", "spike"])
+def test_sample_where_logits_crowd(ops, V, kind):
+    """Rows whose threshold falls among more elements than a row lists (equal logits), that hold -inf, whose logits lie
+    close together, or one far above the rest; tokens as the float64 nucleus in index order gives them."""
+    rows = 24
+    x = rnd(rows, V, s=2.0, seed=V)
+    if kind == "equal":
+        x[:] = 1.5
+    elif kind == "three values":
+        x = torch.round(x / 4.0).clamp(-1, 1) + 0.0                     # (no -0: its key is below that of 0)
+    elif kind == "masked":
+        x[:, V // 50:] = -math.inf
+    elif kind == "flat":
+        x *= 1e-3
+    else:
+        x = (x * 1e-2)
+        x[:, V // 3] = 10.0
+    u = torch.linspace(0.001, 0.999, rows)
+    t, p, pen, ud = _args(rows, 0.9, 0.6, 1.0, u)
+    got = ops.sample(x.clone(), t, p, pen, ud, None).cpu().tolist()
+    for i in range(rows):
+        row = x[i].double().cpu()
+        m = torch.exp((row - row.max()) / 0.9)
+        order = torch.sort(row, descending=True).values                  # equal logits are kept or left together, by their value
+        cum = torch.cumsum(torch.exp((order - row.max()) / 0.9), 0)
+        thr = order[min(V - 1, int((cum < 0.6 * m.sum() * (1 - 1e-6)).sum()))]
+        m[row < thr] = 0.0
+        cdf = torch.cumsum(m, 0) / m.sum()
+        tok = got[i]
+        assert m[tok] > 0, "a token outside the nucleus was drawn"
+        assert float(cdf[tok] - m[tok] / m.sum()) - 1e-4 <= float(u[i]) <= float(cdf[tok]) + 1e-4
+
+
 @pytest.mark.parametrize("V", [500, 20011])
 def test_sample_mixed_rows(ops, V):
     x = rnd(3, V, s=3.0)

@@ -934,7 +934,7 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_p: torch.Tensor,
         need = int(lib.tb_sample_wide_scratch_bytes(c_int(rows), c_int(V)))
         scratch = torch.empty(need, dtype=torch.uint8, device=logits.device)
         _check(lib, lib.tb_sample_wide(ctypes.byref(a), c_int(rows), _ptr(scratch), c_int(1 if nucleus else 0), _stream()),
-               "sample", 10 if nucleus else 4)
+               "sample", 4 if nucleus else 3)
         return out
     _check(lib, lib.tb_sample(ctypes.byref(a), c_int(rows), _stream()), "sample")
     return out

@@ -229,65 +229,118 @@ __global__ void __launch_bounds__(1024) sample_kernel(SampleArgs a) {
 //
 // Masses are fixed-point: m_i = round(2^32 e^((l_i - max) / T)), summed in 64-bit integers.  Integer sums do not
 // depend on their order, so histograms can be built with atomics and the draw still repeats bit for bit.
-// The nucleus threshold is found by a radix search on the order-preserving key of the logit: three passes
-// (11 + 11 + 10 bits), each a histogram of mass per digit among the elements that match the digits found so far,
-// and a scan from the top for the digit at which the mass above reaches top_p x total.
+// The nucleus threshold is the key (the order-preserving bits) of the logit at which the mass of that key and all above
+// reaches top_p x total.  One histogram of mass over 2,048 equal steps of (max - l) / T, which the elements of a row spread
+// over (they fall into few digits of the key, and same-address atomics of a warp wait for one another), finds the step; its
+// elements, a thousandth of a row, are listed, and a CTA of the row finds the key among them by a radix search.
 //
-//   sample_chunk_max  per chunk: repetition penalty on the chunk's ids, then (max, index)   [also the greedy choice];
-//                     clears the row's histograms
-//   sample_hist<R>    per chunk: (R > 0: first the digit of pass R-1, found by every CTA for itself from the
-//                     finished histogram;) mass histogram of pass R            [rows with a nucleus only]
-//   sample_chunk_mass per chunk: the last digit, hence the threshold; mass of the chunk's kept elements
-//   sample_pick       per row: target = u x kept mass; the chunk and then the element at which the running sum
-//                     of kept masses, in index order, passes the target
+//   sample_chunk_max  per chunk: repetition penalty on the chunk's ids, then (max, index) and min  [also the greedy choice];
+//                     clears the row's histogram
+//   sample_hist       per chunk: mass per step; the row's last CTA finds the threshold's  [rows with a nucleus only]
+//   sample_chunk_mass per chunk: mass of the elements above the threshold's step; lists those in it (without a nucleus:
+//                     mass of all)
+//   sample_pick       per row: the threshold from the listed elements (from the row itself if they are too many: equal
+//                     logits), their kept masses added to their chunks', target = u x kept mass; the chunk and then the
+//                     element at which the running sum of kept masses, in index order, passes the target
+// 256,000 logits, top_p 0.95, in a graph: 38 / 45 / 63 / 94 us for 1 / 8 / 32 / 64 rows; six launches that read the row five
+// times (three histograms over the key's digits) took 45 / 76 / 96 / 156.
 // ---------------------------------------------------------------------------
 #define S_CHUNK 8192
 #define S_BINS 2048
+#define S_LIST 4096               // elements of the threshold's step that are listed
 typedef unsigned long long u64;
 
-struct SampleState {              // per row
-    u64 mass_above;               // mass of the elements above the digits found so far
-    u64 want;                     // top_p x total mass
-    unsigned prefix;              // the digits found so far (the high bits of the threshold key)
-    int nucleus;                  // 1: this row searches a threshold; 0: keeps everything (or is greedy)
+struct SampleState {              // per row with a nucleus, left by sample_hist
+    u64 want;                     // what the elements of the threshold's step have to reach
+    int edge;                     // the threshold's step; S_BINS: there are no masses, everything is kept
 };
 
 struct SampleWide {
     SampleArgs a;
-    int n_chunks;
-    float* pmax; int* pidx;       // [rows][n_chunks]
-    u64* hist;                    // [rows][3][S_BINS]
-    u64* cmass;                   // [rows][n_chunks]
-    SampleState* state;           // [rows][3]: after pass 0, 1, 2
+    int n_chunks;                 // chunks of a row
+    int vec;                      // rows start on 16-byte boundaries
+    float* pmax; float* pmin; int* pidx;   // [rows][n_chunks]
+    u64* hist;                    // [rows][S_BINS]
+    u64* cmass;                   // [rows][n_chunks] mass above the threshold's step
+    u64* emass;                   // [rows][n_chunks] mass in it
+    SampleState* state;           // [rows]
+    int* done;                    // [rows] CTAs of sample_hist that have added their masses
+    int* count;                   // [rows] listed elements (those that would be, if they are too many)
+    int* list;                    // [rows][S_LIST] their places
 };
 
 __device__ __forceinline__ u64 fixed_mass(float l, float mx, float invT) {
     return __float2ull_rn(expf((l - mx) * invT) * 4294967296.0f);
 }
-// the row's maximum from the chunk maxima (every thread of the CTA gets it)
-__device__ __forceinline__ float row_max(const SampleWide& w, int row, float* red /* 33 */) {
-    float m = -INFINITY;
-    for (int c = threadIdx.x; c < w.n_chunks; c += blockDim.x) m = fmaxf(m, w.pmax[(size_t)row * w.n_chunks + c]);
-    return block_max(m, red);
+// f(logit, its place) over a chunk by 256 threads, 16 bytes a load and all of a thread's loads on their way together
+// (true: thread t's u-th element is number (u / 4 * 256 + t) * 4 + u % 4 of the chunk; else u * 256 + t)
+template <typename F>
+__device__ __forceinline__ bool each_of_chunk(const SampleWide& w, const float* x, int chunk, F&& f) {
+    const int beg = chunk * S_CHUNK, n = min(w.a.vocab - beg, S_CHUNK);
+    if (w.vec && n == S_CHUNK) {
+        float4 v[S_CHUNK / 1024];
+#pragma unroll
+        for (int u = 0; u < S_CHUNK / 1024; u++) v[u] = *(const float4*)(x + beg + (u * 256 + threadIdx.x) * 4);
+#pragma unroll
+        for (int u = 0; u < S_CHUNK / 1024; u++) {
+            const int i = beg + (u * 256 + threadIdx.x) * 4;
+            f(v[u].x, i); f(v[u].y, i + 1); f(v[u].z, i + 2); f(v[u].w, i + 3);
+        }
+        return true;
+    }
+    for (int i = threadIdx.x; i < n; i += 256) f(x[beg + i], beg + i);
+    return false;
+}
+// the row's maximum and minimum from the chunks' (every thread of the CTA gets them)
+__device__ __forceinline__ void row_range(const SampleWide& w, int row, float* red /* 33 */, float& mx, float& mn) {
+    mx = -INFINITY; mn = INFINITY;
+    for (int c = threadIdx.x; c < w.n_chunks; c += blockDim.x) {
+        mx = fmaxf(mx, w.pmax[(size_t)row * w.n_chunks + c]);
+        mn = fminf(mn, w.pmin[(size_t)row * w.n_chunks + c]);
+    }
+    mx = block_max(mx, red);
+    mn = -block_max(-mn, red);
+}
+__device__ __forceinline__ bool row_has_nucleus(const SampleArgs& a, int row) {
+    return (a.temperature ? a.temperature[row] : 0.f) > 0.f && (a.top_p ? a.top_p[row] : 1.f) < 1.f;
+}
+// Steps of (max - l) / T: from 0 to the row's range, or to 23, from where on a mass is 0 (2^32 e^-23 < 1/2).  Rounding is
+// monotonic, so a larger logit is never in a later step.
+struct Steps { float mx, invT, scale; };
+__device__ __forceinline__ Steps row_steps(float mx, float mn, float T) {
+    Steps s;
+    s.mx = mx; s.invT = 1.f / T;
+    const float reach = fminf((mx - mn) * s.invT, 23.f);            // (a range that is not a number: 23)
+    s.scale = reach > 0.f ? (float)S_BINS / reach : 0.f;
+    return s;
+}
+// the step of a logit; -1: its mass is 0; -2: not a number (a logit that is none, or an infinite one beside an infinite maximum)
+__device__ __forceinline__ int step_of(const Steps& s, float l) {
+    const float x = (s.mx - l) * s.invT;
+    if (x < 23.f) return min((int)(x * s.scale), S_BINS - 1);
+    return x >= 23.f ? -1 : -2;
 }
 
 __global__ void __launch_bounds__(256) sample_chunk_max_kernel(SampleWide w) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ ValIdx red[32];
+    __shared__ float redf[33];
     __shared__ int rec_s[1024];
-    const int row = blockIdx.y, chunk = blockIdx.x, tid = threadIdx.x;
+    const int row = blockIdx.y, tid = threadIdx.x;
     const SampleArgs& a = w.a;
     float* x = a.logits + (size_t)row * a.row_stride;
+    // this CTA's share of the row's histogram starts at zero
+    for (int i = blockIdx.x * 256 + tid; i < S_BINS; i += gridDim.x * 256) w.hist[(size_t)row * S_BINS + i] = 0ull;
+    if (blockIdx.x == 0 && tid == 0) w.count[row] = w.done[row] = 0;
+    const int chunk = blockIdx.x;
     const int beg = chunk * S_CHUNK, end = min(a.vocab, beg + S_CHUNK);
-    // this CTA's share of the row's histograms starts at zero
-    for (int i = chunk * 256 + tid; i < 3 * S_BINS; i += gridDim.x * 256) w.hist[(size_t)row * 3 * S_BINS + i] = 0ull;
-    // repetition penalty, each distinct recent id once; a CTA sees to the ids of its own chunk
+    // repetition penalty, each distinct recent id once; a CTA sees to the ids of its own chunks
     const float pen = a.penalty ? a.penalty[row] : 1.f;
     if (pen > 1.f && a.recent) {
         const int* rec = a.recent + (size_t)row * a.n_recent;
-        for (int j0 = 0; j0 < a.n_recent; j0 += 1024) {            // (lists longer than 1024 in pieces; each id is
-            const int n = min(1024, a.n_recent - j0);               //  compared with the whole list before it)
+        for (int j0 = 0; j0 < a.n_recent; j0 += 1024) {        // (lists longer than 1024 in pieces; each id is
+            const int n = min(1024, a.n_recent - j0);           //  compared with the whole list before it)
             __syncthreads();
             for (int j = tid; j < n; j += 256) rec_s[j] = rec[j0 + j];
             __syncthreads();
@@ -303,167 +356,173 @@ __global__ void __launch_bounds__(256) sample_chunk_max_kernel(SampleWide w) {
         __syncthreads();
     }
     ValIdx b; b.v = -INFINITY; b.i = 0x7fffffff;
-    for (int i = beg + tid; i < end; i += 256) { ValIdx c; c.v = x[i]; c.i = i; b = better(b, c); }
+    float mn = INFINITY;
+    each_of_chunk(w, x, chunk, [&](float l, int i) { ValIdx c; c.v = l; c.i = i; b = better(b, c); mn = fminf(mn, l); });
     b = block_best(b, red);
-    if (tid == 0) { w.pmax[(size_t)row * w.n_chunks + chunk] = b.v; w.pidx[(size_t)row * w.n_chunks + chunk] = b.i; }
+    mn = -block_max(-mn, redf);
+    if (tid == 0) {
+        w.pmax[(size_t)row * w.n_chunks + chunk] = b.v; w.pidx[(size_t)row * w.n_chunks + chunk] = b.i;
+        w.pmin[(size_t)row * w.n_chunks + chunk] = mn;
+    }
 }
 
-// the digit of pass R of a key, and whether the key matches the digits found before it
-template <int R> __device__ __forceinline__ bool digit_of(unsigned key, unsigned prefix, int& bin) {
-    if (R == 0) { bin = key >> 21; return true; }
-    if (R == 1) { bin = (key >> 10) & 2047; return (key >> 21) == prefix; }
-    bin = key & 1023; return (key >> 10) == prefix;
-}
-
-// The digit of pass R from its finished histogram `g` (in shared memory), by a CTA of 256 threads: each thread sums
-// eight digits, warp 0 scans the sums from the top, and the lane in which the mass above reaches `want` walks down
-// its own sums and then the eight digits of one of them.  `*st` (shared memory) is the state before the pass on
-// entry and the state after it on return.
-template <int R>
-__device__ void select_digit(const u64* g, u64* part /* 256 */, SampleState* st_io, float top_p) {
+// Where the running sum of a histogram's masses reaches `want`: the entry, and the mass before it.  `down`: from the last
+// entry to the first.  All zero: entry 0 (the last one).  `g`: S_BINS sums in shared memory; called by the whole CTA.
+struct Reached { u64 before, total; int entry; };
+__device__ void find_entry(const u64* g, u64* part /* 256 */, Reached* out, bool down, u64 want, float top_p) {
     const int tid = threadIdx.x, lane = tid & 31;
-    u64 s = 0ull;
+    auto at = [&](int i) { return g[down ? S_BINS - 1 - i : i]; };
+    if (tid < 256) {
+        u64 s = 0ull;
 #pragma unroll
-    for (int k = 0; k < 8; k++) s += g[tid * 8 + k];
-    part[tid] = s;
+        for (int k = 0; k < 8; k++) s += at(tid * 8 + k);
+        part[tid] = s;
+    }
     __syncthreads();
     if (tid < 32) {
-        SampleState st = *st_io;
         u64 mine = 0ull;
 #pragma unroll
         for (int k = 0; k < 8; k++) mine += part[lane * 8 + k];
-        u64 incl = mine;                             // this lane's sum and those of the lanes above it (higher digits)
-        for (int o = 1; o < 32; o <<= 1) { const u64 v = __shfl_down_sync(0xffffffffu, incl, o); if (lane + o < 32) incl += v; }
-        if (R == 0) {
-            const u64 tot = __shfl_sync(0xffffffffu, incl, 0);       // the total mass, and what the nucleus has to reach
-            const double want = (double)top_p * (double)tot;
-            st.want = want < 1.0 ? 1ull : (u64)want;
-            if (st.want > tot) st.want = tot;
+        u64 incl = mine;
+        for (int o = 1; o < 32; o <<= 1) { const u64 v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+        const u64 tot = __shfl_sync(0xffffffffu, incl, 31);
+        if (top_p > 0.f || want == 0ull) {                          // (the first search: what the nucleus has to reach)
+            const double d = (double)top_p * (double)tot;
+            want = d < 1.0 ? 1ull : (u64)d;
+            if (want > tot) want = tot;
         }
-        const u64 above = st.mass_above + incl - mine;
-        const bool here = above < st.want && above + mine >= st.want;
-        u64 acc = above;
-        int b = 0;
+        const u64 before = incl - mine;
+        const bool here = before < want && incl >= want;
+        u64 acc = before;
+        int i = 0;
         if (here) {
-            int t = lane * 8 + 7;
-            for (; t > lane * 8; t--) { if (acc + part[t] >= st.want) break; acc += part[t]; }
-            b = t * 8 + 7;
-            for (; b > t * 8; b--) { if (acc + g[b] >= st.want) break; acc += g[b]; }
+            int t = lane * 8;
+            for (; t < lane * 8 + 7; t++) { if (acc + part[t] >= want) break; acc += part[t]; }
+            i = t * 8;
+            for (; i < t * 8 + 7; i++) { if (acc + at(i) >= want) break; acc += at(i); }
         }
         const unsigned who = __ballot_sync(0xffffffffu, here);
-        const int src = who ? __ffs(who) - 1 : 0;    // (exactly one lane, unless the masses are all zero)
-        st.mass_above = __shfl_sync(0xffffffffu, acc, src);
-        b = __shfl_sync(0xffffffffu, b, src);
-        st.prefix = (R == 0) ? (unsigned)b : (R == 1) ? ((st.prefix << 11) | (unsigned)b) : ((st.prefix << 10) | (unsigned)b);
-        if (lane == 0) *st_io = st;
+        const int src = who ? __ffs(who) - 1 : 0;                   // (exactly one lane, unless the masses are all zero)
+        acc = __shfl_sync(0xffffffffu, acc, src);
+        i = __shfl_sync(0xffffffffu, i, src);
+        if (lane == 0) { out->before = acc; out->total = want; out->entry = down ? S_BINS - 1 - i : i; }
     }
     __syncthreads();
 }
 
-// The state before pass R for this CTA (R == 0: the start), into shared memory: found from the finished histogram
-// of pass R-1; the CTA of chunk 0 also leaves it in memory for the launches after this one.  `g`: S_BINS sums.
-template <int R>
-__device__ void state_before_pass(const SampleWide& w, int row, u64* g, u64* part, SampleState* out) {
-    if (threadIdx.x == 0) {
-        SampleState st;
-        const float T = w.a.temperature ? w.a.temperature[row] : 0.f;
-        const float tp = w.a.top_p ? w.a.top_p[row] : 1.f;
-        const int nucleus = (T > 0.f && tp < 1.f) ? 1 : 0;
-        st.mass_above = 0ull; st.want = 0ull; st.prefix = 0u;
-        // a row without a nucleus leaves no state behind (its CTAs return before they would write it), so whether a
-        // row has one is taken from its own parameters in every pass, never from that memory
-        if (R > 1 && nucleus) st = w.state[(size_t)row * 3 + (R > 1 ? R - 2 : 0)];
-        st.nucleus = nucleus;
-        *out = st;
-    }
-    __syncthreads();
-    if constexpr (R > 0) {
-        if (!out->nucleus) return;
-        const u64* gg = w.hist + ((size_t)row * 3 + (R - 1)) * S_BINS;
-        for (int j = threadIdx.x; j < S_BINS; j += blockDim.x) g[j] = gg[j];
-        __syncthreads();
-        select_digit<R - 1>(g, part, out, R == 1 ? w.a.top_p[row] : 0.f);
-        if (threadIdx.x == 0 && blockIdx.x == 0) w.state[(size_t)row * 3 + (R - 1)] = *out;
-    }
+// A mass is at most 2^32.  Its low 16 bits and the rest are summed in two 32-bit histograms, whose atomics the shared
+// memory has natively (a 64-bit one is a compare-and-swap loop); the elements of seven chunks cannot overflow either.
+constexpr int S_MOST_CHUNKS = 7;
+__device__ __forceinline__ void add_mass(unsigned* lo, unsigned* hi, int entry, u64 m) {
+    atomicAdd(&lo[entry], (unsigned)(m & 0xffffu));
+    atomicAdd(&hi[entry], (unsigned)(m >> 16));
 }
 
-template <int R>
 __global__ void __launch_bounds__(256) sample_hist_kernel(SampleWide w) {
     pdl_launch_dependents();
     pdl_wait();
-    __shared__ u64 g[S_BINS];
+    __shared__ __align__(8) unsigned lo_hi[2 * S_BINS];
     __shared__ u64 part[256];
-    __shared__ SampleState s_st;
+    __shared__ Reached s_at;
     __shared__ float red[33];
-    const int row = blockIdx.y, chunk = blockIdx.x;
-    state_before_pass<R>(w, row, g, part, &s_st);
-    const SampleState st = s_st;
-    if (!st.nucleus) return;
-    __syncthreads();
-    // A mass is at most 2^32.  Its low 16 bits and the rest are summed in two 32-bit histograms, whose atomics the
-    // shared memory has natively (a 64-bit one is a compare-and-swap loop, slow where most of a row falls into a
-    // few digits); a chunk's 8192 elements cannot overflow either.
-    unsigned* lo = (unsigned*)g;
-    unsigned* hi = lo + S_BINS;
-    for (int i = threadIdx.x; i < 2 * S_BINS; i += blockDim.x) lo[i] = 0u;
+    __shared__ bool last;
+    unsigned* lo = lo_hi;
+    unsigned* hi = lo_hi + S_BINS;
+    const int row = blockIdx.y;
+    if (!row_has_nucleus(w.a, row)) return;
+    for (int i = threadIdx.x; i < S_BINS; i += 256) lo[i] = hi[i] = 0u;
     const float* x = w.a.logits + (size_t)row * w.a.row_stride;
-    const float mx = row_max(w, row, red), invT = 1.f / w.a.temperature[row];   // (block_max has the barriers)
-    const int beg = chunk * S_CHUNK, end = min(w.a.vocab, beg + S_CHUNK);
-    for (int i = beg + threadIdx.x; i < end; i += blockDim.x) {
-        const float l = x[i];
-        int bin;
-        if (!digit_of<R>(f2key(l), st.prefix, bin)) continue;
-        const u64 m = fixed_mass(l, mx, invT);
-        atomicAdd(&lo[bin], (unsigned)(m & 0xffffu));
-        atomicAdd(&hi[bin], (unsigned)(m >> 16));
-    }
+    float mx, mn;
+    row_range(w, row, red, mx, mn);                                 // (has the barriers that the zeros need)
+    const Steps st = row_steps(mx, mn, w.a.temperature[row]);
+    each_of_chunk(w, x, blockIdx.x, [&](float l, int) {
+        const int e = step_of(st, l);
+        if (e >= 0) add_mass(lo, hi, e, fixed_mass(l, st.mx, st.invT));
+    });
     __syncthreads();
-    u64* out = w.hist + ((size_t)row * 3 + R) * S_BINS;
-    for (int i = threadIdx.x; i < S_BINS; i += blockDim.x) {
+    u64* out = w.hist + (size_t)row * S_BINS;
+    for (int i = threadIdx.x; i < S_BINS; i += 256) {
         const u64 m = (u64)lo[i] + ((u64)hi[i] << 16);
         if (m) atomicAdd(&out[i], m);
+    }
+    // the CTA that comes last finds the threshold's step
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&w.done[row], 1) == w.n_chunks - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    u64* g = (u64*)lo_hi;
+    for (int i = threadIdx.x; i < S_BINS; i += 256) g[i] = __ldcg(&out[i]);
+    __syncthreads();
+    find_entry(g, part, &s_at, false, 0ull, w.a.top_p[row]);
+    if (threadIdx.x == 0) {
+        w.state[row].want = s_at.total - s_at.before;
+        w.state[row].edge = s_at.total > 0ull ? s_at.entry : S_BINS;
     }
 }
 
 __global__ void __launch_bounds__(256) sample_chunk_mass_kernel(SampleWide w, int nucleus) {
     pdl_launch_dependents();
     pdl_wait();
-    __shared__ u64 g[S_BINS];
-    __shared__ u64 part[256];
-    __shared__ SampleState s_st;
-    __shared__ u64 red8[8];
+    __shared__ u64 red8[16];
     __shared__ float red[33];
-    const int row = blockIdx.y, chunk = blockIdx.x;
+    const int row = blockIdx.y, chunk = blockIdx.x, lane = threadIdx.x & 31;
     const float T = w.a.temperature ? w.a.temperature[row] : 0.f;
     if (!(T > 0.f)) return;
-    unsigned thr = 0u;                                              // keep everything
-    if (nucleus) {
-        state_before_pass<3>(w, row, g, part, &s_st);
-        if (s_st.nucleus) thr = s_st.prefix;                       // after the last pass the digits are the whole key
-    }
+    const int edge = nucleus && row_has_nucleus(w.a, row) ? w.state[row].edge : S_BINS;
+    float mx, mn;
+    row_range(w, row, red, mx, mn);
+    const Steps st = row_steps(mx, mn, T);
     const float* x = w.a.logits + (size_t)row * w.a.row_stride;
-    const float mx = row_max(w, row, red), invT = 1.f / T;
-    const int beg = chunk * S_CHUNK, end = min(w.a.vocab, beg + S_CHUNK);
-    u64 m = 0ull;
-    for (int i = beg + threadIdx.x; i < end; i += blockDim.x) {
-        const float l = x[i];
-        if (f2key(l) >= thr) m += fixed_mass(l, mx, invT);
+    u64 m = 0ull, in_edge = 0ull;
+    if (edge == S_BINS) {                                           // everything is kept
+        each_of_chunk(w, x, chunk, [&](float l, int) { m += fixed_mass(l, st.mx, st.invT); });
+    } else {
+        unsigned hits = 0u;                                         // which of this thread's elements lie in the threshold's step
+        int k = 0;
+        const bool vec = each_of_chunk(w, x, chunk, [&](float l, int) {
+            const int e = step_of(st, l);
+            if (e >= 0 && e <= edge) { const u64 f = fixed_mass(l, st.mx, st.invT); if (e < edge) m += f; else in_edge += f; }
+            hits |= (unsigned)(e == edge) << k;
+            k++;
+        });
+        // their places go to the row's list, one atomic a warp
+        int before = __popc(hits);
+        for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, before, o); if (lane >= o) before += v; }
+        int base = 0;
+        if (lane == 31 && before > 0) base = atomicAdd(&w.count[row], before);
+        base = __shfl_sync(0xffffffffu, base, 31) + before - __popc(hits);
+        for (; hits; hits &= hits - 1, base++) {
+            const int u = __ffs(hits) - 1;
+            if (base < S_LIST) w.list[(size_t)row * S_LIST + base] = chunk * S_CHUNK + (vec ? ((u >> 2) * 256 + threadIdx.x) * 4 + (u & 3) : u * 256 + threadIdx.x);
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
-    if ((threadIdx.x & 31) == 0) red8[threadIdx.x >> 5] = m;
+    for (int o = 16; o > 0; o >>= 1) { m += __shfl_xor_sync(0xffffffffu, m, o); in_edge += __shfl_xor_sync(0xffffffffu, in_edge, o); }
+    if (lane == 0) { red8[threadIdx.x >> 5] = m; red8[8 + (threadIdx.x >> 5)] = in_edge; }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 2) {
         u64 t = 0ull;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) t += red8[k];
-        w.cmass[(size_t)row * w.n_chunks + chunk] = t;
+        for (int k = 0; k < 8; k++) t += red8[threadIdx.x * 8 + k];
+        (threadIdx.x ? w.emass : w.cmass)[(size_t)row * w.n_chunks + chunk] = t;
     }
 }
 
-__global__ void __launch_bounds__(256) sample_pick_kernel(SampleWide w, int nucleus) {
+// the digit of pass R of a key, and whether the key matches the digits found before it
+__device__ __forceinline__ bool digit_of(int R, unsigned key, unsigned prefix, int& bin) {
+    if (R == 0) { bin = key >> 21; return true; }
+    if (R == 1) { bin = (key >> 10) & 2047; return (key >> 21) == prefix; }
+    bin = key & 1023; return (key >> 10) == prefix;
+}
+
+__global__ void __launch_bounds__(512) sample_pick_kernel(SampleWide w, int nucleus) {
     pdl_launch_dependents();
     pdl_wait();
-    __shared__ u64 part[256];
-    __shared__ u64 cm[256];                                          // the chunks' kept masses: read side by side
+    constexpr int THREADS = 512, PER = S_CHUNK / THREADS;            // consecutive elements per thread: index order
+    __shared__ u64 g[S_BINS];
+    __shared__ u64 part[THREADS];
+    __shared__ u64 cm[256];                                          // the chunks' kept masses
+    __shared__ Reached s_at;
     __shared__ float red[33];
     __shared__ int s_chunk;
     __shared__ u64 s_base, s_target;
@@ -482,11 +541,99 @@ __global__ void __launch_bounds__(256) sample_pick_kernel(SampleWide w, int nucl
         }
         return;
     }
+    for (int c = tid; c < w.n_chunks; c += THREADS) cm[c] = w.cmass[(size_t)row * w.n_chunks + c];
+    const float* x = a.logits + (size_t)row * a.row_stride;
+    float mx, mn;
+    row_range(w, row, red, mx, mn);                                 // (has the barriers that cm needs, too)
+    const Steps st = row_steps(mx, mn, T);
+    const float invT = st.invT;
     unsigned thr = 0u;
-    // (only a row with a nucleus has left a state behind: whether it has one is taken from its own parameters)
-    if (nucleus && (a.top_p ? a.top_p[row] : 1.f) < 1.f) thr = w.state[(size_t)row * 3 + 2].prefix;
-    for (int c = tid; c < w.n_chunks; c += 256) cm[c] = w.cmass[(size_t)row * w.n_chunks + c];
-    const float mx = row_max(w, row, red);                          // (has the barriers that cm needs, too)
+    if (nucleus && row_has_nucleus(a, row)) {
+        const int edge = w.state[row].edge, n = w.count[row];
+        u64 want = w.state[row].want;
+        const bool listed = n <= S_LIST;
+        if (edge < S_BINS) {
+            unsigned prefix = 0u;
+            unsigned* lo = (unsigned*)g;
+            unsigned* hi = lo + S_BINS;
+            bool one_key = false;                                   // too many to list: most likely equal logits, whose key needs no search
+            if (!listed) {
+                float top = -INFINITY, low = INFINITY;
+                auto see = [&](float l) { if (step_of(st, l) == edge) { top = fmaxf(top, l); low = fminf(low, l); } };
+                const int quads = w.vec ? a.vocab / 4 : 0;
+#pragma unroll 8
+                for (int i = tid; i < quads; i += THREADS) {
+                    const float4 l = *(const float4*)(x + 4 * i);
+                    see(l.x); see(l.y); see(l.z); see(l.w);
+                }
+                for (int i = 4 * quads + tid; i < a.vocab; i += THREADS) see(x[i]);
+                top = block_max(top, red);
+                low = -block_max(-low, red);
+                one_key = top == low && top != 0.f;                 // (0 and -0 are two keys)
+                prefix = f2key(top);
+            }
+            for (int R = one_key ? 3 : 0; R < 3; R++) {
+                if (R == 0) prefix = 0u;
+                u64 m[S_BINS / THREADS];
+#pragma unroll
+                for (int u = 0; u < S_BINS / THREADS; u++) m[u] = 0ull;
+                const int total = listed ? n : a.vocab;
+                for (int i0 = 0; i0 < total; i0 += S_MOST_CHUNKS * S_CHUNK) {
+                    const int i1 = min(total, i0 + S_MOST_CHUNKS * S_CHUNK);
+                    __syncthreads();
+                    for (int i = tid; i < 2 * S_BINS; i += THREADS) lo[i] = 0u;
+                    __syncthreads();
+                    if (listed) {
+                        for (int k = i0 + tid; k < i1; k += THREADS) {
+                            const float l = x[w.list[(size_t)row * S_LIST + k]];
+                            int bin;
+                            if (digit_of(R, f2key(l), prefix, bin)) add_mass(lo, hi, bin, fixed_mass(l, mx, invT));
+                        }
+                    } else {
+                        for (int k = i0; k < i1; k += THREADS) {    // (whole warps: a warp whose elements share a digit adds once)
+                            const float l = k + tid < i1 ? x[k + tid] : 0.f;
+                            int bin = -1;
+                            if (k + tid >= i1 || step_of(st, l) != edge || !digit_of(R, f2key(l), prefix, bin)) bin = -1;
+                            u64 add = bin >= 0 ? fixed_mass(l, mx, invT) : 0ull;
+                            if (__all_sync(0xffffffffu, bin == __shfl_sync(0xffffffffu, bin, 0))) {
+                                for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+                                if ((tid & 31) != 0) bin = -1;
+                            }
+                            if (bin >= 0) add_mass(lo, hi, bin, add);
+                        }
+                    }
+                    __syncthreads();
+#pragma unroll
+                    for (int u = 0; u < S_BINS / THREADS; u++) m[u] += (u64)lo[tid + u * THREADS] + ((u64)hi[tid + u * THREADS] << 16);
+                }
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < S_BINS / THREADS; u++) g[tid + u * THREADS] = m[u];
+                __syncthreads();
+                find_entry(g, part, &s_at, true, want, 0.f);
+                want -= s_at.before;
+                prefix = (R == 0) ? (unsigned)s_at.entry : (R == 1) ? ((prefix << 11) | (unsigned)s_at.entry) : ((prefix << 10) | (unsigned)s_at.entry);
+            }
+            thr = prefix;
+            if (listed) {
+                for (int k = tid; k < n; k += THREADS) {
+                    const int i = w.list[(size_t)row * S_LIST + k];
+                    if (f2key(x[i]) >= thr) atomicAdd(&cm[i / S_CHUNK], fixed_mass(x[i], mx, invT));
+                }
+            } else if (one_key) {
+                for (int c = tid; c < w.n_chunks; c += THREADS) cm[c] += w.emass[(size_t)row * w.n_chunks + c];
+            } else {
+                for (int c = tid >> 5; c < w.n_chunks; c += THREADS / 32) {         // a warp a chunk
+                    u64 add = 0ull;
+                    for (int i = c * S_CHUNK + (tid & 31); i < min(a.vocab, (c + 1) * S_CHUNK); i += 32)
+                        if (step_of(st, x[i]) == edge && f2key(x[i]) >= thr) add += fixed_mass(x[i], mx, invT);
+                    for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+                    if ((tid & 31) == 0) cm[c] += add;
+                }
+            }
+            __syncthreads();
+        }
+    }
     if (tid == 0) {
         u64 kept = 0ull;
         for (int c = 0; c < w.n_chunks; c++) kept += cm[c];
@@ -499,43 +646,48 @@ __global__ void __launch_bounds__(256) sample_pick_kernel(SampleWide w, int nucl
         s_chunk = c; s_base = base; s_target = target;
     }
     __syncthreads();
-    const float* x = a.logits + (size_t)row * a.row_stride;
-    const float invT = 1.f / T;
-    constexpr int PER = S_CHUNK / 256;                              // consecutive elements per thread: index order
     const int beg = s_chunk * S_CHUNK + tid * PER, end = min(a.vocab, beg + PER);
+    __align__(16) float v[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k += 4) {
+        if (w.vec && beg + k + 4 <= end) *(float4*)(v + k) = *(const float4*)(x + beg + k);
+        else
+            for (int e = k; e < k + 4; e++) v[e] = beg + e < end ? x[beg + e] : 0.f;
+    }
     u64 mine = 0ull;
-    for (int i = beg; i < end; i++) { const float l = x[i]; if (f2key(l) >= thr) mine += fixed_mass(l, mx, invT); }
+#pragma unroll
+    for (int k = 0; k < PER; k++) if (beg + k < end && f2key(v[k]) >= thr) mine += fixed_mass(v[k], mx, invT);
     part[tid] = mine;
     __syncthreads();
     if (tid < 32) {
-        // exclusive prefix over 256 sums: a lane sums its 8, the lanes scan, each lane writes its 8 prefixes
-        u64 loc[8], sum = 0ull;
+        // exclusive prefix over the threads' sums: a lane sums its 16, the lanes scan, each lane writes its 16 prefixes
+        constexpr int LS = THREADS / 32;
+        u64 loc[LS], sum = 0ull;
 #pragma unroll
-        for (int k = 0; k < 8; k++) { loc[k] = part[tid * 8 + k]; sum += loc[k]; }
+        for (int k = 0; k < LS; k++) { loc[k] = part[tid * LS + k]; sum += loc[k]; }
         u64 incl = sum;
-        for (int o = 1; o < 32; o <<= 1) { const u64 v = __shfl_up_sync(0xffffffffu, incl, o); if (tid >= o) incl += v; }
+        for (int o = 1; o < 32; o <<= 1) { const u64 u = __shfl_up_sync(0xffffffffu, incl, o); if (tid >= o) incl += u; }
         u64 run = s_base + incl - sum;
 #pragma unroll
-        for (int k = 0; k < 8; k++) { part[tid * 8 + k] = run; run += loc[k]; }
+        for (int k = 0; k < LS; k++) { part[tid * LS + k] = run; run += loc[k]; }
     }
     __syncthreads();
     const u64 before = part[tid], target = s_target;
     if (mine > 0ull && target >= before && target < before + mine) {
         u64 run = before; int pick = beg;
-        for (int i = beg; i < end; i++) {
-            const float l = x[i];
-            if (f2key(l) >= thr) { run += fixed_mass(l, mx, invT); pick = i; if (target < run) break; }
-        }
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            if (beg + k < end && target >= run && f2key(v[k]) >= thr) { run += fixed_mass(v[k], mx, invT); pick = beg + k; }
         a.out[row] = pick;
     }
 }
 
 extern "C" long long tb_sample_wide_scratch_bytes(int rows, int vocab) {
     const long long chunks = (vocab + S_CHUNK - 1) / S_CHUNK;
-    return (long long)rows * (chunks * (4 + 4 + 8) + 3LL * S_BINS * 8 + 3LL * (long long)sizeof(SampleState)) + 256;
+    return (long long)rows * (chunks * (4 + 4 + 4 + 8 + 8) + S_BINS * 8LL + (long long)sizeof(SampleState) + (2 + S_LIST) * 4LL) + 256;
 }
 
-// `nucleus`: 0 if the caller knows that every row has top_p >= 1 (the threshold passes are then not launched).
+// `nucleus`: 0 if the caller knows that every row has top_p >= 1 (the threshold's launch is then not made).
 extern "C" int tb_sample_wide(const SampleArgs* args, int rows, void* scratch, int nucleus, cudaStream_t stream) {
     if (rows <= 0) return 0;
     SampleWide w;
@@ -546,21 +698,23 @@ extern "C" int tb_sample_wide(const SampleArgs* args, int rows, void* scratch, i
     if ((w.a.vocab + S_CHUNK - 1) / S_CHUNK > 256) return tb_refuse("sample: a vocabulary of %d is more than this kernel takes", w.a.vocab);
     if (scratch == nullptr || ((uintptr_t)scratch & 15)) return tb_refuse("sample: needs 16-byte aligned scratch");
     w.n_chunks = (w.a.vocab + S_CHUNK - 1) / S_CHUNK;
+    w.vec = ((uintptr_t)w.a.logits & 15) == 0 && w.a.row_stride % 4 == 0;
     char* p = (char*)scratch;
-    w.hist = (u64*)p; p += (size_t)rows * 3 * S_BINS * 8;
+    w.hist = (u64*)p; p += (size_t)rows * S_BINS * 8;
     w.cmass = (u64*)p; p += (size_t)rows * w.n_chunks * 8;
-    w.state = (SampleState*)p; p += (size_t)rows * 3 * sizeof(SampleState);
+    w.emass = (u64*)p; p += (size_t)rows * w.n_chunks * 8;
+    w.state = (SampleState*)p; p += (size_t)rows * sizeof(SampleState);
     w.pmax = (float*)p; p += (size_t)rows * w.n_chunks * 4;
-    w.pidx = (int*)p;
+    w.pmin = (float*)p; p += (size_t)rows * w.n_chunks * 4;
+    w.pidx = (int*)p; p += (size_t)rows * w.n_chunks * 4;
+    w.done = (int*)p; p += (size_t)rows * 4;
+    w.count = (int*)p; p += (size_t)rows * 4;
+    w.list = (int*)p;
     const dim3 per_chunk(w.n_chunks, rows);
     tb_launch(sample_chunk_max_kernel, dim3(per_chunk), dim3(256), 0, stream, w);
-    if (nucleus) {
-        tb_launch(sample_hist_kernel<0>, dim3(per_chunk), dim3(256), 0, stream, w);
-        tb_launch(sample_hist_kernel<1>, dim3(per_chunk), dim3(256), 0, stream, w);
-        tb_launch(sample_hist_kernel<2>, dim3(per_chunk), dim3(256), 0, stream, w);
-    }
+    if (nucleus) tb_launch(sample_hist_kernel, dim3(per_chunk), dim3(256), 0, stream, w);
     tb_launch(sample_chunk_mass_kernel, dim3(per_chunk), dim3(256), 0, stream, w, nucleus);
-    tb_launch(sample_pick_kernel, dim3(rows), dim3(256), 0, stream, w, nucleus);
+    tb_launch(sample_pick_kernel, dim3(rows), dim3(512), 0, stream, w, nucleus);
     return tb_launch_status();
 }
 

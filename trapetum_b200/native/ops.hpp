@@ -398,7 +398,7 @@ public:
         if (logits.cols >= WIDE_SAMPLING_FROM) {
             void* scratch = arena->alloc((size_t)nb((int)logits.rows, (int)logits.cols));
             if (dry()) return out;
-            launched(l, fw(&a, (int)logits.rows, scratch, nucleus ? 1 : 0, stream), "sample", nucleus ? 10 : 4);
+            launched(l, fw(&a, (int)logits.rows, scratch, nucleus ? 1 : 0, stream), "sample", nucleus ? 4 : 3);
             return out;
         }
         if (dry()) return out;
