@@ -272,31 +272,62 @@ __global__ void attn_mixed_decode_kernel(MixedAttnArgs a) {
     }
 }
 
-// out[b, h, :] = sum_s e^(m_s - M) o_s / (unit_sink e^(-M) + sum_s e^(m_s - M) l_s), pieces in ascending order.
-template <typename T>
-__global__ void attn_mixed_fold_kernel(MixedAttnArgs a) {
+// out[b, h, :] = sum_s e^(m_s - M) o_s / (unit_sink e^(-M) + sum_s e^(m_s - M) l_s), pieces in ascending order.  A warp a
+// (row, head), two numbers a lane and load (EVEN: D is even) and all of a piece's on their way together: 2,048 rows of 16 heads
+// in two pieces, 34 MB, in 12 us (a CTA a row and head, a load after the other: 46).
+constexpr int FOLD_WARPS = 4;
+template <typename T, bool EVEN, int NC>
+__global__ void __launch_bounds__(FOLD_WARPS * 32) attn_mixed_fold_kernel(MixedAttnArgs a) {
     pdl_launch_dependents();
     pdl_wait();
-    const int b = blockIdx.x, h = blockIdx.y, D = a.D, n = a.n_pieces;
-    const float* p = a.partial + ((size_t)b * a.H + h) * n * (D + 2);
+    constexpr int W = EVEN ? 2 : 1;                      // numbers a lane and step: columns (lane + 32 k) W and on
+    const long long item = (long long)blockIdx.x * FOLD_WARPS + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, D = a.D, n = a.n_pieces;
+    if (item >= (long long)a.n_tokens * a.H) return;
+    const int b = (int)(item / a.H), h = (int)(item % a.H);
+    const float* p = a.partial + (size_t)item * n * (D + 2);
     float M = a.unit_sink ? 0.f : -INFINITY;
     for (int s = 0; s < n; s++) M = fmaxf(M, p[(size_t)s * (D + 2) + D]);
     float L = a.unit_sink ? expf(-M) : 0.f;
+    float o[NC][W];
+#pragma unroll
+    for (int k = 0; k < NC; k++)
+#pragma unroll
+        for (int e = 0; e < W; e++) o[k][e] = 0.f;
+#pragma unroll 2
     for (int s = 0; s < n; s++) {
-        const float ms = p[(size_t)s * (D + 2) + D];
-        if (ms != -INFINITY) L += p[(size_t)s * (D + 2) + D + 1] * expf(ms - M);
+        const float* ps = p + (size_t)s * (D + 2);
+        const float ms = ps[D];
+        if (ms == -INFINITY) continue;
+        const float f = expf(ms - M);
+        L += ps[D + 1] * f;
+#pragma unroll
+        for (int k = 0; k < NC; k++) {
+            const int d = (lane + 32 * k) * W;
+            if (d >= D) continue;
+            if (EVEN) {
+                const float2 x = *(const float2*)(ps + d);
+                o[k][0] += x.x * f; o[k][W - 1] += x.y * f;
+            } else {
+                o[k][0] += ps[d] * f;
+            }
+        }
     }
     T* orow = (T*)a.out + (size_t)b * a.out_stride + (size_t)h * D;
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        float o = 0.f;
-        for (int s = 0; s < n; s++) {
-            const float ms = p[(size_t)s * (D + 2) + D];
-            if (ms != -INFINITY) o += p[(size_t)s * (D + 2) + d] * expf(ms - M);
-        }
-        orow[d] = from_f<T>(o / L);
+#pragma unroll
+    for (int k = 0; k < NC; k++) {
+        const int d = (lane + 32 * k) * W;
+#pragma unroll
+        for (int e = 0; e < W; e++) if (d + e < D) orow[d + e] = from_f<T>(o[k][e] / L);
     }
 }
-
+template <typename T>
+static void launch_fold(const MixedAttnArgs& a, cudaStream_t stream) {
+    const dim3 grid((unsigned)(((long long)a.n_tokens * a.H + FOLD_WARPS - 1) / FOLD_WARPS)), block(FOLD_WARPS * 32);
+    if (a.D % 2) tb_launch(attn_mixed_fold_kernel<T, false, 16>, grid, block, 0, stream, a);
+    else if (a.D <= 128) tb_launch(attn_mixed_fold_kernel<T, true, 2>, grid, block, 0, stream, a);
+    else tb_launch(attn_mixed_fold_kernel<T, true, 8>, grid, block, 0, stream, a);
+}
 
 // ---------------------------------------------------------------------------
 // Prompts on tensor cores (bfloat16; H <= 32 heads; D = 16 KT).  16 queries a CTA, a warp a head, 32 keys a round.
@@ -593,7 +624,7 @@ extern "C" int tb_attn_mixed_prefill(const MixedAttnArgs* args, int dtype, cudaS
 #undef TB_MP_LAUNCH
         int st = tb_launch_status();
         if (st || am.n_pieces == 1) return st;
-        TB_DISPATCH_1(dtype, T, tb_launch(attn_mixed_fold_kernel<T>, dim3(a.n_tokens, a.H), dim3(128), 0, stream, am));
+        TB_DISPATCH_1(dtype, T, launch_fold<T>(am, stream));
         return tb_launch_status();
     }
     const int nc = pick_nc(a.D);
@@ -630,6 +661,6 @@ extern "C" int tb_attn_mixed_decode(const MixedAttnArgs* args, int dtype, cudaSt
         tb_launch(attn_mixed_decode_kernel<T, NC, false>, dim3(a.n_tokens, a.n_pieces), dim3(a.H * 32), smem, stream, a)));
     int st = tb_launch_status();
     if (st || a.n_pieces == 1) return st;
-    TB_DISPATCH_1(dtype, T, tb_launch(attn_mixed_fold_kernel<T>, dim3(a.n_tokens, a.H), dim3(128), 0, stream, a));
+    TB_DISPATCH_1(dtype, T, launch_fold<T>(a, stream));
     return tb_launch_status();
 }
