@@ -156,6 +156,21 @@ def test_scores_mixed_across_heads_in_a_long_prompt_whose_keys_are_cut_into_piec
     near(got.view(T, H, D), want, dtype, "mixed attention, a long prompt in pieces", rel16=1.5e-2)
 
 
+@pytest.mark.parametrize("n", [1, 15, 17, 33, 500])
+@pytest.mark.parametrize("H, G, D, seen", [(8, 1, 32, 0), (8, 8, 128, -70), (16, 2, 64, 40), (16, 4, 128, -300), (16, 8, 128, 0), (16, 16, 96, -33)])
+def test_scores_mixed_two_pairs_a_thread(H, G, D, seen, n):
+    """8 and 16 heads: with two stages of keys and values (G small), with one, and (16 kv heads of 96) as the other head counts go."""
+    from trapetum_b200.csrc import ops
+    dtype = "bfloat16"
+    g = torch.Generator().manual_seed(H + D + n)
+    q, k, v = (rounded(torch.randn(n, heads, D, generator=g), dtype) for heads in (H, G, G))
+    mix = (torch.eye(H) + 0.4 * torch.randn(H, H, generator=g)).float() * 0.2        # not symmetric: a transposed matrix shows
+    want = _mixed_reference(q, k, v, mix.double(), H, G, seen, True)
+    got = ops.attn_mixed_prefill(dev(q.reshape(n, -1), DTYPES[dtype]), dev(k.reshape(n, -1), DTYPES[dtype]), dev(v.reshape(n, -1), DTYPES[dtype]),
+                                 i32([0, n]), i32([0] * n), H, G, D, dev(mix), seen, True, n)
+    near(got.view(n, H, D), want, dtype, "mixed attention, pairs", rel16=1.5e-2)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H, G, D, seen, ring, sink", [(3, 3, 8, -5, 64, True), (6, 3, 24, -33, 0, True), (4, 2, 64, -64, 64, False),
                                                        (2, 1, 40, 0, 0, True), (5, 1, 16, 70, 128, False), (4, 4, 16, -100, 128, True)])

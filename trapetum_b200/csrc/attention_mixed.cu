@@ -362,8 +362,19 @@ __host__ inline size_t mp_smem(int H, int G, int D, int stages) {
     return (size_t)((H * H + 3) & ~3) * 4 + (size_t)H * MP_BM * MP_RP * 4 + (size_t)stages * (G + mp_value_heads(H, G)) * MP_BN * (D + 8) * 2;
 }
 
+// PAIRS, 8 or 16 heads: a thread mixes two (query, key) pairs for eight heads at once, so that a raw score is read by one or
+// two warps and not by every head's; the mixed scores go back through a buffer of their own.  Shared memory's pipe is what
+// bounds a round: by its addresses a round of 16 heads moves 4,600 rows of 128 bytes for the exchange with a warp a head
+// mixing and 1,800 with pairs.  A score's terms are added in the same order (same results).  One prompt of 2,048 tokens, 16 heads
+// over 4 of 128, blocks of 1,024: 190 -> 174 us with the fold.
+// Rows of 32 scores, eight-column groups exchanged by the query's low bits: no two of a half warp's 8-byte accesses meet.
+__host__ inline size_t mp_smem_pairs(int H, int G, int D, int stages) {
+    return (size_t)H * H * 4 + (size_t)2 * H * MP_BM * MP_BN * 4 + (size_t)stages * 2 * G * MP_BN * (D + 8) * 2;
+}
+__device__ __forceinline__ int mp_pair_at(int g, int i, int j) { return (g * MP_BM + i) * MP_BN + (j ^ ((i & 3) * 8)); }
+
 // MULTI: more than 16 heads (the second paragraph above); else a warp's only raw scores are its own head's.
-template <int KT, bool MULTI>
+template <int KT, bool MULTI, bool PAIRS>
 __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnArgs a) {
     pdl_launch_dependents();
     constexpr int D = 16 * KT, PITCH = D + 8;
@@ -371,7 +382,8 @@ __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnAr
     const int H = a.H, G = a.G, GV = mp_value_heads(H, G);
     float* mix_s = (float*)sm;                                        // [H][H]
     float* raw = mix_s + ((H * H + 3) & ~3);                          // [H][16][MP_RP]
-    bf16* tiles = (bf16*)(raw + H * MP_BM * MP_RP);                   // [stages][K: G | V: GV][32][PITCH]
+    float* mixed = raw + H * MP_BM * MP_BN;                           // PAIRS: as many mixed scores
+    bf16* tiles = (bf16*)(PAIRS ? mixed + H * MP_BM * MP_BN : raw + H * MP_BM * MP_RP);                   // [stages][K: G | V: GV][32][PITCH]
     const size_t k_part = (size_t)G * MP_BN * PITCH, stage = k_part + (size_t)GV * MP_BN * PITCH;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h_raw = warp < H ? warp : 0;
@@ -382,7 +394,7 @@ __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnAr
     const int per_kv = H / G;
     const int kv_lo = (blockIdx.z * 16) / per_kv;                     // the first kv head whose values this CTA needs
     const int kvh = h / per_kv;
-    for (int e = threadIdx.x; e < H * H; e += blockDim.x) mix_s[e] = a.mix[e];
+    for (int e = threadIdx.x; e < H * H; e += blockDim.x) mix_s[e] = a.mix[PAIRS ? e % H * H + e / H : e];     // PAIRS: [raw head][mixed head]
     pdl_wait();
     const int b = blockIdx.y;
     const int s0 = a.seq_start[b], len = a.seq_start[b + 1] - s0;
@@ -467,14 +479,39 @@ __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnAr
             }
 #pragma unroll
             for (int nt = 0; nt < 4; nt++) {
-                float* ra = raw + ((size_t)hr * MP_BM + r) * MP_RP + nt * 8 + c;
+                float* ra = raw + (PAIRS ? mp_pair_at(hr, r, nt * 8 + c) : (hr * MP_BM + r) * MP_RP + nt * 8 + c);
                 *(float2*)ra = make_float2(sc[nt][0], sc[nt][1]);
-                *(float2*)(ra + 8 * MP_RP) = make_float2(sc[nt][2], sc[nt][3]);
+                *(float2*)(ra + 8 * (PAIRS ? MP_BN : MP_RP)) = make_float2(sc[nt][2], sc[nt][3]);
             }
         }
         __syncthreads();
         if (MULTI && !has_out) continue;                               // a warp without a head of its own only made raw scores
         // ---- this head's mixed scores, 32-bit
+        if constexpr (PAIRS) {
+            const int h8 = warp >> 3 << 3;                             // the eight heads; the pairs are of queries 2 (warp % 8) and the next
+            const int at = mp_pair_at(0, (warp & 7) * 2 + (lane >> 4), (lane & 15) * 2);
+            float2 acc[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) acc[e] = make_float2(0.f, 0.f);
+#pragma unroll 4
+            for (int g = 0; g < H; g++) {
+                const float2 x = *(const float2*)(raw + at + g * (MP_BM * MP_BN));
+                float w[8];
+                *(float4*)w = *(const float4*)(mix_s + g * H + h8);
+                *(float4*)(w + 4) = *(const float4*)(mix_s + g * H + h8 + 4);
+#pragma unroll
+                for (int e = 0; e < 8; e++) { acc[e].x = fmaf(w[e], x.x, acc[e].x); acc[e].y = fmaf(w[e], x.y, acc[e].y); }
+            }
+#pragma unroll
+            for (int e = 0; e < 8; e++) *(float2*)(mixed + at + (h8 + e) * (MP_BM * MP_BN)) = acc[e];
+            __syncthreads();
+#pragma unroll
+            for (int nt = 0; nt < 4; nt++) {
+                const float* ma = mixed + mp_pair_at(h, r, nt * 8 + c);
+                const float2 x = *(const float2*)ma, y = *(const float2*)(ma + 8 * MP_BN);
+                sc[nt][0] = x.x; sc[nt][1] = x.y; sc[nt][2] = y.x; sc[nt][3] = y.y;
+            }
+        } else {
 #pragma unroll
         for (int nt = 0; nt < 4; nt++) { sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f; }
         for (int g = 0; g < H; g++) {
@@ -486,6 +523,7 @@ __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnAr
                 sc[nt][0] = fmaf(w, x.x, sc[nt][0]); sc[nt][1] = fmaf(w, x.y, sc[nt][1]);
                 sc[nt][2] = fmaf(w, y.x, sc[nt][2]); sc[nt][3] = fmaf(w, y.y, sc[nt][3]);
             }
+        }
         }
         // ---- who sees whom, and the running softmax of the two rows
         float mx_a = -INFINITY, mx_b = -INFINITY;
@@ -611,17 +649,21 @@ extern "C" int tb_attn_mixed_prefill(const MixedAttnArgs* args, int dtype, cudaS
     if (a.batch > 0 && a.max_seq_len > 0 && aligned && tb_attn_mixed_prefill_mma_takes(dtype, a.H, a.G, a.D)) {
         MixedAttnArgs am = a;
         am.stages = mp_smem(a.H, a.G, a.D, 2) <= 200 * 1024 ? 2 : 1;
-        const size_t sm = mp_smem(a.H, a.G, a.D, am.stages);
+        // pairs wherever they fit beside as many stages as without them (16 heads: 174 against 190 us, see the kernel; 8 heads,
+        // not timed apart, share the kernel)
+        const bool pairs = (a.H == 8 || a.H == 16) && mp_smem_pairs(a.H, a.G, a.D, am.stages) <= 220 * 1024;
+        const size_t sm = pairs ? mp_smem_pairs(a.H, a.G, a.D, am.stages) : mp_smem(a.H, a.G, a.D, am.stages);
         if (am.n_pieces > 1 && a.partial == nullptr) return tb_refuse("attn_mixed: pieces need scratch");
         if (am.n_pieces < 1) am.n_pieces = 1;
         dim3 grid((a.max_seq_len + MP_BM - 1) / MP_BM * am.n_pieces, a.batch, (a.H + 15) / 16);
         const int warps = a.H < 16 ? a.H : 16;
-#define TB_MP_LAUNCH(KT) do { if (a.H > 16) { allow_smem(attn_mixed_prefill_mma_kernel<KT, true>, sm); \
-            tb_launch(attn_mixed_prefill_mma_kernel<KT, true>, grid, dim3(warps * 32), sm, stream, am); } \
-        else { allow_smem(attn_mixed_prefill_mma_kernel<KT, false>, sm); \
-            tb_launch(attn_mixed_prefill_mma_kernel<KT, false>, grid, dim3(warps * 32), sm, stream, am); } } while (0)
+#define TB_MP_LAUNCH_AS(KT, MULTI, PAIRS) do { allow_smem(attn_mixed_prefill_mma_kernel<KT, MULTI, PAIRS>, sm); \
+            tb_launch(attn_mixed_prefill_mma_kernel<KT, MULTI, PAIRS>, grid, dim3(warps * 32), sm, stream, am); } while (0)
+#define TB_MP_LAUNCH(KT) do { if (a.H > 16) TB_MP_LAUNCH_AS(KT, true, false); \
+        else if (pairs) TB_MP_LAUNCH_AS(KT, false, true); else TB_MP_LAUNCH_AS(KT, false, false); } while (0)
         switch (a.D / 16) { case 2: TB_MP_LAUNCH(2); break; case 4: TB_MP_LAUNCH(4); break; case 6: TB_MP_LAUNCH(6); break; default: TB_MP_LAUNCH(8); break; }
 #undef TB_MP_LAUNCH
+#undef TB_MP_LAUNCH_AS
         int st = tb_launch_status();
         if (st || am.n_pieces == 1) return st;
         TB_DISPATCH_1(dtype, T, launch_fold<T>(am, stream));
