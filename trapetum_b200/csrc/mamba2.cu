@@ -102,8 +102,8 @@ __global__ void __launch_bounds__(128, 6) mamba2_conv4_kernel(Mamba2Args a) {
         w[e][0] = x.x; w[e][1] = x.y; w[e][2] = x.z; w[e][3] = x.w;
         bias[e] = ((const float*)a.conv_b)[c + e];
     }
-    int b = a.token_seq[t0], i = t0 - a.seq_start[b];     // (a step's integers are there before its first kernel)
     pdl_wait();
+    int b = a.token_seq[t0], i = t0 - a.seq_start[b];
     const bf16* in = (const bf16*)a.proj + inner + c;
     uint2 rows[CONV_TOK + 3];                        // tokens t0 - 3 .. t0 + 7 (earlier ones only of the same sequence)
 #pragma unroll
