@@ -173,6 +173,54 @@ def test_mamba2_prompts_as_products(ops, heads, P, N, groups, lens, span):
     assert torch.isfinite(got[1][0]).all()
 
 
+@pytest.mark.parametrize("bad", [math.nan, math.inf, -math.inf])
+@pytest.mark.parametrize("at", [0, 17, 127, 128, 200])
+def test_mamba2_prompts_stay_causal(ops, bad, at):
+    """A number that is not finite in one token's x of one channel: the tokens before it give what they give without it,
+    and a NaN shows wherever the recurrence shows it."""
+    heads, P, N, groups, lens = 2, 64, 64, 1, [230, 40]
+    T, B, inner, ch = sum(lens), len(lens), heads * P, heads * P + 2 * groups * N
+    proj, dt = rnd(T, inner + ch, dt=torch.bfloat16), rnd(T, heads, seed=1)
+    small = [rnd(ch, 4, s=0.3, seed=2), rnd(ch, s=0.1, seed=3), rnd(heads, seed=4) - 2, rnd(heads, s=0.5, seed=5), rnd(heads, seed=6)]
+    norm = rnd(inner, s=0.1, seed=7) + 1
+    first = rnd(B, ops.mamba2_state_size(heads, P, N, groups, 4), seed=8)
+    starts, slots = torch.tensor([0, lens[0], T], dtype=torch.int32, device="cuda"), torch.arange(B, dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).to("cuda", torch.int32)
+
+    def run(rows, longest):
+        state = first.clone()
+        return ops.mamba2(rows, dt, heads, P, N, groups, 4, 1, *small, norm, 1e-6, state, starts, seq, slots, B, False, longest)
+    clean, spoilt = run(proj, max(lens)), proj.clone()
+    spoilt[at, inner + 5] = bad
+    got, scan = run(spoilt, max(lens)), run(spoilt, 0)
+    assert torch.equal(got[:at], clean[:at]) and torch.equal(got[lens[0]:], clean[lens[0]:])
+    if math.isnan(bad):
+        assert torch.equal(got.isnan(), scan.isnan())
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf, -math.inf])
+@pytest.mark.parametrize("at", [0, 13, 16, 150])
+def test_gla_prompts_stay_causal(ops, bad, at):
+    """The same of gated linear attention, a value that is not finite."""
+    heads, D, V, rank, lens = 2, 64, 128, 16, [170, 30]
+    T, B = sum(lens), len(lens)
+    proj, low = rnd(T, 2 * heads * (D + V), dt=torch.bfloat16), rnd(1, T, rank, seed=1)
+    a2, bias, norm = rnd(heads * D, rank, s=0.3, seed=2), rnd(heads * D, seed=3) + 2, rnd(V, s=0.1, seed=4) + 1
+    first = rnd(B, heads * D * V, seed=5)
+    starts, slots = torch.tensor([0, lens[0], T], dtype=torch.int32, device="cuda"), torch.arange(B, dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).to("cuda", torch.int32)
+
+    def run(rows, longest):
+        state = first.clone()
+        return ops.gla(rows, low, a2, bias, 8.0, D ** -0.5, norm, 1e-6, heads, D, V, state, starts, seq, slots, B, longest)
+    clean, spoilt = run(proj, max(lens)), proj.clone()
+    spoilt[at, 2 * heads * D + V + 9] = bad
+    got, scan = run(spoilt, max(lens)), run(spoilt, 0)
+    assert torch.equal(got[:at], clean[:at]) and torch.equal(got[lens[0]:], clean[lens[0]:])
+    if math.isnan(bad):
+        assert torch.equal(got.isnan(), scan.isnan())
+
+
 @pytest.mark.parametrize("heads,D,V,lens,span", [(8, 128, 256, [700, 15], 1.0), (2, 72, 128, [16, 33, 1], 0.01), (3, 64, 128, [32], 30.0),
                                                  (1, 8, 144, [300, 257], 1.0), (2, 128, 256, [65], 1e3)])
 def test_gla_prompts_in_blocks(ops, monkeypatch, heads, D, V, lens, span):

@@ -282,7 +282,8 @@ __global__ void gla_fold_kernel(GlaArgs a) {
 // only the order of the 32-bit sums differs from the recurrence's.  The sums c are made in 64 bits and kept as two 32-bit
 // numbers.  Long prompts: a first launch (OUT false) leaves the sums of every chunk but a sequence's last, gla_block_fold_kernel
 // turns them into start states, the second launch (OUT true) writes the outputs, normed and gated: the CTA holds the head.
-// A non-finite v reaches the tokens of its block before it too (0 times it).
+// A non-finite v is seen by its own token and later ones only, as in the recurrence; what it leaves in the state is NaN to the
+// next block's outputs (an infinity has no three parts).
 // Prompts of 1,500 and 548 tokens, 8 heads of 128 x 256, all of ops.gla: 130 us (the recurrence in chunks, its norm a launch
 // of its own: 388; there the chunks of the shorter prompt leave SMs idle too).  A block takes 9.6 us of its CTA: shared
 // memory (14 of 18 thousand cycles), then issue slots; the products are a quarter of the tensor pipe.
@@ -323,6 +324,8 @@ __device__ __forceinline__ void split3(float x, bf16* hi, int step) {      // to
         x -= __bfloat162float(h);
     }
 }
+// A sign bit of the result is set where one of two bfloat16 numbers is infinite or NaN.
+__device__ __forceinline__ uint32_t not_finite(uint32_t v) { return (v & 0x7f807f80u) + 0x00800080u; }
 __device__ __forceinline__ float exp2_fast(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 
 // Shared memory of a CTA, in bytes from its start.
@@ -579,12 +582,30 @@ __global__ void __launch_bounds__(512, 1) gla_block_kernel(GlaArgs a) {
             for (int u2 = 0; u2 < NU; u2++) put(u2);
         }
         if (OUT) {
+            if (__any_sync(0xffffffffu, ((not_finite(vt[0]) | not_finite(vt[1]) | not_finite(vt[2]) | not_finite(vt[3])) & 0x80008000u) != 0)) {
+                // a weight of 0 times such a value of a later token would be NaN: token by token, up to the output's own
+#pragma unroll 1
+                for (int j = 0; j < GB; j++) {
+                    const int from = (lane & ~3) | ((j & 7) >> 1);
+                    const uint32_t a0 = __shfl_sync(0xffffffffu, j < 8 ? vt[0] : vt[2], from), a1 = __shfl_sync(0xffffffffu, j < 8 ? vt[1] : vt[3], from);
+                    const float vj[2] = {__uint_as_float((j & 1) ? a0 & 0xffff0000u : a0 << 16), __uint_as_float((j & 1) ? a1 & 0xffff0000u : a1 << 16)};
+#pragma unroll
+                    for (int x = 0; x < 2; x++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int i = x * 8 + 2 * t + (e & 1);
+                            const bf16* p = (const bf16*)(sm + L::p3 + i * 48) + j;
+                            if (j <= i) o[x][e] = fmaf(__bfloat162float(p[0]) + (__bfloat162float(p[GB * 24]) + __bfloat162float(p[2 * GB * 24])), vj[e >> 1], o[x][e]);
+                        }
+                }
+            } else {
 #pragma unroll
             for (int k = 2; k >= 0; k--) {
                 uint32_t f[4];
                 ldsm_x4(smem_addr(sm + L::p3 + k * GB * 48 + ((lane >> 4) * 8 + (lane & 7)) * 48 + ((lane >> 3) & 1) * 16), f);
                 mma_bf16(o[0], vt, f[0], f[1]);
                 mma_bf16(o[1], vt, f[2], f[3]);
+            }
             }
 #pragma unroll
             for (int x = 0; x < 2; x++)

@@ -425,7 +425,8 @@ __global__ void __launch_bounds__(SCAN_NS * PT / SCAN_PP) mamba2_scan_kernel(Mam
 // outputs.  x, B and C are bfloat16 numbers; what meets them (the weighted scores, the weighted x, the state) is 32-bit and
 // enters as the sum of three bfloat16 numbers, 24 bits, so every product is that of the recurrence and only the order of the
 // 32-bit sums differs.  The running sums are kept as two 32-bit numbers (c_i - c_j of near tokens keeps its digits); a
-// decay below 2^-300 is 0 in any product.  A non-finite x reaches the up to 15 tokens before it too (0 times it).
+// decay below 2^-300 is 0 in any product.  A non-finite x is seen by its own token and later ones only, as in the recurrence;
+// what it leaves in the state is NaN to the next chunk's outputs (an infinity has no three parts).
 // 2,048 tokens, 64 heads of 64 x 128: 31 + 20 + 56 us cold (the recurrence in chunks: 167 + 235); the tensor pipe and the
 // three-way splits share the time of the third launch.  All of ops.mamba2: 486 -> 129 us.
 // ---------------------------------------------------------------------------------------------------------
@@ -457,6 +458,13 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
     lo = pack2(x - __uint_as_float(mid << 16), y - __uint_as_float(mid & 0xffff0000u));
 }
 __device__ __forceinline__ float exp2_fast(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+// A sign bit of the result is set where one of two bfloat16 numbers is infinite or NaN.
+__device__ __forceinline__ uint32_t not_finite(uint32_t v) { return (v & 0x7f807f80u) + 0x00800080u; }
+// What two numbers' three parts add up to: the number in the low halves, in the high halves.
+__device__ __forceinline__ float low3(const uint32_t* p) { return __uint_as_float(p[0] << 16) + (__uint_as_float(p[1] << 16) + __uint_as_float(p[2] << 16)); }
+__device__ __forceinline__ float high3(const uint32_t* p) {
+    return __uint_as_float(p[0] & 0xffff0000u) + (__uint_as_float(p[1] & 0xffff0000u) + __uint_as_float(p[2] & 0xffff0000u));
+}
 
 struct ChunkPlace { int t0, n, c, b, slot; };         // first token, tokens, index in its sequence, sequence, scratch slot
 // A sequence's chunks lie from slot floor(seq_start / 128) + b on, which leaves every sequence enough of them.
@@ -673,6 +681,17 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
             for (int j = 0; j < 8; j++) { o[j][0] *= fa; o[j][1] *= fa; o[j][2] *= fb; o[j][3] *= fb; }
         }
         // ---- the chunk's own tokens, 16 keys at a time up to this warp's last row
+        bool odd = false;                             // an x of this warp's own 16 tokens is not finite
+        {
+            uint32_t any = 0;
+#pragma unroll
+            for (int u = 0; u < MP * 2 / 32; u++) {
+                const uint4 x = *(const uint4*)(sx + (warp * 16 + (lane >> 1)) * MXPITCH + (lane & 1) * MP + u * 16);
+                any |= not_finite(x.x) | not_finite(x.y) | not_finite(x.z) | not_finite(x.w);
+            }
+            odd = __any_sync(0xffffffffu, (any & 0x80008000u) != 0);
+        }
+        uint32_t hi[4], mid[4], lo[4];
         for (int kk = 0; kk <= warp; kk++) {
             float s[2][4];
 #pragma unroll
@@ -684,7 +703,6 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
                 mma_bf16(s[0], q[ks], f[0], f[1]);
                 mma_bf16(s[1], q[ks], f[2], f[3]);
             }
-            uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
             for (int n = 0; n < 2; n++) {
                 const int j = kk * 16 + n * 8 + 2 * t;
@@ -697,6 +715,7 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
                 split3(x0, x1, hi[n * 2], mid[n * 2], lo[n * 2]);
                 split3(x2, x3, hi[n * 2 + 1], mid[n * 2 + 1], lo[n * 2 + 1]);
             }
+            if (odd && kk == warp) break;
 #pragma unroll
             for (int j = 0; j < 8; j += 2) {
                 uint32_t f[4];
@@ -704,6 +723,26 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
                 mma_bf16(o[j], lo, f[0], f[1]); mma_bf16(o[j + 1], lo, f[2], f[3]);
                 mma_bf16(o[j], mid, f[0], f[1]); mma_bf16(o[j + 1], mid, f[2], f[3]);
                 mma_bf16(o[j], hi, f[0], f[1]); mma_bf16(o[j + 1], hi, f[2], f[3]);
+            }
+        }
+        if (odd) {                                    // (0 times a later token's x would be NaN: token by token, up to the row's own)
+            for (int r = 0; r < 16; r++) {
+                const int from = (lane & ~3) | ((r & 7) >> 1);
+                uint32_t wa[3], wb[3];                // the weight of token r in rows ra and rb
+#pragma unroll
+                for (int e = 0; e < 3; e++) {
+                    const uint32_t* part = e == 0 ? hi : e == 1 ? mid : lo;
+                    wa[e] = __shfl_sync(0xffffffffu, r < 8 ? part[0] : part[2], from);
+                    wb[e] = __shfl_sync(0xffffffffu, r < 8 ? part[1] : part[3], from);
+                }
+                const float fa = (r & 1) ? high3(wa) : low3(wa), fb = (r & 1) ? high3(wb) : low3(wb);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const uint32_t x = *(const uint32_t*)(sx + (warp * 16 + r) * MXPITCH + (j * 8 + 2 * t) * 2);
+                    const float xa = __uint_as_float(x << 16), xb = __uint_as_float(x & 0xffff0000u);
+                    if (r <= g) { o[j][0] = fmaf(fa, xa, o[j][0]); o[j][1] = fmaf(fa, xb, o[j][1]); }
+                    if (r <= g + 8) { o[j][2] = fmaf(fb, xa, o[j][2]); o[j][3] = fmaf(fb, xb, o[j][3]); }
+                }
             }
         }
         const float Dh = ((const float*)a.D)[h];
