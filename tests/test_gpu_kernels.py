@@ -269,6 +269,57 @@ def test_latent_decode_pieces(ops, B, heads, C, R, longest, window):
     assert ops.kernel_errors() == {}
 
 
+def state_error(state, want):
+    return float((state.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("n,B,heads,N,log_a", [(100, 1, 4, 128, 0.0), (300, 2, 3, 64, 0.0), (2048, 1, 2, 128, -2.0), (1000, 2, 2, 128, -8.0)])
+def test_mamba2_products_lose_nothing_in_the_state(ops, n, B, heads, N, log_a):
+    """The 32-bit state against 64 bits: as near as the recurrence leaves it (a fifth more: both are sums of the same
+    roundings in another order), also where decays are close to 1 and all terms have one sign, so that sums which are cut
+    off would show.  The convolution copies numbers of 32 to 64, which silu leaves as they are."""
+    P, T, inner, ch = 64, n * B, heads * 64, heads * 64 + 2 * N
+    g = torch.Generator(device="cuda").manual_seed(n + N)
+    proj, dt = (torch.rand(T, inner + ch, device="cuda", generator=g) * 31 + 32).bfloat16(), rnd(T, heads, seed=1)
+    taps = torch.tensor([0.0, 0.0, 0.0, 1.0], device="cuda").repeat(ch, 1)
+    small = [taps, torch.zeros(ch, device="cuda"), rnd(heads, seed=4) - 2, rnd(heads, s=0.5, seed=5) + log_a, rnd(heads, seed=6)]
+    starts, slots = torch.arange(0, T + 1, n, dtype=torch.int32, device="cuda"), torch.arange(B, dtype=torch.int32, device="cuda")
+    seq = torch.arange(B, device="cuda").repeat_interleave(n).to(torch.int32)
+    x, Bm = (t.double().view(B, n, -1) for t in (proj[:, inner:2 * inner], proj[:, 2 * inner:2 * inner + N]))
+    step = torch.nn.functional.softplus(dt.double() + small[2].double()).view(B, n, heads)
+    decay = torch.exp(-torch.exp(small[3].double()) * step)
+    S = torch.zeros(B, heads, P, N, dtype=torch.float64, device="cuda")
+    for t in range(n):
+        S = decay[:, t, :, None, None] * S + (step[:, t, :, None] * x[:, t].view(B, heads, P))[..., None] * Bm[:, t, None, None]
+    err = []
+    for longest in (0, n):
+        state = torch.zeros(B, ops.mamba2_state_size(heads, P, N, 1, 4), device="cuda")
+        ops.mamba2(proj, dt, heads, P, N, 1, 4, 1, *small, torch.ones(inner, device="cuda"), 1e-6, state, starts, seq, slots, B, False, longest)
+        err.append(state_error(state[:, :heads * P * N].view(B, heads, P, N), S))
+    assert err[1] <= 1.2 * err[0], err
+
+
+@pytest.mark.parametrize("n,B,heads,bias", [(100, 1, 4, 0.0), (100, 2, 4, 2.0), (2048, 1, 4, 0.0), (2048, 1, 4, 6.0), (2048, 16, 10, 10.0)])
+def test_gla_blocks_lose_nothing_in_the_state(ops, n, B, heads, bias):
+    """The same of gated linear attention, prompts in several chunks and (16 of them) in one.  ``bias`` 10: decays of 0.99999."""
+    D, V, rank, T = 64, 128, 16, n * B
+    proj, low = rnd(T, 2 * heads * (D + V), dt=torch.bfloat16).abs(), rnd(1, T, rank, seed=1)
+    a2, b2 = rnd(heads * D, rank, s=0.3, seed=2), rnd(heads * D, seed=3) + bias
+    starts, slots = torch.arange(0, T + 1, n, dtype=torch.int32, device="cuda"), torch.arange(B, dtype=torch.int32, device="cuda")
+    seq = torch.arange(B, device="cuda").repeat_interleave(n).to(torch.int32)
+    k, v = (t.double().reshape(B, n, heads, -1) for t in (proj[:, heads * D:2 * heads * D], proj[:, 2 * heads * D:2 * heads * D + heads * V]))
+    decay = torch.exp(torch.nn.functional.logsigmoid(low[0].double() @ a2.double().T + b2.double()) / 8.0).view(B, n, heads, D)
+    S = torch.zeros(B, heads, D, V, dtype=torch.float64, device="cuda")
+    for t in range(n):
+        S = decay[:, t, :, :, None] * S + k[:, t, :, :, None] * v[:, t, :, None, :]
+    err = []
+    for longest in (0, n):
+        state = torch.zeros(B, heads * D * V, device="cuda")
+        ops.gla(proj, low, a2, b2, 8.0, D ** -0.5, torch.ones(V, device="cuda"), 1e-6, heads, D, V, state, starts, seq, slots, B, longest)
+        err.append(state_error(state.view(B, heads, D, V), S))
+    assert err[1] <= 1.2 * err[0], err
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 17, 60), (9, 16, 2048), (16, 1100, 4100), (17, 63, 256), (65, 65, 2052), (70, 130, 8196)])
 def test_gemm_simt_rows_and_tiles(ops, M, N, K):
     """32-bit operands in whole 16-byte pieces: rows that are not full, tails of a k-tile, stage and segment; a row is

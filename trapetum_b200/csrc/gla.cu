@@ -561,18 +561,22 @@ __global__ void __launch_bounds__(512, 1) gla_block_kernel(GlaArgs a) {
             const float* full = (const float*)(sm + L::full);
 #pragma unroll
             for (int ks = 0; ks < KS; ks++) {
+                float u[2][4];                        // (a product's sums are cut off, not rounded: the state is not added to in them)
 #pragma unroll
-                for (int x = 0; x < 2; x++) {
-                    const float2 w = *(const float2*)(full + ks * 16 + x * 8 + 2 * t);
-                    float* s = S[2 * ks + x];
-                    s[0] *= w.x; s[1] *= w.y; s[2] *= w.x; s[3] *= w.y;
-                }
+                for (int e = 0; e < 4; e++) u[0][e] = u[1][e] = 0.f;
 #pragma unroll
                 for (int k = 2; k >= 0; k--) {
                     uint32_t f[4];
                     ldsm_x4_t(smem_addr(sm + L::k3 + k * GB * RP + (((lane >> 3) & 1) * 8 + (lane & 7)) * RP + (ks * 16 + (lane >> 4) * 8) * 2), f);
-                    mma_bf16(S[2 * ks], vt, f[0], f[1]);
-                    mma_bf16(S[2 * ks + 1], vt, f[2], f[3]);
+                    mma_bf16(u[0], vt, f[0], f[1]);
+                    mma_bf16(u[1], vt, f[2], f[3]);
+                }
+#pragma unroll
+                for (int x = 0; x < 2; x++) {
+                    const float2 w = *(const float2*)(full + ks * 16 + x * 8 + 2 * t);
+                    float* s = S[2 * ks + x];
+                    s[0] = fmaf(s[0], w.x, u[x][0]); s[1] = fmaf(s[1], w.y, u[x][1]);
+                    s[2] = fmaf(s[2], w.x, u[x][2]); s[3] = fmaf(s[3], w.y, u[x][3]);
                 }
             }
         }

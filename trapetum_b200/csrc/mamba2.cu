@@ -450,6 +450,11 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// A product's sums are cut off, not rounded, so what comes of 16 terms is added up outside of the products.
+__device__ __forceinline__ void set0(float (*u)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) u[0][e] = u[1][e] = 0.f;
+}
 // Two 32-bit numbers as sums of three bfloat16 numbers each: the remainders are exact, the last one holds what is left.
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     hi = pack2(x, y);
@@ -561,9 +566,13 @@ __global__ void __launch_bounds__(MCT) mamba2_chunk_sum_kernel(Mamba2Args a) {
         for (int j = 0; j < NT; j += 2) {
             uint32_t f[4];
             ldsm_x4_t(smem_addr(sB + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * BPITCH + (n0 + j * 8 + (lane >> 4) * 8) * 2), f);
-            mma_bf16(acc[j], lo, f[0], f[1]); mma_bf16(acc[j + 1], lo, f[2], f[3]);
-            mma_bf16(acc[j], mid, f[0], f[1]); mma_bf16(acc[j + 1], mid, f[2], f[3]);
-            mma_bf16(acc[j], hi, f[0], f[1]); mma_bf16(acc[j + 1], hi, f[2], f[3]);
+            float u[2][4];
+            set0(u);
+            mma_bf16(u[0], lo, f[0], f[1]); mma_bf16(u[1], lo, f[2], f[3]);
+            mma_bf16(u[0], mid, f[0], f[1]); mma_bf16(u[1], mid, f[2], f[3]);
+            mma_bf16(u[0], hi, f[0], f[1]); mma_bf16(u[1], hi, f[2], f[3]);
+#pragma unroll
+            for (int e = 0; e < 4; e++) { acc[j][e] += u[0][e]; acc[j + 1][e] += u[1][e]; }
         }
     }
     float* E = a.chunk_state + (size_t)pl.slot * a.heads * P * N + (size_t)h * P * N;
@@ -663,16 +672,21 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
     for (int j = 0; j < 8; j++) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
     if (warp * 16 < pl.n) {                           // (rows past the end: nothing to write)
 #pragma unroll
-        for (int k = 2; k >= 0; k--)
+        for (int j = 0; j < 8; j += 2)
 #pragma unroll
-            for (int ks = 0; ks < KS; ks++)
+            for (int ks = 0; ks < KS; ks++) {
+                float u[2][4];
+                set0(u);
 #pragma unroll
-                for (int j = 0; j < 8; j += 2) {
+                for (int k = 2; k >= 0; k--) {
                     uint32_t f[4];
                     ldsm_x4(smem_addr(sS + (k * MP + j * 8 + (lane >> 4) * 8 + (lane & 7)) * BPITCH + (ks * 16 + ((lane >> 3) & 1) * 8) * 2), f);
-                    mma_bf16(o[j], q[ks], f[0], f[1]);
-                    mma_bf16(o[j + 1], q[ks], f[2], f[3]);
+                    mma_bf16(u[0], q[ks], f[0], f[1]);
+                    mma_bf16(u[1], q[ks], f[2], f[3]);
                 }
+#pragma unroll
+                for (int e = 0; e < 4; e++) { o[j][e] += u[0][e]; o[j + 1][e] += u[1][e]; }
+            }
         const int ra = warp * 16 + g, rb = ra + 8;
         const float2 ca = scum[ra], cb = scum[rb];
         {
@@ -699,9 +713,13 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
 #pragma unroll
             for (int ks = 0; ks < KS; ks++) {
                 uint32_t f[4];
+                float u[2][4];
                 ldsm_x4(smem_addr(sB + (kk * 16 + (lane >> 4) * 8 + (lane & 7)) * BPITCH + (ks * 16 + ((lane >> 3) & 1) * 8) * 2), f);
-                mma_bf16(s[0], q[ks], f[0], f[1]);
-                mma_bf16(s[1], q[ks], f[2], f[3]);
+                set0(u);
+                mma_bf16(u[0], q[ks], f[0], f[1]);
+                mma_bf16(u[1], q[ks], f[2], f[3]);
+#pragma unroll
+                for (int e = 0; e < 4; e++) { s[0][e] += u[0][e]; s[1][e] += u[1][e]; }
             }
 #pragma unroll
             for (int n = 0; n < 2; n++) {
@@ -720,9 +738,13 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
             for (int j = 0; j < 8; j += 2) {
                 uint32_t f[4];
                 ldsm_x4_t(smem_addr(sx + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * MXPITCH + (j * 8 + (lane >> 4) * 8) * 2), f);
-                mma_bf16(o[j], lo, f[0], f[1]); mma_bf16(o[j + 1], lo, f[2], f[3]);
-                mma_bf16(o[j], mid, f[0], f[1]); mma_bf16(o[j + 1], mid, f[2], f[3]);
-                mma_bf16(o[j], hi, f[0], f[1]); mma_bf16(o[j + 1], hi, f[2], f[3]);
+                float u[2][4];
+                set0(u);
+                mma_bf16(u[0], lo, f[0], f[1]); mma_bf16(u[1], lo, f[2], f[3]);
+                mma_bf16(u[0], mid, f[0], f[1]); mma_bf16(u[1], mid, f[2], f[3]);
+                mma_bf16(u[0], hi, f[0], f[1]); mma_bf16(u[1], hi, f[2], f[3]);
+#pragma unroll
+                for (int e = 0; e < 4; e++) { o[j][e] += u[0][e]; o[j + 1][e] += u[1][e]; }
             }
         }
         if (odd) {                                    // (0 times a later token's x would be NaN: token by token, up to the row's own)
