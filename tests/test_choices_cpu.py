@@ -51,3 +51,33 @@ def test_unevenness_and_the_partition_it_chooses():
     # equal lengths: a stream only where the pieces would take more than two rounds of CTAs
     assert not decode_partition_is_stream(8, 4, 128, 4, 0, 148) and not decode_partition_is_stream(64, 4, 32, 1, 0, 148)
     assert decode_partition_is_stream(64, 16, 32, 1, 0, 148)
+
+
+def test_latent_decode_pieces_are_near_the_best_that_was_timed():
+    """(sequences, heads, bucket of rows) and us a launch by the number of pieces, timed on a B200 at three quarters of
+    the bucket: the chosen number takes at most a sixth more than the best one."""
+    import ctypes
+
+    from trapetum_b200.csrc import build
+    pieces = build.load("attention_latent").tb_latent_decode_pieces
+    timed = {(1, 16, 512): {1: 22.2, 2: 17.0, 3: 16.2, 4: 13.7, 5: 16.2, 6: 16.4},
+             (1, 16, 4096): {8: 21.3, 12: 19.9, 16: 20.0, 18: 20.3, 24: 19.3, 32: 19.6, 40: 21.5, 48: 23.2, 64: 26.1},
+             (2, 32, 4096): {4: 30.8, 8: 21.5, 12: 20.2, 18: 20.8, 24: 19.6, 28: 20.2, 32: 21.4, 40: 24.6, 48: 33.1},
+             (3, 16, 2048): {4: 20.9, 6: 20.6, 7: 19.0, 8: 16.4, 9: 19.3, 12: 17.3, 16: 18.5, 20: 19.2, 24: 18.9},
+             (3, 32, 4096): {4: 31.6, 8: 21.3, 12: 20.4, 16: 20.4, 18: 21.3, 20: 21.1, 24: 28.6, 28: 25.9, 32: 31.4},
+             (5, 16, 4096): {4: 31.9, 8: 21.3, 12: 20.4, 16: 22.3, 18: 22.4, 20: 22.4, 24: 22.3, 28: 23.9, 32: 31.9},
+             (6, 16, 4096): {4: 31.7, 8: 21.3, 12: 21.6, 16: 22.5, 18: 22.5, 20: 22.4, 24: 28.0, 28: 25.9, 32: 32.3},
+             (8, 16, 4096): {4: 31.8, 7: 27.2, 8: 21.4, 9: 25.0, 12: 21.8, 16: 24.0, 18: 26.9, 20: 24.9, 24: 33.7},
+             (5, 32, 2048): {4: 21.9, 7: 19.2, 8: 18.8, 9: 19.7, 10: 20.0, 12: 20.4, 14: 23.8, 16: 28.1, 20: 28.4},
+             (12, 16, 2048): {4: 24.8, 6: 24.4, 7: 21.8, 8: 21.0, 9: 21.3, 10: 21.7, 12: 23.6, 14: 31.9, 20: 34.3},
+             (20, 16, 4096): {2: 65.3, 3: 49.9, 4: 39.1, 6: 33.3, 7: 31.5, 8: 46.5, 12: 42.4, 20: 51.5},
+             (48, 16, 4096): {1: 92.4, 2: 53.2, 3: 44.9, 4: 62.8, 6: 54.3, 8: 66.5},
+             (64, 16, 4096): {1: 120.0, 2: 67.9, 3: 91.4, 4: 78.6, 6: 87.5, 8: 98.3}}
+    for (batch, heads, rows), us in timed.items():
+        n = pieces(*map(ctypes.c_int, (batch, heads, rows, 148)))
+        at = us[min(us, key=lambda k: abs(k - n))]
+        assert at <= min(us.values()) * 7 / 6, (batch, heads, rows, n)
+    for batch in (1, 3, 16, 64, 200, 1000):                        # and any call gets at least one piece of a tile or more
+        for rows in (1, 32, 100, 5000, 1 << 20):
+            n = pieces(*map(ctypes.c_int, (batch, 16, rows, 148)))
+            assert 1 <= n <= 64 and (n == 1 or n * 32 <= rows)

@@ -677,20 +677,24 @@ extern "C" int tb_latent_decode_error() {
 static int latent_units(int batch, int heads) { return batch * ((heads + LD_H - 1) / LD_H); }
 static bool latent_in_cluster(int pieces, int units) { return pieces == 1 || pieces == 2 || pieces == 4 || (pieces == 8 && units <= 8); }
 extern "C" int tb_latent_decode_folds(int pieces, int batch, int heads) { return !latent_in_cluster(pieces, latent_units(batch, heads)); }
-// In how many pieces a launch of `batch` sequences of up to `rows` keys cuts each: the count that wastes least of the last
-// round of CTAs (one an SM), a piece's start and end being worth five turns of its three groups (2.5 us each), with a launch that
-// folds ten; clusters of four and eight do not fill more than one round well (96 units of 3,000 rows in four: 95 us, in three: 79).
+// In how many pieces a launch of `batch` sequences of up to `rows` keys cuts each: the least of a cost in us that was fitted to
+// 236 launches, each timed in up to 21 counts (1 to 64 units of 300 to 8,192 rows of 512 numbers): 6 and 2.4 a turn of the three
+// groups for every round of CTAs (one an SM; contexts lie between their bucket's half and its end: 0.8 of it), and for the launch
+// that folds 3.7, 0.18 a piece and, beyond four fifths of the SMs, up to 2 more (it starts on the free ones).  A piece's share of
+// the start-up alone, as before, cut too finely: 5 sequences of 3,000 rows in 29 pieces 24 to 31 us, in 18: 22, in 12: 20.
+// Clusters of four and eight do not fill more than one round (96 units of 3,000 rows in four: 95 us, in three: 79).
 extern "C" int tb_latent_decode_pieces(int batch, int heads, int rows, int sms) {
     const int units = latent_units(batch, heads), tiles = (rows + LD_BN - 1) / LD_BN;
     int best = 1;
-    double best_eff = 0.0;
-    for (int s = 1; s <= 64 && s * 3 <= tiles + 2; s++) {
-        const long long ctas = (long long)units * s;
-        const double turns = (double)((tiles + s - 1) / s + 2) / 3;
-        const bool cluster = latent_in_cluster(s, units);
-        double eff = (double)ctas / ((double)((ctas + sms - 1) / sms) * sms) * turns / (turns + (cluster ? 5.0 : 10.0));
-        if (cluster && s >= 4 && ctas > sms) eff *= 0.85;
-        if (eff > best_eff + 1e-9) { best = s; best_eff = eff; }
+    double least = 0.0;
+    for (int s = 1; s <= 64 && (s == 1 || s * 3 <= tiles + 2); s++) {
+        const long long ctas = (long long)units * s, rounds = (ctas + sms - 1) / sms;
+        const int usual = (int)((tiles * 4 + 5LL * s - 1) / (5LL * s));          // tiles of a piece
+        double cost = (double)rounds * (6.0 + 2.4 * ((usual + 2) / 3));
+        const double full = (double)ctas / ((double)rounds * sms) - 0.8;
+        if (!latent_in_cluster(s, units)) cost += 3.7 + 0.18 * s + (full > 0.0 ? 10.0 * full : 0.0);
+        else if (s >= 4 && rounds > 1) cost *= 2.0;
+        if (s == 1 || cost < least - 1e-9) { best = s; least = cost; }
     }
     return best;
 }
