@@ -299,6 +299,40 @@ def test_mamba2_products_lose_nothing_in_the_state(ops, n, B, heads, N, log_a):
     assert err[1] <= 1.2 * err[0], err
 
 
+def device_time(call, reps=20):
+    """Least time of ``reps`` calls in a row, of five tries, in ms."""
+    best = math.inf
+    for _ in range(5):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        call()
+        begin.record()
+        for _ in range(reps):
+            call()
+        end.record()
+        torch.cuda.synchronize()
+        best = min(best, begin.elapsed_time(end))
+    return best
+
+
+@pytest.mark.parametrize("lens", [[64] + 63 * [5], [64] + 15 * [5], [8 + 7 * i % 57 for i in range(64)], [300] + 31 * [9]])
+def test_mamba2_short_prompts_are_not_slower_than_the_recurrence(ops, monkeypatch, lens):
+    """Many short prompts in a step whose longest one asks for the product form: no state goes through scratch for them,
+    and the step takes at most a quarter more than the recurrence (five times as much before)."""
+    heads, P, N = 64, 64, 128
+    T, B, inner, ch = sum(lens), len(lens), heads * P, heads * P + 2 * N
+    proj, dt = rnd(T, inner + ch, dt=torch.bfloat16), rnd(T, heads, seed=1)
+    small = [rnd(ch, 4, s=0.3, seed=2), rnd(ch, s=0.1, seed=3), rnd(heads, seed=4) - 2, rnd(heads, s=0.5, seed=5), rnd(heads, seed=6)]
+    starts = torch.tensor([sum(lens[:i]) for i in range(B + 1)], dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).to("cuda", torch.int32)
+    slots = torch.arange(B, dtype=torch.int32, device="cuda")
+    state, norm = torch.zeros(B, ops.mamba2_state_size(heads, P, N, 1, 4), device="cuda"), torch.ones(inner, device="cuda")
+    times = []
+    for least in (ops.MAMBA2_PRODUCTS_FROM, 1 << 30):
+        monkeypatch.setattr(ops, "MAMBA2_PRODUCTS_FROM", least)
+        times.append(device_time(lambda: ops.mamba2(proj, dt, heads, P, N, 1, 4, 1, *small, norm, 1e-6, state, starts, seq, slots, B, False, max(lens))))
+    assert times[0] <= 1.25 * times[1], times
+
+
 @pytest.mark.parametrize("n,B,heads,bias", [(100, 1, 4, 0.0), (100, 2, 4, 2.0), (2048, 1, 4, 0.0), (2048, 1, 4, 6.0), (2048, 16, 10, 10.0)])
 def test_gla_blocks_lose_nothing_in_the_state(ops, n, B, heads, bias):
     """The same of gated linear attention, prompts in several chunks and (16 of them) in one.  ``bias`` 10: decays of 0.99999."""

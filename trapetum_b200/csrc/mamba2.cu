@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(SCAN_NS * PT / SCAN_PP) mamba2_scan_kernel(Mam
 //     y_i = sum_{j <= i} (C_i . B_j) 2^(c_i - c_j) dt_j x_j  +  2^(c_i) S C_i  +  D x_i
 //     S'  = 2^(c_last) S + sum_j 2^(c_last - c_j) dt_j x_j B_j^T
 // in three launches: each chunk's own sum E, the states before the chunks (a scan over chunks, element by element), the
-// outputs.  x, B and C are bfloat16 numbers; what meets them (the weighted scores, the weighted x, the state) is 32-bit and
+// outputs; sequences of one chunk take part in the last one only.  x, B and C are bfloat16 numbers; what meets them (the weighted scores, the weighted x, the state) is 32-bit and
 // enters as the sum of three bfloat16 numbers, 24 bits, so every product is that of the recurrence and only the order of the
 // 32-bit sums differs.  The running sums are kept as two 32-bit numbers (c_i - c_j of near tokens keeps its digits); a
 // decay below 2^-300 is 0 in any product.  A non-finite x is seen by its own token and later ones only, as in the recurrence;
@@ -471,13 +471,14 @@ __device__ __forceinline__ float high3(const uint32_t* p) {
     return __uint_as_float(p[0] & 0xffff0000u) + (__uint_as_float(p[1] & 0xffff0000u) + __uint_as_float(p[2] & 0xffff0000u));
 }
 
-struct ChunkPlace { int t0, n, c, b, slot; };         // first token, tokens, index in its sequence, sequence, scratch slot
+struct ChunkPlace { int t0, n, c, b, slot; bool alone; };   // first token, tokens, index in its sequence, sequence, scratch slot, its sequence's only one
 // A sequence's chunks lie from slot floor(seq_start / 128) + b on, which leaves every sequence enough of them.
 __device__ __forceinline__ ChunkPlace chunk_place(const Mamba2Args& a, int z) {
     ChunkPlace p;
     p.b = z / a.n_chunks; p.c = z % a.n_chunks;
     const int s0 = a.seq_start[p.b], s1 = a.seq_start[p.b + 1];
     p.t0 = s0 + p.c * MC; p.n = min(MC, s1 - p.t0); p.slot = s0 / MC + p.b + p.c;
+    p.alone = a.n_chunks == 1 || s1 - s0 <= MC;       // (without chunks nothing looks for scratch, whatever the lengths)
     return p;
 }
 
@@ -511,52 +512,29 @@ __device__ __forceinline__ void chunk_decays(const Mamba2Args& a, const ChunkPla
     __syncthreads();
 }
 
-// 128 rows of COLS bfloat16 columns, of which `cols` exist, into padded shared rows; rows from n on become zero.
+// n rows of COLS bfloat16 columns, of which `cols` exist, into padded shared rows; up to the next multiple of 16, rows of zeros.
 template <int COLS>
 __device__ __forceinline__ void load_chunk(uint8_t* dst, const bf16* src, long long stride, int n, int cols) {
     constexpr int CPR = COLS / 8, PITCH = COLS * 2 + 16;
 #pragma unroll 4
-    for (int c = threadIdx.x; c < MC * CPR; c += MCT) {
+    for (int c = threadIdx.x; c < (n + 15) / 16 * 16 * CPR; c += MCT) {
         const int r = c / CPR, k = (c % CPR) * 8;
         const bool ok = r < n && k < cols;
         cp_async16(dst + r * PITCH + k * 2, src + (ok ? (size_t)r * stride + k : 0), ok);
     }
 }
 
-// E = sum_j 2^(c_last - c_j) dt_j x_j B_j^T: 64 values of P of one head, all N.  Warp w: 16 rows of P, half of N.
+// sum_j w_j x_j B_j^T of a chunk's n tokens.  Warp w: 16 rows of P, half of N, in accumulators.
 template <int NP>
-__global__ void __launch_bounds__(MCT) mamba2_chunk_sum_kernel(Mamba2Args a) {
-    pdl_launch_dependents();
-    constexpr int BPITCH = NP * 2 + 16, NT = NP / 16;  // 8-column pieces a warp
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* sB = smem;                               // [128][BPITCH]
-    uint8_t* sx = sB + MC * BPITCH;                   // [128][MXPITCH]
-    float2* scum = (float2*)(sx + MC * MXPITCH);      // [128]
-    float* sdt = (float*)(scum + MC);                 // [128], then the weights
-    __shared__ double red[4];
-    const int h = blockIdx.y, p0 = blockIdx.x * MP, N = a.N, P = a.P;
-    const int inner = a.heads * P, ch = inner + 2 * a.groups * N, g_of = h / (a.heads / a.groups);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    pdl_wait();
-    const ChunkPlace pl = chunk_place(a, blockIdx.z);
-    if (pl.n <= 0) return;
-    const bf16* row = (const bf16*)a.xbc + (size_t)pl.t0 * ch;
-    load_chunk<NP>(sB, row + inner + g_of * N, ch, pl.n, N);
-    load_chunk<MP>(sx, row + h * P + p0, ch, pl.n, P - p0);
-    cp_async_commit();
-    chunk_decays(a, pl, h, sdt, scum, red);
-    const float2 last = scum[MC - 1];
-    if (threadIdx.x < MC) sdt[threadIdx.x] *= exp2_fast((last.x - scum[threadIdx.x].x) + (last.y - scum[threadIdx.x].y));
-    if (blockIdx.x == 0 && threadIdx.x == 0) a.chunk_decay[(size_t)pl.slot * a.heads + h] = exp2_fast(last.x + last.y);
-    cp_async_wait<0>();
-    __syncthreads();
+__device__ __forceinline__ void chunk_sum(const uint8_t* sB, const uint8_t* sx, const float* w, int n, float (*acc)[4]) {
+    constexpr int BPITCH = NP * 2 + 16, NT = NP / 16;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
     const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * (NP / 2);
-    float acc[NT][4];
 #pragma unroll
     for (int j = 0; j < NT; j++) { acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f; }
-    const int steps = (pl.n + 15) / 16;
+    const int steps = (n + 15) / 16;
     for (int kk = 0; kk < steps; kk++) {
-        const float2 wa = *(const float2*)(sdt + kk * 16 + 2 * t), wb = *(const float2*)(sdt + kk * 16 + 2 * t + 8);
+        const float2 wa = *(const float2*)(w + kk * 16 + 2 * t), wb = *(const float2*)(w + kk * 16 + 2 * t + 8);
         uint32_t x[4], hi[4], mid[4], lo[4];
         ldsm_x4_t(smem_addr(sx + (kk * 16 + (lane >> 4) * 8 + (lane & 7)) * MXPITCH + (m0 + ((lane >> 3) & 1) * 8) * 2), x);
 #pragma unroll
@@ -575,6 +553,38 @@ __global__ void __launch_bounds__(MCT) mamba2_chunk_sum_kernel(Mamba2Args a) {
             for (int e = 0; e < 4; e++) { acc[j][e] += u[0][e]; acc[j + 1][e] += u[1][e]; }
         }
     }
+}
+
+// E = sum_j 2^(c_last - c_j) dt_j x_j B_j^T: 64 values of P of one head, all N, of a sequence of several chunks.
+template <int NP>
+__global__ void __launch_bounds__(MCT) mamba2_chunk_sum_kernel(Mamba2Args a) {
+    pdl_launch_dependents();
+    constexpr int BPITCH = NP * 2 + 16, NT = NP / 16;  // 8-column pieces a warp
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint8_t* sB = smem;                               // [128][BPITCH]
+    uint8_t* sx = sB + MC * BPITCH;                   // [128][MXPITCH]
+    float2* scum = (float2*)(sx + MC * MXPITCH);      // [128]
+    float* sdt = (float*)(scum + MC);                 // [128], then the weights
+    __shared__ double red[4];
+    const int h = blockIdx.y, p0 = blockIdx.x * MP, N = a.N, P = a.P;
+    const int inner = a.heads * P, ch = inner + 2 * a.groups * N, g_of = h / (a.heads / a.groups);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    pdl_wait();
+    const ChunkPlace pl = chunk_place(a, blockIdx.z);
+    if (pl.n <= 0 || pl.alone) return;
+    const bf16* row = (const bf16*)a.xbc + (size_t)pl.t0 * ch;
+    load_chunk<NP>(sB, row + inner + g_of * N, ch, pl.n, N);
+    load_chunk<MP>(sx, row + h * P + p0, ch, pl.n, P - p0);
+    cp_async_commit();
+    chunk_decays(a, pl, h, sdt, scum, red);
+    const float2 last = scum[MC - 1];
+    if (threadIdx.x < MC) sdt[threadIdx.x] *= exp2_fast((last.x - scum[threadIdx.x].x) + (last.y - scum[threadIdx.x].y));
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.chunk_decay[(size_t)pl.slot * a.heads + h] = exp2_fast(last.x + last.y);
+    cp_async_wait<0>();
+    __syncthreads();
+    float acc[NT][4];
+    chunk_sum<NP>(sB, sx, sdt, pl.n, acc);
+    const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * (NP / 2);
     float* E = a.chunk_state + (size_t)pl.slot * a.heads * P * N + (size_t)h * P * N;
 #pragma unroll
     for (int j = 0; j < NT; j++) {
@@ -595,7 +605,7 @@ __global__ void __launch_bounds__(256) mamba2_chunk_fold_kernel(Mamba2Args a) {
     const int h = (int)(e / per);
     pdl_wait();
     const int s0 = a.seq_start[b], len = a.seq_start[b + 1] - s0, n = (len + MC - 1) / MC, slot = s0 / MC + b;
-    if (n <= 0) return;
+    if (n <= 1) return;                               // (a sequence of one chunk: the outputs' launch)
     float* st = a.state + (size_t)a.slot_ids[b] * a.state_stride + e;
     float4 s = *(const float4*)st;
     float* E = a.chunk_state + (size_t)slot * hpn + e;
@@ -614,7 +624,8 @@ __global__ void __launch_bounds__(256) mamba2_chunk_fold_kernel(Mamba2Args a) {
     *(float4*)st = s;
 }
 
-// y of 128 tokens of one head, 64 values of P.  Warp w: 16 tokens.
+// y of 128 tokens of one head, 64 values of P.  Warp w: 16 tokens.  A sequence of one chunk starts from its slot and leaves its
+// state there, in this launch alone: nobody else reads that part of the slot.
 template <int NP>
 __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) {
     pdl_launch_dependents();
@@ -626,6 +637,7 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
     uint8_t* sx = sB + MC * BPITCH;                   // [128][MXPITCH]
     float2* scum = (float2*)(sx + MC * MXPITCH);      // [128]
     float* sdt = (float*)(scum + MC);                 // [128]
+    float* sw = sdt + MC;                             // [128] the tokens' weights in the state that a sequence of one chunk leaves
     __shared__ double red[4];
     const int h = blockIdx.y, p0 = blockIdx.x * MP, N = a.N, P = a.P;
     const int inner = a.heads * P, ch = inner + 2 * a.groups * N, g_of = h / (a.heads / a.groups);
@@ -640,7 +652,7 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
     load_chunk<MP>(sx, row + h * P + p0, ch, pl.n, P - p0);
     cp_async_commit();
     // the state, on its way through registers meanwhile: thread (p, part of n)
-    const float* S = a.chunk_state + (size_t)pl.slot * a.heads * P * N + ((size_t)h * P + p0) * N;
+    float* S = (pl.alone ? a.state + (size_t)a.slot_ids[pl.b] * a.state_stride : a.chunk_state + (size_t)pl.slot * a.heads * P * N) + ((size_t)h * P + p0) * N;
     constexpr int Q = MP * NP / 4 / MCT;              // groups of four a thread
     float4 sv[Q];
 #pragma unroll
@@ -649,6 +661,8 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
         sv[u] = (p0 + p < P && n < N) ? *(const float4*)(S + (size_t)p * N + n) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     chunk_decays(a, pl, h, sdt, scum, red);
+    const float2 last = scum[MC - 1];
+    if (pl.alone && tid < MC) sw[tid] = sdt[tid] * exp2_fast((last.x - scum[tid].x) + (last.y - scum[tid].y));
     cp_async_wait<1>();
     __syncthreads();
     uint32_t q[KS][4];
@@ -782,6 +796,22 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
             }
         }
     }
+    if (!pl.alone) return;
+    // ---- the state after the sequence (every thread has read its part of the one before, above the last barrier)
+    float acc[NP / 16][4];
+    chunk_sum<NP>(sB, sx, sw, pl.n, acc);
+    const float all = exp2_fast(last.x + last.y);
+    const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * (NP / 2);
+#pragma unroll
+    for (int j = 0; j < NP / 16; j++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int n = n0 + j * 8 + 2 * t, p = m0 + g + e * 8;
+            if (n >= N || p0 + p >= P) continue;
+            float2* to = (float2*)(S + (size_t)p * N + n);
+            const float2 s = *to;
+            *to = make_float2(fmaf(all, s.x, acc[j][2 * e]), fmaf(all, s.y, acc[j][2 * e + 1]));
+        }
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -980,12 +1010,16 @@ extern "C" int tb_mamba2_chunk_slots(int batch, int n_tokens) { return n_tokens 
 
 template <int NP>
 static int run_chunks(const Mamba2Args& a, cudaStream_t stream) {
-    constexpr int BPITCH = NP * 2 + 16, TAIL = MC * MXPITCH + MC * 12;
+    constexpr int BPITCH = NP * 2 + 16, TAIL = MC * MXPITCH + MC * 16;
     constexpr int SUM = MC * BPITCH + TAIL, OUT = (MC * BPITCH > 3 * MP * BPITCH ? MC * BPITCH : 3 * MP * BPITCH) + MC * BPITCH + TAIL;
     cudaError_t e = cudaFuncSetAttribute(mamba2_chunk_sum_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SUM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(mamba2_chunk_out_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT);
     if (e != cudaSuccess) return (int)e;
     const dim3 grid((a.P + MP - 1) / MP, a.heads, a.batch * a.n_chunks);
+    if (a.n_chunks == 1) {
+        tb_launch(mamba2_chunk_out_kernel<NP>, grid, dim3(MCT), OUT, stream, a);
+        return tb_launch_status();
+    }
     tb_launch(mamba2_chunk_sum_kernel<NP>, grid, dim3(MCT), SUM, stream, a);
     int st = tb_launch_status();
     if (st) return st;
@@ -997,7 +1031,7 @@ static int run_chunks(const Mamba2Args& a, cudaStream_t stream) {
     return tb_launch_status();
 }
 
-// n_chunks: of the longest sequence; chunk_state [slots][heads * P * N], chunk_decay [slots][heads].
+// n_chunks: of the longest sequence; chunk_state [slots][heads * P * N] and chunk_decay [slots][heads] if more than one.
 extern "C" int tb_mamba2_chunks(const Mamba2Args* args, int dtype, int w_dtype, cudaStream_t stream) {
     const Mamba2Args& a = *args;
     if (a.n_tokens <= 0 || a.batch <= 0) return 0;
@@ -1005,7 +1039,7 @@ extern "C" int tb_mamba2_chunks(const Mamba2Args* args, int dtype, int w_dtype, 
     const int ch = a.heads * a.P + 2 * a.groups * a.N;
     if (!tb_mamba2_chunks_takes(dtype, a.heads, a.P, a.N, a.groups) || w_dtype != TB_F32)
         return tb_refuse("mamba2: the product form takes bfloat16 with P and N in multiples of 8, N up to 128 (got P=%d N=%d)", a.P, a.N);
-    if (a.chunk_state == nullptr || a.chunk_decay == nullptr || a.n_chunks < 1 || (long long)a.batch * a.n_chunks > 65535)
+    if ((a.n_chunks > 1 && (a.chunk_state == nullptr || a.chunk_decay == nullptr)) || a.n_chunks < 1 || (long long)a.batch * a.n_chunks > 65535)
         return tb_refuse("mamba2: the product form needs its scratch, and at most 65535 chunks (%d sequences of %d)", a.batch, a.n_chunks);
     if (((uintptr_t)a.xbc & 15) || ch % 8 || ((uintptr_t)a.state & 15) || a.state_stride % 4 || ((uintptr_t)a.chunk_state & 15) || ((uintptr_t)a.y & 7))
         return tb_refuse("mamba2: the product form needs 16-byte aligned rows and states");
@@ -1036,4 +1070,13 @@ extern "C" int tb_mamba2_gate_norm(const Mamba2Args* args, int dtype, int w_dtyp
     }
     DISPATCH2(dtype, w_dtype, tb_launch(mamba2_gate_norm_kernel<T, TW>, dim3(a.n_tokens, a.norm_groups), dim3(threads), 0, stream, a));
     return tb_launch_status();
+}
+
+// A step of whole prompts in the product form: convolution, chunks, gated norm in one call (a short prompt's step is bound by the
+// host: 180 tokens of 32 heads 47.6 us with three).
+extern "C" int tb_mamba2_prompts(const Mamba2Args* args, int dtype, int w_dtype, cudaStream_t stream) {
+    int st = tb_mamba2_conv(args, dtype, w_dtype, 0, stream);
+    if (st) return st;
+    st = tb_mamba2_chunks(args, dtype, w_dtype, stream);
+    return st ? st : tb_mamba2_gate_norm(args, dtype, w_dtype, stream);
 }

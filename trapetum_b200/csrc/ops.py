@@ -726,6 +726,7 @@ class _Mamba2Args(ctypes.Structure):
 # Tokens of the longest prompt from which prompts run as products over chunks: 48 / 64 / 96 / 256 tokens take 30.2 / 31.2 /
 # 38.5 / 50.1 us, as a recurrence 30.7 / 36.5 / 52.3 / 111.9 (64 heads of 64 x 128)
 MAMBA2_PRODUCTS_FROM = 64
+MAMBA2_PRODUCTS_MEAN = 16           # ... and of the tokens a sequence, on average
 MAMBA2_PRODUCTS_BYTES = 1 << 30     # ... as long as the states between the chunks (16 KB a token of the medium sizes) stay within this
 
 
@@ -776,16 +777,19 @@ def mamba2(proj: torch.Tensor, dt_raw: torch.Tensor, heads: int, P: int, N: int,
     a.seq_start = seq_start.data_ptr(); a.token_seq = token_seq.data_ptr(); a.slot_ids = slot_ids.data_ptr()
     a.xbc = xbc.data_ptr(); a.y = y.data_ptr(); a.out = out.data_ptr(); a.batch = batch; a.n_tokens = T
     lib = build.load("mamba2")
-    scan_launches, products = 1, False
-    if not one_token_each and max_seq_len >= MAMBA2_PRODUCTS_FROM and lib.tb_mamba2_chunks_takes(c_int(code(dt)), c_int(heads), c_int(P), c_int(N), c_int(groups)) \
-            and state.data_ptr() % 16 == 0 and state.stride(0) % 4 == 0:
-        # whole prompts as products over chunks; not where the chunks' states would take more than MAMBA2_PRODUCTS_BYTES
-        slots, n_chunks = int(lib.tb_mamba2_chunk_slots(c_int(batch), c_int(T))), (max_seq_len + 127) // 128
-        products = slots * heads * P * N * 4 <= MAMBA2_PRODUCTS_BYTES and batch * n_chunks <= 65535
-        if products:
-            chunk_state = torch.empty((slots, heads * P * N), dtype=torch.float32, device=proj.device)
-            chunk_decay = torch.empty((slots, heads), dtype=torch.float32, device=proj.device)
-            a.chunk_state = chunk_state.data_ptr(); a.chunk_decay = chunk_decay.data_ptr(); a.n_chunks = n_chunks
+    scan_launches, products, n_chunks = 1, False, (max_seq_len + 127) // 128
+    if not one_token_each and max_seq_len >= MAMBA2_PRODUCTS_FROM and T >= MAMBA2_PRODUCTS_MEAN * batch and batch * n_chunks <= 65535 and state.data_ptr() % 16 == 0 and state.stride(0) % 4 == 0 \
+            and lib.tb_mamba2_chunks_takes(c_int(code(dt)), c_int(heads), c_int(P), c_int(N), c_int(groups)):
+        # whole prompts as products over chunks; not where the chunks' states would take more than MAMBA2_PRODUCTS_BYTES (prompts
+        # of one chunk need none)
+        products = n_chunks == 1
+        if not products:
+            slots, per_slot = int(lib.tb_mamba2_chunk_slots(c_int(batch), c_int(T))), heads * P * N
+            if slots * per_slot * 4 <= MAMBA2_PRODUCTS_BYTES:
+                scratch = torch.empty(slots * (per_slot + heads), dtype=torch.float32, device=proj.device)
+                a.chunk_state = scratch.data_ptr(); a.chunk_decay = a.chunk_state + slots * per_slot * 4
+                products = True
+        a.n_chunks = n_chunks if products else 0
     if not products and not one_token_each and max_seq_len > 0:
         chunk_len = c_int(0)
         n_chunks = int(lib.tb_mamba2_plan(c_int(heads), c_int(P), c_int(batch), c_int(int(max_seq_len)), ctypes.byref(chunk_len)))
@@ -796,12 +800,12 @@ def mamba2(proj: torch.Tensor, dt_raw: torch.Tensor, heads: int, P: int, N: int,
             a.chunk_len = chunk_len.value; a.n_chunks = n_chunks
             scan_launches = 2
     cd, cw = c_int(code(dt)), c_int(code(wd))
+    if products:
+        _check(lib, lib.tb_mamba2_prompts(ctypes.byref(a), cd, cw, _stream()), "mamba2_prompts", (1 if taps == 1 else 2) + (1 if n_chunks == 1 else 3) + 1)
+        return out
     _check(lib, lib.tb_mamba2_conv(ctypes.byref(a), cd, cw, c_int(int(bool(one_token_each))), _stream()), "mamba2_conv",
            1 if one_token_each or taps == 1 else 2)
-    if products:
-        _check(lib, lib.tb_mamba2_chunks(ctypes.byref(a), cd, cw, _stream()), "mamba2_chunks", 3)
-    else:
-        _check(lib, lib.tb_mamba2_scan(ctypes.byref(a), cd, cw, _stream()), "mamba2_scan", scan_launches)
+    _check(lib, lib.tb_mamba2_scan(ctypes.byref(a), cd, cw, _stream()), "mamba2_scan", scan_launches)
     _check(lib, lib.tb_mamba2_gate_norm(ctypes.byref(a), cd, cw, _stream()), "mamba2_gate_norm")
     return out
 
