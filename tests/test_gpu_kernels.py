@@ -299,6 +299,29 @@ def test_mamba2_products_lose_nothing_in_the_state(ops, n, B, heads, N, log_a):
     assert err[1] <= 1.2 * err[0], err
 
 
+def test_mamba2_prompts_do_not_depend_on_the_step(ops):
+    """A sequence alone and beside others, where a thread of the convolution takes two tokens and eight: the same bits."""
+    heads, P, N, lens = 64, 64, 128, [400, 30, 41]
+    T, inner, ch = sum(lens), heads * P, heads * P + 2 * N
+    proj, dt = rnd(T, inner + ch, dt=torch.bfloat16), rnd(T, heads, seed=1)
+    small = [rnd(ch, 4, s=0.3, seed=2), rnd(ch, s=0.1, seed=3), rnd(heads, seed=4) - 2, rnd(heads, s=0.5, seed=5), rnd(heads, seed=6)]
+    norm, first = rnd(inner, s=0.1, seed=7) + 1, rnd(3, ops.mamba2_state_size(heads, P, N, 1, 4), seed=8)
+
+    def run(which):
+        n = [lens[i] for i in which]
+        rows = torch.cat([torch.arange(sum(lens[:i]), sum(lens[:i + 1])) for i in which]).cuda()
+        starts = torch.tensor([sum(n[:i]) for i in range(len(n) + 1)], dtype=torch.int32, device="cuda")
+        seq = torch.repeat_interleave(torch.arange(len(n)), torch.tensor(n)).to("cuda", torch.int32)
+        state, slots = first.clone(), torch.tensor(which, dtype=torch.int32, device="cuda")
+        out = ops.mamba2(proj[rows], dt[rows], heads, P, N, 1, 4, 1, *small, norm, 1e-6, state, starts, seq, slots, len(n), False, 400)
+        return out, state[which]
+    out, state = run([0, 1, 2])
+    for i in range(3):
+        alone = run([i])
+        assert torch.equal(alone[0], out[sum(lens[:i]):sum(lens[:i + 1])]) and torch.equal(alone[1][0], state[i])
+
+
+
 def device_time(call, reps=20):
     """Least time of ``reps`` calls in a row, of five tries, in ms."""
     best = math.inf

@@ -80,7 +80,6 @@ __global__ void mamba2_conv_kernel(Mamba2Args a) {
 // Four taps in bfloat16: a thread takes four neighbouring channels of eight tokens in a row, whose inputs are on their way
 // together, 8 bytes a load: 18 us for 2,048 tokens x 4,352 channels, cold (a thread per number: 76; eight channels a thread,
 // whose registers leave half the warps: 26; its 36 MB are 5.4).
-constexpr int CONV_TOK = 8;
 __device__ __forceinline__ void unpack4(const uint2& v, float* f) {
     f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
     f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
@@ -89,6 +88,7 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *(uint32_t*)&h;
 }
+template <int CONV_TOK>
 __global__ void __launch_bounds__(128, 6) mamba2_conv4_kernel(Mamba2Args a) {
     pdl_launch_dependents();
     const int inner = a.heads * a.P, ch = inner + 2 * a.groups * a.N;
@@ -919,7 +919,10 @@ extern "C" int tb_mamba2_conv(const Mamba2Args* args, int dtype, int w_dtype, in
     }
     const bool wide = dtype == TB_BF16 && w_dtype == TB_F32 && a.taps == 4 && ch % 4 == 0 && (a.heads * a.P) % 4 == 0 && a.proj_stride % 4 == 0 &&
                       ((uintptr_t)a.proj & 7) == 0 && ((uintptr_t)a.xbc & 7) == 0 && ((uintptr_t)a.conv_w & 15) == 0;
-    if (wide) tb_launch(mamba2_conv4_kernel, dim3((a.n_tokens + CONV_TOK - 1) / CONV_TOK, (ch / 4 + 127) / 128), dim3(128), 0, stream, a);
+    // eight tokens a thread where that leaves three CTAs an SM, else two (100 tokens of 2,176 channels: 65 CTAs of a long chain each)
+    const long long wide_ctas = (long long)((a.n_tokens + 7) / 8) * ((ch / 4 + 127) / 128);
+    if (wide && wide_ctas >= 3 * 148) tb_launch(mamba2_conv4_kernel<8>, dim3((a.n_tokens + 7) / 8, (ch / 4 + 127) / 128), dim3(128), 0, stream, a);
+    else if (wide) tb_launch(mamba2_conv4_kernel<2>, dim3((a.n_tokens + 1) / 2, (ch / 4 + 127) / 128), dim3(128), 0, stream, a);
     else DISPATCH2(dtype, w_dtype, tb_launch(mamba2_conv_kernel<T, TW>, dim3(a.n_tokens, gy), dim3(128), 0, stream, a));
     int st = tb_launch_status();
     if (st) return st;
