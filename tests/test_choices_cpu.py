@@ -81,3 +81,15 @@ def test_latent_decode_pieces_are_near_the_best_that_was_timed():
         for rows in (1, 32, 100, 5000, 1 << 20):
             n = pieces(*map(ctypes.c_int, (batch, 16, rows, 148)))
             assert 1 <= n <= 64 and (n == 1 or n * 32 <= rows)
+
+
+def test_the_gated_norm_of_few_tokens_uses_the_threads_there_are():
+    """A step of few tokens is a chain of waits: 1,024 threads a row, one group of four columns each as long as that goes."""
+    import ctypes
+
+    from trapetum_b200.csrc import build
+    groups = build.load("mamba2").tb_mamba2_gate_norm_groups
+    for tokens, threads in ((1, 1024), (64, 1024), (65, 256), (2048, 256)):
+        for gs in (4, 1000, 1024, 4096, 4100, 8192, 16384):
+            n = groups(ctypes.c_int(tokens), ctypes.c_int(gs))
+            assert n in (1, 2, 4, 8, 16) and gs <= 4 * threads * n and (n == 1 or gs > 2 * threads * n)

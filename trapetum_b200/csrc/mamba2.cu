@@ -841,8 +841,10 @@ __global__ void mamba2_gate_norm_kernel(Mamba2Args a) {
 }
 
 // The same where a thread can keep its NV groups of four columns in registers, so that y and z are read once, 16 bytes of y
-// and four values of z a load (group sizes that are multiples of 4).  Few tokens (the launch's time is a chain of memory
-// round trips): a group a thread.  Many: 256 threads a row, 2,048 rows of 4,096 in 15 us (read twice: 37; 67 MB are 10).
+// and four values of z a load (group sizes that are multiples of 4).  FEW tokens (the launch's time is a chain of memory
+// round trips): up to 1,024 threads a row and the weights fetched ahead of the wait; of a step of one token of 8,192 channels
+// with cold caches, all launches, 13.9 us (256 threads, the weights after the sum: 18.2).  Many: 256 threads a row, 2,048 rows
+// of 4,096 in 15 us (read twice: 37; 67 MB are 10).
 __device__ __forceinline__ float4 four(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ float4 four(const bf16* p) {
     const uint2 u = *(const uint2*)p;
@@ -851,12 +853,20 @@ __device__ __forceinline__ float4 four(const bf16* p) {
 __device__ __forceinline__ void store4(float* p, float4 v) { *(float4*)p = v; }
 __device__ __forceinline__ void store4(bf16* p, float4 v) { *(uint2*)p = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w)); }
 
-template <typename T, int NV>
-__global__ void __launch_bounds__(NV == 1 ? 1024 : NV == 2 ? 512 : 256) mamba2_gate_norm_rows_kernel(Mamba2Args a) {
+template <typename T, int NV, bool FEW>
+__global__ void __launch_bounds__(FEW ? 1024 : 256) mamba2_gate_norm_rows_kernel(Mamba2Args a) {
     pdl_launch_dependents();
     __shared__ float red[33];
     const int inner = a.heads * a.P, gs = inner / a.norm_groups;
     const int t = blockIdx.x, c0 = blockIdx.y * gs;
+    float4 w[NV];
+    if (FEW) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            const int i = (threadIdx.x + k * blockDim.x) * 4;
+            if (i < gs) w[k] = four((const float*)a.norm_w + c0 + i);
+        }
+    }
     pdl_wait();
     const float* y = a.y + (size_t)t * inner + c0;
     const T* z = (const T*)a.proj + (size_t)t * a.proj_stride + c0;
@@ -880,8 +890,8 @@ __global__ void __launch_bounds__(NV == 1 ? 1024 : NV == 2 ? 512 : 256) mamba2_g
     for (int k = 0; k < NV; k++) {
         const int i = (threadIdx.x + k * blockDim.x) * 4;
         if (i < gs) {
-            const float4 w = four((const float*)a.norm_w + c0 + i);
-            store4(out + i, make_float4(v[k].x * r * w.x, v[k].y * r * w.y, v[k].z * r * w.z, v[k].w * r * w.w));
+            if (!FEW) w[k] = four((const float*)a.norm_w + c0 + i);
+            store4(out + i, make_float4(v[k].x * r * w[k].x, v[k].y * r * w[k].y, v[k].z * r * w[k].z, v[k].w * r * w[k].w));
         }
     }
 }
@@ -1049,6 +1059,15 @@ extern "C" int tb_mamba2_chunks(const Mamba2Args* args, int dtype, int w_dtype, 
     return a.N <= 64 ? run_chunks<64>(a, stream) : run_chunks<128>(a, stream);
 }
 
+// Groups of four columns that a thread of the norm takes of rows of `gs` numbers (up to 16,384): for few tokens as few as 1,024
+// threads allow, for many as 256 do.
+constexpr int NORM_FEW = 64;
+extern "C" int tb_mamba2_gate_norm_groups(int n_tokens, int gs) {
+    int nv = 1;
+    while (gs / 4 > nv * (n_tokens <= NORM_FEW ? 1024 : 256)) nv *= 2;
+    return nv;
+}
+
 extern "C" int tb_mamba2_gate_norm(const Mamba2Args* args, int dtype, int w_dtype, cudaStream_t stream) {
     Mamba2Args a = *args;
     if (a.n_tokens <= 0) return 0;
@@ -1060,14 +1079,13 @@ extern "C" int tb_mamba2_gate_norm(const Mamba2Args* args, int dtype, int w_dtyp
     const int es = dtype == TB_BF16 ? 2 : 4;
     if (w_dtype == TB_F32 && gs % 4 == 0 && gs <= 16384 && a.proj_stride % 4 == 0 && ((uintptr_t)a.y & 15) == 0 && ((uintptr_t)a.norm_w & 15) == 0 &&
         ((uintptr_t)a.proj & (4 * es - 1)) == 0 && ((uintptr_t)a.out & (4 * es - 1)) == 0) {
-        const int quads = gs / 4, want = a.n_tokens <= 64 ? 1024 : 256;
-        int nv = 1;
-        while (nv < 16 && quads > nv * (nv == 1 ? 1024 : nv == 2 ? 512 : 256)) nv *= 2;
-        while (nv < 16 && quads > nv * want) nv *= 2;
-        int th = ((quads + nv - 1) / nv + 31) / 32 * 32;
+        const bool few = a.n_tokens <= NORM_FEW;
+        const int nv = tb_mamba2_gate_norm_groups(a.n_tokens, gs);
+        int th = ((gs / 4 + nv - 1) / nv + 31) / 32 * 32;
         if (th < 64) th = 64;
-#define ROWS(NV_) TB_DISPATCH_1(dtype, T, tb_launch(mamba2_gate_norm_rows_kernel<T, NV_>, dim3(a.n_tokens, a.norm_groups), dim3(th), 0, stream, a))
-        if (nv == 1) ROWS(1); else if (nv == 2) ROWS(2); else if (nv == 4) ROWS(4); else if (nv == 8) ROWS(8); else ROWS(16);
+#define ROWS(NV_, FEW_) TB_DISPATCH_1(dtype, T, tb_launch(mamba2_gate_norm_rows_kernel<T, NV_, FEW_>, dim3(a.n_tokens, a.norm_groups), dim3(th), 0, stream, a))
+        if (few) { if (nv == 1) ROWS(1, true); else if (nv == 2) ROWS(2, true); else ROWS(4, true); }
+        else if (nv == 1) ROWS(1, false); else if (nv == 2) ROWS(2, false); else if (nv == 4) ROWS(4, false); else if (nv == 8) ROWS(8, false); else ROWS(16, false);
 #undef ROWS
         return tb_launch_status();
     }
