@@ -322,6 +322,45 @@ def test_mamba2_prompts_do_not_depend_on_the_step(ops):
 
 
 
+@pytest.mark.parametrize("layer", ["mamba2", "gla"])
+def test_prompts_take_the_form_with_less_scratch_where_memory_is_short(ops, monkeypatch, layer):
+    """No memory for the states between the chunks: the recurrence, which needed little before and still does, to the
+    last bit."""
+    heads, lens = 8, [700, 40]
+    T, B = sum(lens), len(lens)
+    starts = torch.tensor([0, lens[0], T], dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).to("cuda", torch.int32)
+    slots, real = torch.arange(B, dtype=torch.int32, device="cuda"), torch.empty
+    if layer == "mamba2":
+        P = N = 64
+        inner, ch = heads * P, heads * P + 2 * N
+        proj, dt = rnd(T, inner + ch, dt=torch.bfloat16), rnd(T, heads, seed=1)
+        small = [rnd(ch, 4, s=0.3, seed=2), rnd(ch, s=0.1, seed=3), rnd(heads, seed=4) - 2, rnd(heads, s=0.5, seed=5), rnd(heads, seed=6)]
+        state, limit, at = torch.zeros(B, ops.mamba2_state_size(heads, P, N, 1, 4), device="cuda"), 7 * heads * P * N, "MAMBA2_PRODUCTS_FROM"
+        run = lambda: ops.mamba2(proj, dt, heads, P, N, 1, 4, 1, *small, torch.ones(inner, device="cuda"), 1e-6, state.zero_(), starts, seq, slots, B, False, 700)
+    else:
+        D, V = 128, 256
+        proj, low = rnd(T, 2 * heads * (D + V), dt=torch.bfloat16), rnd(1, T, 16, seed=1)
+        a2, bias = rnd(heads * D, 16, s=0.3, seed=2), rnd(heads * D, seed=3) + 2
+        state, limit, at = torch.zeros(B, heads * D * V, device="cuda"), 3 * heads * D * V, "GLA_BLOCKS_FROM"
+        run = lambda: ops.gla(proj, low, a2, bias, 8.0, D ** -0.5, torch.ones(V, device="cuda"), 1e-6, heads, D, V, state.zero_(), starts, seq, slots, B, 700)
+
+    def short(*size, **kw):                                              # (the chunks' states are asked for as one row of numbers)
+        if isinstance(size[0], int) and size[0] >= limit:
+            raise torch.OutOfMemoryError("none left")
+        return real(*size, **kw)
+    with monkeypatch.context() as m:
+        m.setattr(ops, at, 1 << 30)
+        scans = [run(), state.clone()]
+    with monkeypatch.context() as m:
+        m.setattr(torch, "empty", short)
+        got = [run(), state.clone()]
+    assert torch.equal(got[0], scans[0]) and torch.equal(got[1], scans[1])
+    run()
+    assert not torch.equal(state, scans[1])                              # with memory: the other form, whose sums are in another order
+
+
+
 def device_time(call, reps=20):
     """Least time of ``reps`` calls in a row, of five tries, in ms."""
     best = math.inf

@@ -730,6 +730,15 @@ MAMBA2_PRODUCTS_MEAN = 16           # ... and of the tokens a sequence, on avera
 MAMBA2_PRODUCTS_BYTES = 1 << 30     # ... as long as the states between the chunks (16 KB a token of the medium sizes) stay within this
 
 
+def _spare(n: int, device) -> Optional[torch.Tensor]:
+    """``n`` float32 numbers of scratch for a form that is only the faster one, or None where memory is too short for it
+    (the caller then takes the form that needs less)."""
+    try:
+        return torch.empty(n, dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 def mamba2_state_size(heads: int, P: int, N: int, groups: int, taps: int) -> int:
     """32-bit numbers of one sequence's state: S [heads, P, N], then the last taps-1 conv inputs [taps-1, channels]."""
     return heads * P * N + (taps - 1) * (heads * P + 2 * groups * N)
@@ -786,9 +795,10 @@ def mamba2(proj: torch.Tensor, dt_raw: torch.Tensor, heads: int, P: int, N: int,
         if not products:
             slots, per_slot = int(lib.tb_mamba2_chunk_slots(c_int(batch), c_int(T))), heads * P * N
             if slots * per_slot * 4 <= MAMBA2_PRODUCTS_BYTES:
-                scratch = torch.empty(slots * (per_slot + heads), dtype=torch.float32, device=proj.device)
-                a.chunk_state = scratch.data_ptr(); a.chunk_decay = a.chunk_state + slots * per_slot * 4
-                products = True
+                scratch = _spare(slots * (per_slot + heads), proj.device)
+                products = scratch is not None
+                if products:
+                    a.chunk_state = scratch.data_ptr(); a.chunk_decay = a.chunk_state + slots * per_slot * 4
         a.n_chunks = n_chunks if products else 0
     if not products and not one_token_each and max_seq_len > 0:
         chunk_len = c_int(0)
@@ -1563,12 +1573,13 @@ def gla(proj: torch.Tensor, low: torch.Tensor, a2: torch.Tensor, a2_bias: torch.
         # whole prompts in blocks; not where the chunks' states would take more than GLA_BLOCKS_BYTES
         chunk = int(lib.tb_gla_blocks_chunk(c_int(heads), c_int(batch), c_int(T), c_int(int(max_seq_len)), c_int(sm_count(proj.device))))
         n_chunks, slots = (max_seq_len + chunk - 1) // chunk, int(lib.tb_gla_blocks_slots(c_int(batch), c_int(T), c_int(chunk)))
-        if (n_chunks == 1 or slots * HD * value_dim * 4 <= GLA_BLOCKS_BYTES) and batch * n_chunks <= 65535 and rank <= 256:
+        per_slot, scratch = HD * value_dim, None
+        if n_chunks > 1 and slots * per_slot * 4 <= GLA_BLOCKS_BYTES:
+            scratch = _spare(slots * (per_slot + HD), proj.device)
+        if (n_chunks == 1 or scratch is not None) and batch * n_chunks <= 65535 and rank <= 256:
             a.chunk_len = chunk; a.n_chunks = n_chunks
-            if n_chunks > 1:
-                chunk_state = torch.empty((slots, HD * value_dim), dtype=torch.float32, device=proj.device)
-                chunk_decay = torch.empty((slots, HD), dtype=torch.float32, device=proj.device)
-                a.chunk_state = chunk_state.data_ptr(); a.chunk_decay = chunk_decay.data_ptr()
+            if scratch is not None:
+                a.chunk_state = scratch.data_ptr(); a.chunk_decay = a.chunk_state + slots * per_slot * 4
             _check(lib, lib.tb_gla_blocks(ctypes.byref(a), c_int(code(dt)), _stream()), "gla_blocks", 2 if n_chunks == 1 else 4)
             return out
     y = torch.empty((T, HV), dtype=torch.float32, device=proj.device)
