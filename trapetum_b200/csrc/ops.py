@@ -723,10 +723,13 @@ class _Mamba2Args(ctypes.Structure):
                 ("chunk_state", c_void_p), ("chunk_decay", c_void_p), ("chunk_len", c_int), ("n_chunks", c_int)]
 
 
-# Tokens of the longest prompt from which prompts run as products over chunks: 48 / 64 / 96 / 256 tokens take 30.2 / 31.2 /
-# 38.5 / 50.1 us, as a recurrence 30.7 / 36.5 / 52.3 / 111.9 (64 heads of 64 x 128)
-MAMBA2_PRODUCTS_FROM = 64
-MAMBA2_PRODUCTS_MEAN = 16           # ... and of the tokens a sequence, on average
+# Tokens of the longest prompt from which prompts run as products over chunks: one of 16 / 24 / 32 / 63 tokens takes 18.4 / 20.3 /
+# 20.5 / 23.9 us, as a recurrence 17.0 / 20.7 / 23.6 / 36.0 (64 heads of 64 x 128; 32 of 64 x 64: 11.6 / 12.8 / 12.9 / 15.3 and
+# 10.9 / 12.9 / 14.6 / 24.1)
+MAMBA2_PRODUCTS_FROM = 24
+# ... and of the tokens a sequence, on average: below, reading and writing the states is all there is (one of 64 tokens and 63 of 5:
+# 196 us, as a recurrence 144; four of 20: 25.3 and 26.3)
+MAMBA2_PRODUCTS_MEAN = 16
 MAMBA2_PRODUCTS_BYTES = 1 << 30     # ... as long as the states between the chunks (16 KB a token of the medium sizes) stay within this
 
 
