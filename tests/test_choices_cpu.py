@@ -83,6 +83,24 @@ def test_latent_decode_pieces_are_near_the_best_that_was_timed():
             assert 1 <= n <= 64 and (n == 1 or n * 32 <= rows)
 
 
+def test_every_way_of_cutting_latent_rows_has_a_test():
+    """The sizes of the GPU tests of decode attention over cached latents reach one, two, four and eight pieces that meet in a
+    cluster, and more that a launch folds."""
+    import ctypes
+
+    import test_gpu_kernels as gpu
+    from trapetum_b200.csrc import build
+    lib = build.load("attention_latent")
+    cases = [(c[0], c[1], min(c[4], c[5] + 31) if c[5] else c[4]) for c in gpu.LATENT_CLUSTERS + gpu.LATENT_FOLDED]
+    seen = set()
+    for i, (batch, heads, rows) in enumerate(cases):
+        n = lib.tb_latent_decode_pieces(*map(ctypes.c_int, (batch, heads, rows, 148)))
+        folds = bool(lib.tb_latent_decode_folds(*map(ctypes.c_int, (n, batch, heads))))
+        assert folds == (i >= len(gpu.LATENT_CLUSTERS))
+        seen.add("folds" if folds else n)
+    assert seen == {1, 2, 4, 8, "folds"}
+
+
 def test_the_gated_norm_of_few_tokens_uses_the_threads_there_are():
     """A step of few tokens is a chain of waits: 1,024 threads a row, one group of four columns each as long as that goes."""
     import ctypes

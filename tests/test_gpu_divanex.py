@@ -96,7 +96,7 @@ def test_head_norm_temperature_and_cache_write(H, G, d, every, dtype):
 @pytest.mark.parametrize("lens", [[37, 1, 18], [530, 1, 300]])
 @pytest.mark.parametrize("heads, P, N, groups, taps, ngroups", [(2, 16, 8, 2, 3, 2), (3, 24, 20, 1, 2, 3), (4, 32, 64, 2, 4, 1),
                                                                 (1, 8, 130, 1, 1, 1), (2, 40, 16, 1, 6, 4)])
-def test_state_space_mixer_between_its_products(heads, P, N, groups, taps, ngroups, lens, dtype):
+def test_state_space_mixer_between_its_products(monkeypatch, heads, P, N, groups, taps, ngroups, lens, dtype):
     """Convolution, recurrence and gated norm: prompts of unequal lengths in slots that are not in order, then three
     single tokens each, against the oracle's functions; the state is carried by the kernels.  The long prompts are cut
     into chunks that run side by side (the short one beside them is a single chunk)."""
@@ -141,6 +141,8 @@ def test_state_space_mixer_between_its_products(heads, P, N, groups, taps, ngrou
                           dev["A_log"], dev["D"], dev["norm"], eps, state, seq_start, token_seq, slots.to(DEV), len(step_lens),
                           one_each, max_seq_len=0 if one_each else max(step_lens))
 
+    ran, check = [], ops._check
+    monkeypatch.setattr(ops, "_check", lambda lib, status, what, kernels=1: (ran.append(what), check(lib, status, what, kernels))[1])
     tol = 2e-5 if dtype == "float32" else 3e-2
     for step in range(4):
         step_lens = lens if step == 0 else [1] * len(lens)
@@ -157,7 +159,10 @@ def test_state_space_mixer_between_its_products(heads, P, N, groups, taps, ngrou
     if max(lens) >= 256:
         chunk_len = __import__("ctypes").c_int(0)
         from trapetum_b200.csrc import build
-        assert build.load("mamba2").tb_mamba2_plan(heads, P, len(lens), max(lens), __import__("ctypes").byref(chunk_len)) > 1
+        lib = build.load("mamba2")
+        products = bool(lib.tb_mamba2_chunks_takes(ops.code(dt), heads, P, N, groups))       # whole pieces in bfloat16
+        assert ran.count("mamba2_prompts") == products and ran.count("mamba2_scan") == 4 - products
+        assert products or lib.tb_mamba2_plan(heads, P, len(lens), max(lens), __import__("ctypes").byref(chunk_len)) > 1
     assert bool((state[1] == 7.0).all()) and bool((state[3] == 0).all()) and bool((state[5] == 0).all())
     S = state[4, :heads * P * N].view(heads, P, N).double().cpu()
     assert float((S - ost[0]["S"].transpose(1, 2)).norm() / ost[0]["S"].norm()) <= tol

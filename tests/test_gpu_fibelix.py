@@ -197,6 +197,13 @@ def test_scores_mixed_across_heads_one_query_against_the_cache(H, G, D, seen, ri
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H, G, D, sink", [(2, 2, 33, True), (4, 1, 160, False), (1, 1, 511, True), (2, 1, 512, False)])
+def test_pieces_of_odd_and_large_heads_are_folded(H, G, D, sink, dtype):
+    """The folding launch where a head's numbers are odd, and where they are more than 128."""
+    test_scores_mixed_across_heads_one_query_against_the_cache(H, G, D, 0, 0, sink, dtype)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H, G, D, block", [(4, 2, 64, 64), (4, 1, 128, 100), (2, 2, 64, 5), (6, 3, 16, 33), (3, 1, 24, 70)])
 def test_blocks_on_the_decode_kernels(H, G, D, block, dtype):
     """The framework's decode kernels with a block in place of a window: lengths around the edges of blocks and pages."""

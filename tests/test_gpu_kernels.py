@@ -148,9 +148,20 @@ def test_gemm_simt_row_does_not_depend_on_the_batch(ops):
     assert torch.equal(full[17:18], one)
 
 
+def recorded(ops, monkeypatch):
+    """The names of the kernel entries that calls go through from here on."""
+    names, check = [], ops._check
+
+    def record(lib, status, what, kernels=1):
+        names.append(what)
+        return check(lib, status, what, kernels)
+    monkeypatch.setattr(ops, "_check", record)
+    return names
+
+
 @pytest.mark.parametrize("heads,P,N,groups,lens,span", [(2, 64, 128, 1, [128], 1.0), (3, 8, 8, 1, [65, 1, 7], 0.1), (4, 72, 40, 2, [129, 300], 1.0),
                                                         (2, 64, 64, 2, [3, 127, 513], 30.0), (1, 16, 120, 1, [64], 1e4)])
-def test_mamba2_prompts_as_products(ops, heads, P, N, groups, lens, span):
+def test_mamba2_prompts_as_products(ops, monkeypatch, heads, P, N, groups, lens, span):
     """The product form against the recurrence (which a step that does not say its longest prompt takes): the same
     convolution, so the states differ by the order of 32-bit sums (up to N + 128 terms and as many products, in rms
     about 1e-6) and the outputs by that and one bfloat16 rounding.  ``span``: how far the decays reach."""
@@ -162,11 +173,12 @@ def test_mamba2_prompts_as_products(ops, heads, P, N, groups, lens, span):
     starts = torch.tensor([sum(lens[:i]) for i in range(B + 1)], dtype=torch.int32, device="cuda")
     seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).to("cuda", torch.int32)
     slots = torch.arange(B, 0, -1, dtype=torch.int32, device="cuda")
-    got = []
+    got, ran = [], recorded(ops, monkeypatch)
     for longest in (0, max(lens)):
         state = first.clone()
         out = ops.mamba2(proj, dt, heads, P, N, groups, 4, 1, *small, norm, 1e-6, state, starts, seq, slots, B, False, longest)
         got.append((out.double(), state.double()))
+    assert ran.count("mamba2_scan") == 1 and ran.count("mamba2_prompts") == 1                       # each form once
     assert torch.equal(got[0][1][0], got[1][1][0])                       # a slot that is not in the step
     assert (got[1][1] - got[0][1]).norm() <= 3e-6 * got[0][1].norm()
     assert (got[1][0] - got[0][0]).norm() <= 3e-3 * got[0][0].norm()
@@ -234,22 +246,27 @@ def test_gla_prompts_in_blocks(ops, monkeypatch, heads, D, V, lens, span):
     starts = torch.tensor([sum(lens[:i]) for i in range(B + 1)], dtype=torch.int32, device="cuda")
     seq = torch.repeat_interleave(torch.arange(B), torch.tensor(lens)).to("cuda", torch.int32)
     slots = torch.arange(B, 0, -1, dtype=torch.int32, device="cuda")
-    got = []
+    got, ran = [], recorded(ops, monkeypatch)
     for longest in (0, max(lens)):
         state = first.clone()
         out = ops.gla(proj, low, a2, bias, 8.0 / span, D ** -0.5, norm, 1e-6, heads, D, V, state, starts, seq, slots, B, longest)
         got.append((out.double(), state.double()))
+    assert ran.count("gla_scan") == 1 and ran.count("gla_blocks") == 1                       # each form once
     assert torch.equal(got[0][1][0], got[1][1][0])                       # a slot that is not in the step
     assert (got[1][1] - got[0][1]).norm() <= 3e-6 * got[0][1].norm()
     assert (got[1][0] - got[0][0]).norm() <= 3e-3 * got[0][0].norm()
     assert torch.isfinite(got[1][0]).all()
 
 
-@pytest.mark.parametrize("B,heads,C,R,longest,window", [(1, 5, 64, 16, 33, 0), (1, 16, 448, 64, 700, 0), (3, 20, 96, 0, 500, 0), (8, 16, 512, 64, 900, 0),
-                                                        (40, 16, 128, 64, 300, 0), (40, 3, 448, 64, 640, 200), (2, 33, 512, 512, 130, 0)])
+# sequences, heads, latent, rotary, rows, window
+LATENT_CLUSTERS = [(1, 5, 64, 16, 33, 0), (1, 16, 448, 64, 700, 0), (3, 20, 96, 0, 500, 0), (8, 16, 512, 64, 900, 0),
+                   (40, 16, 128, 64, 300, 0), (40, 3, 448, 64, 640, 200), (2, 33, 512, 512, 130, 0)]
+
+
+@pytest.mark.parametrize("B,heads,C,R,longest,window", LATENT_CLUSTERS)
 def test_latent_decode_pieces(ops, B, heads, C, R, longest, window):
-    """Every way of cutting the keys (alone, clusters, the folding launch), heads and rows that fill no tile, one to two
-    tiles a ring.  The pool holds NaN wherever no key of the step lies.  Weights and result are rounded to bfloat16 once each."""
+    """Keys cut for clusters (alone, two, four, eight), heads and rows that fill no tile, one to two tiles a ring.  The pool
+    holds NaN wherever no key of the step lies.  Weights and result are rounded to bfloat16 once each."""
     KD, lens = C + R, [max(1, longest - 37 * b % longest) for b in range(B)]
     pages = (longest + PAGE - 1) // PAGE
     pool = torch.full((B * pages, 1, PAGE, KD), float("nan"), dtype=torch.bfloat16, device="cuda")
@@ -321,7 +338,6 @@ def test_mamba2_prompts_do_not_depend_on_the_step(ops):
         assert torch.equal(alone[0], out[sum(lens[:i]):sum(lens[:i + 1])]) and torch.equal(alone[1][0], state[i])
 
 
-
 @pytest.mark.parametrize("layer", ["mamba2", "gla"])
 def test_prompts_take_the_form_with_less_scratch_where_memory_is_short(ops, monkeypatch, layer):
     """No memory for the states between the chunks: the recurrence, which needed little before and still does, to the
@@ -358,7 +374,6 @@ def test_prompts_take_the_form_with_less_scratch_where_memory_is_short(ops, monk
     assert torch.equal(got[0], scans[0]) and torch.equal(got[1], scans[1])
     run()
     assert not torch.equal(state, scans[1])                              # with memory: the other form, whose sums are in another order
-
 
 
 def device_time(call, reps=20):
@@ -414,6 +429,39 @@ def test_gla_blocks_lose_nothing_in_the_state(ops, n, B, heads, bias):
         ops.gla(proj, low, a2, b2, 8.0, D ** -0.5, torch.ones(V, device="cuda"), 1e-6, heads, D, V, state, starts, seq, slots, B, longest)
         err.append(state_error(state.view(B, heads, D, V), S))
     assert err[1] <= 1.2 * err[0], err
+
+
+# sequences, heads, latent, rotary, bucket of rows, window, sink
+LATENT_FOLDED = [(1, 16, 448, 64, 4096, 0, True), (3, 16, 448, 64, 4096, 0, False), (8, 5, 64, 16, 8192, 0, True), (1, 33, 96, 32, 8192, 0, True),
+                 (40, 16, 448, 64, 2048, 0, True), (10, 16, 512, 64, 4096, 3000, False), (12, 20, 128, 0, 4096, 0, True)]
+
+
+@pytest.mark.parametrize("B,heads,C,R,bucket,window,has_sink", LATENT_FOLDED)
+def test_latent_decode_pieces_that_a_launch_folds(ops, monkeypatch, B, heads, C, R, bucket, window, has_sink):
+    """More pieces than a cluster takes, and contexts from one row up to the bucket's last: pieces without a key."""
+    KD, lens, ran = C + R, [[bucket, 1, bucket // 2, 33, 64, bucket - 31, 700][b % 7] for b in range(B)], []
+    pages = (bucket + PAGE - 1) // PAGE
+    pool = torch.full((B * pages, 1, PAGE, KD), float("nan"), dtype=torch.bfloat16, device="cuda")
+    table = torch.arange(B * pages, dtype=torch.int32, device="cuda").flip(0).view(B, pages).contiguous()
+    q, rows = rnd(B, heads * KD, dt=torch.bfloat16), rnd(B, bucket, KD, dt=torch.bfloat16, seed=2)
+    sink = rnd(heads, seed=1) if has_sink else None
+    want = torch.empty(B, heads * C, dtype=torch.float64, device="cuda")
+    for b, n in enumerate(lens):
+        first = max(0, n - window) if window else 0
+        view = pool[table[b].long()].reshape(-1, KD)
+        view[first:n] = rows[b, first:n]
+        pool[table[b].long()] = view.view(pages, 1, PAGE, KD)
+        k = rows[b, first:n].double()
+        s = q[b].double().view(heads, KD) @ k.T * 0.1
+        if has_sink:
+            s = torch.cat([s, sink.double()[:, None]], -1)
+        want[b] = (torch.softmax(s, -1)[:, :n - first] @ k[:, :C]).reshape(-1)
+    check = ops._check
+    monkeypatch.setattr(ops, "_check", lambda lib, status, what, kernels=1: (ran.append((what, kernels)), check(lib, status, what, kernels))[1])
+    got = ops.latent_decode(q, pool, table, torch.tensor(lens, dtype=torch.int32, device="cuda"), sink, heads, C, R, 0.1, bucket, window)
+    assert ran == [("latent_decode_mma", 2)]                             # (with the launch that folds)
+    assert (got.double() - want).norm() <= 4e-3 * want.norm()
+    assert ops.kernel_errors() == {}
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 17, 60), (9, 16, 2048), (16, 1100, 4100), (17, 63, 256), (65, 65, 2052), (70, 130, 8196)])
