@@ -979,7 +979,7 @@ def test_sample_draws_follow_the_inverse_cdf(ops, V, temperature, top_p):
 
 
 @pytest.mark.parametrize("V", [16384, 40001, 256000])
-@pytest.mark.parametrize("kind", ["equal", "three values", "masked", "flat", "spike"])
+@pytest.mark.parametrize("kind", ["equal", "three values", "masked", "flat", "spike", "narrow", "two zeros", "neighbours"])
 def test_sample_where_logits_crowd(ops, V, kind):
     """Rows whose threshold falls among more elements than a row lists (equal logits), that hold -inf, whose logits lie
     close together, or one far above the rest; tokens as the float64 nucleus in index order gives them."""
@@ -993,14 +993,24 @@ def test_sample_where_logits_crowd(ops, V, kind):
         x[:, V // 50:] = -math.inf
     elif kind == "flat":
         x *= 1e-3
-    else:
+    elif kind == "spike":
         x = (x * 1e-2)
         x[:, V // 3] = 10.0
+    elif kind == "narrow":                                              # the bulk in one or two of the steps of the row's range
+        x = (x * 1e-4)
+        x[:, V // 3] = 8.0
+    elif kind == "two zeros":                                           # many of 0, half of them -0, the next lower key
+        x = torch.round(x / 4.0)
+    else:                                                               # thousands each of four numbers that the row's range cannot tell apart
+        x = 1.0 + torch.remainder(torch.arange(V, device="cuda") * 7919, 4).float().expand(rows, V) * 2.0 ** -23
+        x[:, V // 3] = 8.0
     u = torch.linspace(0.001, 0.999, rows)
     t, p, pen, ud = _args(rows, 0.9, 0.6, 1.0, u)
     got = ops.sample(x.clone(), t, p, pen, ud, None).cpu().tolist()
     for i in range(rows):
         row = x[i].double().cpu()
+        if kind == "two zeros":
+            row = torch.where((row == 0) & torch.signbit(row), torch.full_like(row, -1e-30), row)
         m = torch.exp((row - row.max()) / 0.9)
         order = torch.sort(row, descending=True).values                  # equal logits are kept or left together, by their value
         cum = torch.cumsum(torch.exp((order - row.max()) / 0.9), 0)
@@ -1010,6 +1020,18 @@ def test_sample_where_logits_crowd(ops, V, kind):
         tok = got[i]
         assert m[tok] > 0, "a token outside the nucleus was drawn"
         assert float(cdf[tok] - m[tok] / m.sum()) - 1e-4 <= float(u[i]) <= float(cdf[tok]) + 1e-4
+
+
+@pytest.mark.parametrize("rows, V", [(4, 32768), (4, 256000), (32, 256000)])
+def test_sample_takes_about_as_long_where_logits_crowd(ops, rows, V):
+    """Rows with too many elements in the threshold's step to list: within three times the time of ordinary rows (up to
+    24 times before; 1.2 to 2.0 measured)."""
+    ordinary = rnd(rows, V, s=2.0, seed=V)
+    narrow = ordinary * 1e-3
+    narrow[:, V // 3] = 8.0
+    t, p, pen, u = _args(rows, 0.8, 0.95, 1.0, torch.linspace(0.1, 0.9, rows))
+    times = [device_time(lambda: ops.sample(x, t, p, pen, u, None)) for x in (ordinary, narrow, torch.round(ordinary) / 2)]
+    assert max(times[1:]) <= 3.0 * times[0], times
 
 
 @pytest.mark.parametrize("V", [500, 20011])

@@ -21,7 +21,10 @@
 //              wall clock; here the caller owns the generator, so a run repeats.
 //
 // All sums are 32-bit and taken in a fixed order.
+#include <cooperative_groups.h>
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 TB_EXPORT_ERROR()
 
@@ -238,21 +241,26 @@ __global__ void __launch_bounds__(1024) sample_kernel(SampleArgs a) {
 //                     clears the row's histogram
 //   sample_hist       per chunk: mass per step; the row's last CTA finds the threshold's  [rows with a nucleus only]
 //   sample_chunk_mass per chunk: mass of the elements above the threshold's step; lists those in it (without a nucleus:
-//                     mass of all)
-//   sample_pick       per row: the threshold from the listed elements (from the row itself if they are too many: equal
-//                     logits), their kept masses added to their chunks', target = u x kept mass; the chunk and then the
-//                     element at which the running sum of kept masses, in index order, passes the target
-// 256,000 logits, top_p 0.95, in a graph: 38 / 45 / 63 / 94 us for 1 / 8 / 32 / 64 rows; six launches that read the row five
-// times (three histograms over the key's digits) took 45 / 76 / 96 / 156.
+//                     mass of all).  A step of too many to list (CROWDED: equal or coarse logits, or a bulk narrower than a
+//                     thousandth of the row's range beside one far above it) is cut into 512 parts: mass per part and chunk
+//   sample_pick       per row: the threshold from the listed elements, their kept masses added to their chunks', target = u x
+//                     kept mass; the chunk and then the element at which the running sum of kept masses, in index order,
+//                     passes the target.  A crowded row's cluster of CTAs reads it once more, for the elements of the
+//                     threshold's part; if those are too many to list too, they are one number, or 0 and -0, or (a few
+//                     neighbouring numbers, thousands of each) the CTAs search the row by the key's digits
+// 256,000 logits, top_p 0.95, in a graph: 36 / 44 / 93 us for 1 / 8 / 64 rows; six launches that read the row five times (three
+// histograms over the key's digits) took 41 / 73 / 154.  A bulk of 0.002 beside an outlier of 8: 57 / 78 / 208 (39 / 72 / 148).
 // ---------------------------------------------------------------------------
 #define S_CHUNK 8192
 #define S_BINS 2048
-#define S_LIST 4096               // elements of the threshold's step that are listed
+#define S_PARTS 512               // parts of a crowded step
+#define S_LIST 4096               // elements of the threshold's step, or part, that are listed
 typedef unsigned long long u64;
 
 struct SampleState {              // per row with a nucleus, left by sample_hist
     u64 want;                     // what the elements of the threshold's step have to reach
     int edge;                     // the threshold's step; S_BINS: there are no masses, everything is kept
+    int crowded;                  // it may hold more elements (of a mass) than are listed
 };
 
 struct SampleWide {
@@ -261,11 +269,11 @@ struct SampleWide {
     int vec;                      // rows start on 16-byte boundaries
     float* pmax; float* pmin; int* pidx;   // [rows][n_chunks]
     u64* hist;                    // [rows][S_BINS]
+    u64* inner;                   // [rows][n_chunks][S_PARTS] of a crowded row: masses within the threshold's step
     u64* cmass;                   // [rows][n_chunks] mass above the threshold's step
-    u64* emass;                   // [rows][n_chunks] mass in it
     SampleState* state;           // [rows]
     int* done;                    // [rows] CTAs of sample_hist that have added their masses
-    int* count;                   // [rows] listed elements (those that would be, if they are too many)
+    int* count;                   // [rows] listed elements (of a crowded row: those that would be, if they are too many)
     int* list;                    // [rows][S_LIST] their places
 };
 
@@ -319,6 +327,12 @@ __device__ __forceinline__ int step_of(const Steps& s, float l) {
     const float x = (s.mx - l) * s.invT;
     if (x < 23.f) return min((int)(x * s.scale), S_BINS - 1);
     return x >= 23.f ? -1 : -2;
+}
+// the place of a logit within its step, in parts: the remainder of step_of's product, rounded as there (a fused
+// multiply-add would not be, and two kernels have to agree)
+__device__ __forceinline__ int part_of(const Steps& s, float l, int step) {
+    const float t = __fmul_rn((s.mx - l) * s.invT, s.scale);
+    return min((int)(__fsub_rn(t, (float)step) * (float)S_PARTS), S_PARTS - 1);
 }
 
 __global__ void __launch_bounds__(256) sample_chunk_max_kernel(SampleWide w) {
@@ -418,6 +432,19 @@ __device__ __forceinline__ void add_mass(unsigned* lo, unsigned* hi, int entry, 
     atomicAdd(&hi[entry], (unsigned)(m >> 16));
 }
 
+// The same by a whole warp, an entry a lane (-1: none): an entry that all of them share is added to once (equal logits, or
+// digits that a step's elements have in common: their additions would wait for one another).
+__device__ __forceinline__ void add_mass_of_warp(unsigned* lo, unsigned* hi, int entry, u64 m) {
+    const unsigned in = __ballot_sync(0xffffffffu, entry >= 0);
+    if (in == 0u) return;
+    const int first = __shfl_sync(0xffffffffu, entry, __ffs(in) - 1);
+    if (__all_sync(0xffffffffu, entry < 0 || entry == first)) {
+        const unsigned a = __reduce_add_sync(0xffffffffu, entry >= 0 ? (unsigned)(m & 0xffffu) : 0u);
+        const unsigned b = __reduce_add_sync(0xffffffffu, entry >= 0 ? (unsigned)(m >> 16) : 0u);
+        if ((threadIdx.x & 31) == 0) { atomicAdd(&lo[first], a); atomicAdd(&hi[first], b); }
+    } else if (entry >= 0) add_mass(lo, hi, entry, m);
+}
+
 __global__ void __launch_bounds__(256) sample_hist_kernel(SampleWide w) {
     pdl_launch_dependents();
     pdl_wait();
@@ -459,32 +486,53 @@ __global__ void __launch_bounds__(256) sample_hist_kernel(SampleWide w) {
     if (threadIdx.x == 0) {
         w.state[row].want = s_at.total - s_at.before;
         w.state[row].edge = s_at.total > 0ull ? s_at.entry : S_BINS;
+        // no element of the step that has a mass has less than one at the end of the step after it
+        const u64 least = st.scale > 0.f ? __float2ull_rn(expf(-(float)(s_at.entry + 2) / st.scale) * 4294967296.0f) : 1ull;
+        w.state[row].crowded = g[s_at.entry] / (least > 0ull ? least : 1ull) > (u64)S_LIST;
     }
 }
 
 __global__ void __launch_bounds__(256) sample_chunk_mass_kernel(SampleWide w, int nucleus) {
     pdl_launch_dependents();
     pdl_wait();
-    __shared__ u64 red8[16];
+    __shared__ u64 red8[8];
     __shared__ float red[33];
+    __shared__ unsigned lo[S_PARTS], hi[S_PARTS];
     const int row = blockIdx.y, chunk = blockIdx.x, lane = threadIdx.x & 31;
     const float T = w.a.temperature ? w.a.temperature[row] : 0.f;
     if (!(T > 0.f)) return;
     const int edge = nucleus && row_has_nucleus(w.a, row) ? w.state[row].edge : S_BINS;
+    const bool crowded = edge < S_BINS && w.state[row].crowded;
+    if (crowded)
+        for (int i = threadIdx.x; i < S_PARTS; i += 256) lo[i] = hi[i] = 0u;
     float mx, mn;
-    row_range(w, row, red, mx, mn);
+    row_range(w, row, red, mx, mn);                                 // (has the barriers that the zeros need)
     const Steps st = row_steps(mx, mn, T);
     const float* x = w.a.logits + (size_t)row * w.a.row_stride;
-    u64 m = 0ull, in_edge = 0ull;
+    u64 m = 0ull;
     if (edge == S_BINS) {                                           // everything is kept
         each_of_chunk(w, x, chunk, [&](float l, int) { m += fixed_mass(l, st.mx, st.invT); });
+    } else if (crowded) {
+        const bool whole = w.vec && (chunk + 1) * S_CHUNK <= w.a.vocab;       // every lane has every element
+        each_of_chunk(w, x, chunk, [&](float l, int) {
+            const int e = step_of(st, l);
+            const u64 f = e >= 0 && e <= edge ? fixed_mass(l, st.mx, st.invT) : 0ull;
+            int p = -1;
+            if (f > 0ull) { if (e < edge) m += f; else p = part_of(st, l, edge); }
+            if (whole) add_mass_of_warp(lo, hi, p, f);
+            else if (p >= 0) add_mass(lo, hi, p, f);
+        });
+        __syncthreads();
+        for (int i = threadIdx.x; i < S_PARTS; i += 256) w.inner[((size_t)row * w.n_chunks + chunk) * S_PARTS + i] = (u64)lo[i] + ((u64)hi[i] << 16);
     } else {
-        unsigned hits = 0u;                                         // which of this thread's elements lie in the threshold's step
+        unsigned hits = 0u;                                         // which of this thread's elements lie in the threshold's step (and have a mass)
         int k = 0;
         const bool vec = each_of_chunk(w, x, chunk, [&](float l, int) {
             const int e = step_of(st, l);
-            if (e >= 0 && e <= edge) { const u64 f = fixed_mass(l, st.mx, st.invT); if (e < edge) m += f; else in_edge += f; }
-            hits |= (unsigned)(e == edge) << k;
+            if (e >= 0 && e <= edge) {
+                const u64 f = fixed_mass(l, st.mx, st.invT);
+                if (e < edge) m += f; else hits |= (unsigned)(f > 0ull) << k;
+            }
             k++;
         });
         // their places go to the row's list, one atomic a warp
@@ -498,13 +546,13 @@ __global__ void __launch_bounds__(256) sample_chunk_mass_kernel(SampleWide w, in
             if (base < S_LIST) w.list[(size_t)row * S_LIST + base] = chunk * S_CHUNK + (vec ? ((u >> 2) * 256 + threadIdx.x) * 4 + (u & 3) : u * 256 + threadIdx.x);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) { m += __shfl_xor_sync(0xffffffffu, m, o); in_edge += __shfl_xor_sync(0xffffffffu, in_edge, o); }
-    if (lane == 0) { red8[threadIdx.x >> 5] = m; red8[8 + (threadIdx.x >> 5)] = in_edge; }
+    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+    if (lane == 0) red8[threadIdx.x >> 5] = m;
     __syncthreads();
-    if (threadIdx.x < 2) {
+    if (threadIdx.x == 0) {
         u64 t = 0ull;
-        for (int k = 0; k < 8; k++) t += red8[threadIdx.x * 8 + k];
-        (threadIdx.x ? w.emass : w.cmass)[(size_t)row * w.n_chunks + chunk] = t;
+        for (int k = 0; k < 8; k++) t += red8[k];
+        w.cmass[(size_t)row * w.n_chunks + chunk] = t;
     }
 }
 
@@ -515,7 +563,19 @@ __device__ __forceinline__ bool digit_of(int R, unsigned key, unsigned prefix, i
     bin = key & 1023; return (key >> 10) == prefix;
 }
 
-__global__ void __launch_bounds__(512) sample_pick_kernel(SampleWide w, int nucleus) {
+// f(logit, whether it is one) for the elements lo .. hi - 1, whole warps at a time, eight loads of a thread on their way.
+template <int THREADS, typename F>
+__device__ __forceinline__ void each_of_range(const float* x, int lo, int hi, F&& f) {
+    for (int i = lo; i < hi; i += 8 * THREADS) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) { const int k = i + u * THREADS + (int)threadIdx.x; v[u] = k < hi ? x[k] : 0.f; }
+#pragma unroll
+        for (int u = 0; u < 8; u++) if (i + u * THREADS < hi) f(v[u], i + u * THREADS + (int)threadIdx.x < hi);
+    }
+}
+
+__global__ void __launch_bounds__(512, 1) sample_pick_kernel(SampleWide w, int nucleus) {
     pdl_launch_dependents();
     pdl_wait();
     constexpr int THREADS = 512, PER = S_CHUNK / THREADS;            // consecutive elements per thread: index order
@@ -526,9 +586,12 @@ __global__ void __launch_bounds__(512) sample_pick_kernel(SampleWide w, int nucl
     __shared__ float red[33];
     __shared__ int s_chunk;
     __shared__ u64 s_base, s_target;
-    const int row = blockIdx.x, tid = threadIdx.x;
+    const int row = blockIdx.y, tid = threadIdx.x, rank = blockIdx.x, ctas = gridDim.x;
     const SampleArgs& a = w.a;
     const float T = a.temperature ? a.temperature[row] : 0.f;
+    const bool has_edge = nucleus && row_has_nucleus(a, row) && w.state[row].edge < S_BINS;
+    const bool crowded = has_edge && w.state[row].crowded;
+    if (rank > 0 && !crowded) return;                               // (a cluster for the crowded rows)
     if (!(T > 0.f)) {
         // greedy: the best of the chunk maxima, the smallest index on a tie
         if (tid == 0) {
@@ -548,89 +611,186 @@ __global__ void __launch_bounds__(512) sample_pick_kernel(SampleWide w, int nucl
     const Steps st = row_steps(mx, mn, T);
     const float invT = st.invT;
     unsigned thr = 0u;
-    if (nucleus && row_has_nucleus(a, row)) {
-        const int edge = w.state[row].edge, n = w.count[row];
+    if (has_edge) {
+        const int edge = w.state[row].edge;
         u64 want = w.state[row].want;
-        const bool listed = n <= S_LIST;
-        if (edge < S_BINS) {
-            unsigned prefix = 0u;
-            unsigned* lo = (unsigned*)g;
-            unsigned* hi = lo + S_BINS;
-            bool one_key = false;                                   // too many to list: most likely equal logits, whose key needs no search
-            if (!listed) {
-                float top = -INFINITY, low = INFINITY;
-                auto see = [&](float l) { if (step_of(st, l) == edge) { top = fmaxf(top, l); low = fminf(low, l); } };
-                const int quads = w.vec ? a.vocab / 4 : 0;
-#pragma unroll 8
-                for (int i = tid; i < quads; i += THREADS) {
-                    const float4 l = *(const float4*)(x + 4 * i);
-                    see(l.x); see(l.y); see(l.z); see(l.w);
-                }
-                for (int i = 4 * quads + tid; i < a.vocab; i += THREADS) see(x[i]);
-                top = block_max(top, red);
-                low = -block_max(-low, red);
-                one_key = top == low && top != 0.f;                 // (0 and -0 are two keys)
-                prefix = f2key(top);
-            }
-            for (int R = one_key ? 3 : 0; R < 3; R++) {
-                if (R == 0) prefix = 0u;
-                u64 m[S_BINS / THREADS];
+        unsigned* lo = (unsigned*)g;
+        unsigned* hi = lo + S_BINS;
+        auto clear = [&]() {
+            __syncthreads();
+            for (int i = tid; i < 2 * S_BINS; i += THREADS) lo[i] = 0u;
+            __syncthreads();
+        };
+        auto collect = [&](u64* m) {                                // the two halves of the sums
+            __syncthreads();
 #pragma unroll
-                for (int u = 0; u < S_BINS / THREADS; u++) m[u] = 0ull;
-                const int total = listed ? n : a.vocab;
-                for (int i0 = 0; i0 < total; i0 += S_MOST_CHUNKS * S_CHUNK) {
-                    const int i1 = min(total, i0 + S_MOST_CHUNKS * S_CHUNK);
-                    __syncthreads();
-                    for (int i = tid; i < 2 * S_BINS; i += THREADS) lo[i] = 0u;
-                    __syncthreads();
-                    if (listed) {
-                        for (int k = i0 + tid; k < i1; k += THREADS) {
-                            const float l = x[w.list[(size_t)row * S_LIST + k]];
-                            int bin;
-                            if (digit_of(R, f2key(l), prefix, bin)) add_mass(lo, hi, bin, fixed_mass(l, mx, invT));
-                        }
-                    } else {
-                        for (int k = i0; k < i1; k += THREADS) {    // (whole warps: a warp whose elements share a digit adds once)
-                            const float l = k + tid < i1 ? x[k + tid] : 0.f;
-                            int bin = -1;
-                            if (k + tid >= i1 || step_of(st, l) != edge || !digit_of(R, f2key(l), prefix, bin)) bin = -1;
-                            u64 add = bin >= 0 ? fixed_mass(l, mx, invT) : 0ull;
-                            if (__all_sync(0xffffffffu, bin == __shfl_sync(0xffffffffu, bin, 0))) {
-                                for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
-                                if ((tid & 31) != 0) bin = -1;
-                            }
-                            if (bin >= 0) add_mass(lo, hi, bin, add);
+            for (int u = 0; u < S_BINS / THREADS; u++) m[u] += (u64)lo[tid + u * THREADS] + ((u64)hi[tid + u * THREADS] << 16);
+            __syncthreads();
+        };
+        auto advance = [&](int R) {
+            want -= s_at.before;
+            thr = (R == 0) ? (unsigned)s_at.entry : (R == 1) ? ((thr << 11) | (unsigned)s_at.entry) : ((thr << 10) | (unsigned)s_at.entry);
+        };
+        int n = 0;
+        if (!crowded) n = w.count[row];
+        else {
+            __shared__ u64 total[S_BINS];
+            __shared__ u64 from_all[256];                           // first CTA: a number per chunk, from the CTA that has it
+            __shared__ unsigned s_least, s_most;                    // first CTA: the keys of the threshold's part
+            __shared__ int s_many;
+            cg::cluster_group cluster = cg::this_cluster();
+            const int per = (w.n_chunks + ctas - 1) / ctas, c0 = min(w.n_chunks, rank * per), c1 = min(w.n_chunks, c0 + per), lane = tid & 31;
+            const u64* inner = w.inner + (size_t)row * w.n_chunks * S_PARTS;
+            for (int i = tid; i < S_BINS; i += THREADS) {
+                u64 sum = 0ull;
+                if (i < S_PARTS) for (int c = 0; c < w.n_chunks; c++) sum += inner[(size_t)c * S_PARTS + i];
+                total[i] = sum;
+            }
+            if (tid == 0) { s_least = 0xffffffffu; s_most = 0u; s_many = 0; }
+            if (tid < c1 - c0) g[tid] = 0ull;
+            __syncthreads();
+            find_entry(total, part, &s_at, false, want, 0.f);
+            want -= s_at.before;
+            const int level = s_at.entry;
+            if (rank == 0)                                          // what lies above the part is kept
+                for (int c = tid >> 5; c < w.n_chunks; c += THREADS / 32) {
+                    u64 add = 0ull;
+                    for (int i = lane; i < level; i += 32) add += inner[(size_t)c * S_PARTS + i];
+                    for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+                    if (lane == 0) cm[c] += add;
+                }
+            // the part's elements of this CTA's chunks: to the list, until there are too many; the mass of those that are +0
+            const float from = (float)edge + (float)level / S_PARTS;          // (exact)
+            const float to = edge == S_BINS - 1 && level == S_PARTS - 1 ? INFINITY : (float)edge + (float)(level + 1) / S_PARTS;
+            unsigned least = 0xffffffffu, most = 0u;
+            float v[PER], next[PER];
+            auto fetch = [&](int c) {
+#pragma unroll
+                for (int u = 0; u < PER; u++) {
+                    const int i = c * S_CHUNK + u * THREADS + tid;
+                    next[u] = c < c1 && i < a.vocab ? x[i] : 0.f;
+                }
+            };
+            fetch(c0);
+            for (int c = c0; c < c1; c++) {
+#pragma unroll
+                for (int u = 0; u < PER; u++) v[u] = next[u];
+                fetch(c + 1);
+                u64 zeros = 0ull;
+#pragma unroll
+                for (int u = 0; u < PER; u++) {
+                    const float d = (mx - v[u]) * invT, t = __fmul_rn(d, st.scale);
+                    const int i = c * S_CHUNK + u * THREADS + tid;
+                    u64 f = 0ull;
+                    if (i < a.vocab && d < 23.f && t >= from && t < to) {
+                        f = fixed_mass(v[u], mx, invT);
+                        if (f) {
+                            const unsigned key = f2key(v[u]);
+                            least = min(least, key); most = max(most, key);
+                            if (key == 0x80000000u) zeros += f;
                         }
                     }
-                    __syncthreads();
-#pragma unroll
-                    for (int u = 0; u < S_BINS / THREADS; u++) m[u] += (u64)lo[tid + u * THREADS] + ((u64)hi[tid + u * THREADS] << 16);
+                    const unsigned hit = __ballot_sync(0xffffffffu, f > 0ull);
+                    if (hit == 0u) continue;
+                    int at = 0;
+                    if (lane == 0) at = *(volatile int*)&s_many ? S_LIST : atomicAdd(&w.count[row], __popc(hit));
+                    at = __shfl_sync(0xffffffffu, at, 0) + __popc(hit & ((1u << lane) - 1u));
+                    if (f && at < S_LIST) w.list[(size_t)row * S_LIST + at] = i;
+                    if (at >= S_LIST) *(volatile int*)&s_many = 1;
                 }
-                __syncthreads();
+                if (__any_sync(0xffffffffu, zeros > 0ull)) {
+                    for (int o = 16; o > 0; o >>= 1) zeros += __shfl_xor_sync(0xffffffffu, zeros, o);
+                    if (lane == 0) atomicAdd(&g[c - c0], zeros);
+                }
+            }
+            cluster.sync();                                         // (the first CTA's numbers are set up; this one's zeros are added)
+            least = __reduce_min_sync(0xffffffffu, least); most = __reduce_max_sync(0xffffffffu, most);
+            if (lane == 0) { atomicMin(cluster.map_shared_rank(&s_least, 0), least); atomicMax(cluster.map_shared_rank(&s_most, 0), most); }
+            if (tid < c1 - c0) cluster.map_shared_rank(from_all, 0)[c0 + tid] = g[tid];
+            __threadfence();
+            cluster.sync();                                         // all of it is there
+            n = __ldcg(&w.count[row]);
+            if (n > S_LIST) {
+                least = *cluster.map_shared_rank(&s_least, 0); most = *cluster.map_shared_rank(&s_most, 0);
+                cluster.sync();
+                if (least == most || (least == 0x7fffffffu && most == 0x80000000u)) {
+                    if (rank > 0) return;
+                    u64 upper = 0ull;                               // one number; or -0 and +0, the next higher key
+                    if (least != most) for (int c = 0; c < w.n_chunks; c++) upper += from_all[c];
+                    thr = least == most || upper < want ? least : most;
+                    for (int c = tid; c < w.n_chunks; c += THREADS) cm[c] += thr == least ? inner[(size_t)c * S_PARTS + level] : from_all[c];
+                    __syncthreads();
+                } else {
+                    for (int R = 0; R < 3; R++) {
+                        u64 m[S_BINS / THREADS] = {};
+                        for (int c = c0; c < c1; c += S_MOST_CHUNKS) {
+                            clear();
+                            each_of_range<THREADS>(x, c * S_CHUNK, min(a.vocab, min(c1, c + S_MOST_CHUNKS) * S_CHUNK), [&](float l, bool in) {
+                                int bin = -1;
+                                if (!in || step_of(st, l) != edge || part_of(st, l, edge) != level || !digit_of(R, f2key(l), thr, bin)) bin = -1;
+                                add_mass_of_warp(lo, hi, bin, bin >= 0 ? fixed_mass(l, mx, invT) : 0ull);
+                            });
+                            collect(m);
+                        }
+#pragma unroll
+                        for (int u = 0; u < S_BINS / THREADS; u++) g[tid + u * THREADS] = m[u];
+                        cluster.sync();
+                        for (int i = tid; i < S_BINS / ctas; i += THREADS) {      // the sums of a share of the entries, for every CTA
+                            const int e = rank * (S_BINS / ctas) + i;
+                            u64 sum = 0ull;
+                            for (int k = 0; k < ctas; k++) sum += cluster.map_shared_rank(g, k)[e];
+                            for (int k = 0; k < ctas; k++) cluster.map_shared_rank(total, k)[e] = sum;
+                        }
+                        cluster.sync();
+                        find_entry(total, part, &s_at, true, want, 0.f);
+                        advance(R);
+                    }
+                    for (int c = c0; c < c1; c++) {
+                        u64 add = 0ull;
+                        each_of_range<THREADS>(x, c * S_CHUNK, min(a.vocab, (c + 1) * S_CHUNK), [&](float l, bool in) {
+                            if (in && step_of(st, l) == edge && part_of(st, l, edge) == level && f2key(l) >= thr) add += fixed_mass(l, mx, invT);
+                        });
+                        __syncthreads();
+                        if (tid == 0) g[0] = 0ull;
+                        __syncthreads();
+                        for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+                        if (lane == 0 && add) atomicAdd(&g[0], add);
+                        __syncthreads();
+                        if (tid == 0) cluster.map_shared_rank(from_all, 0)[c] = g[0];
+                    }
+                    cluster.sync();
+                    if (rank == 0) for (int c = tid; c < w.n_chunks; c += THREADS) cm[c] += from_all[c];
+                    __syncthreads();
+                }
+            }
+            if (rank > 0) return;
+        }
+        if (n <= S_LIST) {
+            const int* list = w.list + (size_t)row * S_LIST;
+            for (int R = 0; R < 3; R++) {
+                u64 m[S_BINS / THREADS] = {};
+                clear();
+                for (int k = tid; k < (n + 31) / 32 * 32; k += THREADS) {         // (whole warps)
+                    const float l = k < n ? x[__ldcg(&list[k])] : 0.f;
+                    int bin;
+                    if (k >= n || !digit_of(R, f2key(l), thr, bin)) bin = -1;
+                    add_mass_of_warp(lo, hi, bin, bin >= 0 ? fixed_mass(l, mx, invT) : 0ull);
+                }
+                collect(m);
 #pragma unroll
                 for (int u = 0; u < S_BINS / THREADS; u++) g[tid + u * THREADS] = m[u];
                 __syncthreads();
                 find_entry(g, part, &s_at, true, want, 0.f);
-                want -= s_at.before;
-                prefix = (R == 0) ? (unsigned)s_at.entry : (R == 1) ? ((prefix << 11) | (unsigned)s_at.entry) : ((prefix << 10) | (unsigned)s_at.entry);
+                advance(R);
             }
-            thr = prefix;
-            if (listed) {
-                for (int k = tid; k < n; k += THREADS) {
-                    const int i = w.list[(size_t)row * S_LIST + k];
-                    if (f2key(x[i]) >= thr) atomicAdd(&cm[i / S_CHUNK], fixed_mass(x[i], mx, invT));
-                }
-            } else if (one_key) {
-                for (int c = tid; c < w.n_chunks; c += THREADS) cm[c] += w.emass[(size_t)row * w.n_chunks + c];
-            } else {
-                for (int c = tid >> 5; c < w.n_chunks; c += THREADS / 32) {         // a warp a chunk
-                    u64 add = 0ull;
-                    for (int i = c * S_CHUNK + (tid & 31); i < min(a.vocab, (c + 1) * S_CHUNK); i += 32)
-                        if (step_of(st, x[i]) == edge && f2key(x[i]) >= thr) add += fixed_mass(x[i], mx, invT);
-                    for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
-                    if ((tid & 31) == 0) cm[c] += add;
-                }
+            clear();
+            for (int k = tid; k < (n + 31) / 32 * 32; k += THREADS) {
+                const int i = k < n ? __ldcg(&list[k]) : 0;
+                const bool kept = k < n && f2key(x[i]) >= thr;
+                add_mass_of_warp(lo, hi, kept ? i / S_CHUNK : -1, kept ? fixed_mass(x[i], mx, invT) : 0ull);
             }
+            __syncthreads();
+            for (int c = tid; c < w.n_chunks; c += THREADS) cm[c] += (u64)lo[c] + ((u64)hi[c] << 16);
             __syncthreads();
         }
     }
@@ -684,7 +844,7 @@ __global__ void __launch_bounds__(512) sample_pick_kernel(SampleWide w, int nucl
 
 extern "C" long long tb_sample_wide_scratch_bytes(int rows, int vocab) {
     const long long chunks = (vocab + S_CHUNK - 1) / S_CHUNK;
-    return (long long)rows * (chunks * (4 + 4 + 4 + 8 + 8) + S_BINS * 8LL + (long long)sizeof(SampleState) + (2 + S_LIST) * 4LL) + 256;
+    return (long long)rows * (chunks * (4 + 4 + 4 + 8) + S_BINS * 8LL + chunks * S_PARTS * 8LL + (long long)sizeof(SampleState) + (2 + S_LIST) * 4LL) + 256;
 }
 
 // `nucleus`: 0 if the caller knows that every row has top_p >= 1 (the threshold's launch is then not made).
@@ -701,8 +861,8 @@ extern "C" int tb_sample_wide(const SampleArgs* args, int rows, void* scratch, i
     w.vec = ((uintptr_t)w.a.logits & 15) == 0 && w.a.row_stride % 4 == 0;
     char* p = (char*)scratch;
     w.hist = (u64*)p; p += (size_t)rows * S_BINS * 8;
+    w.inner = (u64*)p; p += (size_t)rows * w.n_chunks * S_PARTS * 8;
     w.cmass = (u64*)p; p += (size_t)rows * w.n_chunks * 8;
-    w.emass = (u64*)p; p += (size_t)rows * w.n_chunks * 8;
     w.state = (SampleState*)p; p += (size_t)rows * sizeof(SampleState);
     w.pmax = (float*)p; p += (size_t)rows * w.n_chunks * 4;
     w.pmin = (float*)p; p += (size_t)rows * w.n_chunks * 4;
@@ -714,7 +874,16 @@ extern "C" int tb_sample_wide(const SampleArgs* args, int rows, void* scratch, i
     tb_launch(sample_chunk_max_kernel, dim3(per_chunk), dim3(256), 0, stream, w);
     if (nucleus) tb_launch(sample_hist_kernel, dim3(per_chunk), dim3(256), 0, stream, w);
     tb_launch(sample_chunk_mass_kernel, dim3(per_chunk), dim3(256), 0, stream, w, nucleus);
-    tb_launch(sample_pick_kernel, dim3(rows), dim3(512), 0, stream, w, nucleus);
+    cudaLaunchConfig_t cfg = {};
+    // CTAs of a row's cluster, for crowded rows (the others' all leave but one): as many as leave no row waiting
+    cfg.gridDim = dim3(!nucleus ? 1 : rows <= 18 ? 8 : rows <= 36 ? 4 : rows <= 72 ? 2 : 1, rows); cfg.blockDim = dim3(512); cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cfg.gridDim.x; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, sample_pick_kernel, w, nucleus);
     return tb_launch_status();
 }
 
