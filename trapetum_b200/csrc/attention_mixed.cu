@@ -274,7 +274,7 @@ __global__ void attn_mixed_decode_kernel(MixedAttnArgs a) {
 
 // out[b, h, :] = sum_s e^(m_s - M) o_s / (unit_sink e^(-M) + sum_s e^(m_s - M) l_s), pieces in ascending order.  A warp a
 // (row, head), two numbers a lane and load (EVEN: D is even) and all of a piece's on their way together: 2,048 rows of 16 heads
-// in two pieces, 34 MB, in 12 us (a CTA a row and head, a load after the other: 46).
+// in two pieces, 34 MB, in about 15 us back to back (a CTA a row and head, a load after the other: 46).
 constexpr int FOLD_WARPS = 4;
 template <typename T, bool EVEN, int NC>
 __global__ void __launch_bounds__(FOLD_WARPS * 32) attn_mixed_fold_kernel(MixedAttnArgs a) {
@@ -649,8 +649,9 @@ extern "C" int tb_attn_mixed_prefill(const MixedAttnArgs* args, int dtype, cudaS
     if (a.batch > 0 && a.max_seq_len > 0 && aligned && tb_attn_mixed_prefill_mma_takes(dtype, a.H, a.G, a.D)) {
         MixedAttnArgs am = a;
         am.stages = mp_smem(a.H, a.G, a.D, 2) <= 200 * 1024 ? 2 : 1;
-        // pairs wherever they fit beside as many stages as without them (16 heads: 174 against 190 us, see the kernel; 8 heads,
-        // not timed apart, share the kernel)
+        // pairs wherever they fit beside as many stages as without them: over 48 steps of one to three prompts, 33 to 2,500 tokens,
+        // 16 heads 1.03 to 1.18 times as fast as a warp a head (2,000 tokens, 4 kv heads: 168 against 185 us in a graph), 8 heads
+        // 0.99 to 1.10 (33 tokens: 8.9 against 9.4; 2,000: 111 against 120)
         const bool pairs = (a.H == 8 || a.H == 16) && mp_smem_pairs(a.H, a.G, a.D, am.stages) <= 220 * 1024;
         const size_t sm = pairs ? mp_smem_pairs(a.H, a.G, a.D, am.stages) : mp_smem(a.H, a.G, a.D, am.stages);
         if (am.n_pieces > 1 && a.partial == nullptr) return tb_refuse("attn_mixed: pieces need scratch");

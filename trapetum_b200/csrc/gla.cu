@@ -273,19 +273,21 @@ __global__ void gla_fold_kernel(GlaArgs a) {
 
 // ---------------------------------------------------------------------------------------------------------
 // Prompts in blocks (bfloat16; D up to 128, V up to 256).  A CTA owns a head of a chunk of a sequence, a warp 16 value
-// channels, whose state S^T [16 v][D] stays in the registers of a product's accumulators (mma.sync) while the CTA walks the
+// channels, whose state S^T [16 v][D] stays in registers, as accumulators of mma.sync lie, while the CTA walks the
 // chunk 16 tokens at a time.  With c_i[d] the sum of the log2 decays from the block's start through token i:
 //     o_i = S^T (q_i 2^c_i) + sum_{j <= i} P_ij v_j,     P_ij = sum_d q_i[d] k_j[d] 2^(c_i - c_j)   (32-bit FMA)
 //     S^T <- S^T 2^c_15 + sum_j v_j (k_j 2^(c_15 - c_j))^T
 // No exponent is positive, so nothing overflows whatever the decays.  v is a bfloat16 number; S, P and the decayed q and k
-// are 32-bit and enter as sums of three bfloat16 numbers each (of S times q the six products above 2^-24 are taken), so
-// only the order of the 32-bit sums differs from the recurrence's.  The sums c are made in 64 bits and kept as two 32-bit
-// numbers.  Long prompts: a first launch (OUT false) leaves the sums of every chunk but a sequence's last, gla_block_fold_kernel
-// turns them into start states, the second launch (OUT true) writes the outputs, normed and gated: the CTA holds the head.
+// are 32-bit and enter as sums of three bfloat16 numbers each (of S times q the six products above 2^-24 are taken).  A tensor
+// core's sums are cut off, so a block's are made apart from the state; decays come from ex2 of summed logs.  Against 64 bits
+// the state of 2,048 tokens stands 1.5e-7 off (the recurrence 2.1e-6; with decays of about 0.6 a token 0.7e-7 and 0.5e-7).
+// The sums c are made in 64 bits and kept as two 32-bit numbers.  Long prompts: a first launch (OUT false) leaves the sums of
+// every chunk but a sequence's last, gla_block_fold_kernel turns them into start states, the second launch (OUT true) writes
+// the outputs, normed and gated: the CTA holds the head.
 // A non-finite v is seen by its own token and later ones only, as in the recurrence; what it leaves in the state is NaN to the
 // next block's outputs (an infinity has no three parts).
-// Prompts of 1,500 and 548 tokens, 8 heads of 128 x 256, all of ops.gla: 130 us (the recurrence in chunks, its norm a launch
-// of its own: 388; there the chunks of the shorter prompt leave SMs idle too).  A block takes 9.6 us of its CTA: shared
+// Prompts of 1,500 and 548 tokens, 8 heads of 128 x 256, all of ops.gla, passes back to back: 147.4 us (the recurrence in chunks,
+// its norm a launch of its own: 453; there the chunks of the shorter prompt leave SMs idle too).  A block takes 9.6 us of its CTA: shared
 // memory (14 of 18 thousand cycles), then issue slots; the products are a quarter of the tensor pipe.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int GB = 16;                                // tokens of a block

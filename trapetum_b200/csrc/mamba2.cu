@@ -423,12 +423,15 @@ __global__ void __launch_bounds__(SCAN_NS * PT / SCAN_PP) mamba2_scan_kernel(Mam
 //     S'  = 2^(c_last) S + sum_j 2^(c_last - c_j) dt_j x_j B_j^T
 // in three launches: each chunk's own sum E, the states before the chunks (a scan over chunks, element by element), the
 // outputs; sequences of one chunk take part in the last one only.  x, B and C are bfloat16 numbers; what meets them (the weighted scores, the weighted x, the state) is 32-bit and
-// enters as the sum of three bfloat16 numbers, 24 bits, so every product is that of the recurrence and only the order of the
-// 32-bit sums differs.  The running sums are kept as two 32-bit numbers (c_i - c_j of near tokens keeps its digits); a
-// decay below 2^-300 is 0 in any product.  A non-finite x is seen by its own token and later ones only, as in the recurrence;
-// what it leaves in the state is NaN to the next chunk's outputs (an infinity has no three parts).
-// 2,048 tokens, 64 heads of 64 x 128: 31 + 20 + 56 us cold (the recurrence in chunks: 167 + 235); the tensor pipe and the
-// three-way splits share the time of the third launch.  All of ops.mamba2: 486 -> 129 us.
+// enters as the sum of three bfloat16 numbers, 24 bits.  A tensor core's sums are cut off, so 16 terms at a time are added up in
+// them and those sums outside; decays come from ex2 of summed logs.  Against 64 bits the state of 2,048 tokens stands 0.97e-7 off
+// (the recurrence 0.96e-7; with decays near 1, 1.1e-7 and 5.1e-7), the outputs 0.97e-7 (0.91e-7; 1.4e-7 and 4.8e-7).  The
+// running sums are kept as two 32-bit numbers (c_i - c_j of near tokens keeps its digits); a decay below 2^-300 is 0 in any
+// product.  A non-finite x is seen by its own token and later ones only, as in the recurrence; what it leaves in the state is
+// NaN to the next chunk's outputs (an infinity has no three parts).
+// 2,048 tokens, 64 heads of 64 x 128: 31 + 20 + 56 us cold (the recurrence in chunks: 167 + 235; both before the sums of 16 terms,
+// which take 3 % more); the tensor pipe and the three-way splits share the time of the third launch.  All of ops.mamba2, passes
+// back to back: 489 -> 137.5 us.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int MC = 128, MCT = 256;                    // tokens of a chunk, threads
 constexpr int MP = 64, MXPITCH = MP * 2 + 16;         // values of P a CTA takes; bytes of a shared row of them (no bank conflicts)

@@ -755,7 +755,8 @@ def mamba2(proj: torch.Tensor, dt_raw: torch.Tensor, heads: int, P: int, N: int,
     ``proj`` [T, inner + channels] (compute dtype) and step sizes ``dt_raw`` [T, heads] (float32, before bias and
     softplus; or [splits, T, heads] partial sums) to the gated, normed [T, inner] that the output product reads, with the sequences' states (``state`` [slots, mamba2_state_size] float32, rows picked by ``slot_ids``) carried along.
     ``max_seq_len`` (the longest sequence of a step of whole prompts, 0 if unknown) lets few long prompts be cut into
-    chunks that run side by side."""
+    chunks that run side by side, and prompts in bfloat16 run as matrix products.  A token whose numbers are not finite
+    changes its own outputs and later ones only; an infinity that it leaves in the state shows as NaN there."""
     _cuda(proj, dt_raw, conv_w, conv_b, dt_bias, A_log, D, norm_w, state, seq_start, token_seq, slot_ids)
     inner, ch = heads * P, heads * P + 2 * groups * N
     _rows_contig(proj, "mamba2: proj")
@@ -1538,7 +1539,9 @@ def gla(proj: torch.Tensor, low: torch.Tensor, a2: torch.Tensor, a2_bias: torch.
         seq_start: torch.Tensor, token_seq: torch.Tensor, slot_ids: torch.Tensor, batch: int,
         max_seq_len: int = 0) -> torch.Tensor:
     """Gated linear attention between its products (see gla.cu).  ``max_seq_len`` (the longest sequence of a step of
-    whole prompts, 0 if unknown or one token each) lets few long prompts be cut into chunks that run side by side.  ``proj`` [T, 2 H D + 2 H V]: q, k, v and the output
+    whole prompts, 0 if unknown or one token each) lets few long prompts be cut into chunks that run side by side, and
+    prompts in bfloat16 run as matrix products.  A value that is not finite changes its own token's outputs and later ones only; an
+    infinity that it leaves in the state shows as NaN there.  ``proj`` [T, 2 H D + 2 H V]: q, k, v and the output
     gate's pre-activation, in the compute dtype; ``low`` float32 [splits, T, rank]: partial sums of the decay's first
     product; ``a2`` float32 [H D, rank], ``a2_bias`` float32 [H D], ``norm_w`` float32 [V]; ``state`` float32
     [slots, H D V], rows picked by ``slot_ids``, read and written.  Returns [T, H V] in the compute dtype."""
