@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(1024) sample_kernel(SampleArgs a) {
 //                     passes the target.  A crowded row's cluster of CTAs reads it once more, for the elements of the
 //                     threshold's part; if those are too many to list too, they are one number, or 0 and -0, or (a few
 //                     neighbouring numbers, thousands of each) the CTAs search the row by the key's digits
-// 256,000 logits, top_p 0.95, in a graph: 36 / 44 / 93 us for 1 / 8 / 64 rows; six launches that read the row five times (three
-// histograms over the key's digits) took 41 / 73 / 154.  A bulk of 0.002 beside an outlier of 8: 57 / 78 / 208 (39 / 72 / 148).
+// 256,000 logits, top_p 0.95, in a graph: 36 / 44 / 97 us for 1 / 8 / 64 rows; six launches that read the row five times (three
+// histograms over the key's digits) took 41 / 73 / 154.  A bulk of 0.002 beside an outlier of 8: 60 / 78 / 211 (39 / 72 / 148).
 // ---------------------------------------------------------------------------
 #define S_CHUNK 8192
 #define S_BINS 2048
@@ -492,7 +492,8 @@ __global__ void __launch_bounds__(256) sample_hist_kernel(SampleWide w) {
     }
 }
 
-__global__ void __launch_bounds__(256) sample_chunk_mass_kernel(SampleWide w, int nucleus) {
+// (five CTAs an SM: 64 rows of 256,000 take 97 us in all; with the registers that the crowded rows' branch would take, four, 100)
+__global__ void __launch_bounds__(256, 5) sample_chunk_mass_kernel(SampleWide w, int nucleus) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ u64 red8[8];
