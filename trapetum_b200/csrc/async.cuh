@@ -47,6 +47,35 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
         if (clock64() - t0 > WAIT_CYCLES) return false;
     return true;
 }
+// The same by a whole converged warp, with one answer for all lanes: false if the wait ran out or `abort_flag` was set.
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    if (__all_sync(0xffffffffu, bar_try(bar, parity))) return true;
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, bar_try(bar, parity)))
+        if (__any_sync(0xffffffffu, *abort_flag || clock64() - t0 > WAIT_CYCLES)) return false;
+    return true;
+}
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return warp_wait(smem_u32(bar), parity, abort_flag);
+}
+__device__ __forceinline__ bool warp_test(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test(bar, parity)); }
+// True in one lane of a converged warp.  Copies and MMAs are issued under this and not under `lane == 0`: in a branch that
+// may diverge the compiler makes the operands of each such instruction uniform anew, which took a product's issuing thread
+// about 90 cycles an MMA.
+__device__ __forceinline__ bool elected() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
 // Contiguous global -> shared copy by the TMA unit; both addresses 16-byte aligned, bytes % 16 == 0.
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"

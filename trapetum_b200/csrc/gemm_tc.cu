@@ -199,6 +199,59 @@ __device__ __forceinline__ void store_token_major(const uint32_t* r, int prow, i
     }
 }
 
+// ---------------------------------------------------------------------------
+// The two warps that feed a product (one issues the copies, one the MMAs) run a short loop per k-block, and a chain of
+// dependent instructions in it is paid per k-block whatever the tile.  With one thread of a diverged warp, a stage index
+// modulo the number of stages, 64-bit descriptors made per MMA and a look at the abort flag, an SM spent 620 cycles a
+// k-block for tiles 128, 192 and 256 columns wide alike, although the MMAs need 256 to 512; with 32-bit addresses, a
+// counted stage and stepped descriptors 547; with the whole warp in the loop and one elected lane issuing 414, 430 and
+// 512 (a pair of SMs at 256 x 256: 576 before, 512 now, which is the MMAs' own time).
+// ---------------------------------------------------------------------------
+struct Ring {                            // the stage that comes next, and the phase of its barriers
+    uint32_t s = 0, ph = 0;
+    template <int STAGES> __device__ __forceinline__ void step() { if (++s == STAGES) { s = 0; ph ^= 1; } }
+};
+__device__ __forceinline__ void bar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tile_load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tile_load_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"((uint64_t)map), "r"(cluster_bar), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void commit_to(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void commit_to_pair(uint32_t bar) {
+    asm volatile("{\n\t.reg .b16 m;\n\tmov.b16 m, 3;\n\t"
+                 "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair_lh(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t ab_hi, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"
+        "mov.b64 ad, {%1, %3};\n\t"
+        "mov.b64 bd, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], ad, bd, %4, p;\n\t}"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(ab_hi), "r"(idesc), "r"(acc) : "memory");
+}
+// One k-block: BK / 16 MMAs from the stage whose A starts at a_lo (low half of its descriptor), then the commit that frees it.
+template <bool PAIR>
+__device__ __forceinline__ void issue_kblock(uint32_t d_addr, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t acc, uint32_t empty) {
+#pragma unroll
+    for (int k = 0; k < BK / UMMA_K; k++) {
+        const uint32_t step = k * (UMMA_K * 2 / 16);
+        if (PAIR) umma_bf16_pair_lh(d_addr, a_lo + step, b_lo + step, hi, idesc, k ? 1u : acc);
+        else umma_bf16_lh(d_addr, a_lo + step, b_lo + step, hi, idesc, k ? 1u : acc);
+    }
+    if (PAIR) commit_to_pair(empty); else commit_to(empty);
+}
+
 template <int BN, bool SWAP, typename TOut, bool GATED, bool WIDE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, GemmParams p) {
@@ -239,92 +292,96 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true, waited = false;
-            // the tile that holds weights: the 128-lane operand when swapped, else the BN-column one
-            const CUtensorMap* wmap = SWAP ? &map_p : &map_q;
-            const CUtensorMap* amap = SWAP ? &map_q : &map_p;
-            constexpr int W_OFF = SWAP ? 0 : BM * BK * 2, A_OFF = SWAP ? BM * BK * 2 : 0;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                int tp, tq, sp; decode(item, tp, tq, sp);
-                const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
-                int w_row = SWAP ? tp * BM : tq * BN;
-                const int a_row = SWAP ? tq * BN : tp * BM;
-                if (!SWAP && p.tile_group != nullptr) {
-                    // the table of groups is the preceding kernel's work: nothing is fetched before it is there
-                    if (!waited) { pdl_wait(); waited = true; }
-                    const int g = p.tile_group[tp];
-                    if (g < 0) continue;               // a tile past the last one in use: all three roles leave it out
-                    w_row += g * p.group_rows;
-                }
-                int kb = kb0;
-                if (!waited) {
-                    // Weights do not depend on the kernel before this one: start streaming them into the
-                    // (still empty) stages at once, and only then wait for that kernel, whose output is
-                    // the activation operand.
-                    const int pre = min(kb1 - kb0, C::STAGES);
-                    for (int j = 0; j < pre; j++) {
-                        mbar_expect_tx(&full[j], C::STAGE_BYTES);
-                        tma_load_2d(smem + j * C::STAGE_BYTES + W_OFF, wmap, &full[j], (kb0 + j) * BK, w_row);
-                    }
-                    pdl_wait();
-                    waited = true;
-                    for (int j = 0; j < pre; j++)
-                        tma_load_2d(smem + j * C::STAGE_BYTES + A_OFF, amap, &full[j], (kb0 + j) * BK, a_row);
-                    it = pre; kb = kb0 + pre;
-                }
-                for (; kb < kb1; kb++, it++) {
-                    const int s = it % C::STAGES; const uint32_t ph = (it / C::STAGES) & 1;
-                    if (*abort_flag || !mbar_wait(&empty[s], ph ^ 1)) { ok = false; break; }
-                    uint8_t* st = smem + s * C::STAGE_BYTES;
-                    mbar_expect_tx(&full[s], C::STAGE_BYTES);
-                    tma_load_2d(st + W_OFF, wmap, &full[s], kb * BK, w_row);
-                    tma_load_2d(st + A_OFF, amap, &full[s], kb * BK, a_row);
-                }
+        const uint32_t sm0 = smem_u32(smem), full0 = smem_u32(full), empty0 = smem_u32(empty);
+        uint32_t it = 0;
+        Ring ring;
+        bool ok = true, waited = false;
+        // the tile that holds weights: the 128-lane operand when swapped, else the BN-column one
+        const CUtensorMap* wmap = SWAP ? &map_p : &map_q;
+        const CUtensorMap* amap = SWAP ? &map_q : &map_p;
+        constexpr int W_OFF = SWAP ? 0 : BM * BK * 2, A_OFF = SWAP ? BM * BK * 2 : 0;
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            int tp, tq, sp; decode(item, tp, tq, sp);
+            const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
+            int w_row = SWAP ? tp * BM : tq * BN;
+            const int a_row = SWAP ? tq * BN : tp * BM;
+            if (!SWAP && p.tile_group != nullptr) {
+                // the table of groups is the preceding kernel's work: nothing is fetched before it is there
+                if (!waited) { pdl_wait(); waited = true; }
+                const int g = p.tile_group[tp];
+                if (g < 0) continue;               // a tile past the last one in use: all three roles leave it out
+                w_row += g * p.group_rows;
             }
-            if (!ok) {
-                if (!*abort_flag) { atomicExch(&g_gemm_error, 1); *abort_flag = 1; }
-                // loads already issued still land in this CTA's shared memory: wait for them
-                for (uint32_t back = 1; back <= (uint32_t)C::STAGES && back <= it; back++) {
-                    const uint32_t j = it - back;
-                    mbar_wait(&full[j % C::STAGES], (j / C::STAGES) & 1);
+            int kb = kb0;
+            if (!waited) {
+                // Weights do not depend on the kernel before this one: start streaming them into the
+                // (still empty) stages at once, and only then wait for that kernel, whose output is
+                // the activation operand.
+                const int pre = min(kb1 - kb0, C::STAGES);
+                if (elected())
+                    for (int j = 0; j < pre; j++) {
+                        bar_expect(full0 + 8 * j, C::STAGE_BYTES);
+                        tile_load(sm0 + j * C::STAGE_BYTES + W_OFF, wmap, full0 + 8 * j, (kb0 + j) * BK, w_row);
+                    }
+                pdl_wait();
+                waited = true;
+                if (elected())
+                    for (int j = 0; j < pre; j++)
+                        tile_load(sm0 + j * C::STAGE_BYTES + A_OFF, amap, full0 + 8 * j, (kb0 + j) * BK, a_row);
+                __syncwarp();
+                it = pre; kb = kb0 + pre;
+                ring.s = pre % C::STAGES; ring.ph = pre / C::STAGES;
+            }
+            for (; kb < kb1; kb++, it++) {
+                if (!warp_wait(empty0 + 8 * ring.s, ring.ph ^ 1, abort_flag)) { ok = false; break; }
+                const uint32_t st = sm0 + ring.s * C::STAGE_BYTES, bar = full0 + 8 * ring.s;
+                if (elected()) {
+                    bar_expect(bar, C::STAGE_BYTES);
+                    tile_load(st + W_OFF, wmap, bar, kb * BK, w_row);
+                    tile_load(st + A_OFF, amap, bar, kb * BK, a_row);
                 }
+                ring.step<C::STAGES>();
             }
         }
+        if (!ok && lane == 0) {
+            if (!*abort_flag) { atomicExch(&g_gemm_error, 1); *abort_flag = 1; }
+            // loads already issued still land in this CTA's shared memory: wait for them
+            for (uint32_t back = 1; back <= (uint32_t)C::STAGES && back <= it; back++) {
+                const uint32_t j = it - back;
+                mbar_wait(&full[j % C::STAGES], (j / C::STAGES) & 1);
+            }
+        }
+        __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(BN);
-            uint32_t it = 0, tile_it = 0;
-            bool ok = true;
-            if (!SWAP && p.tile_group != nullptr) pdl_wait();      // the table of groups is the preceding kernel's work
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                int tp, tq, sp; decode(item, tp, tq, sp);
-                if (!SWAP && p.tile_group != nullptr && p.tile_group[tp] < 0) continue;
-                const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
-                const int a = tile_it & 1; const uint32_t aph = (tile_it >> 1) & 1;
-                tile_it++;
-                if (*abort_flag || !mbar_wait(&acc_empty[a], aph ^ 1)) { ok = false; break; }
+        constexpr uint32_t idesc = instr_desc(BN);
+        const uint64_t desc0 = smem_desc(smem_u32(smem));
+        const uint32_t lo0 = desc_lo(desc0), hi = desc_hi(desc0), full0 = smem_u32(full), empty0 = smem_u32(empty);
+        const uint32_t acc_full0 = smem_u32(acc_full), acc_empty0 = smem_u32(acc_empty);
+        uint32_t tile_it = 0;
+        Ring ring;
+        bool ok = true;
+        if (!SWAP && p.tile_group != nullptr) pdl_wait();      // the table of groups is the preceding kernel's work
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            int tp, tq, sp; decode(item, tp, tq, sp);
+            if (!SWAP && p.tile_group != nullptr && p.tile_group[tp] < 0) continue;
+            const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
+            const int a = tile_it & 1; const uint32_t aph = (tile_it >> 1) & 1;
+            tile_it++;
+            if (!warp_wait(acc_empty0 + 8 * a, aph ^ 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t d_addr = tmem_base + a * C::ACC_COLS;
+            for (int kb = kb0; kb < kb1; kb++) {
+                if (!warp_wait(full0 + 8 * ring.s, ring.ph, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t d_addr = tmem_base + a * C::ACC_COLS;
-                for (int kb = kb0; kb < kb1; kb++, it++) {
-                    const int s = it % C::STAGES; const uint32_t ph = (it / C::STAGES) & 1;
-                    if (*abort_flag || !mbar_wait(&full[s], ph)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + s * C::STAGE_BYTES);
-                    const uint32_t sb = sa + BM * BK * 2;
-#pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; k++) {
-                        umma_bf16(d_addr, smem_desc(sa + k * UMMA_K * 2), smem_desc(sb + k * UMMA_K * 2), idesc,
-                                  (kb > kb0 || k > 0) ? 1u : 0u);
-                    }
-                    umma_commit(&empty[s]);            // frees the stage once these MMAs have read it
-                }
-                if (ok) umma_commit(&acc_full[a]);     // the accumulator is complete
+                const uint32_t a_lo = lo0 + ring.s * (C::STAGE_BYTES / 16);
+                if (elected()) issue_kblock<false>(d_addr, a_lo, a_lo + BM * BK * 2 / 16, hi, idesc, kb > kb0, empty0 + 8 * ring.s);
+                ring.step<C::STAGES>();
             }
-            if (!ok && !*abort_flag) { atomicExch(&g_gemm_error, 2); *abort_flag = 1; }
+            if (ok && elected()) commit_to(acc_full0 + 8 * a);     // the accumulator is complete
         }
+        if (!ok && lane == 0 && !*abort_flag) { atomicExch(&g_gemm_error, 2); *abort_flag = 1; }
+        __syncwarp();
     } else {
         // ---------------- epilogue: warps 2..9 ----------------
         const int quarter = warp & 3;                  // the TMEM lanes this warp may read
@@ -465,76 +522,83 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
 
     if (warp == 0) {
         // ---------------- TMA producer, in both CTAs ----------------
-        if (lane == 0) {
-            const uint32_t lead_full = cluster_addr(&full[0], 0);
-            uint32_t it = 0;
-            bool ok = true, waited = false;
-            for (int item = pair; item < n_items && ok; item += n_pairs) {
-                int tp, tq, sp; decode(item, tp, tq, sp);
-                const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
-                const int a_row = tp * 256 + (int)rank * BM, w_row = tq * C::BN + (int)rank * C::HALF;
-                int kb = kb0;
-                if (!waited) {
-                    // weights first, then the wait for the kernel before this one, then its output
-                    const int pre = min(kb1 - kb0, C::STAGES);
+        const uint32_t lead_full = cluster_addr(&full[0], 0);
+        const uint32_t sm0 = smem_u32(smem), full0 = smem_u32(full), empty0 = smem_u32(empty);
+        uint32_t it = 0;
+        Ring ring;
+        bool ok = true, waited = false;
+        for (int item = pair; item < n_items && ok; item += n_pairs) {
+            int tp, tq, sp; decode(item, tp, tq, sp);
+            const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
+            const int a_row = tp * 256 + (int)rank * BM, w_row = tq * C::BN + (int)rank * C::HALF;
+            int kb = kb0;
+            if (!waited) {
+                // weights first, then the wait for the kernel before this one, then its output
+                const int pre = min(kb1 - kb0, C::STAGES);
+                if (elected())
                     for (int j = 0; j < pre; j++) {
-                        if (rank == 0) mbar_expect_tx(&full[j], 2 * C::STAGE_BYTES);
-                        tma_load_2d_pair(smem + j * C::STAGE_BYTES + W_OFF, &map_q, lead_full + 8 * j, (kb0 + j) * BK, w_row);
+                        if (rank == 0) bar_expect(full0 + 8 * j, 2 * C::STAGE_BYTES);
+                        tile_load_pair(sm0 + j * C::STAGE_BYTES + W_OFF, &map_q, lead_full + 8 * j, (kb0 + j) * BK, w_row);
                     }
-                    pdl_wait();
-                    waited = true;
+                pdl_wait();
+                waited = true;
+                if (elected())
                     for (int j = 0; j < pre; j++)
-                        tma_load_2d_pair(smem + j * C::STAGE_BYTES + A_OFF, &map_p, lead_full + 8 * j, (kb0 + j) * BK, a_row);
-                    it = pre; kb = kb0 + pre;
-                }
-                for (; kb < kb1; kb++, it++) {
-                    const int s = it % C::STAGES; const uint32_t ph = (it / C::STAGES) & 1;
-                    if (*abort_flag || !mbar_wait(&empty[s], ph ^ 1)) { ok = false; break; }
-                    uint8_t* st = smem + s * C::STAGE_BYTES;
-                    if (rank == 0) mbar_expect_tx(&full[s], 2 * C::STAGE_BYTES);
-                    tma_load_2d_pair(st + W_OFF, &map_q, lead_full + 8 * s, kb * BK, w_row);
-                    tma_load_2d_pair(st + A_OFF, &map_p, lead_full + 8 * s, kb * BK, a_row);
-                }
+                        tile_load_pair(sm0 + j * C::STAGE_BYTES + A_OFF, &map_p, lead_full + 8 * j, (kb0 + j) * BK, a_row);
+                __syncwarp();
+                it = pre; kb = kb0 + pre;
+                ring.s = pre % C::STAGES; ring.ph = pre / C::STAGES;
             }
-            if (!ok) {
-                if (!*abort_flag) { atomicExch(&g_gemm_error, 4); *abort_flag = 1; }
-                // the leader's barriers count both CTAs' copies: wait for those already issued
-                if (rank == 0)
-                    for (uint32_t back = 1; back <= (uint32_t)C::STAGES && back <= it; back++) {
-                        const uint32_t j = it - back;
-                        mbar_wait(&full[j % C::STAGES], (j / C::STAGES) & 1);
-                    }
+            for (; kb < kb1; kb++, it++) {
+                if (!warp_wait(empty0 + 8 * ring.s, ring.ph ^ 1, abort_flag)) { ok = false; break; }
+                const uint32_t st = sm0 + ring.s * C::STAGE_BYTES, bar = lead_full + 8 * ring.s;
+                if (elected()) {
+                    if (rank == 0) bar_expect(full0 + 8 * ring.s, 2 * C::STAGE_BYTES);
+                    tile_load_pair(st + W_OFF, &map_q, bar, kb * BK, w_row);
+                    tile_load_pair(st + A_OFF, &map_p, bar, kb * BK, a_row);
+                }
+                ring.step<C::STAGES>();
             }
         }
+        if (!ok && lane == 0) {
+            if (!*abort_flag) { atomicExch(&g_gemm_error, 4); *abort_flag = 1; }
+            // the leader's barriers count both CTAs' copies: wait for those already issued
+            if (rank == 0)
+                for (uint32_t back = 1; back <= (uint32_t)C::STAGES && back <= it; back++) {
+                    const uint32_t j = it - back;
+                    mbar_wait(&full[j % C::STAGES], (j / C::STAGES) & 1);
+                }
+        }
+        __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer, in the leader ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             constexpr uint32_t idesc = instr_desc_pair(C::BN);
-            uint32_t it = 0, tile_it = 0;
+            const uint64_t desc0 = smem_desc(smem_u32(smem));
+            const uint32_t lo0 = desc_lo(desc0), hi = desc_hi(desc0), full0 = smem_u32(full), empty0 = smem_u32(empty);
+            const uint32_t acc_full0 = smem_u32(acc_full), acc_empty0 = smem_u32(acc_empty);
+            uint32_t tile_it = 0;
+            Ring ring;
             bool ok = true;
             for (int item = pair; item < n_items && ok; item += n_pairs, tile_it++) {
                 int tp, tq, sp; decode(item, tp, tq, sp);
                 const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
                 const int a = tile_it & 1; const uint32_t aph = (tile_it >> 1) & 1;
-                if (*abort_flag || !mbar_wait(&acc_empty[a], aph ^ 1)) { ok = false; break; }
+                if (!warp_wait(acc_empty0 + 8 * a, aph ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_addr = tmem_base + a * C::BN;
-                for (int kb = kb0; kb < kb1; kb++, it++) {
-                    const int s = it % C::STAGES; const uint32_t ph = (it / C::STAGES) & 1;
-                    if (*abort_flag || !mbar_wait(&full[s], ph)) { ok = false; break; }
+                for (int kb = kb0; kb < kb1; kb++) {
+                    if (!warp_wait(full0 + 8 * ring.s, ring.ph, abort_flag)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + s * C::STAGE_BYTES);
-                    const uint32_t sb = sa + W_OFF;
-#pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; k++) {
-                        umma_bf16_pair(d_addr, smem_desc(sa + k * UMMA_K * 2), smem_desc(sb + k * UMMA_K * 2), idesc,
-                                       (kb > kb0 || k > 0) ? 1u : 0u);
-                    }
-                    umma_commit_pair(&empty[s]);           // frees the stage in both CTAs
+                    const uint32_t a_lo = lo0 + ring.s * (C::STAGE_BYTES / 16);
+                    // the commit frees the stage in both CTAs
+                    if (elected()) issue_kblock<true>(d_addr, a_lo, a_lo + W_OFF / 16, hi, idesc, kb > kb0, empty0 + 8 * ring.s);
+                    ring.step<C::STAGES>();
                 }
-                if (ok) umma_commit_pair(&acc_full[a]);    // the accumulator is complete in both CTAs
+                if (ok && elected()) commit_to_pair(acc_full0 + 8 * a);    // the accumulator is complete in both CTAs
             }
-            if (!ok && !*abort_flag) { atomicExch(&g_gemm_error, 5); *abort_flag = 1; }
+            if (!ok && lane == 0 && !*abort_flag) { atomicExch(&g_gemm_error, 5); *abort_flag = 1; }
+            __syncwarp();
         }
     } else {
         // ---------------- epilogue: warps 2..9 of both CTAs ----------------
