@@ -60,6 +60,7 @@ struct GemmParams {
     // is not in use and nobody touches it.  Null: one group.
     const int* tile_group;
     int group_rows;
+    int staged;                      // the rows of C are made of whole 16-byte pieces: chunks of 32 columns are stored through shared memory
     const float* row_scale;          // grouped products: the sums of token row r times row_scale[r], before the activation; or null
 };
 
@@ -97,14 +98,17 @@ __device__ __forceinline__ float gated(float g, float u, int act, float limit) {
 #ifndef TB_SWAP_HALF_UPTO
 #define TB_SWAP_HALF_UPTO 16
 #endif
+#define EPI_STAGE_BYTES (32 * 128)       // an epilogue warp's 32 rows of a 32-column chunk, on their way through shared memory
 template <int BN, bool SWAP, bool WIDE = false> struct Cfg {
     static constexpr int STAGE_BYTES = BM * BK * 2 + BN * BK * 2;
-    static constexpr int BUDGET = ((SWAP && !WIDE && BN <= TB_SWAP_HALF_UPTO) ? TB_SWAP_KB : 200) * 1024;
+    static constexpr int BUDGET = (!SWAP ? 192 : (!WIDE && BN <= TB_SWAP_HALF_UPTO) ? TB_SWAP_KB : 200) * 1024;
     static constexpr int STAGES_RAW = BUDGET / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 10 ? 10 : STAGES_RAW;
-    static constexpr int ACC_COLS = BN < 32 ? 32 : BN;               // columns of one accumulator stage
+    static constexpr int ACC_COLS = BN < 32 ? 32 : BN;     // columns of one accumulator stage
     static constexpr int TMEM_COLS = 2 * ACC_COLS;                   // a power of two >= 32
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
+    static constexpr int EPI = SWAP ? 0 : EPI_WARPS * EPI_STAGE_BYTES;
+    static constexpr int EPI_OFF = STAGES * STAGE_BYTES + 256 /* barriers */;
+    static constexpr int SMEM = EPI_OFF + EPI + 1024 /* alignment */;
 };
 
 // The exact gelu, v Phi(v), for an output that is rounded to bfloat16.  The tail Q(t) = 1 - Phi(t), t = |v|, is half of
@@ -197,6 +201,50 @@ __device__ __forceinline__ void store_token_major(const uint32_t* r, int prow, i
             }
         }
     }
+}
+
+// The same 32 columns of a warp's 32 rows, rows of whole 16-byte pieces, through 4 KB of shared memory: a row's piece of a
+// chunk then leaves as whole sectors, 8 (float), 4 or 2 lanes side by side.  Written by the thread that holds the row, 16
+// bytes a lane, every store touches 32 lines and the SM takes a line a cycle: a tile of 128 x 256 floats took 11.9 us so,
+// 3.3 this way (the product of 2,048 tokens x 2,304 x 2,048: 25.7 -> 18.2 us).  Pieces are swizzled against bank conflicts.
+template <typename TOut, bool GATED>
+__device__ __forceinline__ void store_staged(const uint32_t* r, uint8_t* stage, int lane, int row0, int q0, const GemmParams& p) {
+    constexpr int RB = GATED ? 32 : 32 * (int)sizeof(TOut), U = RB / 16;
+    auto f = [](int row) { return U == 8 ? row & 7 : U == 4 ? (row >> 1) & 3 : (row >> 2) & 1; };
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        uint32_t w[4];
+        if (GATED) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int j = u * 8 + e * 2;
+                __nv_bfloat162 h2 = __floats2bfloat162_rn(gated(__uint_as_float(r[j]), __uint_as_float(r[j + 16]), p.act, p.limit),
+                                                          gated(__uint_as_float(r[j + 1]), __uint_as_float(r[j + 17]), p.act, p.limit));
+                w[e] = *(uint32_t*)&h2;
+            }
+        } else if (sizeof(TOut) == 2) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int j = u * 8 + e * 2;
+                __nv_bfloat162 h2 = __floats2bfloat162_rn(pointwise(__uint_as_float(r[j]), p) * p.scale, pointwise(__uint_as_float(r[j + 1]), p) * p.scale);
+                w[e] = *(uint32_t*)&h2;
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; e++) w[e] = __float_as_uint(pointwise(__uint_as_float(r[u * 4 + e]), p) * p.scale);
+        }
+        *(uint4*)(stage + lane * RB + ((u ^ f(lane)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    __syncwarp();
+    const int c0 = GATED ? q0 >> 1 : q0;
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+        const int idx = i * 32 + lane, row = idx / U, u = idx % U;
+        const uint4 v = *(const uint4*)(stage + row * RB + ((u ^ f(row)) << 4));
+        if (row0 + row < p.rows_p)
+            *(uint4*)((uint8_t*)p.out + ((size_t)(row0 + row) * p.ld_out + c0) * sizeof(TOut) + u * 16) = v;
+    }
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------------------
@@ -413,7 +461,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
 #pragma unroll
                         for (int j = 0; j < CH; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
                     }
-                    store_token_major<TOut, GATED, CH>(r, prow, q0, sp, p);
+                    if (CH == 32 && p.staged && (GATED ? q0 < p.rows_q : q0 + CH <= p.rows_q))
+                        store_staged<TOut, GATED>(r, smem + C::EPI_OFF + (warp - 2) * EPI_STAGE_BYTES, lane, prow - lane, q0, p);
+                    else store_token_major<TOut, GATED, CH>(r, prow, q0, sp, p);
                 } else if (GATED && SWAP) {
                     // Lanes 0..15 hold gates, lanes 16..31 the ups of the same 16 features.  Two tokens a round: the
                     // lower lanes hand over their gates of the second token and get the ups of the first, so that each
@@ -476,9 +526,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
 struct PairCfg {
     static constexpr int BN = 256, HALF = 128;
     static constexpr int STAGE_BYTES = BM * BK * 2 + HALF * BK * 2;       // per CTA
-    static constexpr int STAGES = (227 * 1024 - 1024 - 256) / STAGE_BYTES;   // 7: all of an SM's shared memory
+    static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;
     static constexpr int TMEM_COLS = 2 * BN;
-    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
+    static constexpr int EPI_OFF = STAGES * STAGE_BYTES + 256 /* barriers */;
+    static constexpr int SMEM = EPI_OFF + EPI_WARPS * EPI_STAGE_BYTES + 1024 /* alignment */;
 };
 
 template <typename TOut, bool GATED>
@@ -621,7 +672,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 uint32_t r[32];
                 tmem_ld32(t_addr + c0, r);
                 tmem_ld_wait();
-                store_token_major<TOut, GATED, 32>(r, prow, tq * C::BN + c0, sp, p);
+                const int q0 = tq * C::BN + c0;
+                if (p.staged && (GATED ? q0 < p.rows_q : q0 + 32 <= p.rows_q))
+                    store_staged<TOut, GATED>(r, smem + C::EPI_OFF + (warp - 2) * EPI_STAGE_BYTES, lane, prow - lane, q0, p);
+                else store_token_major<TOut, GATED, 32>(r, prow, q0, sp, p);
             }
             tc_fence_before();
             __syncwarp();
@@ -833,6 +887,7 @@ static int gemm_tc_run(const void* A, const void* W, void* C, int c_dtype, int M
 
     GemmParams p;
     p.tile_group = nullptr; p.group_rows = 0; p.row_scale = nullptr;
+    p.staged = splits == 1 && C != nullptr && ((uintptr_t)C & 15) == 0 && (ldc * (c_dtype == TB_BF16 ? 2 : 4)) % 16 == 0;
     p.K = K; p.kblocks = kblocks; p.splits = splits; p.kb_per_split = per;
     p.out = C; p.ld_out = ldc; p.partial = scratch; p.cap = splits > 1 ? 0.f : softcap;
     p.act = gated ? gated_act : 0;
@@ -921,6 +976,7 @@ static int gemm_tc_grouped_run(const void* A, const void* W, void* C, int c_dtyp
     p.K = K; p.kblocks = (K + BK - 1) / BK; p.splits = 1; p.kb_per_split = p.kblocks;
     p.out = C; p.ld_out = ldc; p.partial = nullptr; p.cap = 0.f; p.scale = 1.0f;
     p.act = gated ? gated_act : 0; p.limit = 0.f; p.unary = unary;
+    p.staged = ((uintptr_t)C & 15) == 0 && (ldc * (c_dtype == TB_BF16 ? 2 : 4)) % 16 == 0;
     p.rows_p = M; p.rows_q = N;
     CUtensorMap mp, mq;
     if (make_map(&mp, A, M, K, lda, BM) || make_map(&mq, W, groups * N, K, ldw, bn)) return -1;
