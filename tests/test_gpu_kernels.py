@@ -502,6 +502,36 @@ def test_gemm_tc(ops, odt, M, N, K, pair):
         assert float((got.double() - want).norm() / want.norm()) < 4e-3
 
 
+# tokens, weight rows, K and the form that the cost picks on 148 SMs (1000 x CTAs a tile + columns, + 100000 for pairs)
+GEMM_FORMS = [(300, 300, 64, 1128), (1500, 2400, 1032, 1256), (129, 520, 1040, 4128), (200, 2300, 2040, 3128), (300, 2304, 2048, 2128),
+              (300, 3584, 14336, 3256), (257, 2304, 9216, 4256), (700, 2300, 2040, 101128), (1500, 2304, 2048, 101192),
+              (1000, 3580, 4088, 101224), (2047, 2304, 2048, 101256), (513, 18432, 136, 1256)]
+
+
+@pytest.mark.parametrize("M,N,K,form", GEMM_FORMS)
+def test_gemm_tc_forms(ops, M, N, K, form):
+    """Every form of a product of many tokens at sizes with remainders: 32-bit and bfloat16 results, the gate where the
+    rows allow it, a cap, and a result whose rows are not whole 16-byte pieces.  32-bit: sums of K products of which each
+    is exact; bfloat16: one rounding."""
+    from trapetum_b200.csrc import build
+    if ops.sm_count() == 148:
+        assert build.load("gemm_tc").tb_gemm_tc_form(M, N, K, 148) == form
+    a, w = rnd(M, K, dt=torch.bfloat16, s=0.5), rnd(N, K, dt=torch.bfloat16, s=0.5, seed=1)
+    want = a.double() @ w.double().T
+    off = torch.full((M, N + 3), 7.0, device="cuda")
+    for got, truth, tol in ((ops.gemm_tc(a, w, torch.float32), want, 2e-5), (ops.gemm_tc(a, w, torch.bfloat16), want, 4e-3),
+                            (ops.gemm_tc(a, w, torch.float32, 20.0), 20 * torch.tanh(want / 20), 2e-5),
+                            (ops.gemm_tc(a, w, torch.float32, out=off[:, 1:N + 1]), want, 2e-5)):
+        assert float((got.double() - truth).norm() / truth.norm()) < tol
+    assert bool((off[:, 0] == 7).all() and (off[:, N + 1:] == 7).all())
+    if N % 32 == 0:
+        blocks = want.view(M, N // 32, 2, 16)
+        gated = (torch.nn.functional.silu(blocks[:, :, 0]) * blocks[:, :, 1]).reshape(M, N // 2)
+        got = ops.gemm_tc(a, w, torch.bfloat16, gated_act="silu")
+        assert float((got.double() - gated).norm() / gated.norm()) < 4e-3
+    assert ops.gemm_tc_error() == 0
+
+
 @pytest.mark.parametrize("M,N,K,splits", [(8, 2304, 2048, 8), (64, 640, 9216, 5), (1, 136, 1024, 16), (33, 100 * 8, 520, 3)])
 def test_gemm_tc_split_k(ops, M, N, K, splits):
     a, w = rnd(M, K, dt=torch.bfloat16, s=0.5), rnd(N, K, dt=torch.bfloat16, s=0.5, seed=1)

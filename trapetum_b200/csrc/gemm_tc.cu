@@ -1,8 +1,8 @@
 // C[M,N] = A[M,K] * W[N,K]^T in bfloat16 on the 5th-generation tensor cores.
 //
-// tcgen05.mma (kind::f16; cta_group::1 with 128 x BN x 16 per instruction, and for long
-// products of many tokens cta_group::2 with 256 x 256 x 16 over a pair of SMs, see
-// gemm_tc_pair_kernel) issued by one thread, operands staged in shared memory by TMA
+// tcgen05.mma (kind::f16; cta_group::1 with 128 x BN x 16 per instruction, and for most
+// products of many tokens cta_group::2 with 256 x BN x 16 over a pair of SMs, see
+// gemm_tc_pair_kernel) issued by one elected lane, operands staged in shared memory by TMA
 // (128-byte swizzle, K-major), accumulators in tensor memory, read back with tcgen05.ld
 // for the epilogue.
 // The reference has no dense tensor-core product: its linears are 4-bit codebook
@@ -14,7 +14,7 @@
 //   tokens <= 128: swapped, the 128 lanes are weight rows and the BN columns are the
 //                  tokens (BN = 16..128), so a decode step streams every weight
 //                  once through full-height MMA tiles whatever the batch size
-// and optional split-K (small N, large K): each split writes 32-bit partials to
+// (many tokens: single SMs, pairs, or a cluster that cuts a tile's K, and the tile's width, by choose_form) and optional split-K (small N, large K): each split writes 32-bit partials to
 // scratch and tb_splitk_reduce adds them in split order.
 //
 // Roles per CTA (320 threads): warp 0 issues TMA loads, warp 1 owns tensor memory
@@ -61,6 +61,7 @@ struct GemmParams {
     const int* tile_group;
     int group_rows;
     int staged;                      // the rows of C are made of whole 16-byte pieces: chunks of 32 columns are stored through shared memory
+    int cluster;                     // gemm_tc_split_kernel: CTAs that share a tile's K
     const float* row_scale;          // grouped products: the sums of token row r times row_scale[r], before the activation; or null
 };
 
@@ -104,7 +105,7 @@ template <int BN, bool SWAP, bool WIDE = false> struct Cfg {
     static constexpr int BUDGET = (!SWAP ? 192 : (!WIDE && BN <= TB_SWAP_HALF_UPTO) ? TB_SWAP_KB : 200) * 1024;
     static constexpr int STAGES_RAW = BUDGET / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 10 ? 10 : STAGES_RAW;
-    static constexpr int ACC_COLS = BN < 32 ? 32 : BN;     // columns of one accumulator stage
+    static constexpr int ACC_COLS = BN < 32 ? 32 : BN <= 128 ? BN : 256;       // columns of one accumulator stage
     static constexpr int TMEM_COLS = 2 * ACC_COLS;                   // a power of two >= 32
     static constexpr int EPI = SWAP ? 0 : EPI_WARPS * EPI_STAGE_BYTES;
     static constexpr int EPI_OFF = STAGES * STAGE_BYTES + 256 /* barriers */;
@@ -202,6 +203,7 @@ __device__ __forceinline__ void store_token_major(const uint32_t* r, int prow, i
         }
     }
 }
+
 
 // The same 32 columns of a warp's 32 rows, rows of whole 16-byte pieces, through 4 KB of shared memory: a row's piece of a
 // chunk then leaves as whole sectors, 8 (float), 4 or 2 lanes side by side.  Written by the thread that holds the row, 16
@@ -512,9 +514,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
 
 // ---------------------------------------------------------------------------
 // The same product for many tokens on a pair of SMs (cta_group::2): a cluster of two CTAs owns a tile of 256 tokens
-// by 256 weight rows.  Each CTA copies its 128 tokens of A and its 128 of the tile's weight rows into its own shared
-// memory; one thread of the even CTA issues MMAs of 256 x 256 x 16 that read A and half of B from each CTA and leave
-// each CTA's 128 tokens of the result in its own tensor memory.  A k-block of 64 then costs an SM 32 KB of shared
+// by BN weight rows.  Each CTA copies its 128 tokens of A and its half of the tile's weight rows into its own shared
+// memory; a lane of the even CTA issues MMAs of 256 x BN x 16 that read A and half of B from each CTA and leave
+// each CTA's 128 tokens of the result in its own tensor memory.  With BN = 256 a k-block of 64 then costs an SM 32 KB of shared
 // memory and of copies instead of 48 KB: on one SM a 128 x 256 tile reads and refills its operands faster than the
 // shared memory delivers them, which is what bounds the single-CTA kernel above.
 //
@@ -523,20 +525,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
 // on the leader's `acc_empty`.  All waits on these are bounded as above.  The two cluster barriers (after set-up,
 // before the tensor memory is given back) are not: every path reaches them, since every loop before them ends.
 // ---------------------------------------------------------------------------
-struct PairCfg {
-    static constexpr int BN = 256, HALF = 128;
+template <int BN_> struct PairCfg {
+    static constexpr int BN = BN_, HALF = BN / 2;
     static constexpr int STAGE_BYTES = BM * BK * 2 + HALF * BK * 2;       // per CTA
     static constexpr int STAGES = 192 * 1024 / STAGE_BYTES;
-    static constexpr int TMEM_COLS = 2 * BN;
+    static constexpr int ACC_COLS = 256, TMEM_COLS = 2 * ACC_COLS;
     static constexpr int EPI_OFF = STAGES * STAGE_BYTES + 256 /* barriers */;
     static constexpr int SMEM = EPI_OFF + EPI_WARPS * EPI_STAGE_BYTES + 1024 /* alignment */;
 };
 
-template <typename TOut, bool GATED>
+template <int BN, typename TOut, bool GATED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, GemmParams p) {
     pdl_launch_dependents();
-    using C = PairCfg;
+    using C = PairCfg<BN>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = (uint64_t*)(smem + C::STAGES * C::STAGE_BYTES);
@@ -637,7 +639,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 const int a = tile_it & 1; const uint32_t aph = (tile_it >> 1) & 1;
                 if (!warp_wait(acc_empty0 + 8 * a, aph ^ 1, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t d_addr = tmem_base + a * C::BN;
+                const uint32_t d_addr = tmem_base + a * C::ACC_COLS;
                 for (int kb = kb0; kb < kb1; kb++) {
                     if (!warp_wait(full0 + 8 * ring.s, ring.ph, abort_flag)) { ok = false; break; }
                     tc_fence_after();
@@ -666,7 +668,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
             if (!__all_sync(0xffffffffu, mine)) { ok = false; break; }
             tc_fence_after();
             const int prow = tp * 256 + (int)rank * BM + quarter * 32 + lane;
-            const uint32_t t_addr = tmem_base + a * C::BN + ((uint32_t)(quarter * 32) << 16);
+            const uint32_t t_addr = tmem_base + a * C::ACC_COLS + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
             for (int c0 = turn * 32; c0 < C::BN; c0 += (EPI_WARPS / 4) * 32) {
                 uint32_t r[32];
@@ -688,6 +690,155 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
     cluster_sync();
     tc_fence_after();
     if (warp == 1) tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
+}
+
+// ---------------------------------------------------------------------------
+// Many tokens, but fewer tiles than SMs and a long K: a cluster of S CTAs owns one tile of 128 tokens by BN weight rows
+// and each takes a share of K.  The shares meet in distributed shared memory: chunk c (32 columns) of the tile belongs to
+// CTA c mod S; the others write their sums of it into that CTA's stages (idle by then), and the owner adds them in the
+// order of K and runs the epilogue, so that every epilogue works (also those that need the whole sum), nothing passes
+// through memory, and the result does not depend on which CTA was late.
+// ---------------------------------------------------------------------------
+template <int BN, typename TOut, bool GATED>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, GemmParams p) {
+    pdl_launch_dependents();
+    using C = Cfg<BN, false>;
+    constexpr int CHUNKS = BN / 32;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = (uint64_t*)(smem + C::STAGES * C::STAGE_BYTES);
+    uint64_t* full = bars;                       // [STAGES]
+    uint64_t* empty = bars + C::STAGES;          // [STAGES]
+    uint64_t* acc_full = bars + 2 * C::STAGES;
+    uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int S = p.cluster, ks = (int)cluster_ctarank();
+
+    if (threadIdx.x == 32) { tma_prefetch_map(&map_p); tma_prefetch_map(&map_q); }
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < C::STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(acc_full, 1);
+        *abort_flag = 0;
+        mbar_init_fence();
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, BN);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const int tile = blockIdx.x / S, tp = tile % p.tiles_p, tq = tile / p.tiles_p;
+    const int kb0 = ks * p.kblocks / S, n_kb = (ks + 1) * p.kblocks / S - kb0;      // S <= kblocks: every share has work
+    const int quarter = warp & 3, turn = (warp - 2) >> 2;
+    const uint32_t t_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+
+    if (warp == 0) {
+        const int a_row = tp * BM, w_row = tq * BN;
+        const int pre = min(n_kb, C::STAGES);
+        const uint32_t sm0 = smem_u32(smem), full0 = smem_u32(full), empty0 = smem_u32(empty);
+        bool ok = true;
+        // weights first, then the wait for the kernel before this one, then its output
+        if (elected())
+            for (int j = 0; j < pre; j++) {
+                bar_expect(full0 + 8 * j, C::STAGE_BYTES);
+                tile_load(sm0 + j * C::STAGE_BYTES + BM * BK * 2, &map_q, full0 + 8 * j, (kb0 + j) * BK, w_row);
+            }
+        pdl_wait();
+        if (elected())
+            for (int j = 0; j < pre; j++) tile_load(sm0 + j * C::STAGE_BYTES, &map_p, full0 + 8 * j, (kb0 + j) * BK, a_row);
+        __syncwarp();
+        Ring ring;
+        ring.s = pre % C::STAGES; ring.ph = pre / C::STAGES;
+        int it = pre;
+        for (; it < n_kb; it++) {
+            if (!warp_wait(empty0 + 8 * ring.s, ring.ph ^ 1, abort_flag)) { ok = false; break; }
+            const uint32_t st = sm0 + ring.s * C::STAGE_BYTES, bar = full0 + 8 * ring.s;
+            if (elected()) {
+                bar_expect(bar, C::STAGE_BYTES);
+                tile_load(st + BM * BK * 2, &map_q, bar, (kb0 + it) * BK, w_row);
+                tile_load(st, &map_p, bar, (kb0 + it) * BK, a_row);
+            }
+            ring.step<C::STAGES>();
+        }
+        if (!ok && lane == 0) {
+            if (!*abort_flag) { atomicExch(&g_gemm_error, 7); *abort_flag = 1; }
+            for (int back = 1; back <= C::STAGES && back <= it; back++) {
+                const uint32_t j = it - back;
+                mbar_wait(&full[j % C::STAGES], (j / C::STAGES) & 1);
+            }
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = instr_desc(BN);
+        const uint64_t desc0 = smem_desc(smem_u32(smem));
+        const uint32_t lo0 = desc_lo(desc0), hi = desc_hi(desc0), full0 = smem_u32(full), empty0 = smem_u32(empty);
+        Ring ring;
+        bool ok = true;
+        for (int it = 0; it < n_kb; it++) {
+            if (!warp_wait(full0 + 8 * ring.s, ring.ph, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t a_lo = lo0 + ring.s * (C::STAGE_BYTES / 16);
+            if (elected()) issue_kblock<false>(tmem_base, a_lo, a_lo + BM * BK * 2 / 16, hi, idesc, it > 0, empty0 + 8 * ring.s);
+            ring.step<C::STAGES>();
+        }
+        if (ok && elected()) commit_to(smem_u32(acc_full));
+        if (!ok && lane == 0 && !*abort_flag) { atomicExch(&g_gemm_error, 8); *abort_flag = 1; }
+    } else {
+        pdl_wait();                                    // the output may still be read by the kernel before
+        // the decision must be the same in every lane: tcgen05.ld is a warp-wide instruction
+        const bool mine = !*abort_flag && mbar_wait(acc_full, 0);
+        if (!__all_sync(0xffffffffu, mine) && !*abort_flag && lane == 0) { atomicExch(&g_gemm_error, 9); *abort_flag = 1; }
+    }
+    tc_fence_before();
+    cluster_sync();                                    // every share is complete and no CTA's stages are in use any more
+    tc_fence_after();
+    const int row = quarter * 32 + lane;
+    if (warp >= 2) {
+        for (int c = turn; c < CHUNKS; c += EPI_WARPS / 4) {
+            const int owner = c % S;
+            if (owner == ks) continue;
+            uint32_t r[32];
+            tmem_ld32(t_addr + c * 32, r);
+            tmem_ld_wait();
+            // [chunk of the owner][share, without the owner's][column][row]
+            const uint32_t dst = cluster_addr(smem, owner) + ((((c / S) * (S - 1) + (ks < owner ? ks : ks - 1)) * 32) * BM + row) * 4;
+#pragma unroll
+            for (int j = 0; j < 32; j++) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + j * BM * 4), "r"(r[j]) : "memory");
+        }
+    }
+    tc_fence_before();
+    cluster_sync();                                    // all sums are where they are added; nobody touches another CTA any more
+    tc_fence_after();
+    if (warp >= 2) {
+        const float* sums = (const float*)smem;
+        for (int c = turn; c < CHUNKS; c += EPI_WARPS / 4) {
+            if (c % S != ks) continue;
+            uint32_t r[32];
+            tmem_ld32(t_addr + c * 32, r);
+            tmem_ld_wait();
+            const float* src = sums + (size_t)(c / S) * (S - 1) * 32 * BM + row;
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = 0.f;
+            for (int s = 0; s < S; s++) {
+                const float* from = src + (size_t)(s < ks ? s : s - 1) * 32 * BM;
+#pragma unroll
+                for (int j = 0; j < 32; j++) v[j] += s == ks ? __uint_as_float(r[j]) : from[j * BM];
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j++) r[j] = __float_as_uint(v[j]);
+            const int q0 = tq * BN + c * 32;
+            if (p.staged && (GATED ? q0 < p.rows_q : q0 + 32 <= p.rows_q))
+                store_staged<TOut, GATED>(r, smem + C::EPI_OFF + (warp - 2) * EPI_STAGE_BYTES, lane, tp * BM + quarter * 32, q0, p);
+            else store_token_major<TOut, GATED, 32>(r, tp * BM + row, q0, 0, p);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc(tmem_base, BN);
 }
 
 // partial[splits][rows][cols] summed in split order, then cap and conversion.
@@ -769,23 +920,54 @@ static int g_pair_clusters = 0;
 // Sets that policy (for comparisons and tests); returns the previous setting.
 extern "C" int tb_gemm_tc_set_pair(int mode) { const int was = g_pair; g_pair = mode < 0 ? 0 : mode > 2 ? 2 : mode; return was; }
 
-// Where the pair kernel pays.  Its launch costs about a microsecond more (a cluster is placed, two cluster barriers),
-// its main loop runs 5 to 10 % faster.  Measured against the single-SM kernel with weights from memory, 512 to 8,192
-// tokens on the 2B, 9B and 27B shapes: from about 300 k-blocks of work per pair on the pair is 3 to 12 % faster;
-// below, equal or up to 7 % slower.  Whole prompts under sustained load (blocks of twelve repetitions, alternating):
-// 27B shape at 2,048 tokens 98.8 -> 95.0 ms, 2B shape at 8,192 tokens 42.2 -> 41.3 ms, 9B shape at 2,048 equal; the 2B
-// shape at 2,048 tokens has no product that long and does not use it.
-static bool pair_pays(int M, int N, int K) {
-    const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
-    const long long kblocks = (K + BK - 1) / BK;
-    return tiles * kblocks >= 300LL * (g_sms / 2);
+// Which form a product of many tokens takes: the one whose time, by a cost fitted to timed launches, is least.
+//   time = launch + rounds * (round + k-blocks * kblock)      and not less than      launch - 2 + padded operations / rate
+// with a round being as many tiles as the device runs at once.  In microseconds; 249 products of 130 to 3,500 tokens with
+// the 2B, 9B, 27B and a medium model's matrices, weights from memory, in a graph: the form picked takes 0.7 % longer than
+// the best on the mean and 8 % at most, and 13 % less than single SMs and pairs with tiles of 256 alone.  The k-block's
+// time is the MMAs' (128 cycles for 256 x 256 x 16) from 192 columns a pair on, below that the copies'; the rate is what
+// the power cap leaves.  A cluster of two to four CTAs on one tile's K pays where there are few tiles: 384 tokens x 2,304
+// x 9,216: 63 us on single SMs at first, 35 with the loops as they are now, 23 with K cut in two.
+struct TileForm { bool pair; int bn, cluster; };
+static TileForm choose_form(int M, int N, int kblocks) {
+    struct Cost { bool pair; int bn, cluster; double launch, round, kblock, rate; };
+    static const Cost costs[] = {{false, 128, 1, 4.0, 0.9, 0.212, 1.30e9}, {false, 256, 1, 5.0, 0.5, 0.342, 1.50e9},
+                                 {true, 128, 1, 5.0, 0.8, 0.167, 1.45e9},  {true, 192, 1, 6.5, 0.5, 0.227, 1.62e9},
+                                 {true, 224, 1, 7.5, 0.9, 0.254, 1.68e9},  {true, 256, 1, 6.0, 1.0, 0.289, 1.68e9},
+                                 {false, 128, 2, 1.5, 5.0, 0.230, 1.30e9}, {false, 128, 3, 1.5, 5.0, 0.230, 1.30e9},
+                                 {false, 128, 4, 1.5, 5.0, 0.230, 1.30e9}, {false, 256, 3, 1.7, 7.7, 0.375, 1.50e9},
+                                 {false, 256, 4, 1.7, 7.7, 0.375, 1.50e9}};
+    TileForm best = {false, 128, 1};
+    double least = 1e30;
+    for (const Cost& c : costs) {
+        const bool pairs_only = g_pair == 1 && N >= 256;
+        if (c.pair ? (g_pair == 0 || N < 256) : pairs_only) continue;
+        if (c.bn > 128 && N < 256) continue;
+        if (c.cluster > 1 && 2 * c.cluster > kblocks) continue;
+        const long long bm = c.pair ? 256 : BM, tiles = ((M + bm - 1) / bm) * ((N + c.bn - 1) / c.bn);
+        // SMs are handed out a GPC at a time: 45 clusters of three and 33 of four fit the 148 SMs
+        const long long slots = c.pair || c.cluster == 2 ? g_sms / 2 : c.cluster == 1 ? g_sms : c.cluster == 3 ? g_sms * 45 / 148 : g_sms * 33 / 148;
+        const double rounds = (double)((tiles + slots - 1) / (slots > 0 ? slots : 1));
+        const double busy = rounds * (c.round + (kblocks + c.cluster - 1) / c.cluster * c.kblock);
+        const double power = 2.0 * bm * c.bn * BK * (double)tiles * kblocks / c.rate - 2.0;
+        const double t = c.launch + (busy > power ? busy : power);
+        if (t < least) { least = t; best = {c.pair, c.bn, c.cluster}; }
+    }
+    return best;
 }
 
-template <typename TOut, bool GATED>
+// That choice for a product of M > 128 tokens on a device of `sms` SMs: 1000 * CTAs per tile + columns, + 100000 for pairs.
+extern "C" int tb_gemm_tc_form(int M, int N, int K, int sms) {
+    if (!g_sms) g_sms = sms;
+    const TileForm f = choose_form(M, N, (K + BK - 1) / BK);
+    return (f.pair ? 100000 : 0) + 1000 * f.cluster + f.bn;
+}
+
+template <int BN, typename TOut, bool GATED>
 static int launch_pair(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams& p, cudaStream_t stream) {
-    using C = PairCfg;
+    using C = PairCfg<BN>;
     static bool attr_set = false;
-    auto kern = gemm_tc_pair_kernel<TOut, GATED>;
+    auto kern = gemm_tc_pair_kernel<BN, TOut, GATED>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
         if (e != cudaSuccess) return (int)e;
@@ -802,6 +984,28 @@ static int launch_pair(const CUtensorMap& mp, const CUtensorMap& mq, const GemmP
     const int items = p.tiles_p * p.tiles_q * p.splits;
     const int pairs = items < g_pair_clusters ? items : g_pair_clusters;
     tb_launch(kern, dim3(2 * pairs), dim3(GEMM_THREADS), C::SMEM, stream, mp, mq, p);
+    return tb_launch_status();
+}
+
+template <int BN, typename TOut, bool GATED>
+static int launch_split(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams& p, cudaStream_t stream) {
+    using C = Cfg<BN, false>;
+    static bool attr_set = false;
+    auto kern = gemm_tc_split_kernel<BN, TOut, GATED>;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+        if (e != cudaSuccess) return (int)e;
+        attr_set = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.tiles_p * p.tiles_q * p.cluster); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = C::SMEM; cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = p.cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, kern, mp, mq, p);
     return tb_launch_status();
 }
 
@@ -875,18 +1079,17 @@ static int gemm_tc_run(const void* A, const void* W, void* C, int c_dtype, int M
     }
 
     const bool swap = M <= BM;
-    const bool pair = !swap && N >= 256 && (g_pair == 1 || (g_pair == 2 && pair_pays(M, N, K)));
     const bool wide = (long long)N * K * 2 >= (long long)TB_WIDE_FROM_BYTES;
-    int bn;
-    if (swap) bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
-    else {
-        bn = N >= 256 ? 256 : 128;
-        // tiles of 256 weight rows that would leave half of the SMs idle: tiles of 128 finish in about half the time
-        if (bn == 256 && !pair && 2LL * ((M + BM - 1) / BM) * ((N + 255) / 256) <= g_sms) bn = 128;
-    }
+    TileForm form = {false, 128, 1};
+    if (swap) form.bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+    else if (splits > 1) form.bn = N >= 256 ? 256 : 128;               // the caller's own split of K
+    else form = choose_form(M, N, kblocks);
+    const int bn = form.bn;
+    const bool pair = form.pair;
 
     GemmParams p;
     p.tile_group = nullptr; p.group_rows = 0; p.row_scale = nullptr;
+    p.cluster = form.cluster;
     p.staged = splits == 1 && C != nullptr && ((uintptr_t)C & 15) == 0 && (ldc * (c_dtype == TB_BF16 ? 2 : 4)) % 16 == 0;
     p.K = K; p.kblocks = kblocks; p.splits = splits; p.kb_per_split = per;
     p.out = C; p.ld_out = ldc; p.partial = scratch; p.cap = splits > 1 ? 0.f : softcap;
@@ -902,38 +1105,23 @@ static int gemm_tc_run(const void* A, const void* W, void* C, int c_dtype, int M
         if (make_map(&mp, W, N, K, ldw, BM) || make_map(&mq, A, M, K, lda, bn)) return -1;
     } else {
         p.rows_p = M; p.rows_q = N;
-        if (make_map(&mp, A, M, K, lda, BM) || make_map(&mq, W, N, K, ldw, pair ? PairCfg::HALF : bn)) return -1;
+        if (make_map(&mp, A, M, K, lda, BM) || make_map(&mq, W, N, K, ldw, pair ? bn / 2 : bn)) return -1;
     }
     p.tiles_p = (p.rows_p + (pair ? 256 : BM) - 1) / (pair ? 256 : BM);
     p.tiles_q = (p.rows_q + bn - 1) / bn;
 
     int st;
-#define GO(BN_, SW_) (c_dtype == TB_BF16 ? launch<BN_, SW_, bf16>(mp, mq, p, stream) : launch<BN_, SW_, float>(mp, mq, p, stream))
-    if (gated) {
-#define GG(BN_, SW_) launch<BN_, SW_, bf16, true>(mp, mq, p, stream)
-        if (swap) st = bn == 16 ? (wide ? launch<16, true, bf16, true, true>(mp, mq, p, stream) : GG(16, true))
-                     : bn == 32 ? GG(32, true) : bn == 64 ? GG(64, true) : GG(128, true);
-        else if (pair) st = launch_pair<bf16, true>(mp, mq, p, stream);
-        else st = bn == 256 ? GG(256, false) : GG(128, false);
-#undef GG
-    } else if (swap) {
-        switch (bn) {
-        case 16:
-            // a long stream of weights: the kernel's own bytes in flight count for more than the overlap with its
-            // neighbours, so it takes the whole SM
-            if (c_dtype == TB_F32 && wide) st = launch<16, true, float, false, true>(mp, mq, p, stream);
-            else st = GO(16, true);
-            break;
-        case 32: st = GO(32, true); break;
-        case 64: st = GO(64, true); break;
-        default: st = GO(128, true); break;
-        }
-    } else if (pair) {
-        st = c_dtype == TB_BF16 ? launch_pair<bf16, false>(mp, mq, p, stream) : launch_pair<float, false>(mp, mq, p, stream);
-    } else {
-        st = bn == 256 ? GO(256, false) : GO(128, false);
-    }
-#undef GO
+#define OUT3(FN, ...) (gated ? FN<__VA_ARGS__, bf16, true>(mp, mq, p, stream) : c_dtype == TB_BF16 ? FN<__VA_ARGS__, bf16, false>(mp, mq, p, stream) : FN<__VA_ARGS__, float, false>(mp, mq, p, stream))
+    if (swap) {
+        // a long stream of weights: the kernel's own bytes in flight count for more than the overlap with its
+        // neighbours, so it takes the whole SM
+        if (bn == 16) st = wide && gated ? launch<16, true, bf16, true, true>(mp, mq, p, stream)
+                           : wide && c_dtype == TB_F32 ? launch<16, true, float, false, true>(mp, mq, p, stream) : OUT3(launch, 16, true);
+        else st = bn == 32 ? OUT3(launch, 32, true) : bn == 64 ? OUT3(launch, 64, true) : OUT3(launch, 128, true);
+    } else if (p.cluster > 1) st = bn == 256 ? OUT3(launch_split, 256) : OUT3(launch_split, 128);
+    else if (pair) st = bn == 256 ? OUT3(launch_pair, 256) : bn == 224 ? OUT3(launch_pair, 224) : bn == 192 ? OUT3(launch_pair, 192) : OUT3(launch_pair, 128);
+    else st = bn == 256 ? OUT3(launch, 256, false) : OUT3(launch, 128, false);
+#undef OUT3
     if (st) return st;
     if (splits > 1 && reduce) {
         const size_t n = (size_t)M * N;
@@ -976,15 +1164,15 @@ static int gemm_tc_grouped_run(const void* A, const void* W, void* C, int c_dtyp
     p.K = K; p.kblocks = (K + BK - 1) / BK; p.splits = 1; p.kb_per_split = p.kblocks;
     p.out = C; p.ld_out = ldc; p.partial = nullptr; p.cap = 0.f; p.scale = 1.0f;
     p.act = gated ? gated_act : 0; p.limit = 0.f; p.unary = unary;
-    p.staged = ((uintptr_t)C & 15) == 0 && (ldc * (c_dtype == TB_BF16 ? 2 : 4)) % 16 == 0;
+    p.cluster = 1; p.staged = ((uintptr_t)C & 15) == 0 && (ldc * (c_dtype == TB_BF16 ? 2 : 4)) % 16 == 0;
     p.rows_p = M; p.rows_q = N;
     CUtensorMap mp, mq;
     if (make_map(&mp, A, M, K, lda, BM) || make_map(&mq, W, groups * N, K, ldw, bn)) return -1;
     p.tiles_p = (M + BM - 1) / BM;
     p.tiles_q = (N + bn - 1) / bn;
     if (gated) return bn == 256 ? launch<256, false, bf16, true>(mp, mq, p, stream) : launch<128, false, bf16, true>(mp, mq, p, stream);
-    if (c_dtype == TB_BF16) return bn == 256 ? launch<256, false, bf16>(mp, mq, p, stream) : launch<128, false, bf16>(mp, mq, p, stream);
-    return bn == 256 ? launch<256, false, float>(mp, mq, p, stream) : launch<128, false, float>(mp, mq, p, stream);
+    if (c_dtype == TB_BF16) return bn == 256 ? launch<256, false, bf16, false>(mp, mq, p, stream) : launch<128, false, bf16, false>(mp, mq, p, stream);
+    return bn == 256 ? launch<256, false, float, false>(mp, mq, p, stream) : launch<128, false, float, false>(mp, mq, p, stream);
 }
 
 extern "C" int tb_gemm_tc_grouped(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
