@@ -137,65 +137,69 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         // ---------------- loads, and the second product's MMAs ----------------
         // (One thread can issue an MMA every fifty cycles or so; the first product's MMAs run no longer than that.
         //  So the two products have an issuing thread each, and neither waits behind the other's operands.)
-        if (lane == 0) {
-            pdl_wait();
-            constexpr uint32_t idesc_o = instr_desc(HD) | (1u << 16);           // B (= V) is MN-major
-            const uint32_t hi = desc_hi(smem_desc(0));
-            const uint32_t p_lo0 = desc_lo(smem_desc(smem_u32(sP)));
-            // V: panels of 64 dims lie BN * 128 bytes apart (leading-dimension offset, bits 16..29 of the low half);
-            // groups of 8 keys 1024 bytes apart, which is the stride offset that the K-major operands have too
-            const uint32_t v_lo0 = ((smem_u32(sV) & 0x3ffff) >> 4) | ((uint32_t)((BN * 128) >> 4) << 16);
-            bool ok = true;
-            // K tiles, V^T tiles and the second products are started independently, each as soon as it has what it
-            // needs: the scores run up to two blocks ahead of the second product, and so must the K tiles
-            int jk = 0, jv = 0, jp = 0;
-            long long idle_since = clock64();
-            while (ok && jp < nblocks) {
-                bool moved = false;
-                if (jk < nblocks && mbar_test(&k_empty[jk & 1], ((jk >> 1) & 1) ^ 1)) {
-                    const int s = jk & 1, key0 = (nb_lo + jk) * BN;
+        pdl_wait();
+        constexpr uint32_t idesc_o = instr_desc(HD) | (1u << 16);           // B (= V) is MN-major
+        const uint32_t hi = desc_hi(smem_desc(0));
+        const uint32_t p_lo0 = desc_lo(smem_desc(smem_u32(sP)));
+        // V: panels of 64 dims lie BN * 128 bytes apart (leading-dimension offset, bits 16..29 of the low half);
+        // groups of 8 keys 1024 bytes apart, which is the stride offset that the K-major operands have too
+        const uint32_t v_lo0 = ((smem_u32(sV) & 0x3ffff) >> 4) | ((uint32_t)((BN * 128) >> 4) << 16);
+        bool ok = true;
+        // K tiles, V^T tiles and the second products are started independently, each as soon as it has what it
+        // needs: the scores run up to two blocks ahead of the second product, and so must the K tiles
+        int jk = 0, jv = 0, jp = 0;
+        long long idle_since = clock64();
+        while (ok && jp < nblocks) {
+            bool moved = false;
+            if (jk < nblocks && warp_test(&k_empty[jk & 1], ((jk >> 1) & 1) ^ 1)) {
+                const int s = jk & 1, key0 = (nb_lo + jk) * BN;
+                if (elected()) {
                     mbar_expect_tx(&k_full[s], K_BYTES);
                     for (int c = 0; c < QBOXES; c++)
                         tma_load_2d(sK + s * K_BYTES + c * BN * 128, &map_k, &k_full[s], kvh * HD + c * 64, s0 + key0);
-                    jk++; moved = true;
                 }
-                if (jv < nblocks && mbar_test(&v_empty[jv & 1], ((jv >> 1) & 1) ^ 1)) {
-                    const int s = jv & 1, key0 = (nb_lo + jv) * BN;
+                jk++; moved = true;
+            }
+            if (jv < nblocks && warp_test(&v_empty[jv & 1], ((jv >> 1) & 1) ^ 1)) {
+                const int s = jv & 1, key0 = (nb_lo + jv) * BN;
+                if (elected()) {
                     mbar_expect_tx(&v_full[s], V_BYTES);
                     for (int c = 0; c < QBOXES; c++)
                         tma_load_2d(sV + s * V_BYTES + c * BN * 128, &map_v, &v_full[s], kvh * HD + c * 64, s0 + key0);
-                    jv++; moved = true;
                 }
-                if (mbar_test(&v_full[jp & 1], (jp >> 1) & 1) && mbar_test(&p_full[jp & 1], (jp >> 1) & 1)) {
-                    const int s = jp & 1;
-                    tc_fence_after();
-                    const uint32_t p_lo = p_lo0 + s * (P_BYTES >> 4), v_lo = v_lo0 + s * (V_BYTES >> 4);
+                jv++; moved = true;
+            }
+            if (warp_test(&p_full[jp & 1], (jp >> 1) & 1) && warp_test(&v_full[jp & 1], (jp >> 1) & 1)) {
+                const int s = jp & 1;
+                tc_fence_after();
+                const uint32_t p_lo = p_lo0 + s * (P_BYTES >> 4), v_lo = v_lo0 + s * (V_BYTES >> 4);
+                if (elected()) {
 #pragma unroll
                     for (int ks = 0; ks < BN / UMMA_K; ks++)          // 16 keys on: 32 bytes in a row of P, 16 rows of V
                         umma_bf16_lh(tmem_o, p_lo + ks * 2, v_lo + ks * ((UMMA_K * 128) >> 4), hi, idesc_o,
                                      (jp > 0 || ks > 0) ? 1u : 0u);
                     umma_commit(&v_empty[s]);         // V tile and P buffer are free again; O holds blocks 0..jp
-                    jp++; moved = true;
                 }
-                if (moved) idle_since = clock64();
-                else if (*abort_flag || clock64() - idle_since > WAIT_CYCLES) ok = false;
+                jp++; moved = true;
             }
-            if (!ok && !*abort_flag) { atomicExch(&g_attn_tc_error, 1); *abort_flag = 1; }
+            if (moved) idle_since = clock64();
+            else if (__any_sync(0xffffffffu, *abort_flag || clock64() - idle_since > WAIT_CYCLES)) ok = false;
         }
+        if (!ok && lane == 0 && !*abort_flag) { atomicExch(&g_attn_tc_error, 1); *abort_flag = 1; }
     } else if (warp == 1) {
         // ---------------- the first product's MMAs ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = instr_desc(BN);
-            const uint32_t hi = desc_hi(smem_desc(0));
-            const uint32_t k_lo0 = desc_lo(smem_desc(smem_u32(sK)));
-            bool ok = mbar_wait(q_full, 0);
-            // the scores of block j + 2 are issued when S of block j has been read, long before P of block j exists:
-            // the softmax does not wait for them
-            for (int j = 0; j < nblocks && ok; j++) {
-                const int s = j & 1; const uint32_t ph = (j >> 1) & 1;
-                if (*abort_flag || !mbar_wait(&k_full[s], ph) || !mbar_wait(&s_empty[s], ph ^ 1)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t k_lo = k_lo0 + s * (K_BYTES >> 4), d = tmem_s + s * BN;
+        constexpr uint32_t idesc_s = instr_desc(BN);
+        const uint32_t hi = desc_hi(smem_desc(0));
+        const uint32_t k_lo0 = desc_lo(smem_desc(smem_u32(sK)));
+        bool ok = warp_wait(q_full, 0, abort_flag);
+        // the scores of block j + 2 are issued when S of block j has been read, long before P of block j exists:
+        // the softmax does not wait for them
+        for (int j = 0; j < nblocks && ok; j++) {
+            const int s = j & 1; const uint32_t ph = (j >> 1) & 1;
+            if (!warp_wait(&k_full[s], ph, abort_flag) || !warp_wait(&s_empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t k_lo = k_lo0 + s * (K_BYTES >> 4), d = tmem_s + s * BN;
+            if (elected()) {
 #pragma unroll
                 for (int ks = 0; ks < HD / UMMA_K; ks++)
                     umma_bf16_ta_lh(d, tmem_q + ks * (UMMA_K / 2), k_lo + (((ks >> 2) * (BN * 128) + (ks & 3) * 32) >> 4), hi,
@@ -203,8 +207,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 umma_commit(&k_empty[s]);             // K tile may be overwritten once these have run
                 umma_commit(&s_full[s]);              // and S is ready for the softmax
             }
-            if (!ok && !*abort_flag) { atomicExch(&g_attn_tc_error, 2); *abort_flag = 1; }
         }
+        if (!ok && lane == 0 && !*abort_flag) { atomicExch(&g_attn_tc_error, 2); *abort_flag = 1; }
     } else {
         // ---------------- softmax: one thread per query row and group; group g takes the blocks j = g, g + 2, .. ----------------
         const int sw = warp - 2;                                     // 0..7
