@@ -851,6 +851,28 @@ def test_attn_prefill_tc_long(ops, nh, nkv, hd, cap, window, lens):
         close(ref[s].view(n, nh, hd)[sub], want[sub], torch.bfloat16, 2.0)
 
 
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("reach", [0.3, 1.0, 30.0, 3000.0])
+def test_attn_prefill_cap_near_and_far(ops, hd, reach):
+    """The soft cap where all scores lie within half of it, around half of it and far past it (``reach``: scores over the
+    cap at most), every warp with some rows of each; probabilities and the result are rounded to bfloat16 once each."""
+    n, cap = 333, 8.0
+    q, k, v = (rnd(n, hd, dt=torch.bfloat16, seed=i) for i in range(3))
+    most = float((q.double() @ k.double().T).abs().max())
+    scale = reach * cap / most
+    q[::3] *= 0.25
+    starts = torch.tensor([0, n], dtype=torch.int32, device="cuda")
+    got = ops.attn_prefill_tc(q, k, v, starts, [n], 1, 1, hd, scale, cap, 0).double()
+    s = cap * torch.tanh(q.double() @ k.double().T * scale / cap)
+    s = s.masked_fill(torch.ones(n, n, device="cuda", dtype=torch.bool).triu(1), -math.inf)
+    want = torch.softmax(s, -1) @ v.double()
+    assert float((got - want).norm() / want.norm()) < 5e-3
+    # the negative of a query mirrors its scores about 0
+    back = ops.attn_prefill_tc(-q, -k, v, starts, [n], 1, 1, hd, scale, cap, 0).double()
+    assert torch.equal(back, got)
+    assert ops.attn_prefill_tc_error(hd) == 0
+
+
 def test_attn_prefill_far_key_and_window_edge(ops):
     """A key made to stand out is seen from far away without a window, and exactly up to the window's
     edge with one; on tensor cores and on the generic kernel alike."""
