@@ -269,6 +269,19 @@ __device__ __forceinline__ void tile_load(uint32_t dst, const CUtensorMap* map, 
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1) : "memory");
 }
+// The same for data that a step reads once, the first to leave L2: the weights of products of few tokens.  A decode step
+// streams more of them than L2 holds (2B shape: 156 MB a layer), and what went with them were the small kernels between
+// the products: their instructions, the partial sums, keys and values.  Step of one sequence, 2B shape: 1,585 -> 1,450 us.
+__device__ __forceinline__ uint64_t once_policy() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void tile_load_once(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+        ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void tile_load_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int c0, int c1) {
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -344,6 +357,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
         // ---------------- TMA producer ----------------
         const uint32_t sm0 = smem_u32(smem), full0 = smem_u32(full), empty0 = smem_u32(empty);
         uint32_t it = 0;
+        const uint64_t policy = once_policy();
+        auto w_load = [&](uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+            if (SWAP) tile_load_once(dst, map, bar, c0, c1, policy); else tile_load(dst, map, bar, c0, c1);
+        };
         Ring ring;
         bool ok = true, waited = false;
         // the tile that holds weights: the 128-lane operand when swapped, else the BN-column one
@@ -371,7 +388,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                 if (elected())
                     for (int j = 0; j < pre; j++) {
                         bar_expect(full0 + 8 * j, C::STAGE_BYTES);
-                        tile_load(sm0 + j * C::STAGE_BYTES + W_OFF, wmap, full0 + 8 * j, (kb0 + j) * BK, w_row);
+                        w_load(sm0 + j * C::STAGE_BYTES + W_OFF, wmap, full0 + 8 * j, (kb0 + j) * BK, w_row);
                     }
                 pdl_wait();
                 waited = true;
@@ -387,7 +404,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                 const uint32_t st = sm0 + ring.s * C::STAGE_BYTES, bar = full0 + 8 * ring.s;
                 if (elected()) {
                     bar_expect(bar, C::STAGE_BYTES);
-                    tile_load(st + W_OFF, wmap, bar, kb * BK, w_row);
+                    w_load(st + W_OFF, wmap, bar, kb * BK, w_row);
                     tile_load(st + A_OFF, amap, bar, kb * BK, a_row);
                 }
                 ring.step<C::STAGES>();
