@@ -363,7 +363,9 @@ __global__ void __launch_bounds__(DCfg<HD>::NWARP * 32, 1) attn_decode_kernel(De
 #define TW 8                                       // warps that compute: 0..3 the scores, 4..7 the outputs
 #define NTHREADS ((TW + 1) * 32)                   // and one warp that issues the page copies
 #define SROW 72                                    // floats between heads in the score arrays (64 keys + 8: no bank conflicts)
-template <int HD, bool STREAM> struct MCfg {
+// FUSED (split only): q, k and v come as the product's partial sums.  An instance of its own, so that a call with q given
+// does not pay for the registers (43.6 us with it, 43.9 in one kernel, eight contexts of 8,000).
+template <int HD, bool STREAM, bool FUSED = false> struct MCfg {
     static constexpr int BOXES = HD / 64;                            // 64-dim column boxes per page
     static constexpr int BOX_BYTES = PAGE * 128;                     // 64 keys x 128 bytes, swizzled
     static constexpr int TILE_BYTES = BOXES * BOX_BYTES;             // one page of K (or V)
@@ -380,6 +382,7 @@ template <int HD, bool STREAM> struct MCfg {
     static constexpr int SCORE_FLOATS = 2 * 8 * SROW + 2 * 8 * 4;    // two pages' scores, and their maxima per score warp
     static constexpr int SMEM = STAGES * STAGE_BYTES + SCORE_FLOATS * 4 + 192 /* barriers */ + (1024 + 4) * 4 /* stream: page prefix */
                                 + 8 * HD * 2 /* rotated queries */ + 10 * HD * 4 /* this step's q, k, v, summed */
+                                + (FUSED ? 2 * HD * 2 + HD * 4 : 0) /* the new token's k and v, the rotation's cosines and sines */
                                 + 32 /* fold job, abort flag */ + 1024 /* alignment */;
 };
 // byte offset of (key row r, 16-byte chunk c of the head dim) inside a swizzled page
@@ -433,12 +436,12 @@ struct PageCursor {
     int left;                  // pages still to visit
 };
 
-template <int HD, bool STREAM>
-__global__ void __launch_bounds__(NTHREADS, MCfg<HD, STREAM>::CTAS_PER_SM)
+template <int HD, bool STREAM, bool FUSED>
+__global__ void __launch_bounds__(NTHREADS, MCfg<HD, STREAM, FUSED>::CTAS_PER_SM)
 attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, DecodeArgs a,
                        int batch) {
     pdl_launch_dependents();
-    using C = MCfg<HD, STREAM>;
+    using C = MCfg<HD, STREAM, FUSED>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     float* sf = (float*)(smem + C::STAGES * C::STAGE_BYTES);         // [page parity][8 heads][SROW] scores: scaled, capped, masked
@@ -452,7 +455,9 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     bf16* q_s = (bf16*)(pref + 1024 + 4);                            // [8 heads][HD] this run's queries, rotated (fused rotation)
     float* fold_s = (float*)(q_s + 8 * HD);                          // [G heads of q, then k, then v][HD]: the partial sums added up
     // (no static shared memory: two CTAs of this kernel fill an SM's shared memory to the last kilobyte)
-    int* misc = (int*)(fold_s + 10 * HD);
+    bf16* new_s = (bf16*)(fold_s + 10 * HD);                         // fused split: [k, v][HD] of the new token, as they go to the cache
+    float2* turn_s = (float2*)(new_s + 2 * HD);                      // fused split: [HD / 2] cosine and sine of each rotated pair
+    int* misc = FUSED ? (int*)(turn_s + HD / 2) : (int*)(fold_s + 10 * HD);
     int& s_last = misc[0];                          // split: this CTA folds the pair below
     int* s_job = misc + 1;                          // the pair to fold (sequence, kv head, parts)
     volatile int& s_abort = *(volatile int*)(misc + 4);
@@ -556,16 +561,41 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         issued++;
         advance(ahead);
     };
+    static_assert(!(STREAM && FUSED), "the stream partition decides at run time");
+    const bool fused = STREAM ? a.qkv_part != nullptr : FUSED;
+    const int half = (a.inv_freq != nullptr) ? (a.rotary_dim >> 1) : 0;      // rotated pairs per head
+    const int per = HD - half;                                               // items of a head: rotated pairs, then dims beyond them
+    const int k_off = a.n_heads * HD, v_off = (a.n_heads + a.n_kv_heads) * HD;
+    // where the new token's k and v rows of (sequence b, kv head kvh) lie in the pools
+    auto new_row = [&](int b, int kvh) -> size_t {
+        const int pos = a.len_after[b] - 1;
+        const int r = (a.ring_rows > 0) ? pos % a.ring_rows : pos;
+        const int page = a.page_table[(size_t)b * a.pt_stride + r / PAGE];
+        return ((size_t)(page * a.n_kv_heads + kvh) * PAGE + (r % PAGE)) * HD;
+    };
+    // Split, fused: what does not need the product, before the wait: the angles, and where the new token's rows lie.
+    size_t new_off = 0;
+    bool hot_here = false;                           // this CTA's run holds the page of the new token (no other's does)
+    if constexpr (FUSED) {
+        const int hot_rel = cur.hot - cur.first_page;
+        hot_here = cur.left > 0 && hot_rel >= cur.pg && hot_rel < cur.pg + cur.left;
+        if (hot_here) new_off = new_row(cur.b, cur.kvh);
+        if (tid < half) {
+            float sn, cs;
+            sincosf((float)(a.len_after[cur.b] - 1) * a.inv_freq[tid], &sn, &cs);
+            turn_s[tid] = make_float2(cs, sn);
+        }
+    }
     // pages that this step does not write were complete before the step began: fetch them at once
     if (tid == ISSUER)
         while (ahead.left > 0 && issued < C::STAGES && ahead.first_page + ahead.pg != ahead.hot) issue();
     pdl_wait();                                     // the new token's cache rows and q come from earlier kernels
+    // The page of the new token too, now that it is as the step before left it.  (Split, fused: its new row is put into the
+    // stage by the warps that read it; stream: the rows are written to the cache first, below.)
+    if (tid == ISSUER && !(fused && STREAM))
+        while (ahead.left > 0 && issued < C::STAGES) issue();
 
     // ---- fused rotation: this step's q, k, v come as partial sums of their product
-    const bool fused = a.qkv_part != nullptr;
-    const int half = (a.inv_freq != nullptr) ? (a.rotary_dim >> 1) : 0;      // rotated pairs per head
-    const int per = HD - half;                                               // items of a head: rotated pairs, then dims beyond them
-    const int k_off = a.n_heads * HD, v_off = (a.n_heads + a.n_kv_heads) * HD;
     // Adds up partial sums into fold_s: segment g (HD columns) is the piece of sequence seg_b(g)'s row that begins at
     // column seg_col(g).  Every partial sum that is needed is requested at once, four columns a thread and eight
     // splits each, and added in the splits' order: one wait for memory.  For the nthr threads t0 = 0 .. nthr - 1.
@@ -608,13 +638,6 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             dst[x + half] = __float2bfloat16_rn(hsrc[x + half]);
         }
     };
-    // where the new token's k and v rows of (sequence b, kv head kvh) lie in the pools
-    auto new_row = [&](int b, int kvh) -> size_t {
-        const int pos = a.len_after[b] - 1;
-        const int r = (a.ring_rows > 0) ? pos % a.ring_rows : pos;
-        const int page = a.page_table[(size_t)b * a.pt_stride + r / PAGE];
-        return ((size_t)(page * a.n_kv_heads + kvh) * PAGE + (r % PAGE)) * HD;
-    };
     // k (32-bit at ksrc) rotated and v (at vsrc) rounded into the new token's rows, by the nthr threads t0 = 0 .. nthr - 1
     auto append_kv = [&](int b, int kvh, const float* ksrc, const float* vsrc, int t0, int nthr) {
         const size_t off = new_row(b, kvh);
@@ -626,28 +649,49 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             else vd[x - per] = __float2bfloat16_rn(vsrc[x - per]);
         }
     };
-    if (fused && !STREAM) {
+    if constexpr (FUSED) {
         // Split: the CTA has one run.  It needs its G query heads; k and v too if its run holds the page of the new
-        // token, which this CTA and no other reads.
-        const int pos = a.len_after[cur.b] - 1;
-        const int hot_rel = cur.hot - cur.first_page;
-        const bool hot_here = cur.left > 0 && hot_rel >= cur.pg && hot_rel < cur.pg + cur.left;
+        // token, which this CTA and no other reads.  They go to the cache for the steps to come and, for this one, to
+        // shared memory, from where the warps that read the page put them into its stage: waiting for the stores and
+        // only then fetching the page was 3 us of a short context's 11.
         if (warp < TW)
             bulk_sum(G + (hot_here ? 2 : 0), [&](int) { return cur.b; },
                      [&](int g) { return g < G ? (cur.kvh * G + g) * HD : g == G ? k_off + cur.kvh * HD : v_off + cur.kvh * HD; },
                      tid, TW * 32);
         __syncthreads();
         if (warp < TW) {
-            for (int x = tid; x < G * per; x += TW * 32) rotate_from(fold_s + (x / per) * HD, q_s + (x / per) * HD, x % per, pos);
-            if (hot_here) {
-                append_kv(cur.b, cur.kvh, fold_s + G * HD, fold_s + (G + 1) * HD, tid, TW * 32);
-                // the rows were written by ordinary stores and are read by the copy engine next
-                __threadfence();
-                asm volatile("fence.proxy.async;" ::: "memory");
+            auto turned = [&](const float* src, int x, float& lo, float& hi) {       // pair x < half
+                const float2 cs = turn_s[x];
+                const float x0 = src[x], x1 = src[x + half];
+                lo = x0 * cs.x - x1 * cs.y;
+                hi = x1 * cs.x + x0 * cs.y;
+            };
+            for (int y = tid; y < (G + (hot_here ? 1 : 0)) * per; y += TW * 32) {
+                const int g = y / per, x = y % per;
+                const float* src = fold_s + g * HD;
+                bf16* dst = g < G ? q_s + g * HD : new_s;
+                bf16* far = g < G ? nullptr : (bf16*)a.k_pool + new_off;
+                if (x < half) {
+                    float lo, hi;
+                    turned(src, x, lo, hi);
+                    const bf16 l16 = __float2bfloat16_rn(lo), h16 = __float2bfloat16_rn(hi);
+                    dst[x] = l16; dst[x + half] = h16;
+                    if (far) { far[x] = l16; far[x + half] = h16; }
+                } else {
+                    const bf16 v16 = __float2bfloat16_rn(src[x + half]);
+                    dst[x + half] = v16;
+                    if (far) far[x + half] = v16;
+                }
             }
+            if (hot_here)
+                for (int x = tid; x < HD; x += TW * 32) {
+                    const bf16 v16 = __float2bfloat16_rn(fold_s[(G + 1) * HD + x]);
+                    new_s[HD + x] = v16;
+                    ((bf16*)a.v_pool)[new_off + x] = v16;
+                }
         }
         __syncthreads();
-    } else if (fused) {
+    } else if (STREAM && fused) {
         // Stream: the CTA has one run or several.  Those that hold the page of their sequence's new token (this CTA,
         // and no other, reads that page) get the token's k and v rows written first; the first run's query heads go
         // to shared memory.  In passes of up to ten heads' worth of partial sums (what fold_s holds): the first pass
@@ -703,10 +747,13 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         asm volatile("fence.proxy.async;" ::: "memory");
         __syncthreads();
     }
-    if (tid == ISSUER) {
-        if (fused) asm volatile("fence.proxy.async;" ::: "memory");
+    if (tid == ISSUER && fused && STREAM) {
+        asm volatile("fence.proxy.async;" ::: "memory");
         while (ahead.left > 0 && issued < C::STAGES) issue();
     }
+    // split, fused: the page (counted from the run's first) and the row in it that take the new token
+    const int hot_page = hot_here ? cur.hot - cur.first_page - cur.pg : -1;
+    const int hot_row = hot_here ? (int)((new_off / HD) % PAGE) : 0;
 
     const float inv_cap = a.cap > 0.f ? 1.f / a.cap : 0.f;
     const uint32_t smem_base = smem_u32(smem);
@@ -821,6 +868,13 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 const uint32_t stage = smem_base + s * C::STAGE_BYTES;
                 const int row0 = (seg_first + seg_pg0 + j) * PAGE;
                 const bool all_ok = page_all_keys(row0);
+                const bool patch = FUSED && j == hot_page && hot_row / 16 == mt;      // this warp's keys hold the new token's
+                if (patch) {
+                    for (int x = lane; x < HD / 8; x += 32)
+                        *(uint4*)(smem + s * C::STAGE_BYTES + sw_off(hot_row, x)) = *(const uint4*)(new_s + x * 8);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copy engine refills the stage later
+                    __syncwarp();
+                }
                 float c[4][4];                                       // four chains: the MMAs of a chain wait for one another
 #pragma unroll
                 for (int x = 0; x < 4; x++) { c[x][0] = c[x][1] = c[x][2] = c[x][3] = 0.f; }
@@ -923,6 +977,13 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 const uint32_t stage = smem_base + s * C::STAGE_BYTES;
                 const int row0 = (seg_first + seg_pg0 + j) * PAGE;
                 const bool all_ok = page_all_keys(row0);
+                if (FUSED && j == hot_page) {
+                    // the new token's values, in the columns that this warp reads
+                    if (lane < HD / 32)
+                        *(uint4*)(smem + s * C::STAGE_BYTES + C::TILE_BYTES + sw_off(hot_row, d0 / 8 + lane)) = *(const uint4*)(new_s + HD + d0 + lane * 8);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                }
                 if (!all_ok) {
                     // rows of the page that are not keys: their probabilities are 0, but 0 * NaN would still poison O,
                     // so this warp zeroes them in the columns it reads
@@ -1145,11 +1206,11 @@ static int pool_map(CUtensorMap* m, const void* pool, long long rows, int hd) {
     return 0;
 }
 
-template <int HD, bool STREAM>
+template <int HD, bool STREAM, bool FUSED = false>
 static int launch_mma(const DecodeArgs& a, int batch, int n_ctas, cudaStream_t stream) {
-    using C = MCfg<HD, STREAM>;
+    using C = MCfg<HD, STREAM, FUSED>;
     static bool attr_set = false;
-    auto kern = attn_decode_mma_kernel<HD, STREAM>;
+    auto kern = attn_decode_mma_kernel<HD, STREAM, FUSED>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
         if (e != cudaSuccess) return (int)e;
@@ -1255,9 +1316,9 @@ static int run_decode(const DecodeArgs* args, int dtype, int batch, bool tensor_
     } else if (a.q == nullptr) return tb_refuse("attn_decode: q is missing");
     if (tensor_cores) {
         switch (a.hd) {
-        case 64: st = launch_mma<64, false>(a, batch, 0, stream); break;
-        case 128: st = launch_mma<128, false>(a, batch, 0, stream); break;
-        default: st = launch_mma<256, false>(a, batch, 0, stream); break;
+        case 64: st = a.qkv_part ? launch_mma<64, false, true>(a, batch, 0, stream) : launch_mma<64, false>(a, batch, 0, stream); break;
+        case 128: st = a.qkv_part ? launch_mma<128, false, true>(a, batch, 0, stream) : launch_mma<128, false>(a, batch, 0, stream); break;
+        default: st = a.qkv_part ? launch_mma<256, false, true>(a, batch, 0, stream) : launch_mma<256, false>(a, batch, 0, stream); break;
         }
     } else {
     if (!(g == 1 || g == 2 || g == 4 || g == 8))
@@ -1291,11 +1352,11 @@ static int run_decode(const DecodeArgs* args, int dtype, int batch, bool tensor_
 // zeroed counters, which the launch leaves at zero.
 // CTAs of the tensor-core kernel that fit an SM together (the stream partition's shared memory and registers are
 // budgeted for two at heads narrower than 256; one everywhere else); -1 on error.
-template <int HD, bool STREAM> static int mma_occupancy() {
-    using C = MCfg<HD, STREAM>;
+template <int HD, bool STREAM, bool FUSED = false> static int mma_occupancy() {
+    using C = MCfg<HD, STREAM, FUSED>;
     int n = 0;
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD, STREAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<HD, STREAM>, NTHREADS, C::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD, STREAM, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<HD, STREAM, FUSED>, NTHREADS, C::SMEM);
     return e == cudaSuccess ? n : -1;
 }
 extern "C" int tb_attn_decode_occupancy(int hd, int stream_partition) {
