@@ -851,6 +851,42 @@ def test_attn_prefill_tc_long(ops, nh, nkv, hd, cap, window, lens):
         close(ref[s].view(n, nh, hd)[sub], want[sub], torch.bfloat16, 2.0)
 
 
+def moe_rule(ops, T, top, E, W, ff, gated):
+    return ops.moe_tile(T * top, E, (3 if gated else 2) * W * ff * 2)
+
+
+# tokens, experts a token, experts, width, ff, the tile that the rule picks
+MOE_TILES = [(12, 4, 32, 2048, 1024, 16), (33, 4, 8, 136, 48, 32), (200, 2, 16, 96, 208, 64), (700, 2, 6, 72, 16, 128), (128, 1, 40, 264, 144, 16)]
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("on", ["input", "output"])
+@pytest.mark.parametrize("T,top,E,W,ff,tile", MOE_TILES)
+def test_moe_experts_by_tiles(ops, gated, on, T, top, E, W, ff, tile):
+    """Experts' products grouped in tiles of every size: some experts without a pair, one with more than a tile's, sizes
+    that fill no tile of weight rows.  act and the operands are rounded to bfloat16 once each, sums are 32-bit."""
+    assert moe_rule(ops, T, top, E, W, ff, gated) == tile or not gated
+    g = torch.Generator().manual_seed(T)
+    idx = torch.stack([torch.randperm(E - 1, generator=g)[:top] for _ in range(T)])          # the last expert has none
+    idx[: T // 2, 0] = torch.where((idx[: T // 2] == 1).any(1), idx[: T // 2, 0], torch.ones(T // 2, dtype=torch.long))
+    idx, weight = idx.to("cuda", torch.int32), rnd(T, top, seed=3).abs() + 0.1
+    x = rnd(T, W, dt=torch.bfloat16)
+    gw, uw, dw = (rnd(E, *s, dt=torch.bfloat16, s=0.1, seed=i) for i, s in enumerate(((ff, W), (ff, W), (W, ff))))
+    both = torch.stack([ops.interleave_gate_up(gw[e], uw[e]) for e in range(E)]) if gated else None
+    got = ops.moe_experts(x, gw if gated else None, uw, dw, idx, weight, gate_up_w=both, weight_on=on)
+    want = torch.zeros(T, W, dtype=torch.float64, device="cuda")
+    for k in range(top):
+        e, w = idx[:, k].long(), weight[:, k, None].double()
+        xs = x.double() * (w if on == "input" else 1.0)
+        u = torch.stack([uw[e[t]].double() @ xs[t] for t in range(T)])
+        a = torch.relu(u) ** 2
+        if gated:
+            a = torch.nn.functional.silu(torch.stack([gw[e[t]].double() @ xs[t] for t in range(T)])) * u
+        want += torch.stack([dw[e[t]].double() @ a[t] for t in range(T)]) * (1.0 if on == "input" else w)
+    assert float((got.double() - want).norm() / want.norm()) < 4e-3
+    assert ops.kernel_errors() == {}
+
+
 @pytest.mark.parametrize("hd", [64, 128, 256])
 @pytest.mark.parametrize("reach", [0.3, 1.0, 30.0, 3000.0])
 def test_attn_prefill_cap_near_and_far(ops, hd, reach):

@@ -55,9 +55,9 @@ struct GemmParams {
     int act;                         // gated epilogue: 0 gelu_tanh, 1 silu, 2 clamped_swish (only with GATED kernels)
     float limit;                     // clamped_swish: both branches are bounded by it
     int unary;                       // plain epilogues: 0 nothing, 1 every output becomes relu(v)^2, 2 v Phi(v) (never on partial sums)
-    // Grouped products (token-major tiles only): tile tp of the tokens multiplies the weight rows of group
-    // tile_group[tp], which start at row tile_group[tp] * group_rows of the weight operand; a negative entry: the tile
-    // is not in use and nobody touches it.  Null: one group.
+    // Grouped products: a tile of tokens (128 rows, or the BN of swapped tiles) multiplies the weight rows of its group
+    // tile_group[tile], which start at row tile_group[tile] * group_rows of the weight operand; a negative entry: the tile
+    // is not in use and nobody touches it.
     const int* tile_group;
     int group_rows;
     int staged;                      // the rows of C are made of whole 16-byte pieces: chunks of 32 columns are stored through shared memory
@@ -315,7 +315,8 @@ __device__ __forceinline__ void issue_kblock(uint32_t d_addr, uint32_t a_lo, uin
     if (PAIR) commit_to_pair(empty); else commit_to(empty);
 }
 
-template <int BN, bool SWAP, typename TOut, bool GATED, bool WIDE>
+// GROUPED: see GemmParams::tile_group.
+template <int BN, bool SWAP, typename TOut, bool GATED, bool WIDE, bool GROUPED>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_q, GemmParams p) {
     pdl_launch_dependents();
@@ -372,10 +373,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
             const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
             int w_row = SWAP ? tp * BM : tq * BN;
             const int a_row = SWAP ? tq * BN : tp * BM;
-            if (!SWAP && p.tile_group != nullptr) {
+            if constexpr (GROUPED) {
                 // the table of groups is the preceding kernel's work: nothing is fetched before it is there
                 if (!waited) { pdl_wait(); waited = true; }
-                const int g = p.tile_group[tp];
+                const int g = p.tile_group[SWAP ? tq : tp];
                 if (g < 0) continue;               // a tile past the last one in use: all three roles leave it out
                 w_row += g * p.group_rows;
             }
@@ -428,10 +429,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
         uint32_t tile_it = 0;
         Ring ring;
         bool ok = true;
-        if (!SWAP && p.tile_group != nullptr) pdl_wait();      // the table of groups is the preceding kernel's work
+        if (GROUPED) pdl_wait();      // the table of groups is the preceding kernel's work
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
             int tp, tq, sp; decode(item, tp, tq, sp);
-            if (!SWAP && p.tile_group != nullptr && p.tile_group[tp] < 0) continue;
+            if (GROUPED && p.tile_group[SWAP ? tq : tp] < 0) continue;
             const int kb0 = sp * p.kb_per_split, kb1 = min(p.kblocks, kb0 + p.kb_per_split);
             const int a = tile_it & 1; const uint32_t aph = (tile_it >> 1) & 1;
             tile_it++;
@@ -458,7 +459,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
             int tp, tq, sp; decode(item, tp, tq, sp);
-            if (!SWAP && p.tile_group != nullptr && p.tile_group[tp] < 0) continue;
+            if (GROUPED && p.tile_group[SWAP ? tq : tp] < 0) continue;
             const int a = tile_it & 1; const uint32_t aph = (tile_it >> 1) & 1;
             tile_it++;
             // the decision must be the same in every lane: tcgen05.ld is a warp-wide instruction
@@ -474,8 +475,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                 if (CH == 32) tmem_ld32(t_addr + c0, r); else tmem_ld16(t_addr + c0, r);
                 tmem_ld_wait();
                 const int q0 = tq * BN + c0;                           // first row of Q in this chunk
+                if (GROUPED && SWAP && p.row_scale != nullptr) {
+#pragma unroll
+                    for (int j = 0; j < CH; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * p.row_scale[q0 + j]);
+                }
                 if constexpr (!SWAP) {
-                    if (p.row_scale != nullptr) {
+                    if (GROUPED && p.row_scale != nullptr) {
                         const float f = prow < p.rows_p ? p.row_scale[prow] : 0.f;
 #pragma unroll
                         for (int j = 0; j < CH; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
@@ -909,11 +914,11 @@ static int make_map(CUtensorMap* m, const void* base, long long rows, long long 
 
 static int g_sms = 0;
 
-template <int BN, bool SWAP, typename TOut, bool GATED = false, bool WIDE = false>
+template <int BN, bool SWAP, typename TOut, bool GATED = false, bool WIDE = false, bool GROUPED = false>
 static int launch(const CUtensorMap& mp, const CUtensorMap& mq, const GemmParams& p, cudaStream_t stream) {
     using C = Cfg<BN, SWAP, WIDE>;
     static bool attr_set = false;
-    auto kern = gemm_tc_kernel<BN, SWAP, TOut, GATED, WIDE>;
+    auto kern = gemm_tc_kernel<BN, SWAP, TOut, GATED, WIDE, GROUPED>;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
         if (e != cudaSuccess) return (int)e;
@@ -1152,14 +1157,15 @@ static int gemm_tc_run(const void* A, const void* W, void* C, int c_dtype, int M
     return st;
 }
 
-// Grouped products: C[m, :] = A[m, :] W_g^T for the group g = tile_group[m / 128] of the 128-row tile that holds row m.
+// Grouped products: C[m, :] = A[m, :] W_g^T for the group g = tile_group[m / tile] of the tile of rows that holds row m (tile: 128,
+// or 16, 32 or 64 where groups have few rows: swapped tiles, every group's weights streamed once per tile).
 // W holds `groups` matrices of N rows each, one after the other ([groups * N, K]); rows of A are ordered so that every
-// tile of 128 belongs to one group.  gated_act >= 0: the gated epilogue on rows interleaved per group (N = 2 x the
+// tile belongs to one group.  gated_act >= 0: the gated epilogue on rows interleaved per group (N = 2 x the
 // output's width, bfloat16 out); else a plain product into C (bfloat16 or float32).  tile_group: device memory,
-// [ceil(M / 128)] group numbers in [0, groups), or -1 for a tile that is not in use (its rows of C are not written).
+// [ceil(M / tile)] group numbers in [0, groups), or -1 for a tile that is not in use (its rows of C are not written).
 static int gemm_tc_grouped_run(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
                                long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act,
-                               int unary, const float* row_scale, cudaStream_t stream) {
+                               int unary, const float* row_scale, int tile, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || groups <= 0) return 0;
     if (unary < 0 || unary > 2 || (unary && gated_act >= 0)) return tb_refuse("gemm_tc_grouped: unary activation %d (with gate %d)", unary, gated_act);
     if (!tb_gemm_tc_takes(A, W, M, N, K, lda, ldw))
@@ -1170,32 +1176,41 @@ static int gemm_tc_grouped_run(const void* A, const void* W, void* C, int c_dtyp
     const bool gated = gated_act >= 0;
     if (gated && (gated_act > 1 || N % 32 || c_dtype != TB_BF16))
         return tb_refuse("gemm_tc_grouped: the gated epilogue (gelu_tanh or silu) needs a multiple of 32 weight rows and writes bfloat16");
+    if (tile != 16 && tile != 32 && tile != 64 && tile != 128) return tb_refuse("gemm_tc_grouped: tiles of %d rows", tile);
     if (!g_sms) {
         int dev = 0; cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
         if (g_sms <= 0) g_sms = 148;
     }
-    const int bn = N >= 256 ? 256 : 128;
+    const bool swap = tile < BM;
+    const int bn = swap ? tile : N >= 256 ? 256 : 128;
     GemmParams p;
     p.tile_group = tile_group; p.group_rows = N; p.row_scale = row_scale;
     p.K = K; p.kblocks = (K + BK - 1) / BK; p.splits = 1; p.kb_per_split = p.kblocks;
     p.out = C; p.ld_out = ldc; p.partial = nullptr; p.cap = 0.f; p.scale = 1.0f;
     p.act = gated ? gated_act : 0; p.limit = 0.f; p.unary = unary;
     p.cluster = 1; p.staged = ((uintptr_t)C & 15) == 0 && (ldc * (c_dtype == TB_BF16 ? 2 : 4)) % 16 == 0;
-    p.rows_p = M; p.rows_q = N;
     CUtensorMap mp, mq;
-    if (make_map(&mp, A, M, K, lda, BM) || make_map(&mq, W, groups * N, K, ldw, bn)) return -1;
+#define OUT3(...) (gated ? launch<__VA_ARGS__, bf16, true, true, true>(mp, mq, p, stream) : c_dtype == TB_BF16 ? launch<__VA_ARGS__, bf16, false, true, true>(mp, mq, p, stream) : launch<__VA_ARGS__, float, false, true, true>(mp, mq, p, stream))
+    if (swap) {
+        p.rows_p = N; p.rows_q = M;
+        if (make_map(&mp, W, (long long)groups * N, K, ldw, BM) || make_map(&mq, A, M, K, lda, bn)) return -1;
+        p.tiles_p = (N + BM - 1) / BM;
+        p.tiles_q = (M + bn - 1) / bn;
+        return bn == 16 ? OUT3(16, true) : bn == 32 ? OUT3(32, true) : OUT3(64, true);
+    }
+    p.rows_p = M; p.rows_q = N;
+    if (make_map(&mp, A, M, K, lda, BM) || make_map(&mq, W, (long long)groups * N, K, ldw, bn)) return -1;
     p.tiles_p = (M + BM - 1) / BM;
     p.tiles_q = (N + bn - 1) / bn;
-    if (gated) return bn == 256 ? launch<256, false, bf16, true>(mp, mq, p, stream) : launch<128, false, bf16, true>(mp, mq, p, stream);
-    if (c_dtype == TB_BF16) return bn == 256 ? launch<256, false, bf16, false>(mp, mq, p, stream) : launch<128, false, bf16, false>(mp, mq, p, stream);
-    return bn == 256 ? launch<256, false, float, false>(mp, mq, p, stream) : launch<128, false, float, false>(mp, mq, p, stream);
+    return bn == 256 ? OUT3(256, false) : OUT3(128, false);
+#undef OUT3
 }
 
 extern "C" int tb_gemm_tc_grouped(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
                                   long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act,
                                   cudaStream_t stream) {
-    return gemm_tc_grouped_run(A, W, C, c_dtype, M, N, groups, K, lda, ldw, ldc, tile_group, gated_act, 0, nullptr, stream);
+    return gemm_tc_grouped_run(A, W, C, c_dtype, M, N, groups, K, lda, ldw, ldc, tile_group, gated_act, 0, nullptr, BM, stream);
 }
 
 // The same with a unary activation (experts without a gate branch; 0: none) and with a number per row of A that multiplies
@@ -1203,7 +1218,14 @@ extern "C" int tb_gemm_tc_grouped(const void* A, const void* W, void* C, int c_d
 extern "C" int tb_gemm_tc_grouped_ex(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
                                      long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act, int unary,
                                      const float* row_scale, cudaStream_t stream) {
-    return gemm_tc_grouped_run(A, W, C, c_dtype, M, N, groups, K, lda, ldw, ldc, tile_group, gated_act, unary, row_scale, stream);
+    return gemm_tc_grouped_run(A, W, C, c_dtype, M, N, groups, K, lda, ldw, ldc, tile_group, gated_act, unary, row_scale, BM, stream);
+}
+
+// The same with tiles of `tile` rows: 16, 32, 64 or 128.
+extern "C" int tb_gemm_tc_grouped_tiles(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
+                                        long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act, int unary,
+                                        const float* row_scale, int tile, cudaStream_t stream) {
+    return gemm_tc_grouped_run(A, W, C, c_dtype, M, N, groups, K, lda, ldw, ldc, tile_group, gated_act, unary, row_scale, tile, stream);
 }
 
 extern "C" int tb_gemm_tc_ex(const void* A, const void* W, void* C, int c_dtype, int M, int N, int K,

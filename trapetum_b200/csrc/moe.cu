@@ -517,7 +517,7 @@ __global__ void moe_sum_pairs_kernel(const float* __restrict__ pair_out, const f
 
 // ---------------------------------------------------------------------------
 // The same grouping for the tcgen05 product (gemm_tc.cu, grouped mode): the pairs are laid out expert by expert
-// with every expert's stretch padded to whole tiles of 128 rows, so that a tile of the product's token operand
+// with every expert's stretch padded to whole tiles of `tile` rows, so that a tile of the product's token operand
 // belongs to one expert.  tb_moe_group_padded makes the layout (where every pair goes, which pair every row
 // holds, every tile's expert), tb_moe_gather_rows fills the operand (and, if asked for, lays every row's weight out
 // beside it, for weights that multiply the experts' input), and tb_moe_combine_sorted adds a token's
@@ -527,8 +527,8 @@ struct MoePadArgs {
     const int* idx;            // [P] expert of every pair
     int* pos;                  // [P] the pair's row in the padded order
     int* row_pair;             // [max_rows] the pair a row holds, -1 for padding
-    int* tile_group;           // [max_rows / 128] the tile's expert (-1 for tiles past the last one: the product leaves them out)
-    int P, E, max_rows;
+    int* tile_group;           // [max_rows / tile] the tile's expert (-1 for tiles past the last one: the product leaves them out)
+    int P, E, max_rows, tile;
 };
 
 __global__ void __launch_bounds__(1024) moe_group_padded_kernel(MoePadArgs a) {
@@ -539,12 +539,12 @@ __global__ void __launch_bounds__(1024) moe_group_padded_kernel(MoePadArgs a) {
     __syncthreads();
     pdl_wait();
     for (int r = threadIdx.x; r < a.max_rows; r += blockDim.x) a.row_pair[r] = -1;
-    for (int t = threadIdx.x; t < a.max_rows / 128; t += blockDim.x) a.tile_group[t] = -1;     // not in use until an expert claims it
+    for (int t = threadIdx.x; t < a.max_rows / a.tile; t += blockDim.x) a.tile_group[t] = -1;     // not in use until an expert claims it
     for (int p = threadIdx.x; p < a.P; p += blockDim.x) atomicAdd(&cnt[a.idx[p]], 1);
     __syncthreads();
     if (threadIdx.x == 0) {
         int o = 0;
-        for (int e = 0; e < a.E; e++) { off[e] = o; o += (cnt[e] + 127) / 128 * 128; }
+        for (int e = 0; e < a.E; e++) { off[e] = o; o += (cnt[e] + a.tile - 1) / a.tile * a.tile; }
     }
     __syncthreads();
     for (int p = threadIdx.x; p < a.P; p += blockDim.x) {
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(1024) moe_group_padded_kernel(MoePadArgs a) {
         a.pos[p] = r; a.row_pair[r] = p;
     }
     for (int e = threadIdx.x; e < a.E; e += blockDim.x)
-        for (int t = off[e] / 128; t < (off[e] + cnt[e] + 127) / 128; t++) a.tile_group[t] = e;
+        for (int t = off[e] / a.tile; t < (off[e] + cnt[e] + a.tile - 1) / a.tile; t++) a.tile_group[t] = e;
 }
 
 __global__ void __launch_bounds__(128) moe_gather_rows_kernel(const bf16* __restrict__ x, long long x_stride, const int* __restrict__ row_pair,
@@ -591,7 +591,8 @@ __global__ void moe_combine_sorted_kernel(const float* __restrict__ y, const int
 extern "C" int tb_moe_group_padded(const MoePadArgs* args, cudaStream_t stream) {
     const MoePadArgs& a = *args;
     if (a.P <= 0) return 0;
-    if (a.E <= 0 || a.E > 2048 || a.max_rows % 128 || a.max_rows < a.P) return tb_refuse("moe_group_padded: experts=%d rows=%d", a.E, a.max_rows);
+    if (a.E <= 0 || a.E > 2048 || a.tile <= 0 || a.max_rows % a.tile || a.max_rows < a.P)
+        return tb_refuse("moe_group_padded: experts=%d rows=%d tile=%d", a.E, a.max_rows, a.tile);
     tb_launch(moe_group_padded_kernel, dim3(1), dim3(1024), (size_t)3 * a.E * sizeof(int), stream, a);
     return tb_launch_status();
 }

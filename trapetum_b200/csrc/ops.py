@@ -2013,32 +2013,47 @@ def moe_route(logits: torch.Tensor, experts: int, correction: Optional[torch.Ten
     return idx, weight, gate
 
 
-MOE_GROUPED_FROM = 128      # (token, expert) pairs from which the experts' products run grouped on the tensor cores
-MOE_TCGEN05_FROM = 1024     # ... and from which the grouped products are the tcgen05 kernel's (tiles of 128 rows per expert)
+MOE_GROUPED_FROM = 128      # (token, expert) pairs from which the experts' products run grouped by expert
+
+
+def moe_tile(pairs: int, experts: int, expert_bytes: int) -> int:
+    """Rows of a tile of the experts' products grouped on tcgen05, 0 where pair by pair is faster.  By an expert's share of
+    the pairs: tiles of 16, 32 or 64 rows stream the weights as the products of few tokens do, 128 are the token-major ones
+    (32 experts of 12.6 MB, us with tiles of 16 / 32 / 64 / 128: 32 tokens, 4 experts each, 82 / 83 / 83 / 102; 192 tokens
+    100 / 84 / 86 / 104; 512 tokens 179 / 117 / 106 / 120; the grouped kernel on mma.sync 195, 203, -).  Few pairs are
+    grouped (three launches more, two of them short) where they share experts and read much: 12 tokens of the same 69
+    against 98 pair by pair, but 8 tokens 64 against 67, of experts of 6.3 MB 45 against 39, of 3.1 MB 32 against 25."""
+    if pairs < MOE_GROUPED_FROM:
+        if pairs < 48 or pairs * expert_bytes < 150 << 20 or experts > 2048:
+            return 0
+        if experts * (1.0 - (1.0 - 1.0 / experts) ** pairs) > 0.8 * pairs:        # experts that some pair chooses
+            return 0
+    share = pairs / experts
+    return 16 if share <= 12 else 32 if share <= 24 else 64 if share <= 64 else 128
 
 
 class _MoePadArgs(ctypes.Structure):
     _fields_ = [("idx", c_void_p), ("pos", c_void_p), ("row_pair", c_void_p), ("tile_group", c_void_p),
-                ("P", c_int), ("E", c_int), ("max_rows", c_int)]
+                ("P", c_int), ("E", c_int), ("max_rows", c_int), ("tile", c_int)]
 
 
-def _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, ungated=False, on_input=False):
+def _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, ungated=False, on_input=False, tile=128):
     """The experts' products on the tcgen05 kernel: the pairs ordered by expert, each expert's stretch padded to whole
-    tiles of 128 rows (see moe.cu and gemm_tc.cu's grouped mode).  Shapes depend on the sizes only.  ``ungated``:
-    ``gate_up_w`` holds the up rows alone and the first product's epilogue is relu(u)^2.  ``on_input``: a pair's weight
+    tiles of ``tile`` rows (128, or 16, 32 or 64 where an expert has few; see moe.cu and gemm_tc.cu's grouped mode).  Shapes
+    depend on the sizes only.  ``ungated``: ``gate_up_w`` holds the up rows alone and the first product's epilogue is relu(u)^2.  ``on_input``: a pair's weight
     multiplies the first product's sums (the gather lays it out beside the rows) instead of the second's."""
     T, W = x.shape
     E, ff2 = gate_up_w.shape[0], gate_up_w.shape[1]
     ff = ff2 if ungated else ff2 // 2
     top = idx.shape[1]
     P = T * top
-    max_rows = ((P + 127) // 128 + min(E, P)) * 128
-    ints = torch.empty(P + max_rows + max_rows // 128, dtype=torch.int32, device=x.device)
+    max_rows = ((P + tile - 1) // tile + min(E, P)) * tile
+    ints = torch.empty(P + max_rows + max_rows // tile, dtype=torch.int32, device=x.device)
     pos, row_pair, tile_group = ints[:P], ints[P:P + max_rows], ints[P + max_rows:]
     lib = build.load("moe")
     g = _MoePadArgs()
     g.idx = idx.data_ptr(); g.pos = pos.data_ptr(); g.row_pair = row_pair.data_ptr(); g.tile_group = tile_group.data_ptr()
-    g.P = P; g.E = E; g.max_rows = max_rows
+    g.P = P; g.E = E; g.max_rows = max_rows; g.tile = tile
     _check(lib, lib.tb_moe_group_padded(ctypes.byref(g), _stream()), "moe_group_padded")
     xs = torch.empty((max_rows, W), dtype=x.dtype, device=x.device)
     row_weight = torch.empty(max_rows, dtype=torch.float32, device=x.device) if on_input else None
@@ -2047,13 +2062,13 @@ def _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, ungate
     act = torch.empty((max_rows, ff), dtype=x.dtype, device=x.device)
     y = torch.empty((max_rows, W), dtype=torch.float32, device=x.device)
     gl = build.load("gemm_tc")
-    _check(gl, gl.tb_gemm_tc_grouped_ex(_ptr(xs), _ptr(gate_up_w), _ptr(act), c_int(code(x.dtype)), c_int(max_rows), c_int(ff2),
+    _check(gl, gl.tb_gemm_tc_grouped_tiles(_ptr(xs), _ptr(gate_up_w), _ptr(act), c_int(code(x.dtype)), c_int(max_rows), c_int(ff2),
                                         c_int(E), c_int(W), c_longlong(W), c_longlong(W), c_longlong(ff), _ptr(tile_group),
                                         c_int(-1 if ungated else ACTIVATIONS["silu"]), c_int(GEMM_TC_UNARY["relu2"] if ungated else 0),
-                                        _ptr(row_weight), _stream()), "gemm_tc_grouped")
-    _check(gl, gl.tb_gemm_tc_grouped(_ptr(act), _ptr(down_w), _ptr(y), c_int(code(torch.float32)), c_int(max_rows), c_int(W),
+                                        _ptr(row_weight), c_int(tile), _stream()), "gemm_tc_grouped")
+    _check(gl, gl.tb_gemm_tc_grouped_tiles(_ptr(act), _ptr(down_w), _ptr(y), c_int(code(torch.float32)), c_int(max_rows), c_int(W),
                                      c_int(E), c_int(ff), c_longlong(ff), c_longlong(ff), c_longlong(W), _ptr(tile_group),
-                                     c_int(-1), _stream()), "gemm_tc_grouped")
+                                     c_int(-1), c_int(0), _ptr(None), c_int(tile), _stream()), "gemm_tc_grouped")
     _check(lib, lib.tb_moe_combine_sorted(_ptr(y), _ptr(pos), _ptr(None if on_input else weight), _ptr(shared),
                                           c_int(shared.shape[0] if shared is not None else 0),
                                           c_longlong(shared.stride(0) if shared is not None else 0), _ptr(gate), _ptr(out),
@@ -2141,13 +2156,14 @@ def moe_experts(x: torch.Tensor, gate_w: Optional[torch.Tensor], up_w: torch.Ten
                 or gate is None:
             raise KernelError("moe: the shared expert's output must be float32 [splits, T, W] and come with its gate")
     out = torch.empty((T, W), dtype=torch.float32, device=x.device)
-    if x.dtype == torch.bfloat16 and T * top >= MOE_GROUPED_FROM and W % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0 \
-            and x.data_ptr() % 16 == 0:
-        if ungated and T * top >= MOE_TCGEN05_FROM:
-            return _moe_grouped_tc(x, up_w, down_w, idx, weight, shared, gate, out, ungated=True, on_input=on_input)
-        if gate_up_w is not None and T * top >= MOE_TCGEN05_FROM and ff % 16 == 0:
-            return _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, on_input=on_input)
-        return _moe_grouped(x, gate_w, up_w, down_w, idx, weight, shared, gate, out, on_input)
+    if x.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+        tile = moe_tile(T * top, E, (2 if ungated else 3) * W * ff * 2)
+        if tile and ungated:
+            return _moe_grouped_tc(x, up_w, down_w, idx, weight, shared, gate, out, ungated=True, on_input=on_input, tile=tile)
+        if tile and gate_up_w is not None and ff % 16 == 0:
+            return _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, on_input=on_input, tile=tile)
+        if T * top >= MOE_GROUPED_FROM:
+            return _moe_grouped(x, gate_w, up_w, down_w, idx, weight, shared, gate, out, on_input)
     act = torch.empty((T * top, ff), dtype=x.dtype, device=x.device)
     a = _MoeExpertArgs()
     a.x = x.data_ptr(); a.x_stride = x.stride(0)
