@@ -72,6 +72,7 @@ struct F2 { unsigned long long v; };
 __device__ __forceinline__ F2 f2(float x, float y) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y)); return r; }
 __device__ __forceinline__ void unpack(F2 a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); }
 __device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
 __device__ __forceinline__ float rcpf(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
@@ -227,6 +228,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         const float cap2 = a.cap * LOG2E;
         const float cap_x = a.cap > 0.f ? a.scale / a.cap : 0.f;
         const float cap_k = a.cap > 0.f ? 2.f * a.scale / a.cap * LOG2E : 0.f;
+        const bool near_cap = a.cap > 0.f && cap_x > 0.f, plain = a.cap <= 0.f && sc2 > 0.f;
         float m_ref = -INFINITY, l_sum = 0.f;                        // this thread's reference and its share of the row sum
         bool ok = true;
         pdl_wait();
@@ -267,50 +269,66 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_empty[s]);                 // this warp has read its part of S
-            // scale, cap, mask; values in log2 units
+            // The row's maximum in this block, in log2 units.  The other group waits for the reference that
+            // follows from it, so nothing else comes before: what it takes to make probabilities of the scores (scale or
+            // cap, and the exponential) is one pass afterwards (a group's two blocks 3,200 -> 2,800 cycles; 4,000 tokens, 32
+            // heads of 128, with a cap 245 -> 217 us, 2,999 tokens, 16 heads of 256, without a cap: 77 -> 72).  It has to be the
+            // maximum: with a bound (the largest magnitude) the heaviest weight is rounded too, 3 % more error and 4 % less time.
             const int key0 = (nb_lo + j) * BN;
             const bool edge = (key0 + BN - 1 > m0) || (key0 + BN > len) || (a.window > 0 && (m0 + BM - 1) - key0 >= a.window);
-            bool small = false;
-            if (a.cap > 0.f) {
+            const int vis_lo = a.window > 0 ? max(0, i - a.window + 1 - key0) : 0;       // the keys that this row sees: a run of the block's
+            const unsigned vis_n = (unsigned)max(0, min(min(i, len - 1) - key0 + 1, BN) - vis_lo);
+            auto visible = [&](int c) { return (unsigned)(c - vis_lo) < vis_n; };
+            float mx = -INFINITY;
+            bool near = false;
+            if (near_cap) {
                 float ax = 0.f;
 #pragma unroll
-                for (int c = 0; c < BN; c++) ax = fmaxf(ax, fabsf(v[c]));
-                small = __all_sync(0xffffffffu, ax * fabsf(cap_x) <= 0.5f);
+                for (int c = 0; c < BN; c += 2) ax = fmaxf(ax, fmaxf(fabsf(v[c]), fabsf(v[c + 1])));
+                near = __all_sync(0xffffffffu, ax * cap_x <= 0.5f);
             }
-            if (small) {
-                // All of the warp's scores lie within half the cap, as nearly all of a model's do: tanh(t) = t P(t^2), P
-                // fitted to the least largest relative error on |t| <= 0.5 (1.3e-8; 1.1e-7 as evaluated, two scores an
-                // instruction).  The exponential and the reciprocal of the general form keep the special-function unit
-                // busy for 1,024 of a block's 1,536 cycles: 2,048 tokens, 8 heads of 256: 45.4 -> 35.9 us.
-                const F2 k2 = f2(cap_x, cap_x), c0 = f2(0.9999999869f * cap2, 0.9999999869f * cap2),
-                         c1 = f2(-0.3333306939f * cap2, -0.3333306939f * cap2), c2 = f2(0.1332477932f * cap2, 0.1332477932f * cap2),
-                         c3 = f2(-0.05298607529f * cap2, -0.05298607529f * cap2), c4 = f2(0.01713500663f * cap2, 0.01713500663f * cap2);
+            const bool at_once = near && !edge;
+            const F2 k2 = f2(cap_x, cap_x), d0 = f2(0.9999999869f * cap2, 0.9999999869f * cap2), d1 = f2(-0.3333306939f * cap2, -0.3333306939f * cap2),
+                     d2 = f2(0.1332477932f * cap2, 0.1332477932f * cap2), d3 = f2(-0.05298607529f * cap2, -0.05298607529f * cap2),
+                     d4 = f2(0.01713500663f * cap2, 0.01713500663f * cap2);
+            auto tanh_poly = [&](F2 u) { return fma2(fma2(fma2(fma2(d4, u, d3), u, d2), u, d1), u, d0); };
+            if (at_once) {
 #pragma unroll
-                for (int c = 0; c < BN; c += 2) {
-                    const F2 t = mul2(f2(v[c], v[c + 1]), k2), u = mul2(t, t);
-                    const F2 p = fma2(fma2(fma2(fma2(c4, u, c3), u, c2), u, c1), u, c0);
-                    unpack(mul2(t, p), v[c], v[c + 1]);
+                for (int c = 0; c < BN; c += 2) mx = fmaxf(mx, fmaxf(v[c], v[c + 1]));
+                const F2 t = mul2(f2(mx, mx), k2);
+                float x;
+                unpack(mul2(t, tanh_poly(mul2(t, t))), mx, x);
+            } else if (plain) {
+                if (edge) {
+#pragma unroll
+                    for (int c = 0; c < BN; c++) if (!visible(c)) v[c] = -INFINITY;
                 }
-            } else if (a.cap > 0.f) {
-                // cap * tanh(x * scale / cap) = cap - 2 cap / (e^(2 x scale / cap) + 1), in log2 units; 2^(+big) is
-                // inf and its reciprocal 0, 2^(-big) is 0: both ends come out right without a clamp
 #pragma unroll
-                for (int c = 0; c < BN; c++) v[c] = fmaf(-2.f * cap2, rcpf(ex2f(v[c] * cap_k) + 1.f), cap2);
+                for (int c = 0; c < BN; c += 2) mx = fmaxf(mx, fmaxf(v[c], v[c + 1]));
+                mx *= sc2;
             } else {
+                if (near) {
 #pragma unroll
-                for (int c = 0; c < BN; c++) v[c] *= sc2;
-            }
-            if (edge) {
+                    for (int c = 0; c < BN; c += 2) {
+                        const F2 t = mul2(f2(v[c], v[c + 1]), k2);
+                        unpack(mul2(t, tanh_poly(mul2(t, t))), v[c], v[c + 1]);
+                    }
+                } else if (a.cap > 0.f) {
+                    // cap * tanh(x * scale / cap) = cap - 2 cap / (e^(2 x scale / cap) + 1), in log2 units; 2^(+big) is
+                    // inf and its reciprocal 0, 2^(-big) is 0: both ends come out right without a clamp
 #pragma unroll
-                for (int c = 0; c < BN; c++) {
-                    const int jj = key0 + c;
-                    if (!(jj <= i && jj < len && (a.window <= 0 || i - jj < a.window))) v[c] = -INFINITY;
+                    for (int c = 0; c < BN; c++) v[c] = fmaf(-2.f * cap2, rcpf(ex2f(v[c] * cap_k) + 1.f), cap2);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < BN; c++) v[c] *= sc2;
                 }
-            }
-            float mx = -INFINITY;
+                if (edge) {
 #pragma unroll
-            for (int c = 0; c < BN; c += 4)
-                mx = fmaxf(mx, fmaxf(fmaxf(v[c], v[c + 1]), fmaxf(v[c + 2], v[c + 3])));
+                    for (int c = 0; c < BN; c++) if (!visible(c)) v[c] = -INFINITY;
+                }
+#pragma unroll
+                for (int c = 0; c < BN; c += 2) mx = fmaxf(mx, fmaxf(v[c], v[c + 1]));
+            }
             // the row's reference after block j-1, from the other group (a bounded mbarrier wait: no wait here may hang)
             float before = -INFINITY;
             if (j > 0) {
@@ -335,14 +353,40 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             if (lane == 0) mbar_arrive(&ref_full[j & 1]);
             const float mr = (m_ref == -INFINITY) ? 0.f : m_ref;
             uint32_t pk[BN / 2];
-            float ls0 = 0.f, ls1 = 0.f;
-#pragma unroll
-            for (int c = 0; c < BN; c += 2) {
-                const float p0 = ex2f(v[c] - mr), p1 = ex2f(v[c + 1] - mr);
-                ls0 += p0; ls1 += p1;
+            F2 ls = f2(0.f, 0.f);
+            auto put = [&](int c, float x0, float x1) {              // scores c, c + 1 less the reference
+                const float p0 = ex2f(x0), p1 = ex2f(x1);
+                ls = add2(ls, f2(p0, p1));
                 __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
                 pk[c >> 1] = *(uint32_t*)&h2;
+            };
+            const F2 less = f2(-mr, -mr);
+            if (at_once) {
+                // All of the warp's scores lie within half the cap, as nearly all of a model's do: tanh(t) = t P(t^2), P
+                // fitted to the least largest relative error on |t| <= 0.5 (1.3e-8; 1.1e-7 as evaluated, two scores an
+                // instruction).  The exponential and the reciprocal of the general form keep the special-function unit
+                // busy for 1,024 of a block's 1,536 cycles: 2,048 tokens, 8 heads of 256: 45.4 -> 35.9 us.
+#pragma unroll
+                for (int c = 0; c < BN; c += 2) {
+                    const F2 t = mul2(f2(v[c], v[c + 1]), k2);
+                    float x0, x1;
+                    unpack(fma2(t, tanh_poly(mul2(t, t)), less), x0, x1);
+                    put(c, x0, x1);
+                }
+            } else if (plain) {
+                const F2 s2 = f2(sc2, sc2);
+#pragma unroll
+                for (int c = 0; c < BN; c += 2) {
+                    float x0, x1;
+                    unpack(fma2(f2(v[c], v[c + 1]), s2, less), x0, x1);
+                    put(c, x0, x1);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < BN; c += 2) put(c, v[c] - mr, v[c + 1] - mr);
             }
+            float ls0, ls1;
+            unpack(ls, ls0, ls1);
             l_sum = l_sum * factor + (ls0 + ls1);
             // O holds the blocks before j: scale this row if its reference moved (not for the first block: the
             // second product starts O from zero).
