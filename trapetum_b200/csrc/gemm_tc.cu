@@ -282,6 +282,11 @@ __device__ __forceinline__ void tile_load_once(uint32_t dst, const CUtensorMap* 
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
         ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1), "l"(policy) : "memory");
 }
+__device__ __forceinline__ void tile_load_pair_once(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int c0, int c1, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+        ::"r"(dst), "l"((uint64_t)map), "r"(cluster_bar), "r"(c0), "r"(c1), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void tile_load_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int c0, int c1) {
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -360,7 +365,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
         uint32_t it = 0;
         const uint64_t policy = once_policy();
         auto w_load = [&](uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-            if (SWAP) tile_load_once(dst, map, bar, c0, c1, policy); else tile_load(dst, map, bar, c0, c1);
+            tile_load_once(dst, map, bar, c0, c1, policy);
         };
         Ring ring;
         bool ok = true, waited = false;
@@ -600,6 +605,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
         const uint32_t lead_full = cluster_addr(&full[0], 0);
         const uint32_t sm0 = smem_u32(smem), full0 = smem_u32(full), empty0 = smem_u32(empty);
         uint32_t it = 0;
+        const uint64_t policy = once_policy();
         Ring ring;
         bool ok = true, waited = false;
         for (int item = pair; item < n_items && ok; item += n_pairs) {
@@ -613,7 +619,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 if (elected())
                     for (int j = 0; j < pre; j++) {
                         if (rank == 0) bar_expect(full0 + 8 * j, 2 * C::STAGE_BYTES);
-                        tile_load_pair(sm0 + j * C::STAGE_BYTES + W_OFF, &map_q, lead_full + 8 * j, (kb0 + j) * BK, w_row);
+                        tile_load_pair_once(sm0 + j * C::STAGE_BYTES + W_OFF, &map_q, lead_full + 8 * j, (kb0 + j) * BK, w_row, policy);
                     }
                 pdl_wait();
                 waited = true;
@@ -629,7 +635,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_cons
                 const uint32_t st = sm0 + ring.s * C::STAGE_BYTES, bar = lead_full + 8 * ring.s;
                 if (elected()) {
                     if (rank == 0) bar_expect(full0 + 8 * ring.s, 2 * C::STAGE_BYTES);
-                    tile_load_pair(st + W_OFF, &map_q, bar, kb * BK, w_row);
+                    tile_load_pair_once(st + W_OFF, &map_q, bar, kb * BK, w_row, policy);
                     tile_load_pair(st + A_OFF, &map_p, bar, kb * BK, a_row);
                 }
                 ring.step<C::STAGES>();
@@ -762,11 +768,12 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_con
         const int pre = min(n_kb, C::STAGES);
         const uint32_t sm0 = smem_u32(smem), full0 = smem_u32(full), empty0 = smem_u32(empty);
         bool ok = true;
+        const uint64_t policy = once_policy();
         // weights first, then the wait for the kernel before this one, then its output
         if (elected())
             for (int j = 0; j < pre; j++) {
                 bar_expect(full0 + 8 * j, C::STAGE_BYTES);
-                tile_load(sm0 + j * C::STAGE_BYTES + BM * BK * 2, &map_q, full0 + 8 * j, (kb0 + j) * BK, w_row);
+                tile_load_once(sm0 + j * C::STAGE_BYTES + BM * BK * 2, &map_q, full0 + 8 * j, (kb0 + j) * BK, w_row, policy);
             }
         pdl_wait();
         if (elected())
@@ -780,7 +787,7 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_con
             const uint32_t st = sm0 + ring.s * C::STAGE_BYTES, bar = full0 + 8 * ring.s;
             if (elected()) {
                 bar_expect(bar, C::STAGE_BYTES);
-                tile_load(st + BM * BK * 2, &map_q, bar, (kb0 + it) * BK, w_row);
+                tile_load_once(st + BM * BK * 2, &map_q, bar, (kb0 + it) * BK, w_row, policy);
                 tile_load(st, &map_p, bar, (kb0 + it) * BK, a_row);
             }
             ring.step<C::STAGES>();
