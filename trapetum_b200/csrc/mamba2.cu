@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(256) mamba2_chunk_fold_kernel(Mamba2Args a) {
     *(float4*)st = s;
 }
 
-// y of 128 tokens of one head, 64 values of P.  Warp w: 16 tokens.  A sequence of one chunk starts from its slot and leaves its
+// y of 128 tokens of one head, 64 values of P.  A warp: 16 tokens.  A sequence of one chunk starts from its slot and leaves its
 // state there, in this launch alone: nobody else reads that part of the slot.
 template <int NP>
 __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) {
@@ -645,6 +645,9 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
     const int h = blockIdx.y, p0 = blockIdx.x * MP, N = a.N, P = a.P;
     const int inner = a.heads * P, ch = inner + 2 * a.groups * N, g_of = h / (a.heads / a.groups);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    // the 16 tokens of a warp: the later ones see more keys, and the two warps of an SM's quarter (w and w + 4) get nine
+    // sixteens together whichever they are (in order the quarters had 6, 8, 10 and 12)
+    const int wr = warp < 4 ? warp : 11 - warp;
     pdl_wait();
     const ChunkPlace pl = chunk_place(a, blockIdx.z);
     if (pl.n <= 0) return;
@@ -670,7 +673,7 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
     __syncthreads();
     uint32_t q[KS][4];
 #pragma unroll
-    for (int ks = 0; ks < KS; ks++) ldsm_x4(smem_addr(sS + (warp * 16 + (lane & 15)) * BPITCH + (ks * 16 + (lane >> 4) * 8) * 2), q[ks]);
+    for (int ks = 0; ks < KS; ks++) ldsm_x4(smem_addr(sS + (wr * 16 + (lane & 15)) * BPITCH + (ks * 16 + (lane >> 4) * 8) * 2), q[ks]);
     __syncthreads();                                  // C is in registers: its place takes the state
 #pragma unroll
     for (int u = 0; u < Q; u++) {
@@ -687,7 +690,7 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
     float o[8][4];
 #pragma unroll
     for (int j = 0; j < 8; j++) { o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f; }
-    if (warp * 16 < pl.n) {                           // (rows past the end: nothing to write)
+    if (wr * 16 < pl.n) {                           // (rows past the end: nothing to write)
 #pragma unroll
         for (int j = 0; j < 8; j += 2)
 #pragma unroll
@@ -704,7 +707,7 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
 #pragma unroll
                 for (int e = 0; e < 4; e++) { o[j][e] += u[0][e]; o[j + 1][e] += u[1][e]; }
             }
-        const int ra = warp * 16 + g, rb = ra + 8;
+        const int ra = wr * 16 + g, rb = ra + 8;
         const float2 ca = scum[ra], cb = scum[rb];
         {
             const float fa = exp2_fast(ca.x + ca.y), fb = exp2_fast(cb.x + cb.y);
@@ -717,13 +720,13 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
             uint32_t any = 0;
 #pragma unroll
             for (int u = 0; u < MP * 2 / 32; u++) {
-                const uint4 x = *(const uint4*)(sx + (warp * 16 + (lane >> 1)) * MXPITCH + (lane & 1) * MP + u * 16);
+                const uint4 x = *(const uint4*)(sx + (wr * 16 + (lane >> 1)) * MXPITCH + (lane & 1) * MP + u * 16);
                 any |= not_finite(x.x) | not_finite(x.y) | not_finite(x.z) | not_finite(x.w);
             }
             odd = __any_sync(0xffffffffu, (any & 0x80008000u) != 0);
         }
         uint32_t hi[4], mid[4], lo[4];
-        for (int kk = 0; kk <= warp; kk++) {
+        for (int kk = 0; kk <= wr; kk++) {
             float s[2][4];
 #pragma unroll
             for (int n = 0; n < 2; n++) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
@@ -750,7 +753,7 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
                 split3(x0, x1, hi[n * 2], mid[n * 2], lo[n * 2]);
                 split3(x2, x3, hi[n * 2 + 1], mid[n * 2 + 1], lo[n * 2 + 1]);
             }
-            if (odd && kk == warp) break;
+            if (odd && kk == wr) break;
 #pragma unroll
             for (int j = 0; j < 8; j += 2) {
                 uint32_t f[4];
@@ -777,7 +780,7 @@ __global__ void __launch_bounds__(MCT, 2) mamba2_chunk_out_kernel(Mamba2Args a) 
                 const float fa = (r & 1) ? high3(wa) : low3(wa), fb = (r & 1) ? high3(wb) : low3(wb);
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
-                    const uint32_t x = *(const uint32_t*)(sx + (warp * 16 + r) * MXPITCH + (j * 8 + 2 * t) * 2);
+                    const uint32_t x = *(const uint32_t*)(sx + (wr * 16 + r) * MXPITCH + (j * 8 + 2 * t) * 2);
                     const float xa = __uint_as_float(x << 16), xb = __uint_as_float(x & 0xffff0000u);
                     if (r <= g) { o[j][0] = fmaf(fa, xa, o[j][0]); o[j][1] = fmaf(fa, xb, o[j][1]); }
                     if (r <= g + 8) { o[j][2] = fmaf(fb, xa, o[j][2]); o[j][3] = fmaf(fb, xb, o[j][3]); }
