@@ -988,10 +988,10 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                     // rows of the page that are not keys: their probabilities are 0, but 0 * NaN would still poison O,
                     // so this warp zeroes them in the columns it reads
                     uint8_t* v_s = smem + s * C::STAGE_BYTES + C::TILE_BYTES;
-                    for (int x = lane; x < PAGE * (HD / 32); x += 32) {
-                        const int r = x / (HD / 32), cc = d0 / 8 + x % (HD / 32);
-                        if (!is_key(row0 + r)) *(uint4*)(v_s + sw_off(r, cc)) = make_uint4(0, 0, 0, 0);
-                    }
+                    for (int r = lane; r < PAGE; r += 32)
+                        if (!is_key(row0 + r))
+#pragma unroll
+                            for (int cc = 0; cc < HD / 32; cc++) *(uint4*)(v_s + sw_off(r, d0 / 8 + cc)) = make_uint4(0, 0, 0, 0);
                     __syncwarp();
                 }
 #pragma unroll
