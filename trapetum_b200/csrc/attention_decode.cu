@@ -586,6 +586,47 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             turn_s[tid] = make_float2(cs, sn);
         }
     }
+    // geometry of the run that the cursor stands on: which rows (in row space) are keys.  Without a ring, or
+    // before the ring has wrapped: lo <= R < len.  Once it has wrapped (len >= ring_rows) every row holds a token;
+    // too old are the ring_rows - window rows that follow the newest one, a single circular run from old_beg.
+    int len = 0, lo = 0, n_old = 0, old_beg = 0;
+    bool wrapped = false, no_invalid = false;
+    auto set_geometry = [&](int b) {
+        len = a.len_after[b];
+        lo = tb_first_key(a.window, len);
+        wrapped = a.ring_rows > 0 && len >= a.ring_rows;
+        const int newest = wrapped ? (len - 1) % a.ring_rows : 0;
+        n_old = wrapped ? a.ring_rows - a.window : 0;
+        old_beg = wrapped ? (newest + 1 == a.ring_rows ? 0 : newest + 1) : 0;
+        no_invalid = wrapped && n_old == 0;                         // a full ring whose every row is in the window
+    };
+    auto is_key = [&](int R) -> bool {
+        if (wrapped) {
+            int d = R - old_beg;                                    // distance past the start of the old run
+            if (d < 0) d += a.ring_rows;
+            return d >= n_old;
+        }
+        return R >= lo && R < len;
+    };
+    auto page_all_keys = [&](int row0) -> bool {
+        if (no_invalid) return true;
+        bool ok = is_key(row0) && is_key(row0 + PAGE - 1);
+        // in a ring the rows that are too old form one circular run; it may lie inside the page
+        if (wrapped && ok) ok = !(old_beg > row0 && old_beg <= row0 + PAGE - 1);
+        return ok;
+    };
+    // where this lane's ldmatrix rows lie inside a stage: of K (a score warp), of V (an output warp)
+    uint32_t off[C::KS];
+    static_assert(C::KS == C::MT_W * 4, "one array for both");
+    if (warp < TW / 2) {
+#pragma unroll
+        for (int ks = 0; ks < C::KS; ks++) off[ks] = sw_off(warp * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), ks * 2 + (lane >> 4));
+    } else {
+#pragma unroll
+        for (int ks = 0; ks < C::KS; ks++)
+            off[ks] = C::TILE_BYTES + sw_off((ks & 3) * 16 + (lane >> 4) * 8 + (lane & 7), ((warp - TW / 2) & 3) * (HD / 32) + (ks >> 2) * 2 + ((lane >> 3) & 1));
+    }
+    if (FUSED) set_geometry(cur.b);
     // pages that this step does not write were complete before the step began: fetch them at once
     if (tid == ISSUER)
         while (ahead.left > 0 && issued < C::STAGES && ahead.first_page + ahead.pg != ahead.hot) issue();
@@ -773,35 +814,6 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         phase++;
         return ok;
     };
-    // geometry of the run that the cursor stands on: which rows (in row space) are keys.  Without a ring, or
-    // before the ring has wrapped: lo <= R < len.  Once it has wrapped (len >= ring_rows) every row holds a token;
-    // too old are the ring_rows - window rows that follow the newest one, a single circular run from old_beg.
-    int len = 0, lo = 0, n_old = 0, old_beg = 0;
-    bool wrapped = false, no_invalid = false;
-    auto set_geometry = [&](int b) {
-        len = a.len_after[b];
-        lo = tb_first_key(a.window, len);
-        wrapped = a.ring_rows > 0 && len >= a.ring_rows;
-        const int newest = wrapped ? (len - 1) % a.ring_rows : 0;
-        n_old = wrapped ? a.ring_rows - a.window : 0;
-        old_beg = wrapped ? (newest + 1 == a.ring_rows ? 0 : newest + 1) : 0;
-        no_invalid = wrapped && n_old == 0;                         // a full ring whose every row is in the window
-    };
-    auto is_key = [&](int R) -> bool {
-        if (wrapped) {
-            int d = R - old_beg;                                    // distance past the start of the old run
-            if (d < 0) d += a.ring_rows;
-            return d >= n_old;
-        }
-        return R >= lo && R < len;
-    };
-    auto page_all_keys = [&](int row0) -> bool {
-        if (no_invalid) return true;
-        bool ok = is_key(row0) && is_key(row0 + PAGE - 1);
-        // in a ring the rows that are too old form one circular run; it may lie inside the page
-        if (wrapped && ok) ok = !(old_beg > row0 && old_beg <= row0 + PAGE - 1);
-        return ok;
-    };
     auto next_run = [&](PageCursor& c, int n) {                     // the cursor moves past a run of n pages
         c.left -= n;
         c.pg += n;
@@ -829,17 +841,13 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     } else if (warp < TW / 2) {
         // ================= scores: S^T = K Q^T of this warp's 16 keys, scaled, capped, masked =================
         const int mt = warp;
-        uint32_t koff[C::KS];                                       // where this lane's ldmatrix rows lie inside a stage
-#pragma unroll
-        for (int ks = 0; ks < C::KS; ks++)
-            koff[ks] = sw_off(mt * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), ks * 2 + (lane >> 4));
         uint32_t meet_phase = 0;
         int i = 0;                                                  // pages done
         bool first_run = true;
         while (cur.left > 0) {
             const int b = cur.b, kvh = cur.kvh, seg_pg0 = cur.pg, seg_n = min(cur.left, cur.np - cur.pg);
             const int seg_first = cur.first_page;
-            set_geometry(b);
+            if (!FUSED) set_geometry(b);
             // B fragments of Q^T: b0 = Q[head quad][16 ks + 2t, +1], b1 = Q[head quad][16 ks + 8 + 2t, +1]; heads >= G zero
             const bf16* qp = (const bf16*)a.q + (size_t)b * a.q_stride + (size_t)(kvh * G + quad) * HD;
             if (fused) {
@@ -881,7 +889,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
                 for (int ks = 0; ks < C::KS; ks++) {
                     uint32_t a0, a1, a2, a3;
-                    ldsm_x4(stage + koff[ks], a0, a1, a2, a3);
+                    ldsm_x4(stage + off[ks], a0, a1, a2, a3);
                     mma_16816(c[ks & 3], a0, a1, a2, a3, qb[ks][0], qb[ks][1]);
                 }
                 // the accumulators hold keys quad, quad + 8 for heads 2t, 2t + 1
@@ -911,12 +919,6 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         // ================= outputs: running softmax, O^T += V^T P^T for head_dim / 4 dims of this warp =================
         const int ow = warp - TW / 2;
         const int d0 = ow * (HD / 4);
-        uint32_t voff[C::MT_W][4];
-#pragma unroll
-        for (int m = 0; m < C::MT_W; m++)
-#pragma unroll
-            for (int ks = 0; ks < 4; ks++)
-                voff[m][ks] = C::TILE_BYTES + sw_off(ks * 16 + (lane >> 4) * 8 + (lane & 7), (d0 + m * 16) / 8 + ((lane >> 3) & 1));
         uint32_t meet_phase = 0;
         int i = 0;
         bool once = !STREAM;                                        // (split only) an empty piece still reports "nothing here"
@@ -924,7 +926,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             once = false;
             const int b = cur.b, kvh = cur.kvh, seg_pg0 = cur.pg, seg_n = min(cur.left, cur.np - cur.pg), seg_np = cur.np;
             const int seg_first = cur.first_page;
-            set_geometry(b);
+            if (!FUSED) set_geometry(b);
             float o[C::MT_W][4], o2[C::MT_W][4];                    // accumulator rows are dims, columns heads 2t, 2t+1; two chains
 #pragma unroll
             for (int m = 0; m < C::MT_W; m++) { o[m][0] = o[m][1] = o[m][2] = o[m][3] = 0.f; o2[m][0] = o2[m][1] = o2[m][2] = o2[m][3] = 0.f; }
@@ -1001,7 +1003,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
                     for (int ks = 0; ks < 4; ks++) {
                         uint32_t a0, a1, a2, a3;
-                        ldsm_x4_t(stage + voff[m][ks], a0, a1, a2, a3);
+                        ldsm_x4_t(stage + off[m * 4 + ks], a0, a1, a2, a3);
                         mma_16816((ks & 1) ? o2[m] : o[m], a0, a1, a2, a3, pb[ks][0], pb[ks][1]);
                     }
                 }
