@@ -381,7 +381,7 @@ template <int HD, bool STREAM, bool FUSED = false> struct MCfg {
     static constexpr int MT_W = HD / 64;                             // 16-dim tiles of O^T per output warp (head_dim / 4 dims)
     static constexpr int SCORE_FLOATS = 2 * 8 * SROW + 2 * 8 * 4;    // two pages' scores, and their maxima per score warp
     static constexpr int SMEM = STAGES * STAGE_BYTES + SCORE_FLOATS * 4 + 192 /* barriers */ + (1024 + 4) * 4 /* stream: page prefix */
-                                + 8 * HD * 2 /* rotated queries */ + 10 * HD * 4 /* this step's q, k, v, summed */
+                                + 8 * HD * 2 /* rotated queries */ + (FUSED ? 0 : 10 * HD * 4) /* stream: this step's q, k, v, summed */
                                 + (FUSED ? 2 * HD * 2 + HD * 4 : 0) /* the new token's k and v, the rotation's cosines and sines */
                                 + 32 /* fold job, abort flag */ + 1024 /* alignment */;
 };
@@ -455,7 +455,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     bf16* q_s = (bf16*)(pref + 1024 + 4);                            // [8 heads][HD] this run's queries, rotated (fused rotation)
     float* fold_s = (float*)(q_s + 8 * HD);                          // [G heads of q, then k, then v][HD]: the partial sums added up
     // (no static shared memory: two CTAs of this kernel fill an SM's shared memory to the last kilobyte)
-    bf16* new_s = (bf16*)(fold_s + 10 * HD);                         // fused split: [k, v][HD] of the new token, as they go to the cache
+    bf16* new_s = (bf16*)(fold_s + (FUSED ? 0 : 10 * HD));                         // fused split: [k, v][HD] of the new token, as they go to the cache
     float2* turn_s = (float2*)(new_s + 2 * HD);                      // fused split: [HD / 2] cosine and sine of each rotated pair
     int* misc = FUSED ? (int*)(turn_s + HD / 2) : (int*)(fold_s + 10 * HD);
     int& s_last = misc[0];                          // split: this CTA folds the pair below
@@ -585,6 +585,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             sincosf((float)(a.len_after[cur.b] - 1) * a.inv_freq[tid], &sn, &cs);
             turn_s[tid] = make_float2(cs, sn);
         }
+        __syncthreads();
     }
     // geometry of the run that the cursor stands on: which rows (in row space) are keys.  Without a ring, or
     // before the ring has wrapped: lo <= R < len.  Once it has wrapped (len >= ring_rows) every row holds a token;
@@ -695,41 +696,66 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         // token, which this CTA and no other reads.  They go to the cache for the steps to come and, for this one, to
         // shared memory, from where the warps that read the page put them into its stage: waiting for the stores and
         // only then fetching the page was 3 us of a short context's 11.
-        if (warp < TW)
-            bulk_sum(G + (hot_here ? 2 : 0), [&](int) { return cur.b; },
-                     [&](int g) { return g < G ? (cur.kvh * G + g) * HD : g == G ? k_off + cur.kvh * HD : v_off + cur.kvh * HD; },
-                     tid, TW * 32);
-        __syncthreads();
+        // A thread sums, rotates and rounds two items at a time, an item being a rotated pair of a head, a number beyond the
+        // rotary part, or two numbers of v; every partial sum it needs is requested at once, eight splits each.
         if (warp < TW) {
-            auto turned = [&](const float* src, int x, float& lo, float& hi) {       // pair x < half
-                const float2 cs = turn_s[x];
-                const float x0 = src[x], x1 = src[x + half];
-                lo = x0 * cs.x - x1 * cs.y;
-                hi = x1 * cs.x + x0 * cs.y;
-            };
-            for (int y = tid; y < (G + (hot_here ? 1 : 0)) * per; y += TW * 32) {
-                const int g = y / per, x = y % per;
-                const float* src = fold_s + g * HD;
-                bf16* dst = g < G ? q_s + g * HD : new_s;
-                bf16* far = g < G ? nullptr : (bf16*)a.k_pool + new_off;
-                if (x < half) {
-                    float lo, hi;
-                    turned(src, x, lo, hi);
+            const float* base = a.qkv_part + (size_t)cur.b * a.qkv_row_stride;
+            const int n_turned = (G + (hot_here ? 1 : 0)) * per, n_items = n_turned + (hot_here ? HD / 2 : 0);
+            for (int y0 = tid; y0 < n_items; y0 += 2 * TW * 32) {
+                const float* src[2];                                  // the item's first number; its second `apart` numbers on (0: none)
+                int apart[2], seg[2], x[2];
+                float sum[2][2];
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int y = min(y0 + e * TW * 32, n_items - 1);
+                    if (y < n_turned) {
+                        seg[e] = y / per; x[e] = y % per;
+                        apart[e] = x[e] < half ? half : 0;
+                        if (x[e] >= half) x[e] += half;
+                        src[e] = base + (seg[e] < G ? (cur.kvh * G + seg[e]) * HD : k_off + cur.kvh * HD) + x[e];
+                    } else {
+                        seg[e] = G + 1; x[e] = y - n_turned; apart[e] = HD / 2;
+                        src[e] = base + v_off + cur.kvh * HD + x[e];
+                    }
+                }
+                for (int s0 = 0; s0 < a.qkv_splits; s0 += 8) {
+                    float t8[2][2][8];
+#pragma unroll
+                    for (int e = 0; e < 2; e++)
+#pragma unroll
+                        for (int k = 0; k < 8; k++)
+                            if (s0 + k < a.qkv_splits) {
+                                t8[e][0][k] = src[e][(size_t)(s0 + k) * a.qkv_split_stride];
+                                t8[e][1][k] = src[e][(size_t)(s0 + k) * a.qkv_split_stride + apart[e]];
+                            }
+#pragma unroll
+                    for (int e = 0; e < 2; e++)
+#pragma unroll
+                        for (int c = 0; c < 2; c++)
+#pragma unroll
+                            for (int k = 0; k < 8; k++) if (s0 + k < a.qkv_splits) sum[e][c] = (s0 + k == 0) ? t8[e][c][k] : sum[e][c] + t8[e][c][k];
+                }
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    if (y0 + e * TW * 32 >= n_items) break;
+                    float lo = sum[e][0], hi = sum[e][1];
+                    if (seg[e] <= G && apart[e]) {
+                        const float2 cs = turn_s[x[e]];
+                        const float x0 = lo, x1 = hi;
+                        lo = x0 * cs.x - x1 * cs.y;
+                        hi = x1 * cs.x + x0 * cs.y;
+                    }
                     const bf16 l16 = __float2bfloat16_rn(lo), h16 = __float2bfloat16_rn(hi);
-                    dst[x] = l16; dst[x + half] = h16;
-                    if (far) { far[x] = l16; far[x + half] = h16; }
-                } else {
-                    const bf16 v16 = __float2bfloat16_rn(src[x + half]);
-                    dst[x + half] = v16;
-                    if (far) far[x + half] = v16;
+                    bf16* dst = seg[e] < G ? q_s + seg[e] * HD : new_s + (seg[e] - G) * HD;
+                    dst[x[e]] = l16;
+                    if (apart[e]) dst[x[e] + apart[e]] = h16;
+                    if (seg[e] >= G) {
+                        bf16* far = (bf16*)(seg[e] == G ? a.k_pool : a.v_pool) + new_off;
+                        far[x[e]] = l16;
+                        if (apart[e]) far[x[e] + apart[e]] = h16;
+                    }
                 }
             }
-            if (hot_here)
-                for (int x = tid; x < HD; x += TW * 32) {
-                    const bf16 v16 = __float2bfloat16_rn(fold_s[(G + 1) * HD + x]);
-                    new_s[HD + x] = v16;
-                    ((bf16*)a.v_pool)[new_off + x] = v16;
-                }
         }
         __syncthreads();
     } else if (STREAM && fused) {
