@@ -1071,10 +1071,11 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 const float L = e ? L1 : L0, M = e ? m_c1 : m_c0;
                 if (whole) {
                     bf16* dst = (bf16*)a.out + ((size_t)b * a.n_heads + kvh * G + hg) * HD;
+                    const float inv = tb_divided(1.f, L, M, a.sink, kvh * G + hg);      // (a quotient per number was 1 us of a step's launch)
 #pragma unroll
                     for (int m = 0; m < C::MT_W; m++) {
-                        dst[d0 + m * 16 + quad] = __float2bfloat16_rn(tb_divided(o[m][e], L, M, a.sink, kvh * G + hg));
-                        dst[d0 + m * 16 + quad + 8] = __float2bfloat16_rn(tb_divided(o[m][2 + e], L, M, a.sink, kvh * G + hg));
+                        dst[d0 + m * 16 + quad] = __float2bfloat16_rn(o[m][e] * inv);
+                        dst[d0 + m * 16 + quad + 8] = __float2bfloat16_rn(o[m][2 + e] * inv);
                     }
                 } else {
                     float* dst = part_of(my_part, hg);
