@@ -171,6 +171,28 @@ def test_scores_mixed_two_pairs_a_thread(H, G, D, seen, n):
     near(got.view(n, H, D), want, dtype, "mixed attention, pairs", rel16=1.5e-2)
 
 
+@pytest.mark.parametrize("H,G,D,times", [(16, 4, 32, 1), (8, 2, 64, 2), (20, 4, 32, 1)])
+@pytest.mark.parametrize("window", [0, 72, -16, -64, -48, -40, -192, -208])
+def test_scores_mixed_in_steps_with_more_tiles_than_fit_at_once(H, G, D, times, window):
+    """A step with more CTAs than the device holds takes its tiles longest first; every prompt's rows are those of the prompt
+    alone, whose few tiles go by position, bit for bit: no tile is left out or taken twice.  Blocks that are and are not whole
+    tiles, last blocks of one tile up to all, prompts that end within a block."""
+    from trapetum_b200.csrc import ops
+    gen = torch.Generator().manual_seed(7)
+    lens = [193, 1, 200, 64, 15, 129, 177, 16, 190, 100, 48, 65, 192] * times
+    q, k, v = (torch.randn(sum(lens), n * D, generator=gen).bfloat16().cuda() for n in (H, G, G))
+    mix = (torch.randn(H, H, generator=gen) / H).cuda()
+
+    def run(lo, hi):
+        part = lens[lo:hi]
+        starts = torch.tensor([0] + part).cumsum(0)
+        rows = slice(sum(lens[:lo]), sum(lens[:hi]))
+        seq = torch.repeat_interleave(torch.arange(len(part)), torch.tensor(part)).int().cuda()
+        return ops.attn_mixed_prefill(q[rows], k[rows], v[rows], starts.int().cuda(), seq, H, G, D, mix, window, True, max(part))
+
+    assert torch.equal(run(0, len(lens)), torch.cat([run(b, b + 1) for b in range(len(lens))]))
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H, G, D, seen, ring, sink", [(3, 3, 8, -5, 64, True), (6, 3, 24, -33, 0, True), (4, 2, 64, -64, 64, False),
                                                        (2, 1, 40, 0, 0, True), (5, 1, 16, 70, 128, False), (4, 4, 16, -100, 128, True)])

@@ -366,16 +366,30 @@ __host__ inline size_t mp_smem(int H, int G, int D, int stages) {
 // two warps and not by every head's; the mixed scores go back through a buffer of their own.  Shared memory's pipe is what
 // bounds a round: by its addresses a round of 16 heads moves 4,600 rows of 128 bytes for the exchange with a warp a head
 // mixing and 1,800 with pairs.  A score's terms are added in the same order (same results).  One prompt of 2,048 tokens, 16 heads
-// over 4 of 128, blocks of 1,024: 190 -> 174 us with the fold.
+// over 4 of 128, blocks of 1,024, in the order of positions: 190 -> 174 us with the fold.
 // Rows of 32 scores, eight-column groups exchanged by the query's low bits: no two of a half warp's 8-byte accesses meet.
 __host__ inline size_t mp_smem_pairs(int H, int G, int D, int stages) {
     return (size_t)H * H * 4 + (size_t)2 * H * MP_BM * MP_BN * 4 + (size_t)stages * 2 * G * MP_BN * (D + 8) * 2;
 }
 __device__ __forceinline__ int mp_pair_at(int g, int i, int j) { return (g * MP_BM + i) * MP_BN + (j ^ ((i & 3) * 8)); }
 
+// The tile of queries that the x-th of n takes: those that see most keys first, since what starts last ends last.  Within
+// blocks of positions that is the blocks' last tiles, then the ones before them; else the last tiles.
+// One prompt of 2,048 tokens, in the order of positions -> so (us): 16 heads over 4 of 128, blocks of 1,024 173 -> 114 (29
+// -> 19 rounds of the longest tile's keys, by simulation), of 512 107 -> 76; 8 heads over 2 94 -> 78 and 56 -> 49.
+__device__ __forceinline__ int mp_tile(int x, int n, int window) {
+    const int per = window < 0 && -window % MP_BM == 0 ? -window / MP_BM : n;        // tiles of a block
+    if (per >= n) return n - 1 - x;
+    const int blocks = (n + per - 1) / per, rest = n - (blocks - 1) * per;           // the last block has `rest` tiles
+    const int ahead = (per - rest) * (blocks - 1);                                   // tiles at places that the last block has not
+    if (x < ahead) return x % (blocks - 1) * per + per - 1 - x / (blocks - 1);
+    x -= ahead;
+    return x % blocks * per + rest - 1 - x / blocks;
+}
+
 // MULTI: more than 16 heads (the second paragraph above); else a warp's only raw scores are its own head's.
 template <int KT, bool MULTI, bool PAIRS>
-__global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnArgs a) {
+__global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnArgs a, unsigned flip) {
     pdl_launch_dependents();
     constexpr int D = 16 * KT, PITCH = D + 8;
     extern __shared__ __align__(16) unsigned char sm[];
@@ -387,22 +401,27 @@ __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnAr
     const size_t k_part = (size_t)G * MP_BN * PITCH, stage = k_part + (size_t)GV * MP_BN * PITCH;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h_raw = warp < H ? warp : 0;
-    const int h_out = blockIdx.z * 16 + warp;                         // the head this warp mixes, weighs and writes
+    // which work: the launch's CTAs in order, `flip` of them backwards, go round the sequences and groups of heads, so that
+    // every sequence's longest tiles come first
+    const unsigned cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    const unsigned turn = cta < flip ? flip - 1 - cta : cta, round = gridDim.y * gridDim.z;
+    const int nth = turn / round, b = turn % round % gridDim.y, z = turn % round / gridDim.y;
+    const int h_out = z * 16 + warp;                         // the head this warp mixes, weighs and writes
     const bool has_out = h_out < H;
     const int h = has_out ? h_out : h_raw;                            // the head whose queries stay in registers
     const int r = lane >> 2, c = (lane & 3) * 2;                      // this thread's rows r and r + 8, columns c and c + 1 of a tile of 8
     const int per_kv = H / G;
-    const int kv_lo = (blockIdx.z * 16) / per_kv;                     // the first kv head whose values this CTA needs
+    const int kv_lo = (z * 16) / per_kv;                              // the first kv head whose values this CTA needs
     const int kvh = h / per_kv;
     for (int e = threadIdx.x; e < H * H; e += blockDim.x) mix_s[e] = a.mix[PAIRS ? e % H * H + e / H : e];     // PAIRS: [raw head][mixed head]
     pdl_wait();
-    const int b = blockIdx.y;
     const int s0 = a.seq_start[b], len = a.seq_start[b + 1] - s0;
     // a tile's keys may be cut into pieces that CTAs of their own take (a short prompt then fills the GPU); their
     // partial (max, sum, o) are folded by attn_mixed_fold_kernel, in piece order
     const int P = a.n_pieces > 1 ? a.n_pieces : 1;
-    const int i0 = (blockIdx.x / P) * MP_BM, piece = blockIdx.x % P;
-    if (i0 >= len) return;
+    const int tiles_of_b = (len + MP_BM - 1) / MP_BM, piece = nth % P;
+    if (nth / P >= tiles_of_b) return;
+    const int i0 = mp_tile(nth / P, tiles_of_b, a.window) * MP_BM;
     const int i_last = min(i0 + MP_BM - 1, len - 1);
     const int ia = i0 + r, ib = i0 + r + 8;                           // the two queries whose scores this thread holds
     // the queries of this head as the products' left operand, kept in registers
@@ -658,8 +677,20 @@ extern "C" int tb_attn_mixed_prefill(const MixedAttnArgs* args, int dtype, cudaS
         if (am.n_pieces < 1) am.n_pieces = 1;
         dim3 grid((a.max_seq_len + MP_BM - 1) / MP_BM * am.n_pieces, a.batch, (a.H + 15) / 16);
         const int warps = a.H < 16 ? a.H : 16;
+        static int sms = 0;
+        if (!sms) {
+            int dev = 0; cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (sms <= 0) sms = 148;
+        }
+        // Where an SM holds two CTAs (up to eight heads: registers for 16 warps, shared memory), the first of each SM start with
+        // the shortest of the longest, so that the second of an SM, which is short, meets one that is not long
+        // (700 tokens, 8 heads, blocks of 512: 31.4 us, by length alone 33.4).
+        const bool two = warps <= 8 && 2 * (sm + 1024) <= 228 * 1024;
+        const unsigned long long total = (unsigned long long)grid.x * grid.y * grid.z;
+        const unsigned flip = two ? (unsigned)(total < (unsigned long long)sms ? total : sms) : 0u;
 #define TB_MP_LAUNCH_AS(KT, MULTI, PAIRS) do { allow_smem(attn_mixed_prefill_mma_kernel<KT, MULTI, PAIRS>, sm); \
-            tb_launch(attn_mixed_prefill_mma_kernel<KT, MULTI, PAIRS>, grid, dim3(warps * 32), sm, stream, am); } while (0)
+            tb_launch(attn_mixed_prefill_mma_kernel<KT, MULTI, PAIRS>, grid, dim3(warps * 32), sm, stream, am, flip); } while (0)
 #define TB_MP_LAUNCH(KT) do { if (a.H > 16) TB_MP_LAUNCH_AS(KT, true, false); \
         else if (pairs) TB_MP_LAUNCH_AS(KT, false, true); else TB_MP_LAUNCH_AS(KT, false, false); } while (0)
         switch (a.D / 16) { case 2: TB_MP_LAUNCH(2); break; case 4: TB_MP_LAUNCH(4); break; case 6: TB_MP_LAUNCH(6); break; default: TB_MP_LAUNCH(8); break; }
