@@ -932,6 +932,26 @@ def test_attn_prefill_far_key_and_window_edge(ops):
             assert hit(250) == (window == 0)
 
 
+@pytest.mark.parametrize("nh,nkv,hd,rot,n", [(24, 16, 128, 128, 129), (20, 20, 256, 256, 128), (5, 1, 80, 32, 131), (32, 17, 512, 512, 128)])
+def test_rope_kv_of_many_heads(ops, nh, nkv, hd, rot, n):
+    """Prompts whose tokens have more work items and copied pieces than their threads hold at a time, against the same rows in
+    pieces of fewer than 128 tokens, which another kernel takes: both round 32-bit results once (two units of bfloat16's last
+    place, 2^-7, where a product is contracted in one and not in the other)."""
+    qkv = rnd(n, (nh + 2 * nkv) * hd, dt=torch.bfloat16)
+    pos, seq, after = torch.arange(n).int().cuda() + 40, torch.zeros(n).int().cuda(), torch.tensor([n + 40]).int().cuda()
+    table = torch.tensor([[3, 0, 2]]).int().cuda()
+    inv = (1e4 ** -(torch.arange(0, rot, 2).float() / rot)).cuda()
+    pools = [torch.zeros(4, nkv, PAGE, hd, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    want = qkv.clone()
+    ops.rope_kv(qkv, nh, nkv, hd, rot, inv, pos, seq, after, *pools[:2], table, 0)
+    for lo in range(0, n, 100):
+        part = slice(lo, min(n, lo + 100))
+        ops.rope_kv(want[part], nh, nkv, hd, rot, inv, pos[part], seq[part], after, *pools[2:], table, 0)
+    for got, ref in ((qkv, want), (pools[0], pools[2]), (pools[1], pools[3])):
+        torch.testing.assert_close(got.float(), ref.float(), rtol=2 ** -7, atol=1e-6)
+    assert torch.equal(pools[1], pools[3])
+
+
 @pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("hd,rot,ring,theta", [(16, 16, 0, 1e4), (48, 48, 128, 5e4), (256, 256, 64, 1e4), (32, 16, 0, 1e3), (64, 0, 0, 1.0),
                                                (640, 640, 0, 1e4), (576, 530, 64, 1e4)])     # more pairs than a CTA has threads for

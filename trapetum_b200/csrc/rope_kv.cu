@@ -138,20 +138,60 @@ __global__ void rope_kv_kernel(RopeKvArgs a) {
 }
 
 // The same for many tokens (a prompt), bfloat16, head_dim a multiple of 16 with the whole head rotated or
-// rotary_dim a multiple of 16: one warp per token, 16-byte accesses.  A lane owns eight neighbouring pairs
-// (dims i..i+7 and i+half..i+half+7) of every second head slot; their sines and cosines are computed once and
-// reused for all the heads the lane visits.
-__global__ void __launch_bounds__(256, 2) rope_kv_rows_kernel(RopeKvArgs a, int n_tokens) {
+// rotary_dim a multiple of 16: a CTA of ROPE_TH threads a token, 16-byte accesses.  The threads make the token's sines and
+// cosines once, one or two angles each, and leave them in shared memory; then each takes work items of eight neighbouring
+// pairs of one head (dims i..i+7 and i+half..i+half+7).  What a thread reads of the row first is requested before its angles
+// are made.  Up to about a thousand tokens the launch lasts as long as one token's chain (a warp a token made eight angles a lane
+// and then went through its heads), beyond that as long as its bytes: us in a graph, a warp a token -> so, tokens 128 / 384 /
+// 1,024 / 2,048 / 8,192: 8 heads over 4 of 256 5.3 / 5.4 / 6.9 / 8.6 / 32.4 -> 2.7 / 3.9 / 4.5 / 8.7 / 28.8, 32 over 16 of 128 8.0 /
+// 8.3 / 13.0 / 15.1 / 61.5 -> 4.0 / 5.9 / 8.0 / 13.5 / 49.6.
+constexpr int ROPE_TH = 128, ROPE_GROUPS = 32;          // threads; most groups of eight pairs of a head
+__global__ void __launch_bounds__(ROPE_TH, 8) rope_kv_rows_kernel(RopeKvArgs a) {
     pdl_launch_dependents();
-    pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (t >= n_tokens) return;
+    __shared__ float4 turn_s[2][2][ROPE_GROUPS];        // [sine, cosine][first, last four pairs][group]
+    const int t = blockIdx.x, tid = threadIdx.x;
     const int hd = a.head_dim, half = a.rotary_dim >> 1;
     const int groups = half >> 3;                       // groups of eight pairs per head (0: no rotation)
     const int chunks = hd >> 3;                         // 16-byte chunks per head
     bf16* row = (bf16*)a.qkv + (size_t)t * a.row_stride;
+    auto unpack = [](const uint4& w, float* f) {
+        const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) { f[2 * i] = __uint_as_float(u[i] << 16); f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
+    };
+    auto pack = [](const float* f) -> uint4 {
+        uint32_t u[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) { __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]); u[i] = *(uint32_t*)&h2; }
+        return make_uint4(u[0], u[1], u[2], u[3]);
+    };
+    const int n_turn = (a.n_heads + a.n_kv_heads) * groups;
+    // what is only copied to the cache: k dims beyond the rotary part, and v
+    const int k_tail = chunks - 2 * groups;             // chunks per k head that pass through
+    const int n_copy = a.k_pool != nullptr ? a.n_kv_heads * (k_tail + chunks) : 0;
+    auto copy_src = [&](int x) -> const bf16* {
+        const int kvh = x / (k_tail + chunks), c = x % (k_tail + chunks);
+        return c < k_tail ? row + a.k_off + kvh * hd + 2 * half + c * 8 : row + a.v_off + kvh * hd + (c - k_tail) * 8;
+    };
+    auto turn_at = [&](int x) -> bf16* {
+        const int hs = x / groups, g = x % groups;
+        return row + (hs < a.n_heads ? a.q_off + hs * hd : a.k_off + (hs - a.n_heads) * hd) + g * 8;
+    };
+    constexpr int TURN = 2, HELD = 2;                   // items and copied chunks that a thread holds in registers
+    uint4 lo[TURN], hi[TURN], held[HELD];
+    auto fetch = [&](int x0) {
+#pragma unroll
+        for (int u = 0; u < TURN; u++) {
+            const int x = x0 + u * ROPE_TH;
+            if (x < n_turn) { const bf16* p = turn_at(x); lo[u] = *(const uint4*)p; hi[u] = *(const uint4*)(p + half); }
+        }
+    };
+    pdl_wait();
     const int pos = a.positions[t];
+    fetch(tid);
+#pragma unroll
+    for (int i = 0; i < HELD; i++)
+        if (tid + ROPE_TH * i < n_copy) held[i] = *(const uint4*)copy_src(tid + ROPE_TH * i);
     size_t cache_off = 0;
     bool store = false;
     if (a.k_pool != nullptr) {
@@ -164,91 +204,49 @@ __global__ void __launch_bounds__(256, 2) rope_kv_rows_kernel(RopeKvArgs a, int 
             cache_off = ((size_t)page * a.n_kv_heads * a.page_rows + (r % a.page_rows)) * hd;
         }
     }
-    auto unpack = [](const uint4& w, float* f) {
-        const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+    for (int i = tid; i < half; i += ROPE_TH) {
+        float sn, cs;
+        sincosf((float)pos * a.inv_freq[i], &sn, &cs);
+        ((float*)&turn_s[0][(i >> 2) & 1][i >> 3])[i & 3] = sn;
+        ((float*)&turn_s[1][(i >> 2) & 1][i >> 3])[i & 3] = cs;
+    }
+    __syncthreads();
+    for (int x0 = tid; x0 < n_turn; x0 += TURN * ROPE_TH) {
+        if (x0 != tid) fetch(x0);
 #pragma unroll
-        for (int i = 0; i < 4; i++) { f[2 * i] = __uint_as_float(u[i] << 16); f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
-    };
-    auto pack = [](const float* f) -> uint4 {
-        uint32_t u[4];
+        for (int u = 0; u < TURN; u++) {
+            const int x = x0 + u * ROPE_TH;
+            if (x < n_turn) {
+                const int hs = x / groups, g = x % groups;
+                float v0[8], v1[8], y0[8], y1[8];
+                __align__(16) float sn[8], cs[8];
+                *(float4*)sn = turn_s[0][0][g]; *(float4*)(sn + 4) = turn_s[0][1][g];
+                *(float4*)cs = turn_s[1][0][g]; *(float4*)(cs + 4) = turn_s[1][1][g];
+                unpack(lo[u], v0); unpack(hi[u], v1);
 #pragma unroll
-        for (int i = 0; i < 4; i++) { __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]); u[i] = *(uint32_t*)&h2; }
-        return make_uint4(u[0], u[1], u[2], u[3]);
-    };
-    const int qk_slots = a.n_heads + a.n_kv_heads;
-    // ---- what is only copied to the cache (k dims beyond the rotary part, and v): requested first, stored last, so
-    // that the token's row is on its way while the sines and cosines are made
-    const int k_tail = chunks - 2 * groups;             // chunks per k head that pass through
-    const int n_copy = store ? a.n_kv_heads * (k_tail + chunks) : 0;
-    auto copy_src = [&](int x) -> const bf16* {
-        const int kvh = x / (k_tail + chunks), c = x % (k_tail + chunks);
-        return c < k_tail ? row + a.k_off + kvh * hd + 2 * half + c * 8 : row + a.v_off + kvh * hd + (c - k_tail) * 8;
-    };
+                for (int e = 0; e < 8; e++) { y0[e] = v0[e] * cs[e] - v1[e] * sn[e]; y1[e] = v1[e] * cs[e] + v0[e] * sn[e]; }
+                const uint4 w0 = pack(y0), w1 = pack(y1);
+                bf16* p = turn_at(x);
+                *(uint4*)p = w0;
+                *(uint4*)(p + half) = w1;
+                if (hs >= a.n_heads && store) {
+                    bf16* dst = (bf16*)a.k_pool + cache_off + (size_t)(hs - a.n_heads) * a.page_rows * hd + g * 8;
+                    *(uint4*)dst = w0;
+                    *(uint4*)(dst + half) = w1;
+                }
+            }
+        }
+    }
+    if (!store) return;
     auto copy_dst = [&](int x) -> bf16* {
         const int kvh = x / (k_tail + chunks), c = x % (k_tail + chunks);
         return c < k_tail ? (bf16*)a.k_pool + cache_off + (size_t)kvh * a.page_rows * hd + 2 * half + c * 8
                           : (bf16*)a.v_pool + cache_off + (size_t)kvh * a.page_rows * hd + (c - k_tail) * 8;
     };
-    constexpr int HELD = 4;                             // copied chunks a lane holds in registers (more go round a loop at the end)
-    uint4 held[HELD];
 #pragma unroll
     for (int i = 0; i < HELD; i++)
-        if (lane + 32 * i < n_copy) held[i] = *(const uint4*)copy_src(lane + 32 * i);
-    // ---- rotated part of q and k heads: work items (head slot, group of eight pairs)
-    if (groups > 0) {
-        const int lanes_per_head = groups < 32 ? groups : 32;          // groups <= 16 for head_dim <= 256
-        const int heads_at_once = 32 / lanes_per_head;
-        const int g = lane % lanes_per_head, h0 = lane / lanes_per_head;
-        if (h0 < heads_at_once) {
-            // four head slots at a time: their loads are requested together, and the next four before these are
-            // worked on, so that a warp waits for memory once and not once per head
-            auto fetch = [&](int hs0, uint4* wlo, uint4* whi) {
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int hs = hs0 + u * heads_at_once;
-                    if (hs < qk_slots) {
-                        const int col0 = hs < a.n_heads ? a.q_off + hs * hd : a.k_off + (hs - a.n_heads) * hd;
-                        wlo[u] = *(const uint4*)(row + col0 + g * 8);
-                        whi[u] = *(const uint4*)(row + col0 + half + g * 8);
-                    }
-                }
-            };
-            uint4 wlo[4], whi[4], nlo[4], nhi[4];
-            fetch(h0, wlo, whi);
-            float sn[8], cs[8];
-#pragma unroll
-            for (int e = 0; e < 8; e++) sincosf((float)pos * a.inv_freq[g * 8 + e], &sn[e], &cs[e]);
-            for (int hs0 = h0; hs0 < qk_slots; hs0 += 4 * heads_at_once) {
-                fetch(hs0 + 4 * heads_at_once, nlo, nhi);
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int hs = hs0 + u * heads_at_once;
-                    if (hs < qk_slots) {
-                        const bool is_q = hs < a.n_heads;
-                        const int col0 = is_q ? a.q_off + hs * hd : a.k_off + (hs - a.n_heads) * hd;
-                        float x0[8], x1[8], y0[8], y1[8];
-                        unpack(wlo[u], x0); unpack(whi[u], x1);
-#pragma unroll
-                        for (int e = 0; e < 8; e++) { y0[e] = x0[e] * cs[e] - x1[e] * sn[e]; y1[e] = x1[e] * cs[e] + x0[e] * sn[e]; }
-                        const uint4 w0 = pack(y0), w1 = pack(y1);
-                        *(uint4*)(row + col0 + g * 8) = w0;
-                        *(uint4*)(row + col0 + half + g * 8) = w1;
-                        if (!is_q && store) {
-                            bf16* dst = (bf16*)a.k_pool + cache_off + (size_t)(hs - a.n_heads) * a.page_rows * hd;
-                            *(uint4*)(dst + g * 8) = w0;
-                            *(uint4*)(dst + half + g * 8) = w1;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) { wlo[u] = nlo[u]; whi[u] = nhi[u]; }
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < HELD; i++)
-        if (lane + 32 * i < n_copy) *(uint4*)copy_dst(lane + 32 * i) = held[i];
-    for (int x = lane + 32 * HELD; x < n_copy; x += 32) *(uint4*)copy_dst(x) = *(const uint4*)copy_src(x);
+        if (tid + ROPE_TH * i < n_copy) *(uint4*)copy_dst(tid + ROPE_TH * i) = held[i];
+    for (int x = tid + ROPE_TH * HELD; x < n_copy; x += ROPE_TH) *(uint4*)copy_dst(x) = *(const uint4*)copy_src(x);
 }
 
 extern "C" int tb_rope_kv(const RopeKvArgs* args, int dtype, int n_tokens, cudaStream_t stream) {
@@ -261,14 +259,14 @@ extern "C" int tb_rope_kv(const RopeKvArgs* args, int dtype, int n_tokens, cudaS
         return tb_refuse("rope: a cache write needs page_rows > 0, a page table and both pools");
     if (a.ring_rows > 0 && a.ring_rows % a.page_rows != 0)
         return tb_refuse("rope: ring_rows=%d must be a multiple of page_rows=%d", a.ring_rows, a.page_rows);
-    // many tokens in bfloat16 with 16-byte aligned rows and heads: the warp-per-token kernel
+    // many tokens in bfloat16 with 16-byte aligned rows and heads: the kernel of 16-byte items
     if (dtype == TB_BF16 && n_tokens >= 128 && a.partial == nullptr && a.head_dim % 16 == 0 &&
         (a.inv_freq == nullptr || a.rotary_dim == 0 || a.rotary_dim % 16 == 0) && a.rotary_dim / 16 <= 32 &&
         a.row_stride % 8 == 0 && a.q_off % 8 == 0 && a.k_off % 8 == 0 && a.v_off % 8 == 0 && ((uintptr_t)a.qkv & 15) == 0 &&
         ((uintptr_t)a.k_pool & 15) == 0 && ((uintptr_t)a.v_pool & 15) == 0) {
         RopeKvArgs b = a;
         if (b.inv_freq == nullptr) b.rotary_dim = 0;
-        tb_launch(rope_kv_rows_kernel, dim3((n_tokens + 7) / 8), dim3(256), 0, stream, b, n_tokens);
+        tb_launch(rope_kv_rows_kernel, dim3(n_tokens), dim3(ROPE_TH), 0, stream, b);
         return tb_launch_status();
     }
     const int slots = a.n_heads + 2 * a.n_kv_heads;
