@@ -4,7 +4,7 @@
 // Same formula as attention_prefill.cu (and as the reference's one-query attn_k,
 // runtime/cuda/codebook_gemv.cu:240-270); what differs is where the work runs:
 //   * one CTA = 128 queries of one head of one sequence; S = Q K^T and O += P V are tcgen05.mma
-//     (128 x 64 x 16 and 128 x head_dim x 16) issued by one thread, with S and O in tensor memory;
+//     (128 x 64 x 16 and 128 x head_dim x 16) issued by one elected lane, with S and O in tensor memory;
 //   * tensor memory's lanes are the query rows, so a row's running maximum, exponentials and row sum
 //     stay with the row's threads: no shuffles across a warp;
 //   * K and V tiles arrive by tiled TMA (128-byte swizzle); P is written to shared
@@ -46,7 +46,7 @@ constexpr int P_BYTES = BM * 128;                     // 128 rows x 64 keys
 constexpr int TILE_BYTES = 2 * K_BYTES + 2 * V_BYTES + 2 * P_BYTES;
 constexpr int ROWX_BYTES = 2 * 2 * BM * 4;         // the softmax threads' exchange: references [2][BM], row sums [2][BM]
 constexpr int USED_BYTES = TILE_BYTES + ROWX_BYTES + 256;
-constexpr int SMEM_BYTES = USED_BYTES + 512;       // head_dim 256 uses all but 256 bytes of an SM's shared memory
+constexpr int SMEM_BYTES = USED_BYTES + 512;       // head_dim 256: 163 KB; a CTA an SM (tensor memory)
 static_assert(SMEM_BYTES <= 232448, "does not fit an SM's shared memory");
 constexpr int Q_COLS = HD / 2;                        // Q in tensor memory: two bf16 per column
 constexpr int TMEM_COLS = (2 * BN + HD + Q_COLS) <= 256 ? 256 : 512;

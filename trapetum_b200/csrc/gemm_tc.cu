@@ -9,12 +9,13 @@
 // GEMVs (runtime/cuda/codebook_gemv.cu:86-114) with a fixed-order second stage
 // for determinism (:178-184); the same rule holds here (no atomics anywhere).
 //
-// One kernel, two orientations, chosen by the host:
-//   tokens >  128: the 128 lanes of a tile are tokens, its BN columns weight rows
+// Two orientations:
+//   tokens >  128: the 128 lanes of a tile are tokens, its BN columns weight rows; single SMs, pairs of SMs or a cluster
+//                  that cuts a tile's K, and the tile's width, by the least of the fitted costs in choose_form
 //   tokens <= 128: swapped, the 128 lanes are weight rows and the BN columns are the
 //                  tokens (BN = 16..128), so a decode step streams every weight
 //                  once through full-height MMA tiles whatever the batch size
-// (many tokens: single SMs, pairs, or a cluster that cuts a tile's K, and the tile's width, by choose_form) and optional split-K (small N, large K): each split writes 32-bit partials to
+// and optional split-K (small N, large K): each split writes 32-bit partials to
 // scratch and tb_splitk_reduce adds them in split order.
 //
 // Roles per CTA (320 threads): warp 0 issues TMA loads, warp 1 owns tensor memory

@@ -26,27 +26,13 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
-}
-// The same with the A operand in tensor memory: row i of A in lane i, two bf16 of the row per 32-bit column (K-major),
-// so that the 16 elements of one instruction are 8 columns.
-__device__ __forceinline__ void umma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
-}
-// The same two with the shared-memory descriptors given as their 32-bit halves.  One thread issues every MMA, and a
-// small MMA runs no longer than the few instructions that make its descriptors: stepping through a tile then adds a
-// constant to the low half (the start address in 16-byte units) and leaves the high half alone.
+// The shared-memory descriptors are given as their 32-bit halves: one lane issues every MMA, and a small MMA runs no longer
+// than the few instructions that make its descriptors, so stepping through a tile adds a constant to the low half (the
+// start address in 16-byte units) and leaves the high half alone.
 __device__ __forceinline__ uint32_t desc_lo(uint64_t d) { return (uint32_t)d; }
 __device__ __forceinline__ uint32_t desc_hi(uint64_t d) { return (uint32_t)(d >> 32); }
+// The A operand lies in tensor memory: row i of A in lane i, two bf16 of the row per 32-bit column (K-major), so that the 16
+// elements of one instruction are 8 columns.
 __device__ __forceinline__ void umma_bf16_ta_lh(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                                                 uint32_t acc) {
     asm volatile(
@@ -56,6 +42,7 @@ __device__ __forceinline__ void umma_bf16_ta_lh(uint32_t tmem_d, uint32_t tmem_a
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc) : "memory");
 }
+// Both operands in shared memory.
 __device__ __forceinline__ void umma_bf16_lh(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t ab_hi, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"
@@ -122,7 +109,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
-// A pair of CTAs on one tile (cta_group::2): a cluster of two CTAs on neighbouring SMs.  One thread of the even CTA
+// A pair of CTAs on one tile (cta_group::2): a cluster of two CTAs on neighbouring SMs.  One lane of the even CTA
 // (the leader) issues MMAs of 256 rows: each CTA holds its 128 rows of A and its half of B's rows in its own shared
 // memory, at the same offsets, and its 128 rows of the accumulator in its own tensor memory, at the same address.
 // Both CTAs' copies report to the leader's barrier; a commit reaches the same barrier in both CTAs.
@@ -146,13 +133,6 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
-// A tiled copy into this CTA's shared memory whose bytes are counted on a barrier of either CTA of the pair
-// (given by its address in the cluster's window).  No multicast: each CTA fetches what it needs itself.
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t cluster_bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(cluster_bar), "r"(c0), "r"(c1) : "memory");
-}
 // Executed by the same warp of both CTAs, with the same destination offset.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols) : "memory");
@@ -160,21 +140,6 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t col
 }
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t addr, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
-}
-// Arrives, once the pair's MMAs issued so far are complete, on the barrier at this offset in both CTAs.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-    asm volatile(
-        "{\n\t.reg .b16 m;\n\t"
-        "mov.b16 m, 3;\n\t"
-        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}"
-        ::"r"(smem_u32(bar)) : "memory");
 }
 // Instruction descriptor of the pair's MMA: bf16 x bf16 -> f32, both operands K-major, M = 256 over the two CTAs.
 __host__ __device__ constexpr uint32_t instr_desc_pair(int n) {
