@@ -959,7 +959,7 @@ extern "C" int tb_gemm_tc_set_pair(int mode) { const int was = g_pair; g_pair = 
 // the power cap leaves.  A cluster of two to four CTAs on one tile's K pays where there are few tiles: 384 tokens x 2,304
 // x 9,216: 63 us on single SMs at first, 35 with the loops as they are now, 23 with K cut in two.
 struct TileForm { bool pair; int bn, cluster; };
-static TileForm choose_form(int M, int N, int kblocks) {
+static TileForm choose_form(int M, int N, int kblocks, int sms) {
     struct Cost { bool pair; int bn, cluster; double launch, round, kblock, rate; };
     static const Cost costs[] = {{false, 128, 1, 4.0, 0.9, 0.212, 1.30e9}, {false, 256, 1, 5.0, 0.5, 0.342, 1.50e9},
                                  {true, 128, 1, 5.0, 0.8, 0.167, 1.45e9},  {true, 192, 1, 6.5, 0.5, 0.227, 1.62e9},
@@ -976,7 +976,7 @@ static TileForm choose_form(int M, int N, int kblocks) {
         if (c.cluster > 1 && 2 * c.cluster > kblocks) continue;
         const long long bm = c.pair ? 256 : BM, tiles = ((M + bm - 1) / bm) * ((N + c.bn - 1) / c.bn);
         // SMs are handed out a GPC at a time: 45 clusters of three and 33 of four fit the 148 SMs
-        const long long slots = c.pair || c.cluster == 2 ? g_sms / 2 : c.cluster == 1 ? g_sms : c.cluster == 3 ? g_sms * 45 / 148 : g_sms * 33 / 148;
+        const long long slots = c.pair || c.cluster == 2 ? sms / 2 : c.cluster == 1 ? sms : c.cluster == 3 ? sms * 45 / 148 : sms * 33 / 148;
         const double rounds = (double)((tiles + slots - 1) / (slots > 0 ? slots : 1));
         const double busy = rounds * (c.round + (kblocks + c.cluster - 1) / c.cluster * c.kblock);
         const double power = 2.0 * bm * c.bn * BK * (double)tiles * kblocks / c.rate - 2.0;
@@ -988,8 +988,7 @@ static TileForm choose_form(int M, int N, int kblocks) {
 
 // That choice for a product of M > 128 tokens on a device of `sms` SMs: 1000 * CTAs per tile + columns, + 100000 for pairs.
 extern "C" int tb_gemm_tc_form(int M, int N, int K, int sms) {
-    if (!g_sms) g_sms = sms;
-    const TileForm f = choose_form(M, N, (K + BK - 1) / BK);
+    const TileForm f = choose_form(M, N, (K + BK - 1) / BK, sms);
     return (f.pair ? 100000 : 0) + 1000 * f.cluster + f.bn;
 }
 
@@ -1113,7 +1112,7 @@ static int gemm_tc_run(const void* A, const void* W, void* C, int c_dtype, int M
     TileForm form = {false, 128, 1};
     if (swap) form.bn = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
     else if (splits > 1) form.bn = N >= 256 ? 256 : 128;               // the caller's own split of K
-    else form = choose_form(M, N, kblocks);
+    else form = choose_form(M, N, kblocks, g_sms);
     const int bn = form.bn;
     const bool pair = form.pair;
 
