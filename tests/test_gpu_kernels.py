@@ -909,6 +909,33 @@ def test_attn_prefill_cap_near_and_far(ops, hd, reach):
     assert ops.attn_prefill_tc_error(hd) == 0
 
 
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("spread", [0.5, 1.3, 20.0])
+def test_attn_prefill_cap_of_a_row_goes_by_its_own_keys(ops, hd, window, spread):
+    """What the soft cap makes of a score must not depend on scores that the query does not see: a prompt's rows are the
+    same bits alone, before a prompt of huge scores and behind one, and with huge queries, keys and values from some later
+    token on (also one that shares a tile, a warp and a block of keys with them).  ``spread``: the scores' standard
+    deviation, with which all rows, some of them or none stay within half the cap."""
+    n, cap, scale = 333, 8.0, spread / math.sqrt(hd)
+    q, k, v = (rnd(n, hd, dt=torch.bfloat16, seed=i) for i in range(3))
+
+    def run(prompts):
+        qs, ks, vs = (torch.cat(x) for x in zip(*prompts))
+        lens = [p[0].shape[0] for p in prompts]
+        starts = torch.tensor([0] + lens, dtype=torch.int32, device="cuda").cumsum(0).int()
+        return ops.attn_prefill_tc(qs, ks, vs, starts, lens, 1, 1, hd, scale, cap, window)
+
+    alone = run([(q, k, v)])
+    huge = tuple(rnd(77, hd, dt=torch.bfloat16, s=100.0, seed=9 + i) for i in range(3))
+    assert torch.equal(run([(q, k, v), huge])[:n], alone)
+    assert torch.equal(run([huge, (q, k, v)])[77:], alone)
+    for at in (300, 273, 129, 70):
+        later = tuple(torch.cat([x[:at], x[at:] * 100]) for x in (q, k, v))
+        assert torch.equal(run([later])[:at], alone[:at]), at
+    assert ops.attn_prefill_tc_error(hd) == 0
+
+
 def test_attn_prefill_far_key_and_window_edge(ops):
     """A key made to stand out is seen from far away without a window, and exactly up to the window's
     edge with one; on tensor cores and on the generic kernel alike."""

@@ -67,15 +67,16 @@ struct PrefillTcArgs {
 };
 
 __device__ __forceinline__ float ex2f(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-// Two 32-bit floats in one register pair, and the packed instructions on them (each half rounded as the plain one rounds).
+// Two 32-bit floats in one register pair, and the packed instruction on them (each half rounded as the plain one rounds).
 struct F2 { unsigned long long v; };
 __device__ __forceinline__ F2 f2(float x, float y) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y)); return r; }
 __device__ __forceinline__ void unpack(F2 a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); }
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
 __device__ __forceinline__ float rcpf(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
+// PLAIN: no cap, and a scale above 0.  An instance of its own: in one kernel the forms' code and registers cost each other
+// (4,000 tokens, 32 heads of 128, no cap: 191 us in one kernel, 171 so).
+template <bool PLAIN>
 __global__ void __launch_bounds__(320, 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, PrefillTcArgs a) {
     pdl_launch_dependents();
@@ -226,9 +227,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         const float LOG2E = 1.4426950408889634f;
         const float sc2 = a.scale * LOG2E;                           // scores in log2 units
         const float cap2 = a.cap * LOG2E;
-        const float cap_x = a.cap > 0.f ? a.scale / a.cap : 0.f;
         const float cap_k = a.cap > 0.f ? 2.f * a.scale / a.cap * LOG2E : 0.f;
-        const bool near_cap = a.cap > 0.f && cap_x > 0.f, plain = a.cap <= 0.f && sc2 > 0.f;
         float m_ref = -INFINITY, l_sum = 0.f;                        // this thread's reference and its share of the row sum
         bool ok = true;
         pdl_wait();
@@ -269,51 +268,25 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_empty[s]);                 // this warp has read its part of S
-            // The row's maximum in this block, in log2 units.  The other group waits for the reference that
-            // follows from it, so nothing else comes before: what it takes to make probabilities of the scores (scale or
-            // cap, and the exponential) is one pass afterwards (a group's two blocks 3,200 -> 2,800 cycles; 4,000 tokens, 32
-            // heads of 128, with a cap 245 -> 217 us, 2,999 tokens, 16 heads of 256, without a cap: 77 -> 72).  It has to be the
-            // maximum: with a bound (the largest magnitude) the heaviest weight is rounded too, 3 % more error and 4 % less time.
+            // The row's maximum in this block, in log2 units.  The other group waits for the reference that follows from it.
+            // Without a cap nothing else comes before: scale, reference and exponential are one pass afterwards (a group's two
+            // blocks 3,200 -> 2,800 cycles).  It has to be the maximum: with a bound (the largest magnitude) the heaviest weight
+            // is rounded too, 3 % more error and 4 % less time.
             const int key0 = (nb_lo + j) * BN;
             const bool edge = (key0 + BN - 1 > m0) || (key0 + BN > len) || (a.window > 0 && (m0 + BM - 1) - key0 >= a.window);
-            const int vis_lo = a.window > 0 ? max(0, i - a.window + 1 - key0) : 0;       // the keys that this row sees: a run of the block's
-            const unsigned vis_n = (unsigned)max(0, min(min(i, len - 1) - key0 + 1, BN) - vis_lo);
-            auto visible = [&](int c) { return (unsigned)(c - vis_lo) < vis_n; };
             float mx = -INFINITY;
-            bool near = false;
-            if (near_cap) {
-                float ax = 0.f;
-#pragma unroll
-                for (int c = 0; c < BN; c += 2) ax = fmaxf(ax, fmaxf(fabsf(v[c]), fabsf(v[c + 1])));
-                near = __all_sync(0xffffffffu, ax * cap_x <= 0.5f);
-            }
-            const bool at_once = near && !edge;
-            const F2 k2 = f2(cap_x, cap_x), d0 = f2(0.9999999869f * cap2, 0.9999999869f * cap2), d1 = f2(-0.3333306939f * cap2, -0.3333306939f * cap2),
-                     d2 = f2(0.1332477932f * cap2, 0.1332477932f * cap2), d3 = f2(-0.05298607529f * cap2, -0.05298607529f * cap2),
-                     d4 = f2(0.01713500663f * cap2, 0.01713500663f * cap2);
-            auto tanh_poly = [&](F2 u) { return fma2(fma2(fma2(fma2(d4, u, d3), u, d2), u, d1), u, d0); };
-            if (at_once) {
-#pragma unroll
-                for (int c = 0; c < BN; c += 2) mx = fmaxf(mx, fmaxf(v[c], v[c + 1]));
-                const F2 t = mul2(f2(mx, mx), k2);
-                float x;
-                unpack(mul2(t, tanh_poly(mul2(t, t))), mx, x);
-            } else if (plain) {
+            if constexpr (PLAIN) {
+                const int vis_lo = a.window > 0 ? max(0, i - a.window + 1 - key0) : 0;   // the keys that this row sees: a run of the block's
+                const unsigned vis_n = (unsigned)max(0, min(min(i, len - 1) - key0 + 1, BN) - vis_lo);
                 if (edge) {
 #pragma unroll
-                    for (int c = 0; c < BN; c++) if (!visible(c)) v[c] = -INFINITY;
+                    for (int c = 0; c < BN; c++) if ((unsigned)(c - vis_lo) >= vis_n) v[c] = -INFINITY;
                 }
 #pragma unroll
-                for (int c = 0; c < BN; c += 2) mx = fmaxf(mx, fmaxf(v[c], v[c + 1]));
+                for (int c = 0; c < BN; c += 4) mx = fmaxf(mx, fmaxf(fmaxf(v[c], v[c + 1]), fmaxf(v[c + 2], v[c + 3])));
                 mx *= sc2;
             } else {
-                if (near) {
-#pragma unroll
-                    for (int c = 0; c < BN; c += 2) {
-                        const F2 t = mul2(f2(v[c], v[c + 1]), k2);
-                        unpack(mul2(t, tanh_poly(mul2(t, t))), v[c], v[c + 1]);
-                    }
-                } else if (a.cap > 0.f) {
+                if (a.cap > 0.f) {
                     // cap * tanh(x * scale / cap) = cap - 2 cap / (e^(2 x scale / cap) + 1), in log2 units; 2^(+big) is
                     // inf and its reciprocal 0, 2^(-big) is 0: both ends come out right without a clamp
 #pragma unroll
@@ -324,10 +297,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 }
                 if (edge) {
 #pragma unroll
-                    for (int c = 0; c < BN; c++) if (!visible(c)) v[c] = -INFINITY;
+                    for (int c = 0; c < BN; c++) {
+                        const int jj = key0 + c;
+                        if (!(jj <= i && jj < len && (a.window <= 0 || i - jj < a.window))) v[c] = -INFINITY;
+                    }
                 }
 #pragma unroll
-                for (int c = 0; c < BN; c += 2) mx = fmaxf(mx, fmaxf(v[c], v[c + 1]));
+                for (int c = 0; c < BN; c += 4)
+                    mx = fmaxf(mx, fmaxf(fmaxf(v[c], v[c + 1]), fmaxf(v[c + 2], v[c + 3])));
             }
             // the row's reference after block j-1, from the other group (a bounded mbarrier wait: no wait here may hang)
             float before = -INFINITY;
@@ -353,28 +330,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             if (lane == 0) mbar_arrive(&ref_full[j & 1]);
             const float mr = (m_ref == -INFINITY) ? 0.f : m_ref;
             uint32_t pk[BN / 2];
-            F2 ls = f2(0.f, 0.f);
+            float ls0 = 0.f, ls1 = 0.f;
             auto put = [&](int c, float x0, float x1) {              // scores c, c + 1 less the reference
                 const float p0 = ex2f(x0), p1 = ex2f(x1);
-                ls = add2(ls, f2(p0, p1));
+                ls0 += p0; ls1 += p1;
                 __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
                 pk[c >> 1] = *(uint32_t*)&h2;
             };
-            const F2 less = f2(-mr, -mr);
-            if (at_once) {
-                // All of the warp's scores lie within half the cap, as nearly all of a model's do: tanh(t) = t P(t^2), P
-                // fitted to the least largest relative error on |t| <= 0.5 (1.3e-8; 1.1e-7 as evaluated, two scores an
-                // instruction).  The exponential and the reciprocal of the general form keep the special-function unit
-                // busy for 1,024 of a block's 1,536 cycles: 2,048 tokens, 8 heads of 256: 45.4 -> 35.9 us.
-#pragma unroll
-                for (int c = 0; c < BN; c += 2) {
-                    const F2 t = mul2(f2(v[c], v[c + 1]), k2);
-                    float x0, x1;
-                    unpack(fma2(t, tanh_poly(mul2(t, t)), less), x0, x1);
-                    put(c, x0, x1);
-                }
-            } else if (plain) {
-                const F2 s2 = f2(sc2, sc2);
+            if constexpr (PLAIN) {
+                const F2 less = f2(-mr, -mr), s2 = f2(sc2, sc2);
 #pragma unroll
                 for (int c = 0; c < BN; c += 2) {
                     float x0, x1;
@@ -385,8 +349,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
                 for (int c = 0; c < BN; c += 2) put(c, v[c] - mr, v[c + 1] - mr);
             }
-            float ls0, ls1;
-            unpack(ls, ls0, ls1);
             l_sum = l_sum * factor + (ls0 + ls1);
             // O holds the blocks before j: scale this row if its reference moved (not for the first block: the
             // second product starts O from zero).
@@ -531,14 +493,16 @@ extern "C" int tb_attn_prefill_tc_ex(const void* q, const void* k, const void* v
     a.q = (const bf16*)q; a.q_stride = q_stride; a.n_tokens = n_tokens;
     a.seq_start = seq_start; a.out = (bf16*)out;
     a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.window = window; a.scale = scale; a.cap = cap; a.sink = sink;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    const bool plain = cap <= 0.f && scale > 0.f;
+    auto kern = plain ? attn_prefill_tc_kernel<true> : attn_prefill_tc_kernel<false>;
+    static bool attr_set[2] = {false, false};
+    if (!attr_set[plain]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         if (e != cudaSuccess) return (int)e;
-        attr_set = true;
+        attr_set[plain] = true;
     }
     dim3 grid(n_heads, batch, (max_seq_len + BM - 1) / BM);
-    tb_launch(attn_prefill_tc_kernel, grid, dim3(320), SMEM_BYTES, stream, mk, mv, a);
+    tb_launch(kern, grid, dim3(320), SMEM_BYTES, stream, mk, mv, a);
     return tb_launch_status();
 }
 
