@@ -887,6 +887,60 @@ def test_moe_experts_by_tiles(ops, gated, on, T, top, E, W, ff, tile):
     assert ops.kernel_errors() == {}
 
 
+def off_16_bytes(t):
+    """The same numbers, contiguous, in memory that begins 2 bytes past a 16-byte boundary."""
+    room = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    room[1:] = t.reshape(-1)
+    return room[1:].view(t.shape)
+
+
+def moe_case(ops, T, top, E, W, ff, gated):
+    g = torch.Generator().manual_seed(T)
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to("cuda", torch.int32)
+    weight, x = rnd(T, top, seed=3).abs() + 0.1, rnd(T, W, dt=torch.bfloat16)
+    gw, uw, dw = (rnd(E, *s, dt=torch.bfloat16, s=0.1, seed=i) for i, s in enumerate(((ff, W), (ff, W), (W, ff))))
+    both = torch.stack([ops.interleave_gate_up(gw[e], uw[e]) for e in range(E)]) if gated else None
+    want = torch.zeros(T, W, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        t, k = torch.nonzero(idx == e, as_tuple=True)
+        u = x[t].double() @ uw[e].double().T
+        a = torch.nn.functional.silu(x[t].double() @ gw[e].double().T) * u if gated else torch.relu(u) ** 2
+        want.index_add_(0, t, a @ dw[e].double().T * weight[t, k, None].double())
+    return idx, weight, x, gw if gated else None, uw, dw, both, want
+
+
+@pytest.mark.parametrize("which", ["gate and up", "gate and up alone", "down", "joint", "up without a gate", "down without a gate"])
+@pytest.mark.parametrize("T,top,E,W,ff", [(16, 4, 16, 2048, 1024), (60, 4, 12, 136, 48), (300, 4, 12, 136, 48)])
+def test_moe_experts_whose_matrices_begin_off_16_bytes(ops, which, T, top, E, W, ff):
+    """Contiguous matrices may begin anywhere: what the tensor cores' copies cannot fetch is read another way, at counts of
+    pairs that run pair by pair (where such matrices were always taken) and at those that run grouped."""
+    gated = "without" not in which
+    idx, weight, x, gw, uw, dw, both, want = moe_case(ops, T, top, E, W, ff, gated)
+    assert moe_rule(ops, T, top, E, W, ff, gated) > 0
+    if which.startswith("gate and up") or which.startswith("up"):
+        gw, uw = off_16_bytes(gw) if gated else None, off_16_bytes(uw)
+    elif which.startswith("down"):
+        dw = off_16_bytes(dw)
+    else:
+        both = off_16_bytes(both)
+    got = ops.moe_experts(x, gw, uw, dw, idx, weight, gate_up_w=None if which.endswith("alone") else both)
+    assert float((got.double() - want).norm() / want.norm()) < 4e-3
+    assert ops.kernel_errors() == {}
+
+
+@pytest.mark.parametrize("T", [16, 60, 300])
+def test_moe_experts_leave_a_joint_matrix_that_is_not_packed_unread(ops, T):
+    """The interleaved gate and up rows only speed the products up: if they are not [E, 2 ff, W], packed, of x's dtype the
+    single matrices are read."""
+    idx, weight, x, gw, uw, dw, both, want = moe_case(ops, T, 4, 12, 1024, 512, True)
+    wide = torch.zeros(12, 1024, 1024 + 64, dtype=torch.bfloat16, device="cuda")
+    wide[:, :, :1024] = both
+    for joint in (wide[:, :, :1024], both.float(), both[:, :512].contiguous(), None):
+        got = ops.moe_experts(x, gw, uw, dw, idx, weight, gate_up_w=joint)
+        assert float((got.double() - want).norm() / want.norm()) < 4e-3
+    assert ops.kernel_errors() == {}
+
+
 @pytest.mark.parametrize("hd", [64, 128, 256])
 @pytest.mark.parametrize("reach", [0.3, 1.0, 30.0, 3000.0])
 def test_attn_prefill_cap_near_and_far(ops, hd, reach):

@@ -629,8 +629,9 @@ extern "C" int tb_moe_grouped(const MoeGroupedArgs* args, const float* shared, i
                               const float* gate, float* out, int n_tokens, int max_tiles, cudaStream_t stream) {
     const MoeGroupedArgs& a = *args;
     if (n_tokens <= 0) return 0;
-    if (a.W % 8 || a.ff % 8 || ((uintptr_t)a.x & 15) || (a.x_stride % 8))
-        return tb_refuse("moe_grouped: W=%d and ff=%d must be multiples of 8 and the rows 16-byte aligned", a.W, a.ff);
+    if (a.W % 8 || a.ff % 8 || (a.x_stride % 8) ||
+        (((uintptr_t)a.x | (uintptr_t)a.gate_w | (uintptr_t)a.up_w | (uintptr_t)a.down_w) & 15))
+        return tb_refuse("moe_grouped: W=%d and ff=%d must be multiples of 8 and the rows and matrices 16-byte aligned", a.W, a.ff);
     constexpr int SMEM = MG_STAGES * MG_STAGE_BYTES;
     static bool attr_set = false;
     if (!attr_set) {

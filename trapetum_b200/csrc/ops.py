@@ -2125,14 +2125,20 @@ class _MoeExpertArgs(ctypes.Structure):
                 ("n_tokens", c_int), ("W", c_int), ("ff", c_int), ("top", c_int), ("ungated", c_int), ("weight_in", c_int)]
 
 
+def _at_16_bytes(*tensors: torch.Tensor) -> bool:
+    """Whether all begin where the kernels' 16-byte copies can."""
+    return all(t.data_ptr() % 16 == 0 for t in tensors)
+
+
 def moe_experts(x: torch.Tensor, gate_w: Optional[torch.Tensor], up_w: torch.Tensor, down_w: torch.Tensor, idx: torch.Tensor,
                 weight: torch.Tensor, shared: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
                 gate_up_w: Optional[torch.Tensor] = None, weight_on: str = "output") -> torch.Tensor:
     """The weighted sum of every token's chosen experts ``down_e(silu(gate_e x) * up_e x)`` plus ``gate[t] * shared[t]``
     (``shared`` float32 partial sums [splits, T, W]); returns float32 [T, W].  Expert matrices: ``gate_w``, ``up_w``
     [E, ff, W] and ``down_w`` [E, W, ff] of x's dtype; ``gate_up_w`` [E, 2 ff, W]: every expert's gate and up rows
-    interleaved (``interleave_gate_up``), which lets many tokens run on the tcgen05 product.  ``gate_w`` None: the
-    experts have no gate matrix and are ``down_e(relu(up_e x)^2)``.  ``weight_on`` "input": a winner's weight w multiplies
+    interleaved (``interleave_gate_up``), which lets many tokens run on the tcgen05 product; one that is not packed like
+    that, or of another dtype, is not read.  ``gate_w`` None: the experts have no gate matrix and are
+    ``down_e(relu(up_e x)^2)``.  Matrices that do not begin on 16 bytes are read pair by pair, whatever the count.  ``weight_on`` "input": a winner's weight w multiplies
     what its expert reads, ``down_e(silu(w gate_e x) * w up_e x)``, and not what it returns (the first products are
     linear, so their 32-bit sums are multiplied)."""
     if weight_on not in ("input", "output"):
@@ -2156,13 +2162,14 @@ def moe_experts(x: torch.Tensor, gate_w: Optional[torch.Tensor], up_w: torch.Ten
                 or gate is None:
             raise KernelError("moe: the shared expert's output must be float32 [splits, T, W] and come with its gate")
     out = torch.empty((T, W), dtype=torch.float32, device=x.device)
-    if x.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
+    if x.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0 and _at_16_bytes(x, down_w):
         tile = moe_tile(T * top, E, (2 if ungated else 3) * W * ff * 2)
-        if tile and ungated:
+        if tile and ungated and _at_16_bytes(up_w):
             return _moe_grouped_tc(x, up_w, down_w, idx, weight, shared, gate, out, ungated=True, on_input=on_input, tile=tile)
-        if tile and gate_up_w is not None and ff % 16 == 0:
+        if tile and not ungated and ff % 16 == 0 and gate_up_w is not None and tuple(gate_up_w.shape) == (E, 2 * ff, W) \
+                and gate_up_w.dtype == x.dtype and gate_up_w.is_contiguous() and _at_16_bytes(gate_up_w):
             return _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, on_input=on_input, tile=tile)
-        if T * top >= MOE_GROUPED_FROM:
+        if T * top >= MOE_GROUPED_FROM and not ungated and _at_16_bytes(gate_w, up_w):
             return _moe_grouped(x, gate_w, up_w, down_w, idx, weight, shared, gate, out, on_input)
     act = torch.empty((T * top, ff), dtype=x.dtype, device=x.device)
     a = _MoeExpertArgs()
