@@ -765,6 +765,31 @@ def test_attn_decode_that_rotates_and_appends_by_itself(ops, nh, nkv, hd, rot, c
     assert ops.attn_decode_error() == 0
 
 
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("n", [14, 30, 56])
+def test_attn_decode_divides_with_one_rounding(ops, hd, n):
+    """n keys of equal score, half of them with the value a and half with the next bfloat16 number b: weights, sums and
+    their number are exact and the mean is the midpoint of a and b, so the result is the even one of the two.  The sum
+    times a rounded 1 / n passes the midpoint for a third of the a's."""
+    nh, nkv, dt = 4, 2, torch.bfloat16
+    a = 1.0 + (torch.arange(hd) % 128) / 128.0
+    v = torch.stack([a + (i % 2) / 128.0 for i in range(n)])[:, None, :].expand(n, nkv, hd).to(dt)
+    assert torch.equal(v.float()[0, 0], a) and torch.equal(v.float()[1, 0], a + 1 / 128)
+    kp, vp, table = paged([torch.zeros(n, nkv, hd, dtype=dt).cuda()], [v.cuda()], [n], 0, 4, seed=1)
+    la = torch.tensor([n], dtype=torch.int32, device="cuda")
+    q = rnd(1, nh * hd, dt=dt)
+    want = (a + 1 / 256).to(dt).expand(nh, hd)                          # ties go to the even one
+    part = torch.zeros(2, 1, (nh + 2 * nkv) * hd, device="cuda")
+    part[0, 0, :nh * hd] = q.float()[0]
+    part[1, 0, (nh + nkv) * hd:] = v[n - 1].reshape(-1).float().cuda()
+    for name, got in (("split", ops.attn_decode_tma(q, kp, vp, table, la, nh, nkv, hd, 1.0, 0.0, 0, 0, 1)),
+                      ("stream", ops.attn_decode_stream(q, kp, vp, table, la, nh, nkv, hd, 1.0, 0.0, 0, 0)),
+                      ("fused split", ops.attn_decode_tma(part, kp, vp, table, la, nh, nkv, hd, 1.0, 0.0, 0, 0, 1, "mma", (None, 0))),
+                      ("fused stream", ops.attn_decode_stream(part, kp, vp, table, la, nh, nkv, hd, 1.0, 0.0, 0, 0, None, (None, 0)))):
+        assert torch.equal(got.view(nh, hd).cpu(), want), name
+    assert ops.attn_decode_error() == 0
+
+
 @pytest.mark.parametrize("dt", DT)
 def test_attn_decode_far_key_and_window_edge(ops, dt):
     """One key is made to stand out.  Among hundreds it must win the softmax; one step outside the

@@ -41,12 +41,17 @@ __device__ __forceinline__ int tb_first_key(int window, int len) {
     return 0;
 }
 
-// What a weighted sum at reference M is divided by: L, or with a sink (a.sink) L + exp(sink - M).  When the sink stands far
-// above every score the quotient is taken at the sink instead, so that nothing overflows.
-__device__ __forceinline__ float tb_divided(float acc, float L, float M, const float* sink, int h) {
-    if (sink == nullptr) return acc / L;
+// What a weighted sum at reference M is multiplied and then divided by: 1 and L, or with a sink (a.sink) L + exp(sink - M).  When
+// the sink stands far above every score the quotient is taken at the sink instead, so that nothing overflows.
+struct Divisor { float f, d; };
+__device__ __forceinline__ Divisor tb_divisor(float L, float M, const float* sink, int h) {
+    if (sink == nullptr) return {1.f, L};
     const float s = sink[h], top = fmaxf(M, s), f = __expf(M - top);
-    return acc * f / (L * f + __expf(s - top));
+    return {f, L * f + __expf(s - top)};
+}
+__device__ __forceinline__ float tb_divided(float acc, float L, float M, const float* sink, int h) {
+    const Divisor by = tb_divisor(L, M, sink, h);
+    return acc * by.f / by.d;
 }
 
 template <int HD> struct DCfg {
@@ -1071,11 +1076,12 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 const float L = e ? L1 : L0, M = e ? m_c1 : m_c0;
                 if (whole) {
                     bf16* dst = (bf16*)a.out + ((size_t)b * a.n_heads + kvh * G + hg) * HD;
-                    const float inv = tb_divided(1.f, L, M, a.sink, kvh * G + hg);      // (a quotient per number was 1 us of a step's launch)
+                    // a quotient a number: times a rounded 1 / L it would be rounded twice
+                    const Divisor by = tb_divisor(L, M, a.sink, kvh * G + hg);
 #pragma unroll
                     for (int m = 0; m < C::MT_W; m++) {
-                        dst[d0 + m * 16 + quad] = __float2bfloat16_rn(o[m][e] * inv);
-                        dst[d0 + m * 16 + quad + 8] = __float2bfloat16_rn(o[m][2 + e] * inv);
+                        dst[d0 + m * 16 + quad] = __float2bfloat16_rn(o[m][e] * by.f / by.d);
+                        dst[d0 + m * 16 + quad + 8] = __float2bfloat16_rn(o[m][2 + e] * by.f / by.d);
                     }
                 } else {
                     float* dst = part_of(my_part, hg);
