@@ -168,6 +168,30 @@ def test_state_space_mixer_between_its_products(monkeypatch, heads, P, N, groups
     assert float((S - ost[0]["S"].transpose(1, 2)).norm() / ost[0]["S"].norm()) <= tol
 
 
+@pytest.mark.parametrize("n", [1, 3, 40, 500])
+@pytest.mark.parametrize("conv, gate", [(-88.0, 2.0), (2.0, -88.0), (-30.0, -30.0)])
+def test_state_space_gates_far_below_zero(n, conv, gate):
+    """silu(-88) = -88 e^-88 is a bfloat16 number (-5e-37).  One function for the convolution and the gate of steps and of
+    prompts of every length: with B = C = 0 the scan is y = D x, so out = silu(conv) silu(gate) / sqrt(mean square + eps)."""
+    from trapetum_b200.csrc import ops
+    heads, P, N, taps, eps = 4, 64, 64, 4, 1e-5
+    inner, ch = heads * P, heads * P + 2 * N
+    proj = torch.zeros(n, inner + ch, dtype=torch.bfloat16, device=DEV)
+    proj[:, :inner] = gate
+    bias = torch.zeros(ch, device=DEV)
+    bias[:inner] = conv
+    one = torch.ones(inner, device=DEV)
+    state = torch.zeros(1, ops.mamba2_state_size(heads, P, N, 1, taps), device=DEV)
+    got = ops.mamba2(proj, torch.zeros(n, heads, device=DEV), heads, P, N, 1, taps, 1, torch.zeros(ch, taps, device=DEV), bias,
+                     torch.zeros(heads, device=DEV), torch.zeros(heads, device=DEV), one[:heads].contiguous(), one, eps, state,
+                     torch.tensor([0, n]).int().to(DEV), torch.zeros(n).int().to(DEV), torch.zeros(1).int().to(DEV), 1, n == 1,
+                     max_seq_len=0 if n == 1 else n)
+    silu = lambda x: x / (1.0 + math.exp(-x))
+    y = silu(conv) * silu(gate)
+    want = y / math.sqrt(y * y + eps)
+    assert float((got.double() / want - 1.0).abs().max()) < 2.1 * 2.0 ** -8           # x and the result are rounded to bfloat16, 2^-8 of the number at most
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_clamped_swish_token_gate_fold_norm_and_scaled_products(dtype):
     from trapetum_b200.csrc import ops

@@ -28,9 +28,6 @@
 TB_EXPORT_ERROR()
 
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
-// The same where the result is about to be rounded to bfloat16 (2^-9): fast exponential and reciprocal, relative error near
-// 2^-21.  With expf and the divide, 45 instructions a number bounded the kernels of many tokens, not the memory.
-__device__ __forceinline__ float silu_fast(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
 struct Mamba2Args {
@@ -143,7 +140,7 @@ __global__ void __launch_bounds__(128, 6) mamba2_conv4_kernel(Mamba2Args a) {
             acc[e] = bias[e] + w[e][0] * h[0][e];
             acc[e] += w[e][1] * h[1][e];
             acc[e] += w[e][2] * h[2][e];
-            acc[e] = silu_fast(acc[e] + w[e][3] * cur[e]);
+            acc[e] = silu_f(acc[e] + w[e][3] * cur[e]);
             h[0][e] = h[1][e]; h[1][e] = h[2][e]; h[2][e] = cur[e];
         }
         *(uint2*)((bf16*)a.xbc + (size_t)(t0 + r) * ch + c) = make_uint2(pack2(acc[0], acc[1]), pack2(acc[2], acc[3]));
@@ -889,8 +886,7 @@ __global__ void __launch_bounds__(FEW ? 1024 : 256) mamba2_gate_norm_rows_kernel
     float ss = 0.f;
 #pragma unroll
     for (int k = 0; k < NV; k++) {
-        if (sizeof(T) == 2) { v[k].x *= silu_fast(u[k].x); v[k].y *= silu_fast(u[k].y); v[k].z *= silu_fast(u[k].z); v[k].w *= silu_fast(u[k].w); }
-        else { v[k].x *= silu_f(u[k].x); v[k].y *= silu_f(u[k].y); v[k].z *= silu_f(u[k].z); v[k].w *= silu_f(u[k].w); }
+        v[k].x *= silu_f(u[k].x); v[k].y *= silu_f(u[k].y); v[k].z *= silu_f(u[k].z); v[k].w *= silu_f(u[k].w);
         ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
     }
     ss = block_sum(ss, red);
