@@ -123,6 +123,26 @@ def test_gated_linear_attention_between_its_products(H, D, V, rank, lens, dtype)
             near(state[slots[b]].view(H, D, V), want_state[b], dtype, "gla state", rel32=3e-5, rel16=1e-2)
 
 
+@pytest.mark.parametrize("n", [1, 3, 40, 500])
+def test_gated_linear_gates_far_below_zero(n):
+    """silu(-88) = -88 e^-88 is a bfloat16 number (-5e-37), in steps and in prompts of every length: the same outputs as with
+    a gate of 1, times silu(-88) / silu(1)."""
+    from trapetum_b200.csrc import ops
+    H, D, V, rank = 2, 64, 128, 16
+    g = torch.Generator().manual_seed(n)
+    proj = torch.randn(n, 2 * H * D + 2 * H * V, generator=g).to(DEV, torch.bfloat16)
+    low, a2 = torch.randn(n, rank, generator=g).to(DEV), torch.randn(H * D, rank, generator=g).to(DEV)
+    out = []
+    for gate in (1.0, -88.0):
+        proj[:, 2 * H * D + H * V:] = gate
+        out.append(ops.gla(proj, low, a2, torch.ones(H * D, device=DEV), 3.0, D ** -0.5, torch.ones(V, device=DEV), 1e-4, H, D, V,
+                           torch.zeros(1, H * D * V, device=DEV), torch.tensor([0, n]).int().to(DEV), torch.zeros(n).int().to(DEV),
+                           torch.zeros(1).int().to(DEV), 1, max_seq_len=n).double())
+    silu = lambda x: x / (1.0 + math.exp(-x))
+    want = out[0] * (silu(-88.0) / silu(1.0))
+    assert float((out[1] - want).abs().max() / want.abs().max()) < 2.1 * 2.0 ** -8         # both rounded to bfloat16 once, 2^-8 of the number at most
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H, C, R, dims", [(2, 40, 8, 8), (3, 24, 16, 8), (4, 112, 16, 16), (1, 200, 64, 64), (20, 128, 32, 32),
                                            (8, 448, 64, 64), (5, 80, 0, 0)])

@@ -341,8 +341,6 @@ __device__ __forceinline__ void split3(float x, bf16* hi, int step) {      // to
 }
 // A sign bit of the result is set where one of two bfloat16 numbers is infinite or NaN.
 __device__ __forceinline__ uint32_t not_finite(uint32_t v) { return (v & 0x7f807f80u) + 0x00800080u; }
-// v / (1 + e^-v) where the result is about to be rounded to bfloat16: fast exponential and reciprocal, relative error near 2^-21.
-__device__ __forceinline__ float silu_fast(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 __device__ __forceinline__ float exp2_fast(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 
 // Shared memory of a CTA, in bytes from its start.
@@ -489,7 +487,7 @@ __global__ void __launch_bounds__(512, 1) gla_block_kernel(GlaArgs a) {
                 for (int e = 0; e < 4; e++) {
                     const float g0 = __uint_as_float(gu[e] << 16), g1 = __uint_as_float(gu[e] & 0xffff0000u);
                     const float w0 = a.norm_w != nullptr ? a.norm_w[v8 + 2 * e] : 1.f, w1 = a.norm_w != nullptr ? a.norm_w[v8 + 2 * e + 1] : 1.f;
-                    out[e] = pack2(y[2 * e] * r * w0 * silu_fast(g0), y[2 * e + 1] * r * w1 * silu_fast(g1));
+                    out[e] = pack2(y[2 * e] * r * w0 * (g0 / (1.f + expf(-g0))), y[2 * e + 1] * r * w1 * (g1 / (1.f + expf(-g1))));
                 }
                 *(uint4*)((bf16*)a.out + tok * HV + (size_t)h * V + v8) = make_uint4(out[0], out[1], out[2], out[3]);
             }
