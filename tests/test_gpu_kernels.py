@@ -966,6 +966,22 @@ def test_moe_experts_leave_a_joint_matrix_that_is_not_packed_unread(ops, T):
     assert ops.kernel_errors() == {}
 
 
+@pytest.mark.parametrize("T", [4, 16, 60, 300, 700])
+def test_moe_gate_far_below_zero(ops, T):
+    """silu(-88) = -88 e^-88 is a bfloat16 number (-5e-37), whichever way the experts' products run."""
+    E, W, ff, top = 12, 1024, 512, 4
+    x = torch.zeros(T, W, dtype=torch.bfloat16, device="cuda")
+    x[:, 0] = 1.0
+    gw, uw = (torch.zeros(E, ff, W, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    gw[:, :, 0], uw[:, :, 0] = -88.0, 1.0
+    dw = torch.ones(E, W, ff, dtype=torch.bfloat16, device="cuda")
+    both = torch.stack([ops.interleave_gate_up(gw[e], uw[e]) for e in range(E)])
+    idx = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(t))[:top] for t in range(T)]).to("cuda", torch.int32)
+    got = ops.moe_experts(x, gw, uw, dw, idx, torch.ones(T, top, device="cuda"), gate_up_w=both)
+    want = -88.0 * math.exp(-88.0) * ff * top
+    assert float((got.double() / want - 1.0).abs().max()) < 4e-3          # the activations are rounded to bfloat16
+
+
 @pytest.mark.parametrize("hd", [64, 128, 256])
 @pytest.mark.parametrize("reach", [0.3, 1.0, 30.0, 3000.0])
 def test_attn_prefill_cap_near_and_far(ops, hd, reach):

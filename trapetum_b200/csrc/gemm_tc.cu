@@ -74,7 +74,11 @@ struct GemmParams {
 // The result is rounded to bfloat16, so tanh and the logistic function are taken through the fast exponential
 // and division (relative error near 2^-21): 0.5 (1 + tanh(y)) = 1 / (1 + e^(-2y)).
 // clamped_swish: g' = min(g, L), u' = clamp(u, -L, L), g' / (1 + e^(-1.702 g')) * (u' + 1).
+// That error grows with the gate, to 2^-19 at -30, and below -87.3, where the divisor passes 2^126, the quotient is 0.  EXACT
+// (the experts' grouped products): silu by expf and a true quotient, the function of the experts' other kernels.
+template <bool EXACT>
 __device__ __forceinline__ float gated(float g, float u, int act, float limit) {
+    if (EXACT && act == 1) return g / (1.0f + expf(-g)) * u;
     if (act == 2) {
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit) + 1.0f;
@@ -136,7 +140,7 @@ __device__ __forceinline__ float pointwise(float v, const GemmParams& p) {
     return v;
 }
 
-template <typename TOut, bool GATED, int CH>
+template <typename TOut, bool GATED, int CH, bool EXACT = false>
 __device__ __forceinline__ void store_token_major(const uint32_t* r, int prow, int q0, int sp, const GemmParams& p) {
     static_assert(!GATED || CH == 32, "a gate and its up value lie 16 columns apart");
     if (GATED) {
@@ -146,8 +150,8 @@ __device__ __forceinline__ void store_token_major(const uint32_t* r, int prow, i
             uint32_t w[8];
 #pragma unroll
             for (int j = 0; j < 16; j += 2) {
-                const float v0 = gated(__uint_as_float(r[j]), __uint_as_float(r[j + 16]), p.act, p.limit);
-                const float v1 = gated(__uint_as_float(r[j + 1]), __uint_as_float(r[j + 17]), p.act, p.limit);
+                const float v0 = gated<EXACT>(__uint_as_float(r[j]), __uint_as_float(r[j + 16]), p.act, p.limit);
+                const float v1 = gated<EXACT>(__uint_as_float(r[j + 1]), __uint_as_float(r[j + 17]), p.act, p.limit);
                 __nv_bfloat162 h2 = __floats2bfloat162_rn(v0, v1);
                 w[j >> 1] = *(uint32_t*)&h2;
             }
@@ -210,7 +214,7 @@ __device__ __forceinline__ void store_token_major(const uint32_t* r, int prow, i
 // chunk then leaves as whole sectors, 8 (float), 4 or 2 lanes side by side.  Written by the thread that holds the row, 16
 // bytes a lane, every store touches 32 lines and the SM takes a line a cycle: a tile of 128 x 256 floats took 11.9 us so,
 // 3.3 this way (the product of 2,048 tokens x 2,304 x 2,048: 25.7 -> 18.2 us).  Pieces are swizzled against bank conflicts.
-template <typename TOut, bool GATED>
+template <typename TOut, bool GATED, bool EXACT = false>
 __device__ __forceinline__ void store_staged(const uint32_t* r, uint8_t* stage, int lane, int row0, int q0, const GemmParams& p) {
     constexpr int RB = GATED ? 32 : 32 * (int)sizeof(TOut), U = RB / 16;
     auto f = [](int row) { return U == 8 ? row & 7 : U == 4 ? (row >> 1) & 3 : (row >> 2) & 1; };
@@ -221,8 +225,8 @@ __device__ __forceinline__ void store_staged(const uint32_t* r, uint8_t* stage, 
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const int j = u * 8 + e * 2;
-                __nv_bfloat162 h2 = __floats2bfloat162_rn(gated(__uint_as_float(r[j]), __uint_as_float(r[j + 16]), p.act, p.limit),
-                                                          gated(__uint_as_float(r[j + 1]), __uint_as_float(r[j + 17]), p.act, p.limit));
+                __nv_bfloat162 h2 = __floats2bfloat162_rn(gated<EXACT>(__uint_as_float(r[j]), __uint_as_float(r[j + 16]), p.act, p.limit),
+                                                          gated<EXACT>(__uint_as_float(r[j + 1]), __uint_as_float(r[j + 17]), p.act, p.limit));
                 w[e] = *(uint32_t*)&h2;
             }
         } else if (sizeof(TOut) == 2) {
@@ -492,8 +496,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                         for (int j = 0; j < CH; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
                     }
                     if (CH == 32 && p.staged && (GATED ? q0 < p.rows_q : q0 + CH <= p.rows_q))
-                        store_staged<TOut, GATED>(r, smem + C::EPI_OFF + (warp - 2) * EPI_STAGE_BYTES, lane, prow - lane, q0, p);
-                    else store_token_major<TOut, GATED, CH>(r, prow, q0, sp, p);
+                        store_staged<TOut, GATED, GROUPED>(r, smem + C::EPI_OFF + (warp - 2) * EPI_STAGE_BYTES, lane, prow - lane, q0, p);
+                    else store_token_major<TOut, GATED, CH, GROUPED>(r, prow, q0, sp, p);
                 } else if (GATED && SWAP) {
                     // Lanes 0..15 hold gates, lanes 16..31 the ups of the same 16 features.  Two tokens a round: the
                     // lower lanes hand over their gates of the second token and get the ups of the first, so that each
@@ -507,7 +511,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant_
                         const float u = low ? got : __uint_as_float(r[j + 1]);
                         const int tok = q0 + j + (low ? 0 : 1);
                         if (tok < p.rows_q && prow < p.rows_p)
-                            ((bf16*)p.out)[(size_t)tok * p.ld_out + feat] = __float2bfloat16_rn(gated(g, u, p.act, p.limit));
+                            ((bf16*)p.out)[(size_t)tok * p.ld_out + feat] = __float2bfloat16_rn(gated<GROUPED>(g, u, p.act, p.limit));
                     }
                 } else {
                     // weight rows on lanes (prow), tokens on columns (q0 + j): lanes write neighbours
