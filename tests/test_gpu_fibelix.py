@@ -174,9 +174,9 @@ def test_scores_mixed_two_pairs_a_thread(H, G, D, seen, n):
 @pytest.mark.parametrize("H,G,D,times", [(16, 4, 32, 1), (8, 2, 64, 2), (20, 4, 32, 1)])
 @pytest.mark.parametrize("window", [0, 72, -16, -64, -48, -40, -192, -208])
 def test_scores_mixed_in_steps_with_more_tiles_than_fit_at_once(H, G, D, times, window):
-    """A step with more CTAs than the device holds takes its tiles longest first; every prompt's rows are those of the prompt
-    alone, whose few tiles go by position, bit for bit: no tile is left out or taken twice.  Blocks that are and are not whole
-    tiles, last blocks of one tile up to all, prompts that end within a block."""
+    """A step with more CTAs than the device holds takes its tiles longest first, and goes round the sequences: every row against
+    the oracle (a tile left out or taken in another's place shows), and the same bits as the prompt alone.  Blocks that are
+    and are not whole tiles, last blocks of one tile up to all, prompts that end within a block."""
     from trapetum_b200.csrc import ops
     gen = torch.Generator().manual_seed(7)
     lens = [193, 1, 200, 64, 15, 129, 177, 16, 190, 100, 48, 65, 192] * times
@@ -190,7 +190,12 @@ def test_scores_mixed_in_steps_with_more_tiles_than_fit_at_once(H, G, D, times, 
         seq = torch.repeat_interleave(torch.arange(len(part)), torch.tensor(part)).int().cuda()
         return ops.attn_mixed_prefill(q[rows], k[rows], v[rows], starts.int().cuda(), seq, H, G, D, mix, window, True, max(part))
 
-    assert torch.equal(run(0, len(lens)), torch.cat([run(b, b + 1) for b in range(len(lens))]))
+    got = run(0, len(lens))
+    assert torch.equal(got, torch.cat([run(b, b + 1) for b in range(len(lens))]))
+    want = torch.cat([_mixed_reference(a.view(-1, H, D).cpu().double(), b.view(-1, G, D).cpu().double(), c.view(-1, G, D).cpu().double(),
+                                       mix.cpu().double(), H, G, window, True) for a, b, c in zip(*(x.split(lens) for x in (q, k, v)))])
+    rows = (got.view(-1, H, D).double().cpu() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
+    assert float(rows.max()) < 1.5e-2                        # weights and results are rounded to bfloat16, 2^-8 of the number at most
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])

@@ -728,10 +728,11 @@ def test_attn_decode_in_many_pieces(ops, splits):
 def test_attn_decode_that_rotates_and_appends_by_itself(ops, nh, nkv, hd, rot, cap, window):
     """Given the partial sums of the q/k/v product, the tensor-core decode kernel must do what the rotation kernel
     followed by the attention kernel does: the same output, and the same new rows in the cache, bit for bit (same
-    sums in the same order).  The new token lies on a page's first row, last row and in the middle; in a ring it
-    overwrites the oldest row."""
+    sums in the same order).  The new token lies on a page's first row, last row and in the middle, among the 16 rows
+    of each of the four warps that put it into the page's copy in shared memory; in a ring it overwrites the oldest row."""
     dt = torch.bfloat16
-    lens = [1, 64, 65, 200, 333, 128]
+    lens = [1, 64, 65, 200, 333, 128, 21, 175]
+    assert {(n - 1) % PAGE // 16 for n in lens} == {0, 1, 2, 3}
     ring = ((window + PAGE - 1) // PAGE) * PAGE if window else 0
     ks = [rnd(n, nkv, hd, dt=dt, seed=i).cpu() for i, n in enumerate(lens)]
     vs = [rnd(n, nkv, hd, dt=dt, seed=10 + i).cpu() for i, n in enumerate(lens)]
@@ -993,14 +994,12 @@ def test_attn_prefill_cap_near_and_far(ops, hd, reach):
     scale = reach * cap / most
     q[::3] *= 0.25
     starts = torch.tensor([0, n], dtype=torch.int32, device="cuda")
-    got = ops.attn_prefill_tc(q, k, v, starts, [n], 1, 1, hd, scale, cap, 0).double()
-    s = cap * torch.tanh(q.double() @ k.double().T * scale / cap)
-    s = s.masked_fill(torch.ones(n, n, device="cuda", dtype=torch.bool).triu(1), -math.inf)
-    want = torch.softmax(s, -1) @ v.double()
-    assert float((got - want).norm() / want.norm()) < 5e-3
-    # the negative of a query mirrors its scores about 0
-    back = ops.attn_prefill_tc(-q, -k, v, starts, [n], 1, 1, hd, scale, cap, 0).double()
-    assert torch.equal(back, got)
+    for sign in (1.0, -1.0):                                            # the negative of a query mirrors its scores about 0
+        got = ops.attn_prefill_tc(sign * q, k, v, starts, [n], 1, 1, hd, scale, cap, 0).double()
+        s = cap * torch.tanh(sign * q.double() @ k.double().T * scale / cap)
+        s = s.masked_fill(torch.ones(n, n, device="cuda", dtype=torch.bool).triu(1), -math.inf)
+        want = torch.softmax(s, -1) @ v.double()
+        assert float((got - want).norm() / want.norm()) < 5e-3
     assert ops.attn_prefill_tc_error(hd) == 0
 
 
@@ -1289,9 +1288,10 @@ def test_refusals(ops):
 def test_attn_decode_ctas_per_sm(ops):
     """The tensor-core decode kernel's stream partition is budgeted (shared memory to the byte, registers by its
     launch bounds) for two CTAs an SM at heads narrower than 256: if a change breaks the budget the kernel still
-    computes the same, only slower, so the fit is checked here."""
+    computes the same, only slower, so the fit is checked here.  (2: the split partition that adds up, rotates and appends.)"""
     from trapetum_b200.csrc import build
     lib = build.load("attention_decode")
     for hd in (64, 128, 256):
         assert lib.tb_attn_decode_occupancy(hd, 0) == 1, hd
         assert lib.tb_attn_decode_occupancy(hd, 1) == (2 if hd <= 128 else 1), hd
+        assert lib.tb_attn_decode_occupancy(hd, 2) == 1, hd

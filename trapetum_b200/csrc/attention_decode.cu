@@ -1394,11 +1394,15 @@ template <int HD, bool STREAM, bool FUSED = false> static int mma_occupancy() {
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_decode_mma_kernel<HD, STREAM, FUSED>, NTHREADS, C::SMEM);
     return e == cudaSuccess ? n : -1;
 }
-extern "C" int tb_attn_decode_occupancy(int hd, int stream_partition) {
+// partition 0: split, 1: stream, 2: split, from the product's partial sums.
+template <int HD> static int mma_occupancy_of(int partition) {
+    return partition == 1 ? mma_occupancy<HD, true>() : partition == 2 ? mma_occupancy<HD, false, true>() : mma_occupancy<HD, false>();
+}
+extern "C" int tb_attn_decode_occupancy(int hd, int partition) {
     switch (hd) {
-    case 64: return stream_partition ? mma_occupancy<64, true>() : mma_occupancy<64, false>();
-    case 128: return stream_partition ? mma_occupancy<128, true>() : mma_occupancy<128, false>();
-    case 256: return stream_partition ? mma_occupancy<256, true>() : mma_occupancy<256, false>();
+    case 64: return mma_occupancy_of<64>(partition);
+    case 128: return mma_occupancy_of<128>(partition);
+    case 256: return mma_occupancy_of<256>(partition);
     default: return -1;
     }
 }
