@@ -274,9 +274,11 @@ __device__ __forceinline__ void tile_load(uint32_t dst, const CUtensorMap* map, 
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(c0), "r"(c1) : "memory");
 }
-// The same for data that a step reads once, the first to leave L2: the weights of products of few tokens.  A decode step
-// streams more of them than L2 holds (2B shape: 156 MB a layer), and what went with them were the small kernels between
-// the products: their instructions, the partial sums, keys and values.  Step of one sequence, 2B shape: 1,585 -> 1,450 us.
+// The same for data that a step reads once, the first to leave L2: the weights.  A decode step streams more of them than L2
+// holds (2B shape: 156 MB a layer), and what went with them were the small kernels between the products: their
+// instructions, the partial sums, keys and values.  Step of one sequence, 2B shape: 1,585 -> 1,450 us.  With many tokens
+// several CTAs read a weight tile, but at about the same time (tiles of tokens are the inner index of a launch's order), and
+// what the next launches read again is tokens.
 __device__ __forceinline__ uint64_t once_policy() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
@@ -979,7 +981,8 @@ static TileForm choose_form(int M, int N, int kblocks, int sms) {
         if (c.bn > 128 && N < 256) continue;
         if (c.cluster > 1 && 2 * c.cluster > kblocks) continue;
         const long long bm = c.pair ? 256 : BM, tiles = ((M + bm - 1) / bm) * ((N + c.bn - 1) / c.bn);
-        // SMs are handed out a GPC at a time: 45 clusters of three and 33 of four fit the 148 SMs
+        // SMs are handed out a GPC at a time: of these kernels, one CTA an SM, the runtime reports 74 clusters of two, 45 of
+        // three and 33 of four at once on a B200's 148 SMs.  (Elsewhere in proportion: an estimate in a cost, not a limit.)
         const long long slots = c.pair || c.cluster == 2 ? sms / 2 : c.cluster == 1 ? sms : c.cluster == 3 ? sms * 45 / 148 : sms * 33 / 148;
         const double rounds = (double)((tiles + slots - 1) / (slots > 0 ? slots : 1));
         const double busy = rounds * (c.round + (kblocks + c.cluster - 1) / c.cluster * c.kblock);
@@ -1174,9 +1177,11 @@ static int gemm_tc_run(const void* A, const void* W, void* C, int c_dtype, int M
 // tile belongs to one group.  gated_act >= 0: the gated epilogue on rows interleaved per group (N = 2 x the
 // output's width, bfloat16 out); else a plain product into C (bfloat16 or float32).  tile_group: device memory,
 // [ceil(M / tile)] group numbers in [0, groups), or -1 for a tile that is not in use (its rows of C are not written).
-static int gemm_tc_grouped_run(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
-                               long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act,
-                               int unary, const float* row_scale, int tile, cudaStream_t stream) {
+// unary: an activation of experts without a gate branch (0: none); row_scale [M] or null: a number per row of A that multiplies
+// its sums before any activation.
+extern "C" int tb_gemm_tc_grouped_tiles(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
+                                        long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act,
+                                        int unary, const float* row_scale, int tile, cudaStream_t stream) {
     if (M <= 0 || N <= 0 || groups <= 0) return 0;
     if (unary < 0 || unary > 2 || (unary && gated_act >= 0)) return tb_refuse("gemm_tc_grouped: unary activation %d (with gate %d)", unary, gated_act);
     if (!tb_gemm_tc_takes(A, W, M, N, K, lda, ldw))
@@ -1216,27 +1221,6 @@ static int gemm_tc_grouped_run(const void* A, const void* W, void* C, int c_dtyp
     p.tiles_q = (N + bn - 1) / bn;
     return bn == 256 ? OUT3(256, false) : OUT3(128, false);
 #undef OUT3
-}
-
-extern "C" int tb_gemm_tc_grouped(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
-                                  long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act,
-                                  cudaStream_t stream) {
-    return gemm_tc_grouped_run(A, W, C, c_dtype, M, N, groups, K, lda, ldw, ldc, tile_group, gated_act, 0, nullptr, BM, stream);
-}
-
-// The same with a unary activation (experts without a gate branch; 0: none) and with a number per row of A that multiplies
-// its sums before any activation (row_scale [M], or null).
-extern "C" int tb_gemm_tc_grouped_ex(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
-                                     long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act, int unary,
-                                     const float* row_scale, cudaStream_t stream) {
-    return gemm_tc_grouped_run(A, W, C, c_dtype, M, N, groups, K, lda, ldw, ldc, tile_group, gated_act, unary, row_scale, BM, stream);
-}
-
-// The same with tiles of `tile` rows: 16, 32, 64 or 128.
-extern "C" int tb_gemm_tc_grouped_tiles(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K,
-                                        long long lda, long long ldw, long long ldc, const int* tile_group, int gated_act, int unary,
-                                        const float* row_scale, int tile, cudaStream_t stream) {
-    return gemm_tc_grouped_run(A, W, C, c_dtype, M, N, groups, K, lda, ldw, ldc, tile_group, gated_act, unary, row_scale, tile, stream);
 }
 
 extern "C" int tb_gemm_tc_ex(const void* A, const void* W, void* C, int c_dtype, int M, int N, int K,

@@ -370,15 +370,14 @@ struct MoeGroupedArgs {
 };
 extern "C" int tb_moe_grouped_args_bytes() { return (int)sizeof(MoeGroupedArgs); }  // for the Python mirror's check
 
-// MODE 1: rows of x (by pair / top) times [G_e ; U_e] for 64 columns of ff, then silu(g) * u  ->  act[pair]
-// MODE 2: rows of x (by pair / top) times U_e for 128 columns of ff, then relu(u)^2            ->  act[pair]
-// MODE 0: rows of act (by pair) times D_e for 128 columns of W, times the pair's weight        ->  pair_out[pair]
+// GATED: rows of x (by pair / top) times [G_e ; U_e] for 64 columns of ff, then silu(g) * u  ->  act[pair]
+// else:  rows of act (by pair) times D_e for 128 columns of W, times the pair's weight       ->  pair_out[pair]
+// (Experts without a gate matrix have a tile on tcgen05 at every count that is grouped.)
 // A tile is 128 pairs x 128 weight rows, eight warps (4 x 2) of 32 x 64 each, k in blocks of 64 through a three-stage
 // cp.async ring.  GATED lays the weight rows out so that a warp holds a gate column and its up column in one thread:
 // rows 64w .. 64w+31 of the tile are gate rows n0 + 32w .., rows 64w+32 .. 64w+63 the up rows of the same columns.
-template <int MODE>
+template <bool GATED>
 __global__ void __launch_bounds__(MG_THREADS, 2) moe_grouped_kernel(MoeGroupedArgs a) {
-    constexpr bool GATED = MODE == 1, FROM_X = MODE != 0;
     pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char mg_ring[];
     __shared__ int row_src[MG_BM];
@@ -387,22 +386,22 @@ __global__ void __launch_bounds__(MG_THREADS, 2) moe_grouped_kernel(MoeGroupedAr
     pdl_wait();
     if (tile >= *a.n_tiles) return;
     const int e = a.tile_expert[tile], row0 = a.tile_row0[tile], rows = a.tile_rows[tile];
-    const int K = FROM_X ? a.W : a.ff;
-    const int N = FROM_X ? a.ff : a.W;
+    const int K = GATED ? a.W : a.ff;
+    const int N = GATED ? a.ff : a.W;
     const int n0 = blockIdx.y * (GATED ? MG_BN / 2 : MG_BN);
     if (threadIdx.x < MG_BM) row_src[threadIdx.x] = threadIdx.x < rows ? a.perm[row0 + threadIdx.x] : -1;
     __syncthreads();
-    const bf16* A = FROM_X ? a.x : a.act;
-    const long long a_stride = FROM_X ? a.x_stride : a.ff;
+    const bf16* A = GATED ? a.x : a.act;
+    const long long a_stride = GATED ? a.x_stride : a.ff;
     const bf16* B1 = a.up_w + (size_t)e * a.ff * a.W;
-    const bf16* B0 = MODE == 1 ? a.gate_w + (size_t)e * a.ff * a.W : (MODE == 2 ? B1 : a.down_w + (size_t)e * a.W * a.ff);
+    const bf16* B0 = GATED ? a.gate_w + (size_t)e * a.ff * a.W : a.down_w + (size_t)e * a.W * a.ff;
     auto load = [&](int s, int k0) {
         unsigned char* sa = mg_ring + (size_t)s * MG_STAGE_BYTES; unsigned char* sb = sa + MG_BM * MG_PITCH;
         for (int c = threadIdx.x; c < MG_BM * (MG_BK / 8); c += MG_THREADS) {
             const int r = c >> 3, ch = c & 7, k = k0 + ch * 8;
             const int p = row_src[r];
             const bool ok = p >= 0 && k < K;
-            const bf16* src = A + (size_t)(ok ? (FROM_X ? p / a.top : p) : 0) * a_stride + (ok ? k : 0);
+            const bf16* src = A + (size_t)(ok ? (GATED ? p / a.top : p) : 0) * a_stride + (ok ? k : 0);
             mg_cp16(sa + r * MG_PITCH + ch * 16, src, ok);
         }
         for (int c = threadIdx.x; c < MG_BN * (MG_BK / 8); c += MG_THREADS) {
@@ -452,7 +451,7 @@ __global__ void __launch_bounds__(MG_THREADS, 2) moe_grouped_kernel(MoeGroupedAr
     for (int m = 0; m < 2; m++) {
         const int ra = wm * 32 + m * 16 + (lane >> 2), rb = ra + 8;
         const int pa = row_src[ra], pb = row_src[rb];
-        if (FROM_X && a.weight_in) {
+        if (GATED && a.weight_in) {
             const float ia = pa >= 0 ? a.weight[pa] : 0.f, ib = pb >= 0 ? a.weight[pb] : 0.f;
 #pragma unroll
             for (int n = 0; n < 8; n++) { acc[m][n][0] *= ia; acc[m][n][1] *= ia; acc[m][n][2] *= ib; acc[m][n][3] *= ib; }
@@ -467,18 +466,6 @@ __global__ void __launch_bounds__(MG_THREADS, 2) moe_grouped_kernel(MoeGroupedAr
                     const float ga = acc[m][n][j], ua = acc[m][n + 4][j], gb = acc[m][n][2 + j], ub = acc[m][n + 4][2 + j];
                     if (pa >= 0) a.act[(size_t)pa * a.ff + col] = __float2bfloat16_rn(ga / (1.f + expf(-ga)) * ua);
                     if (pb >= 0) a.act[(size_t)pb * a.ff + col] = __float2bfloat16_rn(gb / (1.f + expf(-gb)) * ub);
-                }
-            }
-        } else if (MODE == 2) {
-#pragma unroll
-            for (int n = 0; n < 8; n++) {
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const int col = n0 + wn * 64 + n * 8 + cq + j;
-                    if (col >= N) continue;
-                    const float ua = fmaxf(acc[m][n][j], 0.f), ub = fmaxf(acc[m][n][2 + j], 0.f);
-                    if (pa >= 0) a.act[(size_t)pa * a.ff + col] = __float2bfloat16_rn(ua * ua);
-                    if (pb >= 0) a.act[(size_t)pb * a.ff + col] = __float2bfloat16_rn(ub * ub);
                 }
             }
         } else {
@@ -629,23 +616,22 @@ extern "C" int tb_moe_grouped(const MoeGroupedArgs* args, const float* shared, i
                               const float* gate, float* out, int n_tokens, int max_tiles, cudaStream_t stream) {
     const MoeGroupedArgs& a = *args;
     if (n_tokens <= 0) return 0;
+    if (a.gate_w == nullptr) return tb_refuse("moe_grouped: the experts need a gate matrix");
     if (a.W % 8 || a.ff % 8 || (a.x_stride % 8) ||
         (((uintptr_t)a.x | (uintptr_t)a.gate_w | (uintptr_t)a.up_w | (uintptr_t)a.down_w) & 15))
         return tb_refuse("moe_grouped: W=%d and ff=%d must be multiples of 8 and the rows and matrices 16-byte aligned", a.W, a.ff);
     constexpr int SMEM = MG_STAGES * MG_STAGE_BYTES;
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e1 = cudaFuncSetAttribute(moe_grouped_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        cudaError_t e2 = cudaFuncSetAttribute(moe_grouped_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        cudaError_t e3 = cudaFuncSetAttribute(moe_grouped_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-        if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) return (int)(e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3));
+        cudaError_t e1 = cudaFuncSetAttribute(moe_grouped_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaError_t e2 = cudaFuncSetAttribute(moe_grouped_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e1 != cudaSuccess || e2 != cudaSuccess) return (int)(e1 != cudaSuccess ? e1 : e2);
         attr_set = true;
     }
-    if (a.gate_w != nullptr) tb_launch(moe_grouped_kernel<1>, dim3(max_tiles, (a.ff + 63) / 64), dim3(MG_THREADS), SMEM, stream, a);
-    else tb_launch(moe_grouped_kernel<2>, dim3(max_tiles, (a.ff + MG_BN - 1) / MG_BN), dim3(MG_THREADS), SMEM, stream, a);   // experts without a gate matrix
+    tb_launch(moe_grouped_kernel<true>, dim3(max_tiles, (a.ff + 63) / 64), dim3(MG_THREADS), SMEM, stream, a);
     int st = tb_launch_status();
     if (st) return st;
-    tb_launch(moe_grouped_kernel<0>, dim3(max_tiles, (a.W + MG_BN - 1) / MG_BN), dim3(MG_THREADS), SMEM, stream, a);
+    tb_launch(moe_grouped_kernel<false>, dim3(max_tiles, (a.W + MG_BN - 1) / MG_BN), dim3(MG_THREADS), SMEM, stream, a);
     st = tb_launch_status();
     if (st) return st;
     const long long n = (long long)n_tokens * a.W;

@@ -2089,7 +2089,7 @@ class _MoeGroupedArgs(ctypes.Structure):
 
 
 def _moe_grouped(x, gate_w, up_w, down_w, idx, weight, shared, gate, out, on_input=False):
-    """The experts' products with the pairs grouped by expert (bfloat16, tensor cores; see moe.cu).  The grid holds the
+    """The products of experts with a gate, the pairs grouped by expert (bfloat16, tensor cores; see moe.cu).  The grid holds the
     most tiles there can be, so nothing the host does depends on which experts were chosen."""
     T, W = x.shape
     E, ff = up_w.shape[0], up_w.shape[1]
@@ -2108,7 +2108,7 @@ def _moe_grouped(x, gate_w, up_w, down_w, idx, weight, shared, gate, out, on_inp
     _check(lib, lib.tb_moe_group(ctypes.byref(g), _stream()), "moe_group")
     a = _MoeGroupedArgs()
     a.x = x.data_ptr(); a.x_stride = x.stride(0)
-    a.gate_w = gate_w.data_ptr() if gate_w is not None else None; a.up_w = up_w.data_ptr(); a.down_w = down_w.data_ptr()
+    a.gate_w = gate_w.data_ptr(); a.up_w = up_w.data_ptr(); a.down_w = down_w.data_ptr()
     a.perm = perm.data_ptr(); a.tile_expert = te.data_ptr(); a.tile_row0 = tr0.data_ptr(); a.tile_rows = trn.data_ptr()
     a.n_tiles = nt.data_ptr(); a.weight = weight.data_ptr(); a.act = act.data_ptr(); a.pair_out = pair_out.data_ptr()
     a.W = W; a.ff = ff; a.top = top; a.weight_in = int(on_input)
