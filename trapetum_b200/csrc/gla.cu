@@ -299,7 +299,7 @@ __global__ void gla_fold_kernel(GlaArgs a) {
 // the outputs, normed and gated: the CTA holds the head.
 // A non-finite v is seen by its own token and later ones only, as in the recurrence; what it leaves in the state is NaN to the
 // next block's outputs (an infinity has no three parts).
-// Prompts of 1,500 and 548 tokens, 8 heads of 128 x 256, all of ops.gla, passes back to back: 147.4 us (the recurrence in chunks,
+// Prompts of 1,500 and 548 tokens, 8 heads of 128 x 256, all of ops.gla, passes back to back: 141.7 us (the recurrence in chunks,
 // its norm a launch of its own: 453; there the chunks of the shorter prompt leave SMs idle too).  A block takes 9.6 us of its CTA: shared
 // memory (14 of 18 thousand cycles), then issue slots; the products are a quarter of the tensor pipe.
 // ---------------------------------------------------------------------------------------------------------

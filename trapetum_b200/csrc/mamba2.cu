@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(SCAN_NS * PT / SCAN_PP) mamba2_scan_kernel(Mam
 // NaN to the next chunk's outputs (an infinity has no three parts).
 // 2,048 tokens, 64 heads of 64 x 128: 31 + 20 + 56 us cold (the recurrence in chunks: 167 + 235; both before the sums of 16 terms,
 // which take 3 % more); the tensor pipe and the three-way splits share the time of the third launch.  All of ops.mamba2, passes
-// back to back: 489 -> 137.5 us.
+// back to back: 489 -> 136.8 us.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int MC = 128, MCT = 256;                    // tokens of a chunk, threads
 constexpr int MP = 64, MXPITCH = MP * 2 + 16;         // values of P a CTA takes; bytes of a shared row of them (no bank conflicts)
