@@ -881,6 +881,14 @@ def moe_rule(ops, T, top, E, W, ff, gated):
     return ops.moe_tile(T * top, E, (3 if gated else 2) * W * ff * 2)
 
 
+def test_moe_few_pairs_are_grouped_where_they_share_enough(ops):
+    """Pairs, experts, an expert's bytes: on either side of the lines that the rule draws for fewer than 128 pairs."""
+    mb = 1 << 20
+    for pairs, experts, size, tile in ((48, 32, 12 * mb, 16), (47, 32, 12 * mb, 0), (64, 64, 3 * mb, 0), (96, 64, 3 * mb, 16),
+                                       (64, 128, 4 * mb, 0), (96, 128, 4 * mb, 16), (127, 2048, 12 * mb, 0), (127, 4096, 12 * mb, 0), (128, 4096, mb, 16)):
+        assert ops.moe_tile(pairs, experts, size) == tile, (pairs, experts, size)
+
+
 # tokens, experts a token, experts, width, ff, the tile that the rule picks
 MOE_TILES = [(12, 4, 32, 2048, 1024, 16), (33, 4, 8, 136, 48, 32), (200, 2, 16, 96, 208, 64), (700, 2, 6, 72, 16, 128), (128, 1, 40, 264, 144, 16)]
 

@@ -2022,11 +2022,15 @@ def moe_tile(pairs: int, experts: int, expert_bytes: int) -> int:
     (32 experts of 12.6 MB, us with tiles of 16 / 32 / 64 / 128: 32 tokens, 4 experts each, 82 / 83 / 83 / 102; 192 tokens
     100 / 84 / 86 / 104; 512 tokens 179 / 117 / 106 / 120; the grouped kernel on mma.sync 195, 203, -).  Few pairs are
     grouped (three launches more, two of them short) where they share experts and read much: 12 tokens of the same 69
-    against 98 pair by pair, but 8 tokens 64 against 67, of experts of 6.3 MB 45 against 39, of 3.1 MB 32 against 25."""
+    against 98 pair by pair, but 8 tokens 64 against 67, of experts of 6.3 MB 45 against 39, of 3.1 MB 32 against 25.  What
+    is not read again has to outweigh about 17 us: 64 pairs over 64 experts of 3.1 MB save 74 MB, 39 against 36; 96 pairs
+    of these 145 MB, 42 against 53; 64 pairs over 128 ungated ones of 4.2 MB 57 MB, 55 against 48; 96 over these 119 MB, 66
+    against 74."""
     if pairs < MOE_GROUPED_FROM:
         if pairs < 48 or pairs * expert_bytes < 150 << 20 or experts > 2048:
             return 0
-        if experts * (1.0 - (1.0 - 1.0 / experts) ** pairs) > 0.8 * pairs:        # experts that some pair chooses
+        chosen = experts * (1.0 - (1.0 - 1.0 / experts) ** pairs)                   # experts that some pair chooses
+        if chosen > 0.8 * pairs or (pairs - chosen) * expert_bytes < 90 << 20:
             return 0
     share = pairs / experts
     return 16 if share <= 12 else 32 if share <= 24 else 64 if share <= 64 else 128
