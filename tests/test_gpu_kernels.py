@@ -975,10 +975,11 @@ def test_moe_experts_leave_a_joint_matrix_that_is_not_packed_unread(ops, T):
     assert ops.kernel_errors() == {}
 
 
-@pytest.mark.parametrize("T", [4, 16, 60, 300, 700])
-def test_moe_gate_far_below_zero(ops, T):
-    """silu(-88) = -88 e^-88 is a bfloat16 number (-5e-37), whichever way the experts' products run."""
-    E, W, ff, top = 12, 1024, 512, 4
+@pytest.mark.parametrize("T, E, tile", [(4, 12, 0), (16, 12, 16), (60, 12, 32), (120, 12, 64), (255, 12, 128)])
+def test_moe_gate_far_below_zero(ops, T, E, tile):
+    """silu(-88) = -88 e^-88 is a bfloat16 number (-5e-37), pair by pair and in tiles of every size below 1,024 pairs."""
+    W, ff, top = 1024, 512, 4
+    assert moe_rule(ops, T, top, E, W, ff, True) == tile and T * top < ops.MOE_EXACT_BELOW
     x = torch.zeros(T, W, dtype=torch.bfloat16, device="cuda")
     x[:, 0] = 1.0
     gw, uw = (torch.zeros(E, ff, W, dtype=torch.bfloat16, device="cuda") for _ in range(2))

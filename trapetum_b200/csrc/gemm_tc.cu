@@ -74,11 +74,11 @@ struct GemmParams {
 // The result is rounded to bfloat16, so tanh and the logistic function are taken through the fast exponential
 // and division (relative error near 2^-21): 0.5 (1 + tanh(y)) = 1 / (1 + e^(-2y)).
 // clamped_swish: g' = min(g, L), u' = clamp(u, -L, L), g' / (1 + e^(-1.702 g')) * (u' + 1).
-// That error grows with the gate, to 2^-19 at -30, and below -87.3, where the divisor passes 2^126, the quotient is 0.  EXACT
-// (the experts' grouped products): silu by expf and a true quotient, the function of the experts' other kernels.
+// That error grows with the gate, to 2^-19 at -30, and below -87.3, where the divisor passes 2^126, the quotient is 0.  Act 3
+// (EXACT, the grouped products of experts): silu by expf and a true quotient, the function of the experts' other kernels.
 template <bool EXACT>
 __device__ __forceinline__ float gated(float g, float u, int act, float limit) {
-    if (EXACT && act == 1) return g / (1.0f + expf(-g)) * u;
+    if (EXACT && act == 3) return g / (1.0f + expf(-g)) * u;
     if (act == 2) {
         g = fminf(g, limit);
         u = fminf(fmaxf(u, -limit), limit) + 1.0f;
@@ -1190,8 +1190,8 @@ extern "C" int tb_gemm_tc_grouped_tiles(const void* A, const void* W, void* C, i
     if (tile_group == nullptr) return tb_refuse("gemm_tc_grouped: no table of groups");
     if ((long long)groups * N > 2147483647LL) return tb_refuse("gemm_tc_grouped: %d groups of %d rows", groups, N);
     const bool gated = gated_act >= 0;
-    if (gated && (gated_act > 1 || N % 32 || c_dtype != TB_BF16))
-        return tb_refuse("gemm_tc_grouped: the gated epilogue (gelu_tanh or silu) needs a multiple of 32 weight rows and writes bfloat16");
+    if (gated && ((gated_act > 1 && gated_act != 3) || N % 32 || c_dtype != TB_BF16))
+        return tb_refuse("gemm_tc_grouped: the gated epilogue (gelu_tanh, silu or exact silu) needs a multiple of 32 weight rows and writes bfloat16");
     if (tile != 16 && tile != 32 && tile != 64 && tile != 128) return tb_refuse("gemm_tc_grouped: tiles of %d rows", tile);
     if (!g_sms) {
         int dev = 0; cudaGetDevice(&dev);

@@ -2014,6 +2014,9 @@ def moe_route(logits: torch.Tensor, experts: int, correction: Optional[torch.Ten
 
 
 MOE_GROUPED_FROM = 128      # (token, expert) pairs from which the experts' products run grouped by expert
+MOE_EXACT_BELOW = 1024      # ... and below which grouped products on tcgen05 take silu by expf and a true quotient, as pair by pair
+                            # (many pairs: by the fast forms; 1,024 pairs of 8 experts of 12.6 MB 45 us, with the exact ones 64)
+GEMM_TC_SILU_EXACT = 3
 
 
 def moe_tile(pairs: int, experts: int, expert_bytes: int) -> int:
@@ -2068,7 +2071,7 @@ def _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, ungate
     gl = build.load("gemm_tc")
     _check(gl, gl.tb_gemm_tc_grouped_tiles(_ptr(xs), _ptr(gate_up_w), _ptr(act), c_int(code(x.dtype)), c_int(max_rows), c_int(ff2),
                                         c_int(E), c_int(W), c_longlong(W), c_longlong(W), c_longlong(ff), _ptr(tile_group),
-                                        c_int(-1 if ungated else ACTIVATIONS["silu"]), c_int(GEMM_TC_UNARY["relu2"] if ungated else 0),
+                                        c_int(-1 if ungated else GEMM_TC_SILU_EXACT if P < MOE_EXACT_BELOW else ACTIVATIONS["silu"]), c_int(GEMM_TC_UNARY["relu2"] if ungated else 0),
                                         _ptr(row_weight), c_int(tile), _stream()), "gemm_tc_grouped")
     _check(gl, gl.tb_gemm_tc_grouped_tiles(_ptr(act), _ptr(down_w), _ptr(y), c_int(code(torch.float32)), c_int(max_rows), c_int(W),
                                      c_int(E), c_int(ff), c_longlong(ff), c_longlong(ff), c_longlong(W), _ptr(tile_group),
