@@ -138,15 +138,18 @@ __global__ void rope_kv_kernel(RopeKvArgs a) {
 }
 
 // The same for many tokens (a prompt), bfloat16, head_dim a multiple of 16 with the whole head rotated or
-// rotary_dim a multiple of 16: a CTA of ROPE_TH threads a token, 16-byte accesses.  The threads make the token's sines and
+// rotary_dim a multiple of 16: a CTA of 128 threads a token, 16-byte accesses (64
+// threads where a token has no more work items than that and there are many tokens: 12 heads over 2 of 64, 1,024 / 2,048 / 8,192
+// tokens 3.0 / 4.8 / 14.5 us with 128, 3.5 / 4.2 / 10.9 with 64).  The threads make the token's sines and
 // cosines once, one or two angles each, and leave them in shared memory; then each takes work items of eight neighbouring
 // pairs of one head (dims i..i+7 and i+half..i+half+7).  What a thread reads of the row first is requested before its angles
 // are made.  Up to about a thousand tokens the launch lasts as long as one token's chain (a warp a token made eight angles a lane
 // and then went through its heads), beyond that as long as its bytes: us in a graph, a warp a token -> so, tokens 128 / 384 /
 // 1,024 / 2,048 / 8,192: 8 heads over 4 of 256 5.3 / 5.4 / 6.9 / 8.6 / 32.4 -> 2.7 / 3.9 / 4.5 / 8.7 / 28.8, 32 over 16 of 128 8.0 /
 // 8.3 / 13.0 / 15.1 / 61.5 -> 4.0 / 5.9 / 8.0 / 13.5 / 49.6.
-constexpr int ROPE_TH = 128, ROPE_GROUPS = 32;          // threads; most groups of eight pairs of a head
-__global__ void __launch_bounds__(ROPE_TH, 8) rope_kv_rows_kernel(RopeKvArgs a) {
+constexpr int ROPE_GROUPS = 32;                         // most groups of eight pairs of a head
+template <int ROPE_TH>
+__global__ void __launch_bounds__(ROPE_TH, 1024 / ROPE_TH) rope_kv_rows_kernel(RopeKvArgs a) {
     pdl_launch_dependents();
     __shared__ float4 turn_s[2][2][ROPE_GROUPS];        // [sine, cosine][first, last four pairs][group]
     const int t = blockIdx.x, tid = threadIdx.x;
@@ -266,7 +269,10 @@ extern "C" int tb_rope_kv(const RopeKvArgs* args, int dtype, int n_tokens, cudaS
         ((uintptr_t)a.k_pool & 15) == 0 && ((uintptr_t)a.v_pool & 15) == 0) {
         RopeKvArgs b = a;
         if (b.inv_freq == nullptr) b.rotary_dim = 0;
-        tb_launch(rope_kv_rows_kernel, dim3(n_tokens), dim3(ROPE_TH), 0, stream, b);
+        const int groups = b.rotary_dim / 16, chunks = b.head_dim / 8;
+        const int items = max((b.n_heads + b.n_kv_heads) * groups, b.k_pool ? b.n_kv_heads * (2 * chunks - 2 * groups) : 0);
+        if (items <= 64 && n_tokens > 1536) tb_launch(rope_kv_rows_kernel<64>, dim3(n_tokens), dim3(64), 0, stream, b);
+        else tb_launch(rope_kv_rows_kernel<128>, dim3(n_tokens), dim3(128), 0, stream, b);
         return tb_launch_status();
     }
     const int slots = a.n_heads + 2 * a.n_kv_heads;
