@@ -387,6 +387,7 @@ __device__ __forceinline__ int mp_tile(int x, int n, int window) {
     return x % blocks * per + rest - 1 - x / blocks;
 }
 
+constexpr unsigned IN_ORDER = ~0u;
 // MULTI: more than 16 heads (the second paragraph above); else a warp's only raw scores are its own head's.
 template <int KT, bool MULTI, bool PAIRS>
 __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnArgs a, unsigned flip) {
@@ -402,10 +403,17 @@ __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnAr
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h_raw = warp < H ? warp : 0;
     // which work: the launch's CTAs in order, `flip` of them backwards, go round the sequences and groups of heads, so that
-    // every sequence's longest tiles come first
-    const unsigned cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    const unsigned turn = cta < flip ? flip - 1 - cta : cta, round = gridDim.y * gridDim.z;
-    const int nth = turn / round, b = turn % round % gridDim.y, z = turn % round / gridDim.y;
+    // every sequence's longest tiles come first; a last group of fewer heads (H above 16, no multiple of it) is shorter work and
+    // comes after the others (1,000 tokens, 24 heads, window 256: 72.0 us going round it too, 69.3 so).  IN_ORDER: all start at once.
+    int nth = blockIdx.x, b = blockIdx.y, z = blockIdx.z;
+    if (flip != IN_ORDER) {
+        const unsigned cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+        unsigned turn = cta < flip ? flip - 1 - cta : cta, zs = gridDim.z;
+        z = 0;
+        if (MULTI && H % 16) { const unsigned group = gridDim.x * gridDim.y; z = turn / group; turn %= group; zs = 1; }
+        const unsigned round = gridDim.y * zs;
+        nth = turn / round; b = turn % round % gridDim.y; z += turn % round / gridDim.y;
+    }
     const int h_out = z * 16 + warp;                         // the head this warp mixes, weighs and writes
     const bool has_out = h_out < H;
     const int h = has_out ? h_out : h_raw;                            // the head whose queries stay in registers
@@ -421,7 +429,7 @@ __global__ void __launch_bounds__(512) attn_mixed_prefill_mma_kernel(MixedAttnAr
     const int P = a.n_pieces > 1 ? a.n_pieces : 1;
     const int tiles_of_b = (len + MP_BM - 1) / MP_BM, piece = nth % P;
     if (nth / P >= tiles_of_b) return;
-    const int i0 = mp_tile(nth / P, tiles_of_b, a.window) * MP_BM;
+    const int i0 = (flip == IN_ORDER ? nth / P : mp_tile(nth / P, tiles_of_b, a.window)) * MP_BM;
     const int i_last = min(i0 + MP_BM - 1, len - 1);
     const int ia = i0 + r, ib = i0 + r + 8;                           // the two queries whose scores this thread holds
     // the queries of this head as the products' left operand, kept in registers
@@ -685,10 +693,11 @@ extern "C" int tb_attn_mixed_prefill(const MixedAttnArgs* args, int dtype, cudaS
         }
         // Where an SM holds two CTAs (up to eight heads: registers for 16 warps, shared memory), the first of each SM start with
         // the shortest of the longest, so that the second of an SM, which is short, meets one that is not long
-        // (700 tokens, 8 heads, blocks of 512: 31.4 us, by length alone 33.4).
-        const bool two = warps <= 8 && 2 * (sm + 1024) <= 228 * 1024;
+        // (700 tokens, 8 heads, blocks of 512: 31.4 us, by length alone 33.4; up to four heads only if every other SM has a second: 176
+        // CTAs 14.6 us by length alone and 15.5 so, 256 CTAs 38.3 and 36.6).
         const unsigned long long total = (unsigned long long)grid.x * grid.y * grid.z;
-        const unsigned flip = two ? (unsigned)(total < (unsigned long long)sms ? total : sms) : 0u;
+        const bool two = (warps > 4 ? warps <= 8 : 2 * total > 3ull * sms) && 2 * (sm + 1024) <= 228 * 1024;
+        const unsigned flip = total <= (unsigned long long)sms ? IN_ORDER : two ? (unsigned)sms : 0u;
 #define TB_MP_LAUNCH_AS(KT, MULTI, PAIRS) do { allow_smem(attn_mixed_prefill_mma_kernel<KT, MULTI, PAIRS>, sm); \
             tb_launch(attn_mixed_prefill_mma_kernel<KT, MULTI, PAIRS>, grid, dim3(warps * 32), sm, stream, am, flip); } while (0)
 #define TB_MP_LAUNCH(KT) do { if (a.H > 16) TB_MP_LAUNCH_AS(KT, true, false); \
