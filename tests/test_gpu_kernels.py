@@ -884,7 +884,8 @@ def moe_rule(ops, T, top, E, W, ff, gated):
 def test_moe_few_pairs_are_grouped_where_they_share_enough(ops):
     """Pairs, experts, an expert's bytes: on either side of the lines that the rule draws for fewer than 128 pairs."""
     mb = 1 << 20
-    for pairs, experts, size, tile in ((48, 32, 12 * mb, 16), (47, 32, 12 * mb, 0), (64, 64, 3 * mb, 0), (96, 64, 3 * mb, 16),
+    for pairs, experts, size, tile in ((48, 32, 12 * mb, 16), (47, 32, 12 * mb, 0), (79, 32, 3 * mb, 0), (80, 32, 3 * mb, 16), (64, 64, 4 * mb, 16),
+                                       (64, 64, 3 * mb, 0), (96, 64, 3 * mb, 16),
                                        (64, 128, 4 * mb, 0), (96, 128, 4 * mb, 16), (127, 2048, 12 * mb, 0), (127, 4096, 12 * mb, 0), (128, 4096, mb, 16)):
         assert ops.moe_tile(pairs, experts, size) == tile, (pairs, experts, size)
 
@@ -962,7 +963,15 @@ def test_moe_experts_whose_matrices_begin_off_16_bytes(ops, which, T, top, E, W,
     assert ops.kernel_errors() == {}
 
 
-@pytest.mark.parametrize("T", [16, 60, 300])
+def test_moe_tiles_refuse_scratch_that_is_too_small(ops, monkeypatch):
+    idx, weight, x, gw, uw, dw, both, want = moe_case(ops, 60, 4, 12, 136, 48, True)
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *s, **k: empty(s[0] - 256, **k) if k.get("dtype") == torch.uint8 else empty(*s, **k))
+    with pytest.raises(ops.KernelError, match="scratch"):
+        ops.moe_experts(x, gw, uw, dw, idx, weight, gate_up_w=both)
+
+
+@pytest.mark.parametrize("T", [24, 60, 300])
 def test_moe_experts_leave_a_joint_matrix_that_is_not_packed_unread(ops, T):
     """The interleaved gate and up rows only speed the products up: if they are not [E, 2 ff, W], packed, of x's dtype the
     single matrices are read."""
@@ -975,7 +984,7 @@ def test_moe_experts_leave_a_joint_matrix_that_is_not_packed_unread(ops, T):
     assert ops.kernel_errors() == {}
 
 
-@pytest.mark.parametrize("T, E, tile", [(4, 12, 0), (16, 12, 16), (60, 12, 32), (120, 12, 64), (255, 12, 128)])
+@pytest.mark.parametrize("T, E, tile", [(4, 12, 0), (24, 12, 16), (60, 12, 32), (120, 12, 64), (255, 12, 128)])
 def test_moe_gate_far_below_zero(ops, T, E, tile):
     """silu(-88) = -88 e^-88 is a bfloat16 number (-5e-37), pair by pair and in tiles of every size below 1,024 pairs."""
     W, ff, top = 1024, 512, 4

@@ -505,9 +505,9 @@ __global__ void moe_sum_pairs_kernel(const float* __restrict__ pair_out, const f
 // ---------------------------------------------------------------------------
 // The same grouping for the tcgen05 product (gemm_tc.cu, grouped mode): the pairs are laid out expert by expert
 // with every expert's stretch padded to whole tiles of `tile` rows, so that a tile of the product's token operand
-// belongs to one expert.  tb_moe_group_padded makes the layout (where every pair goes, which pair every row
-// holds, every tile's expert), tb_moe_gather_rows fills the operand (and, if asked for, lays every row's weight out
-// beside it, for weights that multiply the experts' input), and tb_moe_combine_sorted adds a token's
+// belongs to one expert.  moe_group_padded_kernel makes the layout (where every pair goes, which pair every row
+// holds, every tile's expert), moe_gather_rows_kernel fills the operand (and, if asked for, lays every row's weight out
+// beside it, for weights that multiply the experts' input), and moe_combine_sorted_kernel adds a token's
 // weighted expert outputs (and the shared expert) back up.
 // ---------------------------------------------------------------------------
 struct MoePadArgs {
@@ -575,32 +575,60 @@ __global__ void moe_combine_sorted_kernel(const float* __restrict__ y, const int
     out[i] = acc;
 }
 
-extern "C" int tb_moe_group_padded(const MoePadArgs* args, cudaStream_t stream) {
-    const MoePadArgs& a = *args;
-    if (a.P <= 0) return 0;
-    if (a.E <= 0 || a.E > 2048 || a.tile <= 0 || a.max_rows % a.tile || a.max_rows < a.P)
-        return tb_refuse("moe_group_padded: experts=%d rows=%d tile=%d", a.E, a.max_rows, a.tile);
-    tb_launch(moe_group_padded_kernel, dim3(1), dim3(1024), (size_t)3 * a.E * sizeof(int), stream, a);
-    return tb_launch_status();
-}
+// The five launches by one call: made one by one from Python, with an allocation for each intermediate, they and the routing took the
+// host 66 us, longer than the device takes for small experts; so 41.  The product is tb_gemm_tc_grouped_tiles, which lives in another library.
+typedef int (*GroupedProduct)(const void* A, const void* W, void* C, int c_dtype, int M, int N, int groups, int K, long long lda,
+                              long long ldw, long long ldc, const int* tile_group, int gated_act, int unary, const float* row_scale,
+                              int tile, cudaStream_t stream);
+struct MoeTilesArgs {
+    const bf16* x; long long x_stride;         // [T][W]
+    const int* idx; const float* weight;       // [T][top]
+    const bf16* first_w; const bf16* down_w;   // [E][2 ff or ff][W], [E][W][ff]
+    const float* shared; long long shared_split_stride; const float* gate;
+    float* out;                                // [T][W]
+    GroupedProduct product;
+    unsigned char* scratch; long long scratch_bytes;
+    int shared_splits, n_tokens, W, ff, top, E, tile;
+    int gated_act, unary;                      // of the first product: a gate's activation, or -1 and a unary one
+    int weight_in;                             // the weight multiplies the first product's sums, not the second's
+    int in_product;                            // set on return: the status is the product's, with its library's message
+};
+extern "C" int tb_moe_tiles_args_bytes() { return (int)sizeof(MoeTilesArgs); }      // for the Python mirror's check
 
-extern "C" int tb_moe_gather_rows(const void* x, long long x_stride, const int* row_pair, void* out, int rows, int W, int top,
-                                  const float* weight, float* row_weight, cudaStream_t stream) {
-    if (rows <= 0) return 0;
-    if (row_weight != nullptr && weight == nullptr) return tb_refuse("moe_gather_rows: no weights to lay out");
-    if (W % 8 || x_stride % 8 || ((uintptr_t)x & 15) || ((uintptr_t)out & 15)) return tb_refuse("moe_gather_rows: rows must be 16-byte aligned");
-    tb_launch(moe_gather_rows_kernel, dim3(rows), dim3(128), 0, stream, (const bf16*)x, x_stride, row_pair, (bf16*)out, W, top,
-              weight, row_weight);
-    return tb_launch_status();
-}
-
-extern "C" int tb_moe_combine_sorted(const float* y, const int* pos, const float* weight, const float* shared, int shared_splits,
-                                     long long shared_split_stride, const float* gate, float* out, int n_tokens, int W, int top,
-                                     cudaStream_t stream) {
-    const long long n = (long long)n_tokens * W;
-    if (n <= 0) return 0;
-    tb_launch(moe_combine_sorted_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, y, pos, weight, shared, shared_splits,
-              shared_split_stride, gate, out, n, W, top);
+extern "C" int tb_moe_tiles(MoeTilesArgs* args, cudaStream_t stream) {
+    MoeTilesArgs& a = *args;
+    a.in_product = 0;
+    if (a.n_tokens <= 0 || a.top <= 0) return 0;
+    if (a.W % 8 || a.ff % 8 || a.x_stride % 8 || ((uintptr_t)a.x & 15)) return tb_refuse("moe_tiles: rows must be 16-byte aligned");
+    MoePadArgs g;
+    g.P = a.n_tokens * a.top; g.E = a.E; g.tile = a.tile; g.idx = a.idx;
+    if (a.E <= 0 || a.E > 2048 || a.tile <= 0) return tb_refuse("moe_tiles: experts=%d tile=%d", a.E, a.tile);
+    g.max_rows = ((g.P + a.tile - 1) / a.tile + (a.E < g.P ? a.E : g.P)) * a.tile;
+    const long long rows = g.max_rows;
+    long long at = 0;
+    auto take = [&](long long bytes) { unsigned char* p = a.scratch + at; at += (bytes + 255) / 256 * 256; return p; };
+    g.pos = (int*)take(4 * (g.P + rows + rows / a.tile));
+    g.row_pair = g.pos + g.P; g.tile_group = g.row_pair + rows;
+    float* row_weight = a.weight_in ? (float*)take(4 * rows) : nullptr;
+    bf16* xs = (bf16*)take(2 * rows * a.W);
+    bf16* act = (bf16*)take(2 * rows * a.ff);
+    float* y = (float*)take(4 * rows * a.W);
+    if (at > a.scratch_bytes || a.scratch == nullptr || ((uintptr_t)a.scratch & 15))
+        return tb_refuse("moe_tiles: %lld bytes of scratch are needed, %lld given", at, a.scratch_bytes);
+    tb_launch(moe_group_padded_kernel, dim3(1), dim3(1024), (size_t)3 * a.E * sizeof(int), stream, g);
+    int st = tb_launch_status();
+    if (st) return st;
+    tb_launch(moe_gather_rows_kernel, dim3(g.max_rows), dim3(128), 0, stream, a.x, a.x_stride, (const int*)g.row_pair, xs, a.W, a.top,
+              a.weight_in ? a.weight : (const float*)nullptr, row_weight);
+    st = tb_launch_status();
+    if (st) return st;
+    st = a.product(xs, a.first_w, act, TB_BF16, g.max_rows, a.gated_act >= 0 ? 2 * a.ff : a.ff, a.E, a.W, a.W, a.W, a.ff, g.tile_group,
+                   a.gated_act, a.unary, row_weight, a.tile, stream);
+    if (!st) st = a.product(act, a.down_w, y, TB_F32, g.max_rows, a.W, a.E, a.ff, a.ff, a.ff, a.W, g.tile_group, -1, 0, nullptr, a.tile, stream);
+    if (st) { a.in_product = 1; return st; }
+    const long long n = (long long)a.n_tokens * a.W;
+    tb_launch(moe_combine_sorted_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, (const float*)y, (const int*)g.pos,
+              a.weight_in ? (const float*)nullptr : a.weight, a.shared, a.shared_splits, a.shared_split_stride, a.gate, a.out, n, a.W, a.top);
     return tb_launch_status();
 }
 

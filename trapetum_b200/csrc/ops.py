@@ -84,7 +84,7 @@ def args_mirrors():
     return (("gla", "tb_gla_args_bytes", _GlaArgs), ("mamba2", "tb_mamba2_args_bytes", _Mamba2Args), ("retention", "tb_retention_args_bytes", _RetentionArgs),
             ("projnorm_kv", "tb_projnorm_kv_args_bytes", _ProjNormKvArgs), ("norm", "tb_add_terms_args_bytes", _AddTermsArgs),
             ("dyt", "tb_dyt_args_bytes", _DytArgs), ("moe", "tb_moe_route_args_bytes", _MoeRouteArgs),
-            ("moe", "tb_moe_expert_args_bytes", _MoeExpertArgs), ("moe", "tb_moe_grouped_args_bytes", _MoeGroupedArgs))
+            ("moe", "tb_moe_expert_args_bytes", _MoeExpertArgs), ("moe", "tb_moe_grouped_args_bytes", _MoeGroupedArgs), ("moe", "tb_moe_tiles_args_bytes", _MoeTilesArgs))
 
 
 def _rows_contig(t: torch.Tensor, what: str) -> None:
@@ -2014,6 +2014,7 @@ def moe_route(logits: torch.Tensor, experts: int, correction: Optional[torch.Ten
 
 
 MOE_GROUPED_FROM = 128      # (token, expert) pairs from which the experts' products run grouped by expert
+MOE_SHARED_FROM = 48        # ... and from which they may, where they share enough (moe_tile)
 MOE_EXACT_BELOW = 1024      # ... and below which grouped products on tcgen05 take silu by expf and a true quotient, as pair by pair
                             # (many pairs: by the fast forms; 1,024 pairs of 8 experts of 12.6 MB 45 us, with the exact ones 64)
 GEMM_TC_SILU_EXACT = 3
@@ -2025,12 +2026,14 @@ def moe_tile(pairs: int, experts: int, expert_bytes: int) -> int:
     (32 experts of 12.6 MB, us with tiles of 16 / 32 / 64 / 128: 32 tokens, 4 experts each, 82 / 83 / 83 / 102; 192 tokens
     100 / 84 / 86 / 104; 512 tokens 179 / 117 / 106 / 120; the grouped kernel on mma.sync 195, 203, -).  Few pairs are
     grouped (three launches more, two of them short) where they share experts and read much: 12 tokens of the same 69
-    against 98 pair by pair, but 8 tokens 64 against 67, of experts of 6.3 MB 45 against 39, of 3.1 MB 32 against 25.  What
-    is not read again has to outweigh about 17 us: 64 pairs over 64 experts of 3.1 MB save 74 MB, 39 against 36; 96 pairs
+    against 98 pair by pair, but 8 tokens 64 against 67, of experts of 6.3 MB 45 against 39, of 3.1 MB 32 against 25.
+    What is not read again has to outweigh about 17 us: 64 pairs over 64 experts of 3.1 MB save 74 MB, 39 against 36; 96 pairs
     of these 145 MB, 42 against 53; 64 pairs over 128 ungated ones of 4.2 MB 57 MB, 55 against 48; 96 over these 119 MB, 66
-    against 74."""
+    against 74.  And called outside a graph routing and a grouped pass take the host 41 us, pair by pair 30 to 36: 64 pairs
+    over 32 experts of 3.1 MB 43 against 37, 80 pairs 42 against 52; 80 pairs of ungated ones of 2.1 MB 41 against 30, 124 pairs
+    41 against 41."""
     if pairs < MOE_GROUPED_FROM:
-        if pairs < 48 or pairs * expert_bytes < 150 << 20 or experts > 2048:
+        if pairs < MOE_SHARED_FROM or pairs * expert_bytes < 240 << 20 or experts > 2048:
             return 0
         chosen = experts * (1.0 - (1.0 - 1.0 / experts) ** pairs)                   # experts that some pair chooses
         if chosen > 0.8 * pairs or (pairs - chosen) * expert_bytes < 90 << 20:
@@ -2039,9 +2042,12 @@ def moe_tile(pairs: int, experts: int, expert_bytes: int) -> int:
     return 16 if share <= 12 else 32 if share <= 24 else 64 if share <= 64 else 128
 
 
-class _MoePadArgs(ctypes.Structure):
-    _fields_ = [("idx", c_void_p), ("pos", c_void_p), ("row_pair", c_void_p), ("tile_group", c_void_p),
-                ("P", c_int), ("E", c_int), ("max_rows", c_int), ("tile", c_int)]
+class _MoeTilesArgs(ctypes.Structure):
+    _fields_ = [("x", c_void_p), ("x_stride", c_longlong), ("idx", c_void_p), ("weight", c_void_p), ("first_w", c_void_p),
+                ("down_w", c_void_p), ("shared", c_void_p), ("shared_split_stride", c_longlong), ("gate", c_void_p), ("out", c_void_p),
+                ("product", c_void_p), ("scratch", c_void_p), ("scratch_bytes", c_longlong), ("shared_splits", c_int),
+                ("n_tokens", c_int), ("W", c_int), ("ff", c_int), ("top", c_int), ("E", c_int), ("tile", c_int),
+                ("gated_act", c_int), ("unary", c_int), ("weight_in", c_int), ("in_product", c_int)]
 
 
 def _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, ungated=False, on_input=False, tile=128):
@@ -2050,36 +2056,27 @@ def _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, ungate
     depend on the sizes only.  ``ungated``: ``gate_up_w`` holds the up rows alone and the first product's epilogue is relu(u)^2.  ``on_input``: a pair's weight
     multiplies the first product's sums (the gather lays it out beside the rows) instead of the second's."""
     T, W = x.shape
-    E, ff2 = gate_up_w.shape[0], gate_up_w.shape[1]
-    ff = ff2 if ungated else ff2 // 2
+    E, ff = gate_up_w.shape[0], down_w.shape[2]
     top = idx.shape[1]
     P = T * top
-    max_rows = ((P + tile - 1) // tile + min(E, P)) * tile
-    ints = torch.empty(P + max_rows + max_rows // tile, dtype=torch.int32, device=x.device)
-    pos, row_pair, tile_group = ints[:P], ints[P:P + max_rows], ints[P + max_rows:]
-    lib = build.load("moe")
-    g = _MoePadArgs()
-    g.idx = idx.data_ptr(); g.pos = pos.data_ptr(); g.row_pair = row_pair.data_ptr(); g.tile_group = tile_group.data_ptr()
-    g.P = P; g.E = E; g.max_rows = max_rows; g.tile = tile
-    _check(lib, lib.tb_moe_group_padded(ctypes.byref(g), _stream()), "moe_group_padded")
-    xs = torch.empty((max_rows, W), dtype=x.dtype, device=x.device)
-    row_weight = torch.empty(max_rows, dtype=torch.float32, device=x.device) if on_input else None
-    _check(lib, lib.tb_moe_gather_rows(_ptr(x), c_longlong(x.stride(0)), _ptr(row_pair), _ptr(xs), c_int(max_rows), c_int(W),
-                                       c_int(top), _ptr(weight if on_input else None), _ptr(row_weight), _stream()), "moe_gather_rows")
-    act = torch.empty((max_rows, ff), dtype=x.dtype, device=x.device)
-    y = torch.empty((max_rows, W), dtype=torch.float32, device=x.device)
-    gl = build.load("gemm_tc")
-    _check(gl, gl.tb_gemm_tc_grouped_tiles(_ptr(xs), _ptr(gate_up_w), _ptr(act), c_int(code(x.dtype)), c_int(max_rows), c_int(ff2),
-                                        c_int(E), c_int(W), c_longlong(W), c_longlong(W), c_longlong(ff), _ptr(tile_group),
-                                        c_int(-1 if ungated else GEMM_TC_SILU_EXACT if P < MOE_EXACT_BELOW else ACTIVATIONS["silu"]), c_int(GEMM_TC_UNARY["relu2"] if ungated else 0),
-                                        _ptr(row_weight), c_int(tile), _stream()), "gemm_tc_grouped")
-    _check(gl, gl.tb_gemm_tc_grouped_tiles(_ptr(act), _ptr(down_w), _ptr(y), c_int(code(torch.float32)), c_int(max_rows), c_int(W),
-                                     c_int(E), c_int(ff), c_longlong(ff), c_longlong(ff), c_longlong(W), _ptr(tile_group),
-                                     c_int(-1), c_int(0), _ptr(None), c_int(tile), _stream()), "gemm_tc_grouped")
-    _check(lib, lib.tb_moe_combine_sorted(_ptr(y), _ptr(pos), _ptr(None if on_input else weight), _ptr(shared),
-                                          c_int(shared.shape[0] if shared is not None else 0),
-                                          c_longlong(shared.stride(0) if shared is not None else 0), _ptr(gate), _ptr(out),
-                                          c_int(T), c_int(W), c_int(top), _stream()), "moe_combine_sorted")
+    rows = ((P + tile - 1) // tile + min(E, P)) * tile
+    # layout, rows' weights, operand, activations, the second product's 32-bit rows; each from a 256-byte boundary
+    need = sum(-(-n // 256) * 256 for n in (4 * (P + rows + rows // tile), 4 * rows if on_input else 0, 2 * rows * W, 2 * rows * ff, 4 * rows * W))
+    scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
+    lib, gl = build.load("moe"), build.load("gemm_tc")
+    a = _MoeTilesArgs()
+    a.x = x.data_ptr(); a.x_stride = x.stride(0); a.idx = idx.data_ptr(); a.weight = weight.data_ptr()
+    a.first_w = gate_up_w.data_ptr(); a.down_w = down_w.data_ptr()
+    if shared is not None:
+        a.shared = shared.data_ptr(); a.shared_splits = shared.shape[0]; a.shared_split_stride = shared.stride(0)
+    a.gate = gate.data_ptr() if gate is not None else None
+    a.out = out.data_ptr(); a.product = ctypes.cast(gl.tb_gemm_tc_grouped_tiles, c_void_p).value
+    a.scratch = scratch.data_ptr(); a.scratch_bytes = need
+    a.n_tokens = T; a.W = W; a.ff = ff; a.top = top; a.E = E; a.tile = tile; a.weight_in = int(on_input)
+    a.gated_act = -1 if ungated else GEMM_TC_SILU_EXACT if P < MOE_EXACT_BELOW else ACTIVATIONS["silu"]
+    a.unary = GEMM_TC_UNARY["relu2"] if ungated else 0
+    status = lib.tb_moe_tiles(ctypes.byref(a), _stream())
+    _check(gl if a.in_product else lib, status, "moe_tiles", 5)
     return out
 
 
@@ -2169,7 +2166,8 @@ def moe_experts(x: torch.Tensor, gate_w: Optional[torch.Tensor], up_w: torch.Ten
                 or gate is None:
             raise KernelError("moe: the shared expert's output must be float32 [splits, T, W] and come with its gate")
     out = torch.empty((T, W), dtype=torch.float32, device=x.device)
-    if x.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0 and _at_16_bytes(x, down_w):
+    if T * top >= MOE_SHARED_FROM and x.dtype == torch.bfloat16 and W % 8 == 0 and ff % 8 == 0 and x.stride(0) % 8 == 0 \
+            and _at_16_bytes(x, down_w):
         tile = moe_tile(T * top, E, (2 if ungated else 3) * W * ff * 2)
         if tile and ungated and _at_16_bytes(up_w):
             return _moe_grouped_tc(x, up_w, down_w, idx, weight, shared, gate, out, ungated=True, on_input=on_input, tile=tile)
