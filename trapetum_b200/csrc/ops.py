@@ -2071,7 +2071,7 @@ def _moe_grouped_tc(x, gate_up_w, down_w, idx, weight, shared, gate, out, ungate
         a.shared = shared.data_ptr(); a.shared_splits = shared.shape[0]; a.shared_split_stride = shared.stride(0)
     a.gate = gate.data_ptr() if gate is not None else None
     a.out = out.data_ptr(); a.product = ctypes.cast(gl.tb_gemm_tc_grouped_tiles, c_void_p).value
-    a.scratch = scratch.data_ptr(); a.scratch_bytes = need
+    a.scratch = scratch.data_ptr(); a.scratch_bytes = scratch.numel()
     a.n_tokens = T; a.W = W; a.ff = ff; a.top = top; a.E = E; a.tile = tile; a.weight_in = int(on_input)
     a.gated_act = -1 if ungated else GEMM_TC_SILU_EXACT if P < MOE_EXACT_BELOW else ACTIVATIONS["silu"]
     a.unary = GEMM_TC_UNARY["relu2"] if ungated else 0
