@@ -171,7 +171,7 @@ def test_scores_mixed_two_pairs_a_thread(H, G, D, seen, n):
     near(got.view(n, H, D), want, dtype, "mixed attention, pairs", rel16=1.5e-2)
 
 
-@pytest.mark.parametrize("H,G,D,times", [(16, 4, 32, 1), (8, 2, 64, 2), (20, 4, 32, 1)])
+@pytest.mark.parametrize("H,G,D,times", [(16, 4, 32, 1), (8, 2, 64, 2), (20, 4, 32, 1), (4, 2, 64, 1), (4, 2, 64, 2)])
 @pytest.mark.parametrize("window", [0, 72, -16, -64, -48, -40, -192, -208])
 def test_scores_mixed_in_steps_with_more_tiles_than_fit_at_once(H, G, D, times, window):
     """A step with more CTAs than the device holds takes its tiles longest first, and goes round the sequences: every row against

@@ -1091,6 +1091,23 @@ def test_rope_kv_of_many_heads(ops, nh, nkv, hd, rot, n):
     assert torch.equal(pools[1], pools[3])
 
 
+@pytest.mark.parametrize("nh,nkv,hd,rot", [(12, 2, 64, 64), (14, 2, 64, 64), (3, 1, 128, 32), (2, 4, 64, 0)])
+def test_rope_kv_of_few_heads(ops, nh, nkv, hd, rot):
+    """More than 1,536 tokens of up to 64 work items take 64 threads a token: the same bits as in pieces that take 128."""
+    n = 1600
+    qkv = rnd(n, (nh + 2 * nkv) * hd, dt=torch.bfloat16)
+    pos, seq, after = torch.arange(n).int().cuda(), torch.zeros(n).int().cuda(), torch.tensor([n]).int().cuda()
+    table = torch.arange(n // PAGE - 1, -1, -1).int().cuda()[None].contiguous()
+    inv = (1e4 ** -(torch.arange(0, rot, 2).float() / rot)).cuda() if rot else None
+    pools = [torch.zeros(n // PAGE, nkv, PAGE, hd, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    want = qkv.clone()
+    ops.rope_kv(qkv, nh, nkv, hd, rot, inv, pos, seq, after, *pools[:2], table, 0)
+    for part in (slice(0, 1400), slice(1400, n)):
+        ops.rope_kv(want[part], nh, nkv, hd, rot, inv, pos[part], seq[part], after, *pools[2:], table, 0)
+    assert torch.equal(qkv, want) and torch.equal(pools[0], pools[2]) and torch.equal(pools[1], pools[3])
+    assert torch.equal(pools[1].transpose(1, 2).flip(0).reshape(n, nkv * hd), qkv[:, (nh + nkv) * hd:])
+
+
 @pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("hd,rot,ring,theta", [(16, 16, 0, 1e4), (48, 48, 128, 5e4), (256, 256, 64, 1e4), (32, 16, 0, 1e3), (64, 0, 0, 1.0),
                                                (640, 640, 0, 1e4), (576, 530, 64, 1e4)])     # more pairs than a CTA has threads for
